@@ -219,7 +219,9 @@ int it_matmul_t2_launch(it_ctx* c, const it_mat* w, int ntok, const it_q8* x, fl
     // most SMs; smaller matrices keep the finer tiles of the kernel in this file.  IT_MATMUL=legacy / tc forces one.
     const char* fv = getenv("IT_MATMUL");      // read on every call so that a test can exercise both kernels on one shape
     const int force = !fv ? 0 : !strcmp(fv, "legacy") ? 1 : !strcmp(fv, "tc") ? 2 : 0;
-    if (force != 1 && (force == 2 || wr == 4)) {
+    // 5120-row matrices at 33 to 64 activation rows too: their 160 row groups are one wave and twelve CTAs of 32-row tiles here
+    // (5120 x 17408 x 64: 67.6 us, 57.6 there; x 40: 58.9 and 57.3; x 12: 44.3 and 50.0; 2560 rows x 64, K 5120: 14.8 and 19.9)
+    if (force != 1 && (force == 2 || wr == 4 || (rg > c->sm_count && ntok > MM_TOK / 2))) {
         const int r = it_matmul_tc_launch(c, w, ntok, x, y, y_stride, accum); if (r <= 0) return r;
     }
     if (wr == 4) return mm_launch<4, 4>(c, w, ntok, x, y, y_stride, accum);

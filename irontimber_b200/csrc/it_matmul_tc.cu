@@ -3,21 +3,28 @@
 // (src/cpu.rs:48-63); it takes the place of the 64x64 tile kernels VkEngine::mv selects for prompt chunks
 // (src/vk/mod.rs:655-677).
 //
-// A CTA owns 128 matrix rows (four 32-row groups) x 64 activation rows (x 128 when the launch has more than 64: one
-// expanded tile and one issue sequence then feed twice the columns) and walks the 128-column blocks in order.
-//   warp 24  producer: per block one stage = four weight tiles (bulk copies) + the 64 x 128 int8 activations as one
-//            box of a tiled tensor map with the 128-byte swizzle, i.e. already in the K-major layout the MMA reads
-//   warps 16-23 expanders (two sets of four, alternating blocks): turn the packed 2-bit codes of a stage into a 128 x 128 tile of unsigned bytes (codes 0..3)
-//            in the same K-major 128-byte-swizzled layout (row r at 128 r, 16-byte piece p at (p ^ (r & 7)) * 16),
-//            and the f16 block scales of the 128 rows into f32
-//   warp 25  one thread issues four tcgen05.mma (M 128, N 64, K 32, u8 x s8 -> s32) per block into one of eight
-//            64-column accumulators in tensor memory and commits them to mbarriers (accumulator ready; A tile and
-//            stage free again)
-//   warps 0-15 epilogue, four groups of four warps: group q owns activation rows 16 q .. 16 q + 15, its thread r reads
-//            those columns of row r of the accumulator (tcgen05.ld 32x32b; warp w may touch lanes 32 (w % 4) ..), forms
+// A CTA walks tiles of 128 matrix rows (four 32-row groups) x 64 activation rows (x 128 when the launch has more than 64: one
+// expanded tile and one issue sequence then feed twice the columns); one CTA per SM, a tile's 128-column blocks in order, two
+// blocks (the 256 columns of a q8k scale) a step.
+//   warp 16  weight producer: per stage four weight tiles of each of the four row groups (bulk copies)
+//   warp 18  activation producer: per step the int8 activations as boxes of a tiled tensor map with the 128-byte swizzle,
+//            i.e. already in the K-major layout the MMA reads
+//   warps 8-15 expanders (two sets of four, alternating steps): turn the packed 2-bit codes into 128 x 128 tiles of signed bytes
+//            code - 1 in the same K-major 128-byte-swizzled layout (row r at 128 r, 16-byte piece p at (p ^ (r & 7)) * 16), so that
+//            the accumulator is S - sum128 at once, and the f16 block scales of the 128 rows into f32
+//   warp 17  one thread issues eight tcgen05.mma (M 128, K 32, s8 x s8 -> s32) per step into the step's two accumulators in tensor
+//            memory and commits them to one mbarrier (accumulators ready; tiles and boxes free again)
+//   warp 19  fetches the next tile's activation scales
+//   warps 0-7 epilogue: reads the accumulators (a thread gets four rows x every fourth column), forms
 //            (d_w * d_x) * float(S - sum128) for each and adds it to an f32 accumulator it keeps in registers for the
-//            whole row of blocks: ascending block order, one thread per (row, activation row) pair - the CPU's order,
-//            bit for bit.  The MMA of block b + 1 runs while block b is folded.
+//            whole row of blocks: ascending block order, one thread per (row, activation row) pair - the CPU's order, bit for bit.
+// What bounds it: per block and SM sub-core the epilogue's 64 pairs of values cost about 6.5 cycles each (conversion, two products, one
+// addition, every one rounded; a two-value instruction takes two cycles of the f32 pipe) = 420 cycles, the MMAs 256 plus their
+// operands' share of the shared-memory port; measured 970 cycles a block with everything running (1900 before).  What the steps
+// gave, 34816 x 5120 x 512 rows: 310 us with a row per epilogue thread (256 broadcast loads of scales a block: 1024 cycles of the
+// shared-memory port); 251 with the fragment layout and two-value arithmetic; 242 with conversions instead of biased accumulators; 217 with
+// CTAs that walk several tiles (7 us of 31 per tile were fill and drain); 202 with two blocks a step and eight epilogue warps; 197 with
+// the 16x128b read-out.
 // Integer block sums are exact whatever the hardware's summation order, so only the f32 epilogue decides the bits.
 //
 // Every wait is bounded; when one runs out the CTA raises the context's error flag (IT_ETIMEOUT), every role leaves
@@ -43,10 +50,9 @@ constexpr int TC_EPI_REGS = 168, TC_OTHER_REGS = 48;
 template <int NH> struct Tc {
     static constexpr int TOK = 64 * NH;                  // activation rows per CTA (N of the MMA)
     static constexpr int X_BYTES = TOK * 128;            // the activation tile of one block: NH boxes of the tensor map, one under the other
-    static constexpr int XS = NH == 1 ? 3 : 2;           // steps of activation tiles in flight (they come from L2)
     static constexpr int ND = 256 / TOK;                 // steps of accumulators in tensor memory
     static constexpr int EPI_TOK = TOK / 2;              // activation rows per epilogue warp
-    static constexpr int CG = EPI_TOK / 8;               // 8-column groups per epilogue warp
+    static constexpr int CC = EPI_TOK / 32;              // 32-column chunks per epilogue warp
     static constexpr int NDW = 2 * (TC_NA + ND);         // ring of per-block row scales: the expanders run at most NA + ND steps ahead of the epilogue
     // kind::i8 instruction descriptor: D s32, A signed 8 bit, B signed 8 bit, both K-major, N = TOK, M = 128
     static constexpr unsigned IDESC = (2u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(TOK >> 3) << 17) | ((unsigned)(TC_ROWS >> 4) << 24);
@@ -54,14 +60,14 @@ template <int NH> struct Tc {
 
 // Weight stages and activation boxes have rings of their own: the weights come from HBM, the boxes from L2.
 struct TcSmem { int x, a, w, dx, dx_bytes, dw, bars, tmem, flag, total; };
-template <int NH> __host__ __device__ inline TcSmem tc_layout(int nb, int wstages, int dxbufs) {
+template <int NH> __host__ __device__ inline TcSmem tc_layout(int nb, int wstages, int dxbufs, int xsteps) {
     TcSmem L; int o = 0;
-    L.x = o; o += Tc<NH>::XS * 2 * Tc<NH>::X_BYTES;    // 1024-byte aligned (128-byte swizzle)
+    L.x = o; o += xsteps * 2 * Tc<NH>::X_BYTES;    // 1024-byte aligned (128-byte swizzle)
     L.a = o; o += TC_NA * 2 * TC_A_BYTES;              // 1024-byte aligned
     L.w = o; o += wstages * TC_W_BYTES;
     L.dx = o; L.dx_bytes = (nb / 2) * Tc<NH>::TOK * 4; o += dxbufs * L.dx_bytes;
-    L.dw = o; o += Tc<NH>::NDW * TC_ROWS * 8;
-    L.bars = o; o += (2 * wstages + Tc<NH>::XS + TC_NA + 2 * Tc<NH>::ND + 4) * 8;
+    L.dw = o; o += Tc<NH>::NDW * TC_ROWS * 4;
+    L.bars = o; o += (2 * wstages + xsteps + TC_NA + 2 * Tc<NH>::ND + 4) * 8;
     o = (o + 15) & ~15;
     L.tmem = o; o += 16;
     L.flag = o; o += 16;
@@ -83,19 +89,20 @@ __device__ __forceinline__ void tc_mma(unsigned d_tmem, unsigned long long adesc
 __device__ __forceinline__ void tc_commit(unsigned bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" :: "r"(bar) : "memory");
 }
-// Accumulator read-out in the fragment shape 16x256b: of 16 lanes (matrix rows) x 32 columns (activation rows) thread 4 g + t gets, for
-// each of the four column groups c, rows g and g + 8, columns 8 c + 2 t and 8 c + 2 t + 1.
-__device__ __forceinline__ void tc_ld_frag(unsigned taddr, int (&v)[16]) {
-    asm volatile("tcgen05.ld.sync.aligned.16x256b.x4.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]),
-                   "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-                 : "r"(taddr) : "memory");
+// Accumulator read-out of 32 lanes (matrix rows) x 32 columns (activation rows) in the fragment shape 16x128b: of 16 lanes x 4 columns
+// thread 4 g + t gets rows g and g + 8 of column t, side by side.  v[16 hf + 2 c + e]: row g + 16 hf + 8 e, column 4 c + t.
+// Measured per register and warp: 1.0 cycle, against 2.0 for the shape 16x256b and 0.6 for 32x32b, whose threads would need
+// the scales of 32 columns each.
+__device__ __forceinline__ void tc_ld_chunk(unsigned taddr, int (&v)[32]) {
+    asm volatile("tcgen05.ld.sync.aligned.16x128b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%32];\n\t"
+                 "tcgen05.ld.sync.aligned.16x128b.x8.b32 {%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%33];"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
+                 : "r"(taddr), "r"(taddr + (16u << 16)) : "memory");
 }
 // Waits for the loads; the values pass through it so that nothing that uses them moves in front.
-__device__ __forceinline__ void tc_ld_wait(int (&v)[16]) {
+__device__ __forceinline__ void tc_ld_wait(int (&v)[32]) {
     asm volatile("tcgen05.wait::ld.sync.aligned;"
-                 : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7]), "+r"(v[8]), "+r"(v[9]), "+r"(v[10]), "+r"(v[11]),
-                   "+r"(v[12]), "+r"(v[13]), "+r"(v[14]), "+r"(v[15]) :: "memory");
+                 : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7]), "+r"(v[8]), "+r"(v[9]), "+r"(v[10]), "+r"(v[11]), "+r"(v[12]), "+r"(v[13]), "+r"(v[14]), "+r"(v[15]), "+r"(v[16]), "+r"(v[17]), "+r"(v[18]), "+r"(v[19]), "+r"(v[20]), "+r"(v[21]), "+r"(v[22]), "+r"(v[23]), "+r"(v[24]), "+r"(v[25]), "+r"(v[26]), "+r"(v[27]), "+r"(v[28]), "+r"(v[29]), "+r"(v[30]), "+r"(v[31]) :: "memory");
 }
 __device__ __forceinline__ void mbar_arrive_n(unsigned bar, unsigned n) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0], %1;" :: "r"(bar), "r"(n) : "memory"); }
 
@@ -112,23 +119,20 @@ __device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) { f32x2 r; asm("add.rn.f
 // the constant is not known at compile time.
 __device__ __forceinline__ f32x2 mul2_rounded(f32x2 a, f32x2 b, f32x2 mz) { f32x2 r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(mz)); return r; }
 
-// Place of activation row m's scale inside a step's TOK of them: the 2 * CG rows of one epilogue thread (8 c + 2 t + e) lie side by side.
-template <int NH> __device__ __forceinline__ int tc_dx_slot(int m) {
-    constexpr int E = Tc<NH>::EPI_TOK;
-    return m / E * E + ((m & 7) >> 1) * (E / 4) + 2 * ((m % E) >> 3) + (m & 1);
-}
+// Place of activation row m's scale inside a step's TOK of them: of every 16 rows the four of one epilogue thread (4 c + t) lie side by side.
+__device__ __forceinline__ int tc_dx_slot(int m) { return (m & ~15) + (m & 3) * 4 + ((m >> 2) & 3); }
 template <int N> __device__ __forceinline__ void reg_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" :: "n"(N)); }
 template <int N> __device__ __forceinline__ void reg_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" :: "n"(N)); }
 
 template <int NH>
 __global__ void __launch_bounds__(TC_THREADS, 1)
-k_matmul_tc(const __grid_constant__ CUtensorMap xmap, const uint8_t* __restrict__ tiles, int nb, int rows, int row_groups, int wstages, int ntiles, int tok_tiles, int dxbufs,
+k_matmul_tc(const __grid_constant__ CUtensorMap xmap, const uint8_t* __restrict__ tiles, int nb, int rows, int row_groups, int wstages, int ntiles, int tok_tiles, int dxbufs, int xsteps,
             const float* __restrict__ xd, int x_stride, int ntok,
             float* arena, size_t y_off, size_t y_stride, int accum, int* error_flag, const it_peers* peers, const it_rowmap map, float minus_zero) {
-    constexpr int TC_TOK = Tc<NH>::TOK, TC_X_BYTES = Tc<NH>::X_BYTES, TC_XS = Tc<NH>::XS, TC_ND = Tc<NH>::ND, TC_EPI_TOK = Tc<NH>::EPI_TOK, CG = Tc<NH>::CG, NDW = Tc<NH>::NDW;
+    constexpr int TC_TOK = Tc<NH>::TOK, TC_X_BYTES = Tc<NH>::X_BYTES, TC_ND = Tc<NH>::ND, TC_EPI_TOK = Tc<NH>::EPI_TOK, CC = Tc<NH>::CC, NDW = Tc<NH>::NDW;
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
-    const TcSmem L = tc_layout<NH>(nb, wstages, dxbufs);
+    const TcSmem L = tc_layout<NH>(nb, wstages, dxbufs, xsteps);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, np = nb / 2;      // np: steps (pairs of blocks) of a tile
     volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + L.flag);
     unsigned* tmem_slot = reinterpret_cast<unsigned*>(smem + L.tmem);
@@ -137,7 +141,7 @@ k_matmul_tc(const __grid_constant__ CUtensorMap xmap, const uint8_t* __restrict_
     // step (full / empty), activation scales (full / empty).  "Accumulators d full" is the one commit of a step: it also tells the
     // expanders and the activation producer that the tiles and boxes the step read may be reused.
     const unsigned wfull0 = bars, wempty0 = wfull0 + 8 * wstages, xfull0 = wempty0 + 8 * wstages,
-                   afull0 = xfull0 + 8 * TC_XS, dfull0 = afull0 + 8 * TC_NA, dempty0 = dfull0 + 8 * TC_ND, sfull0 = dempty0 + 8 * TC_ND, sempty0 = sfull0 + 16;
+                   afull0 = xfull0 + 8 * xsteps, dfull0 = afull0 + 8 * TC_NA, dempty0 = dfull0 + 8 * TC_ND, sfull0 = dempty0 + 8 * TC_ND, sempty0 = sfull0 + 16;
     // The CTA's tiles: blockIdx.x, + gridDim.x, ...; the activation tiles of one group of matrix rows are neighbours.  Every role walks
     // the same tiles with its ring positions running on, so the next tile's weights, boxes and products are under way while
     // the epilogue still stores the last one's results.
@@ -146,7 +150,7 @@ k_matmul_tc(const __grid_constant__ CUtensorMap xmap, const uint8_t* __restrict_
     if (tid == 0) {
         *abort_flag = 0;
         for (int s = 0; s < wstages; s++) { mbar_init(wfull0 + 8 * s, 1); mbar_init(wempty0 + 8 * s, 8); }
-        for (int s = 0; s < TC_XS; s++) mbar_init(xfull0 + 8 * s, 1);
+        for (int s = 0; s < xsteps; s++) mbar_init(xfull0 + 8 * s, 1);
         for (int a = 0; a < TC_NA; a++) mbar_init(afull0 + 8 * a, 4);
         for (int d = 0; d < TC_ND; d++) { mbar_init(dfull0 + 8 * d, 1); mbar_init(dempty0 + 8 * d, TC_EPI_WARPS); }
         for (int k = 0; k < 2; k++) { mbar_init(sfull0 + 8 * k, 1); mbar_init(sempty0 + 8 * k, TC_EPI_WARPS); }
@@ -198,8 +202,8 @@ k_matmul_tc(const __grid_constant__ CUtensorMap xmap, const uint8_t* __restrict_
             for (int tile = tile0; ok && tile < ntiles; tile += tstep) {
                 const int tok0 = tile % tok_tiles * TC_TOK;
                 for (int p = 0; p < np; p++) {
-                    // the slot was last read TC_XS steps ago: wait for that step's commit
-                    if (issued >= TC_XS) {
+                    // the slot was last read xsteps steps ago: wait for that step's commit
+                    if (issued >= xsteps) {
                         if (!mbar_wait(dfull0 + 8 * dp, dpp, abort_flag, error_flag, 19)) { ok = false; break; }
                         if (++dp == TC_ND) { dp = 0; dpp ^= 1u; }
                     }
@@ -208,14 +212,14 @@ k_matmul_tc(const __grid_constant__ CUtensorMap xmap, const uint8_t* __restrict_
                     for (int k = 0; k < 2 * NH; k++)     // 64 rows per box; the boxes of a block lie one under the other like one box of TOK rows
                         tma_load_2d(smem_u32(smem + L.x + s * 2 * TC_X_BYTES + k * 64 * 128), &xmap, (2 * p + k / NH) * 128, tok0 + 64 * (k % NH), xfull0 + 8 * s);
                     issued++;
-                    if (++s == TC_XS) s = 0;
+                    if (++s == xsteps) s = 0;
                 }
             }
             if (*abort_flag) {
-                const int first = issued > TC_XS ? issued - TC_XS : 0;
+                const int first = issued > xsteps ? issued - xsteps : 0;
                 for (int k = first; k < issued; k++) {
                     const long long t0 = clock64();
-                    while (!mbar_test(xfull0 + 8 * (k % TC_XS), (unsigned)(k / TC_XS) & 1u) && clock64() - t0 < WAIT_CLOCKS) { }
+                    while (!mbar_test(xfull0 + 8 * (k % xsteps), (unsigned)(k / xsteps) & 1u) && clock64() - t0 < WAIT_CLOCKS) { }
                 }
             }
         }
@@ -241,7 +245,7 @@ k_matmul_tc(const __grid_constant__ CUtensorMap xmap, const uint8_t* __restrict_
                     tc_mma<true>(dt, ad + 6, bd + 6, Tc<NH>::IDESC);
                 }
                 tc_commit(dfull0 + 8 * d);        // accumulators complete; tiles and boxes of this step may be reused
-                if (++s == TC_XS) { s = 0; xph ^= 1u; }
+                if (++s == xsteps) { s = 0; xph ^= 1u; }
                 if (++a == TC_NA) { a = 0; aph ^= 1u; }
                 if (++d == TC_ND) { d = 0; dph ^= 1u; }
             }
@@ -258,7 +262,7 @@ k_matmul_tc(const __grid_constant__ CUtensorMap xmap, const uint8_t* __restrict_
             float* dxs = reinterpret_cast<float*>(smem + L.dx + k * L.dx_bytes);
             for (int m = lane; m < TC_TOK; m += 32) {
                 const float* src = xd + (size_t)(tok0 + m) * (x_stride / 256);
-                float* dst = dxs + tc_dx_slot<NH>(m);
+                float* dst = dxs + tc_dx_slot(m);
 #pragma unroll 8
                 for (int bb = 0; bb < np; bb++) dst[bb * TC_TOK] = m < ntv ? src[bb] : 0.f;
             }
@@ -272,7 +276,7 @@ k_matmul_tc(const __grid_constant__ CUtensorMap xmap, const uint8_t* __restrict_
         unsigned char* const at = smem + L.a + 2 * eset * TC_A_BYTES + (rgl * 32 + g) * 128;
         unsigned char* const plo = at + (((2 * t) ^ g) << 4);          // columns 32 t .. 32 t + 15 of row g; the other rows 1024 bytes apart
         unsigned char* const phi = at + (((2 * t + 1) ^ g) << 4);      // columns 32 t + 16 .. 32 t + 31
-        float* const dws = reinterpret_cast<float*>(smem + L.dw) + rgl * 64 + 8 * g;
+        float* const dws = reinterpret_cast<float*>(smem + L.dw) + rgl * 32 + 4 * g;
         const unsigned char* const src0 = smem + L.w + rgl * TC_KB * IT_TILE_BYTES;
         int s = 0, dp = eset, r = 0, gp = 0; unsigned sph = 0, dpp = 0; bool ok = true;
         for (int tile = tile0; ok && tile < ntiles; tile += tstep)
@@ -297,12 +301,11 @@ k_matmul_tc(const __grid_constant__ CUtensorMap xmap, const uint8_t* __restrict_
                         *reinterpret_cast<uint4*>(plo + h * TC_A_BYTES + i * 1024) = make_uint4(sgn(wa.x), sgn(wa.y), sgn(wa.z), sgn(wa.w));
                         *reinterpret_cast<uint4*>(phi + h * TC_A_BYTES + i * 1024) = make_uint4(sgn(wb.x), sgn(wb.y), sgn(wb.z), sgn(wb.w));
                     }
-                    if (t == 0) {                         // row scales, each one twice (the operand pair of the epilogue's two-value products)
+                    if (t == 0) {
                         const uint2 sc = *reinterpret_cast<const uint2*>(src + 1024 + 8 * g);
                         const __half2 h01 = *reinterpret_cast<const __half2*>(&sc.x), h23 = *reinterpret_cast<const __half2*>(&sc.y);
-                        const float d0 = __low2float(h01), d1 = __high2float(h01), d2 = __low2float(h23), d3 = __high2float(h23);
-                        float4* dw = reinterpret_cast<float4*>(dws + (r + h) * 2 * TC_ROWS);
-                        dw[0] = make_float4(d0, d0, d1, d1); dw[1] = make_float4(d2, d2, d3, d3);      // rows g, g + 8, g + 16, g + 24: the rows of one epilogue thread
+                        *reinterpret_cast<float4*>(dws + (r + h) * TC_ROWS) =      // rows g, g + 8, g + 16, g + 24: the rows of one epilogue thread
+                            make_float4(__low2float(h01), __high2float(h01), __low2float(h23), __high2float(h23));
                     }
                 }
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");     // generic-proxy stores before the MMA's async-proxy reads
@@ -317,14 +320,14 @@ k_matmul_tc(const __grid_constant__ CUtensorMap xmap, const uint8_t* __restrict_
         }
     } else {
         // ---------------- epilogue: warp 4 q + i owns row group i x activation rows EPI_TOK q ..; its thread 4 g + t owns rows
-        // g, g + 8, g + 16, g + 24 of the group and, of every eight activation rows, the two at 2 t.  Two 16-byte loads of row
-        // scales and EPI_TOK / 16 of activation scales then serve EPI_TOK results per block: with a row per thread and all columns
+        // g, g + 8, g + 16, g + 24 of the group and every fourth activation row.  One 16-byte load of row scales per block and one of
+        // activation scales per 16 columns and step then serve all of a thread's results: with a row per thread and all columns
         // (one broadcast 16-byte load per four results) the shared-memory read port was what bounded the kernel.
         constexpr int NEPI = TC_EPI_WARPS * 32;
         reg_inc<TC_EPI_REGS>();
         const int grp = warp >> 2, rgl = warp & 3, g = lane >> 2, t = lane & 3, m0 = grp * TC_EPI_TOK;
         const unsigned tquad = tmem_base + ((unsigned)(rgl * 32) << 16) + (unsigned)m0;
-        const ulonglong2* const dws = reinterpret_cast<const ulonglong2*>(smem + L.dw) + rgl * 16 + 2 * g;
+        const ulonglong2* const dws = reinterpret_cast<const ulonglong2*>(smem + L.dw) + rgl * 8 + g;
         asm volatile("griddepcontrol.wait;" ::: "memory");            // q8 scales and (when accumulating) y come from earlier kernels
         asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
         {
@@ -333,7 +336,7 @@ k_matmul_tc(const __grid_constant__ CUtensorMap xmap, const uint8_t* __restrict_
 #pragma unroll 4
             for (int i = tid; i < np * TC_TOK; i += NEPI) {
                 const int m = i % TC_TOK, bb = i / TC_TOK;
-                dxs[bb * TC_TOK + tc_dx_slot<NH>(m)] = m < ntv ? xd[(size_t)(tok0 + m) * (x_stride / 256) + bb] : 0.f;
+                dxs[bb * TC_TOK + tc_dx_slot(m)] = m < ntv ? xd[(size_t)(tok0 + m) * (x_stride / 256) + bb] : 0.f;
             }
             asm volatile("bar.sync 1, %0;" :: "n"(NEPI) : "memory");
         }
@@ -345,50 +348,49 @@ k_matmul_tc(const __grid_constant__ CUtensorMap xmap, const uint8_t* __restrict_
             const int rg0 = tile / tok_tiles * 4, tok0 = tile % tok_tiles * TC_TOK, ntv = min(TC_TOK, ntok - tok0);
             const bool active = m0 < ntv;              // groups past the last activation row only release the accumulators
             if (j > 0 && !mbar_wait(sfull0 + 8 * k, (unsigned)((j - 1) >> 1) & 1u, abort_flag, error_flag, 18)) break;
-            const ulonglong2* dx2 = reinterpret_cast<const ulonglong2*>(smem + L.dx + k * L.dx_bytes + (m0 + t * 2 * CG) * 4);
-            f32x2 acc[4][CG];                          // [row g + 8 i][column pair of group c]
+            const float4* dxs = reinterpret_cast<const float4*>(smem + L.dx + k * L.dx_bytes) + m0 / 4 + t;
+            f32x2 acc[2][8 * CC];                      // rows g + 16 hf and g + 8 + 16 hf of column 4 c + t
 #pragma unroll
-            for (int i = 0; i < 4; i++)
+            for (int hf = 0; hf < 2; hf++)
 #pragma unroll
-                for (int c = 0; c < CG; c++) acc[i][c] = 0ull;
+                for (int c = 0; c < 8 * CC; c++) acc[hf][c] = 0ull;
             for (int p = 0; p < np; p++) {             // two blocks at a time: they share the activation scale, the wait and the release
                 if (!mbar_wait(dfull0 + 8 * d, dph, abort_flag, error_flag, 17)) { ok = false; break; }
                 __syncwarp();
                 if (active) {
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    // chunks of 16 lanes x 32 columns; the next one is on its way while one is folded
-                    constexpr int NCC = CG / 4, NCH = 4 * NCC;
+                    // chunks of 32 columns of one block; the next one is on its way while one is folded
                     const unsigned ta = tquad + (unsigned)(2 * d * TC_TOK);
-                    auto chunk = [&](int ch) { return ta + (unsigned)(ch / (2 * NCC) * TC_TOK) + ((unsigned)(ch / NCC % 2) << 20) + (unsigned)(32 * (ch % NCC)); };
-                    int S[2][16];
-                    tc_ld_frag(chunk(0), S[0]);
-                    f32x2 dx[CG];
+                    auto chunk = [&](int ch) { return ta + (unsigned)((ch & 1) * TC_TOK + (ch >> 1) * 32); };
+                    int S[2][32];
+                    tc_ld_chunk(chunk(0), S[0]);
+                    // row scales of both blocks: stored by the expanders before they released the tiles to the MMAs whose completion we just saw
+                    const ulonglong2 dwb[2] = { dws[r * TC_ROWS / 4], dws[(r + 1) * TC_ROWS / 4] };
+                    f32x2 dx[8];
 #pragma unroll
-                    for (int c = 0; c < CG / 2; c++) { const ulonglong2 v = dx2[c]; dx[2 * c] = v.x; dx[2 * c + 1] = v.y; }
-                    ulonglong2 dw[2];
-#pragma unroll
-                    for (int ch = 0; ch < NCH; ch++) {
-                        const int h = ch / (2 * NCC), hf = ch / NCC % 2, cc = ch % NCC;
-                        // row scales of this block: stored by the expanders before they released the tile to the MMA whose completion we just saw
-                        if (ch % (2 * NCC) == 0) { dw[0] = dws[(r + h) * TC_ROWS / 2]; dw[1] = dws[(r + h) * TC_ROWS / 2 + 1]; }
-                        int (&v)[16] = S[ch & 1];
+                    for (int ch = 0; ch < 2 * CC; ch++) {
+                        if (!(ch & 1)) {                                      // both blocks of these columns share the activation scales
+                            const float4 xa = dxs[(ch >> 1) * 8], xb = dxs[(ch >> 1) * 8 + 4];
+                            dx[0] = pkf(xa.x, xa.x); dx[1] = pkf(xa.y, xa.y); dx[2] = pkf(xa.z, xa.z); dx[3] = pkf(xa.w, xa.w);
+                            dx[4] = pkf(xb.x, xb.x); dx[5] = pkf(xb.y, xb.y); dx[6] = pkf(xb.z, xb.z); dx[7] = pkf(xb.w, xb.w);
+                        }
+                        int (&v)[32] = S[ch & 1];
                         tc_ld_wait(v);
-                        if (ch + 1 < NCH) tc_ld_frag(chunk(ch + 1), S[(ch + 1) & 1]);
+                        if (ch + 1 < 2 * CC) tc_ld_chunk(chunk(ch + 1), S[(ch + 1) & 1]);
                         else {
                             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                             __syncwarp();
                             if (lane == 0) mbar_arrive(dempty0 + 8 * d);      // the MMAs of step p + ND may use the accumulators
                         }
 #pragma unroll
-                        for (int c = 0; c < 4; c++) {
-                            f32x2 (&a0)[CG] = acc[2 * hf], (&a1)[CG] = acc[2 * hf + 1];
-                            const f32x2 x = dx[4 * cc + c];
-                            a0[4 * cc + c] = add2(a0[4 * cc + c], mul2_rounded(mul2(dw[hf].x, x), pkf((float)v[4 * c], (float)v[4 * c + 1]), mz));
-                            a1[4 * cc + c] = add2(a1[4 * cc + c], mul2_rounded(mul2(dw[hf].y, x), pkf((float)v[4 * c + 2], (float)v[4 * c + 3]), mz));
+                        for (int c = 0; c < 8; c++) {
+                            const int cc = (ch >> 1) * 8 + c;
+                            acc[0][cc] = add2(acc[0][cc], mul2_rounded(mul2(dwb[ch & 1].x, dx[c]), pkf((float)v[2 * c], (float)v[2 * c + 1]), mz));
+                            acc[1][cc] = add2(acc[1][cc], mul2_rounded(mul2(dwb[ch & 1].y, dx[c]), pkf((float)v[16 + 2 * c], (float)v[16 + 2 * c + 1]), mz));
                         }
                     }
                 } else if (lane == 0) mbar_arrive(dempty0 + 8 * d);
-                dx2 += TC_TOK / 4;
+                dxs += TC_TOK / 4;
                 if (++d == TC_ND) { d = 0; dph ^= 1u; }
                 r = r + 2 == NDW ? 0 : r + 2;
             }
@@ -401,28 +403,22 @@ k_matmul_tc(const __grid_constant__ CUtensorMap xmap, const uint8_t* __restrict_
                 const int row = (rg0 + rgl) * 32 + g + 8 * i;
                 if (row >= rows) continue;
                 const int grow = it_map_row(map, row);
-                const size_t off = y_off + (size_t)(tok0 + m0 + 2 * t) * y_stride + grow;     // first of this thread's activation rows
+                const size_t off = y_off + (size_t)(tok0 + m0 + t) * y_stride + grow;     // first of this thread's activation rows
+                float old[8 * CC];
                 if (!peers) {
                     float* y = arena + off;
-                    float old[2 * CG];
 #pragma unroll
-                    for (int c = 0; c < CG; c++)
+                    for (int c = 0; c < 8 * CC; c++) old[c] = accum && m0 + 4 * c + t < ntv ? __ldcg(y + (size_t)(4 * c) * y_stride) : 0.f;
 #pragma unroll
-                        for (int e = 0; e < 2; e++) old[2 * c + e] = accum && m0 + 8 * c + 2 * t + e < ntv ? __ldcg(y + (size_t)(8 * c + e) * y_stride) : 0.f;
-#pragma unroll
-                    for (int c = 0; c < CG; c++) {
-                        const float2 v = upk(acc[i][c]);
-                        const int m = m0 + 8 * c + 2 * t;
-                        if (m < ntv) y[(size_t)(8 * c) * y_stride] = accum ? __fadd_rn(old[2 * c], v.x) : v.x;
-                        if (m + 1 < ntv) y[(size_t)(8 * c + 1) * y_stride] = accum ? __fadd_rn(old[2 * c + 1], v.y) : v.y;
+                    for (int c = 0; c < 8 * CC; c++) {
+                        const float2 v2 = upk(acc[i >> 1][c]); const float v = i & 1 ? v2.y : v2.x;
+                        if (m0 + 4 * c + t < ntv) y[(size_t)(4 * c) * y_stride] = accum ? __fadd_rn(old[c], v) : v;
                     }
                 } else {
 #pragma unroll
-                    for (int c = 0; c < CG; c++) {
-                        const float2 v = upk(acc[i][c]);
-                        const int m = m0 + 8 * c + 2 * t;
-                        if (m < ntv) it_result_store(peers, arena, off + (size_t)(8 * c) * y_stride, v.x, accum);
-                        if (m + 1 < ntv) it_result_store(peers, arena, off + (size_t)(8 * c + 1) * y_stride, v.y, accum);
+                    for (int c = 0; c < 8 * CC; c++) {
+                        const float2 v2 = upk(acc[i >> 1][c]); const float v = i & 1 ? v2.y : v2.x;
+                        if (m0 + 4 * c + t < ntv) it_result_store(peers, arena, off + (size_t)(4 * c) * y_stride, v, accum);
                     }
                 }
             }
@@ -445,13 +441,16 @@ template <int NH>
 static int tc_launch(it_ctx* c, const it_mat* w, int ntok, const it_q8* x, float* y, size_t y_stride, int accum) {
     const int nb = (int)(w->cols / 128);
     const int tok_tiles = (ntok + Tc<NH>::TOK - 1) / Tc<NH>::TOK, ntiles = (int)((w->row_groups + 3) / 4) * tok_tiles;
-    // one CTA per SM walks its tiles, with two buffers of activation scales; where those do not fit (wide rows), a CTA per tile
+    // One CTA per SM walks its tiles, with two buffers of activation scales; where those do not fit (wide rows), a CTA per tile.
     int grid = ntiles < c->sm_count ? ntiles : c->sm_count, dxbufs = ntiles > grid ? 2 : 1;
-    if (tc_layout<NH>(nb, 2, dxbufs).total + 1024 > TC_SMEM_MAX) { grid = ntiles; dxbufs = 1; }
-    int stages = 5;                        // weight stages of TC_KB blocks: as deep as shared memory allows
-    while (stages > 2 && tc_layout<NH>(nb, stages, dxbufs).total + 1024 > TC_SMEM_MAX) stages--;
-    const TcSmem L = tc_layout<NH>(nb, stages, dxbufs);
-    if (L.total + 1024 > TC_SMEM_MAX) return 1;
+    auto fits = [&](int wst, int xst) { return tc_layout<NH>(nb, wst, dxbufs, xst).total + 1024 <= TC_SMEM_MAX; };
+    if (!fits(2, 2)) { grid = ntiles; dxbufs = 1; }
+    if (!fits(2, 2)) return 1;
+    // Activation boxes three steps deep where they fit (two left the MMA waiting 375 cycles a step), then weight stages of TC_KB blocks
+    const int xsteps = fits(2, 3) ? 3 : 2;
+    int stages = 5;
+    while (!fits(stages, xsteps)) stages--;
+    const TcSmem L = tc_layout<NH>(nb, stages, dxbufs, xsteps);
     static bool attr_set[16] = {};
     if (!attr_set[c->device & 15]) { IT_CUDA(cudaFuncSetAttribute(k_matmul_tc<NH>, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM_MAX)); attr_set[c->device & 15] = true; }
     cudaLaunchConfig_t cfg = {};
@@ -460,7 +459,7 @@ static int tc_launch(it_ctx* c, const it_mat* w, int ntok, const it_q8* x, float
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization; attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr; cfg.numAttrs = 1;
-    IT_CUDA(cudaLaunchKernelEx(&cfg, k_matmul_tc<NH>, x->tmap, (const uint8_t*)w->tiles, nb, (int)w->rows, (int)w->row_groups, stages, ntiles, tok_tiles, dxbufs,
+    IT_CUDA(cudaLaunchKernelEx(&cfg, k_matmul_tc<NH>, x->tmap, (const uint8_t*)w->tiles, nb, (int)w->rows, (int)w->row_groups, stages, ntiles, tok_tiles, dxbufs, xsteps,
         (const float*)x->d, (int)x->max_n, ntok, c->arena, (size_t)(y - c->arena), y_stride, accum, c->error_flag_dev,
         (const it_peers*)(w->sharded ? c->peers_dev : nullptr), w->map, -0.0f));
     c->pdl_safe_q8 = x;
@@ -468,7 +467,7 @@ static int tc_launch(it_ctx* c, const it_mat* w, int ntok, const it_q8* x, float
 }
 
 // Returns IT_OK after launching, or a positive value when the shape does not suit this kernel (the caller then uses k_matmul_t2).
-// More than 64 activation rows go to the 128-row variant when its buffers fit (rows of up to about 12,000 columns).
+// More than 64 activation rows go to the 128-row variant when its buffers fit (rows of up to about 28,000 columns).
 int it_matmul_tc_launch(it_ctx* c, const it_mat* w, int ntok, const it_q8* x, float* y, size_t y_stride, int accum) {
     static const bool wide = []{ const char* v = getenv("IT_MATMUL_WIDE"); return !v || atoi(v) != 0; }();
     if (wide && ntok > 64) { const int r = tc_launch<2>(c, w, ntok, x, y, y_stride, accum); if (r != 1) return r; }

@@ -173,6 +173,18 @@ def test_matmul_t2_tile_kernel_bit_exact(be, orc, rows, cols, ntok, acc, kernel,
     assert np.array_equal(bits(got), bits(want))
 
 
+@pytest.mark.parametrize("rows,cols,ntok,acc", [(19200, 1024, 200, True), (9590, 2048, 300, False), (18950, 1024, 40, True), (19072, 16384, 65, False)])
+def test_matmul_t2_several_tiles_per_cta_bit_exact(be, orc, rows, cols, ntok, acc):
+    """More 128-row tiles than SMs: a CTA of the tensor-memory kernel walks two or three of them with its rings running on (ragged
+    last row groups and activation tiles among them); the widest rows leave no room for the second buffer of scales and get a
+    CTA per tile."""
+    rng = np.random.default_rng(rows + cols + ntok)
+    raw = synth_pq2(rows * 3 + cols, rows, cols)
+    X = rng.standard_normal((ntok, cols)).astype(np.float32)
+    got, want = run_mv(be, orc, raw, rows, cols, X, acc=acc)
+    assert np.array_equal(bits(got), bits(want))
+
+
 def test_matvec_t2_integer_accumulators_bit_exact(be, orc):
     rng = np.random.default_rng(77)
     rows, cols, ntok = 333, 2048, 4
