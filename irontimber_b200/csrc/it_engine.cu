@@ -242,6 +242,8 @@ int it_engine_build(int device, const it_model_config* cfg, uint64_t seed, int w
         E_TRY(dev_alloc(e, (void**)&e->mkc, (size_t)c.ctx_len * kvd * 4, true)); E_TRY(dev_alloc(e, (void**)&e->mvc, (size_t)c.ctx_len * kvd * 4, true));
     }
     E_TRY(it_q8_create(e->ctx, (size_t)std::max(std::max(e_, ff), std::max(inner, nh * hd)), IT_MAXT, &e->q8));
+    e->att_scratch_floats = std::min(IT_ATT_SCRATCH_FLOATS, (size_t)IT_MAXT * nh * (((size_t)c.ctx_len + 127) / 128 * 128));
+    E_TRY(dev_alloc(e, (void**)&e->att_scratch, e->att_scratch_floats * sizeof(float), false));
     E_TRY(dev_alloc(e, (void**)&e->toks_dev, (2 * IT_MAXT + 8) * sizeof(uint32_t), true));
     E_TRY(dev_alloc(e, (void**)&e->pos_dev, 64, true));
     if (cudaHostAlloc((void**)&e->host_pin, (size_t)IT_PIN_SLOTS * IT_PIN_WORDS * sizeof(uint32_t), cudaHostAllocDefault) != cudaSuccess) return fail(it_fail(IT_ENOMEM, "engine: pinned staging allocation failed"));

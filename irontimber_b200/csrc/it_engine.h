@@ -54,6 +54,7 @@ struct it_engine {
     int* pos_dev;                                    // position read by the recorded decode step
     it_arena_layout lay;
     float theta_scale;
+    float* att_scratch; size_t att_scratch_floats;   // attention scores of a block of prompt rows (it_sup_attention_tiled)
     std::vector<void*> owned;                        // plain device allocations to free
     int pos, mpos;                                   // trunk position; next MTP position (src/vk/mod.rs: pos, mpos)
     size_t hp_off; int hp_n;                         // pending h rows for the next draft (arena offset, count)
@@ -69,6 +70,7 @@ struct it_engine {
     int small_next;
     bool record_passes;                              // environment IT_PASS_GRAPHS (default on)
 };
+#define IT_ATT_SCRATCH_FLOATS ((size_t)32 << 20)     // 128 MB: the scores of a block of rows and what reads them again stay about the size of L2
 #define IT_PIN_SLOTS 8
 #define IT_PIN_WORDS (2 * IT_MAXT + 8)
 #define IT_SMALL_ROWS 8

@@ -112,7 +112,11 @@ int it_engine_run_chunk(it_engine* e, const uint32_t* toks, int nt, int logit_ro
             // prompt passes: one CTA per group of query heads and pair of rows that share their K / V reads; else one per (head, row)
             int ar = 1;
             static const bool grouped = []{ const char* v = getenv("IT_ATTN_GROUPED"); return !v || atoi(v) != 0; }();
-            if (grouped && nt > 8 && !pos_ptr) { ar = it_sup_attention_prefill(cx, q, 2 * hd, s_att, q + hd, l.kc, l.vc, hd, nh, nkv, pos0, A + L.o, (size_t)nh * hd, nt); if (ar < 0) return ar; }
+            if (grouped && nt > 8 && !pos_ptr) {
+                ar = it_sup_attention_tiled(cx, q, 2 * hd, s_att, q + hd, l.kc, l.vc, hd, nh, nkv, pos0, A + L.o, (size_t)nh * hd, nt, e->att_scratch, e->att_scratch_floats);
+                if (ar == 1) ar = it_sup_attention_prefill(cx, q, 2 * hd, s_att, q + hd, l.kc, l.vc, hd, nh, nkv, pos0, A + L.o, (size_t)nh * hd, nt);
+                if (ar < 0) return ar;
+            }
             if (ar == 1) IT_TRY(it_sup_attention(cx, q, 2 * hd, s_att, q + hd, l.kc, l.vc, kvd, hd, nh, nkv, pos0, pos_ptr, c.ctx_len, A + L.o, (size_t)nh * hd, nt, 1));
             IT_TRY(had_mv(e, l.o, nt, L.o, (size_t)nh * hd, L.x, e_, 1, true));
         }

@@ -52,6 +52,11 @@ int it_sup_attention_max_positions(int hd);
 int it_sup_attention_prefill(it_ctx* c, const float* q, size_t q_hs, size_t q_ts, const float* gate, const void* kc, const void* vc, int hd, int nh, int nkv, int slot0,
                              float* out, size_t o_ts, int nt);
 
+// The same for long prompt passes (it_attention_tiled.cu): scores go through `scratch` a block of rows at a time.  Returns 1 when the shape
+// or the scratch does not suit or the pass is too small for it (nothing launched), a negative code on error.
+int it_sup_attention_tiled(it_ctx* c, const float* q, size_t q_hs, size_t q_ts, const float* gate, const void* kc, const void* vc, int hd, int nh, int nkv, int slot0,
+                           float* out, size_t o_ts, int nt, float* scratch, size_t scratch_floats);
+
 // Fused forms for passes of up to 8 rows (same arithmetic and order as the separate kernels; see it_support.cu).
 int it_sup_attn_prep(it_ctx* c, float* qkv, size_t ts, int nh, int nkv, int hd, const float* q_norm, const float* k_norm, float eps, int pos0, const int* pos_ptr,
                      int n_rot, float theta_scale, const int* sections, void* kc, void* vc, int nt);
