@@ -81,7 +81,11 @@ int it_engine_run_chunk(it_engine* e, const uint32_t* toks, int nt, int logit_ro
                 IT_TRY(it_sup_conv(cx, A + L.big1, s_gdn, l.conv_w, l.conv_st, A + L.conv, cd, cd, c.conv_k, nt, l.ck_conv, csz, nck));
                 IT_TRY(it_sup_norm_head(cx, A + L.conv, sd, cd, A + L.conv, sd, cd, sd, 2 * nk, nullptr, 2, c.eps, nullptr, 0, 0, nt));
             }
-            if (sd == 128) {
+            // prompt passes: state rows spread over the GPU, then the gated norm; short passes and passes with checkpoints: both in one launch
+            const int gr = nt > 8 && nck == 0 ? it_sup_gdn_rows(cx, A + L.conv, cd, A + L.beta, A + L.alpha, nv, l.dt, l.a, l.ssm_st, A + L.o, inner, nv, nk, sd, qk, nt) : 1;
+            if (gr < 0) return gr;
+            if (gr == 0) IT_TRY(it_sup_norm_head(cx, A + L.o, sd, inner, A + L.o, sd, inner, sd, nv, l.ssm_norm, 1, c.eps, A + L.big1 + cd, sd, s_gdn, nt));
+            else if (sd == 128) {
                 // [delta rule | gated norm] in one launch, for any number of rows (the state stays in shared memory across the rows)
                 // (the kernel stages up to IT_GDN_MAXROWS rows at a time; the state carries over from one launch to the next)
                 for (int t0 = 0; t0 < nt; t0 += IT_GDN_MAXROWS) {

@@ -57,6 +57,10 @@ int it_sup_attention_prefill(it_ctx* c, const float* q, size_t q_hs, size_t q_ts
 int it_sup_attention_tiled(it_ctx* c, const float* q, size_t q_hs, size_t q_ts, const float* gate, const void* kc, const void* vc, int hd, int nh, int nkv, int slot0,
                            float* out, size_t o_ts, int nt, float* scratch, size_t scratch_floats);
 
+// The delta rule alone over the rows of a prompt pass (it_gdn_prefill.cu); returns 1 when the shape does not suit it (nothing launched).
+int it_sup_gdn_rows(it_ctx* c, const float* co, size_t co_ts, const float* beta, const float* alpha, size_t ba_ts, const float* dt, const float* a, float* state, float* o, size_t o_ts,
+                    int nv, int nk, int sd, int qk, int nt);
+
 // Fused forms for passes of up to 8 rows (same arithmetic and order as the separate kernels; see it_support.cu).
 int it_sup_attn_prep(it_ctx* c, float* qkv, size_t ts, int nh, int nkv, int hd, const float* q_norm, const float* k_norm, float eps, int pos0, const int* pos_ptr,
                      int n_rot, float theta_scale, const int* sections, void* kc, void* vc, int nt);
