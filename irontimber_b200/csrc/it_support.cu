@@ -135,6 +135,37 @@ __global__ void __launch_bounds__(1024) k_conv_wide(const float* mixed, size_t m
     if (live && threadIdx.y == 0) for (int i = 0; i < kk - 1; i++) state[(size_t)i * cd + ch] = keep[i];
 }
 
+// The same with every input read once: a thread walks CONV_ROWS rows of its channel with the last KK - 1 inputs in registers.  The kernel
+// above reads each input KK times on 80 of the SMs (27B shape); 256 rows of 10240 channels: 10 us against 37.  Only the CTAs of the first
+// rows read the old state, so they also write the new one (the last KK - 1 inputs of the pass).
+constexpr int CONV_ROWS = 16;
+template <int KK>
+__global__ void __launch_bounds__(128) k_conv_rows(const float* __restrict__ mixed, size_t m_ts, const float* __restrict__ w, float* state, float* __restrict__ out, size_t o_ts, int cd, int nt) {
+    IT_PDL_TRIGGER(); IT_PDL_WAIT();
+    const int ch = blockIdx.x * 128 + threadIdx.x, r0 = blockIdx.y * CONV_ROWS;
+    if (ch >= cd) return;
+    float wt[KK], win[KK + CONV_ROWS - 1];                   // win[i]: input of row r0 - (KK - 1) + i
+#pragma unroll
+    for (int i = 0; i < KK; i++) wt[i] = w[ch * KK + i];
+#pragma unroll
+    for (int i = 0; i < KK + CONV_ROWS - 1; i++) {
+        const int r = r0 - (KK - 1) + i;
+        win[i] = r < 0 ? state[(size_t)(KK - 1 + r) * cd + ch] : r < nt ? mixed[(size_t)r * m_ts + ch] : 0.f;
+    }
+#pragma unroll
+    for (int t = 0; t < CONV_ROWS; t++) {
+        if (r0 + t >= nt) break;
+        float s = 0.f;
+#pragma unroll
+        for (int i = 0; i < KK; i++) s = it_add(s, it_mul(win[t + i], wt[i]));
+        out[(size_t)(r0 + t) * o_ts + ch] = it_silu(s);
+    }
+    if (r0 == 0) {
+#pragma unroll
+        for (int i = 0; i < KK - 1; i++) state[(size_t)i * cd + ch] = mixed[(size_t)(nt - (KK - 1) + i) * m_ts + ch];
+    }
+}
+
 // Dense f32 rows (ssm_beta / ssm_alpha; cpu::matvec's f32 arm under Numerics::Ggml, src/cpu.rs:36-43: f32 products,
 // f64 accumulation).  One CTA of 256 threads per row: thread i adds the products i, i+256, ... in f64, each warp folds
 // with a butterfly, the eight warp sums are added in ascending order.  Rows [0, rows) use w0 / y0, rows [rows, 2 rows) w1 / y1.
@@ -155,6 +186,54 @@ __global__ void __launch_bounds__(256) k_dense_rows(const float* __restrict__ w0
         double tt = wsum[0];
         for (int k = 1; k < 8; k++) tt += wsum[k];
         (r < rows ? y0 : y1)[t * y_ts + row] = (float)tt;
+    }
+}
+
+// The same for many rows of activations: a CTA forms DR_W x DR_T results, every one with the additions of k_dense_rows in its order, so
+// that a loaded weight or activation serves four or eight products (one result per CTA moves 1 GB through L2 at 256 rows of
+// 96 x 5120: 70 us; here 55, most of it the conversions to f64).
+constexpr int DR_W = 8, DR_T = 4;
+__global__ void __launch_bounds__(256) k_dense_tile(const float* __restrict__ w0, const float* __restrict__ w1, int rows, int cols, const float* __restrict__ x, size_t x_ts,
+                                                    float* y0, float* y1, size_t y_ts, int nt) {
+    IT_PDL_TRIGGER(); IT_PDL_WAIT();
+    __shared__ double wsum[8][DR_W * DR_T];
+    const int r0 = blockIdx.x * DR_W, t0 = blockIdx.y * DR_T, tid = threadIdx.x;
+    const float* wp[DR_W]; const float* xp[DR_T];
+#pragma unroll
+    for (int r = 0; r < DR_W; r++) { const int g = min(r0 + r, 2 * rows - 1); wp[r] = (g < rows ? w0 + (size_t)g * cols : w1 + (size_t)(g - rows) * cols); }
+#pragma unroll
+    for (int t = 0; t < DR_T; t++) xp[t] = x + (size_t)min(t0 + t, nt - 1) * x_ts;
+    double s[DR_W][DR_T];
+#pragma unroll
+    for (int r = 0; r < DR_W; r++)
+#pragma unroll
+        for (int t = 0; t < DR_T; t++) s[r][t] = 0.0;
+    for (int i = tid; i < cols; i += 256) {
+        float a[DR_W], b[DR_T];
+#pragma unroll
+        for (int r = 0; r < DR_W; r++) a[r] = wp[r][i];
+#pragma unroll
+        for (int t = 0; t < DR_T; t++) b[t] = xp[t][i];
+#pragma unroll
+        for (int r = 0; r < DR_W; r++)
+#pragma unroll
+            for (int t = 0; t < DR_T; t++) s[r][t] += (double)it_mul(a[r], b[t]);
+    }
+#pragma unroll
+    for (int r = 0; r < DR_W; r++)
+#pragma unroll
+        for (int t = 0; t < DR_T; t++) {
+            double v = s[r][t];
+#pragma unroll
+            for (int m = 16; m >= 1; m >>= 1) v += __shfl_xor_sync(0xffffffffu, v, m);
+            if ((tid & 31) == 0) wsum[tid >> 5][r * DR_T + t] = v;
+        }
+    __syncthreads();
+    if (tid < DR_W * DR_T) {
+        const int g = r0 + tid / DR_T, t = t0 + tid % DR_T;
+        double v = wsum[0][tid];
+        for (int k = 1; k < 8; k++) v += wsum[k][tid];
+        if (g < 2 * rows && t < nt) (g < rows ? y0 : y1)[(size_t)t * y_ts + (g < rows ? g : g - rows)] = (float)v;
     }
 }
 
@@ -606,13 +685,18 @@ int it_sup_rope(it_ctx* c, float* x, size_t hs, size_t ts, int nheads, int nt, i
 int it_sup_conv(it_ctx* c, const float* mixed, size_t m_ts, const float* w, float* state, float* out, size_t o_ts, int cd, int kk, int nt, float* ck, size_t ck_stride, int nck) {
     if (kk < 2 || kk > 9) return it_fail(IT_EINVAL, "conv kernel size %d not supported", kk);
     it_note_op(c);
-    if (nt > 8 && nck == 0) {   // prompt passes: rows in parallel
+    if (nt > 8 && nck == 0 && kk == 4) {   // prompt passes: rows in parallel
+        it_pdl(k_conv_rows<4>, dim3((cd + 127) / 128, (nt + CONV_ROWS - 1) / CONV_ROWS), dim3(128), 0, c->stream, mixed, m_ts, w, state, out, o_ts, cd, nt); KCHK("conv_rows"); return IT_OK;
+    }
+    if (nt > 8 && nck == 0) {
         it_pdl(k_conv_wide, dim3((cd + 127) / 128), dim3(128, 8), 0, c->stream, mixed, m_ts, w, state, out, o_ts, cd, kk, nt); KCHK("conv_wide"); return IT_OK;
     }
     it_pdl(k_conv, dim3((cd + 127) / 128), dim3(128), 0, c->stream, mixed, m_ts, w, state, out, o_ts, cd, kk, nt, ck, ck_stride, nck); KCHK("conv"); return IT_OK;
 }
 int it_sup_dense_rows(it_ctx* c, const float* w0, const float* w1, int rows, int cols, const float* x, size_t x_ts, float* y0, float* y1, size_t y_ts, int nt) {
-    it_note_op(c); it_pdl(k_dense_rows, dim3(dim3(2 * rows, nt)), dim3(256), 0, c->stream, w0, w1, rows, cols, x, x_ts, y0, y1, y_ts); KCHK("dense_rows"); return IT_OK;
+    it_note_op(c);
+    if (nt >= 8) { it_pdl(k_dense_tile, dim3((2 * rows + DR_W - 1) / DR_W, (nt + DR_T - 1) / DR_T), dim3(256), 0, c->stream, w0, w1, rows, cols, x, x_ts, y0, y1, y_ts, nt); KCHK("dense_tile"); return IT_OK; }
+    it_pdl(k_dense_rows, dim3(dim3(2 * rows, nt)), dim3(256), 0, c->stream, w0, w1, rows, cols, x, x_ts, y0, y1, y_ts); KCHK("dense_rows"); return IT_OK;
 }
 int it_sup_gdn(it_ctx* c, const float* co, size_t co_ts, const float* beta, const float* alpha, size_t ba_ts, const float* dt, const float* a, float* state, float* o, size_t o_ts,
                int nv, int nk, int sd, int qk, int nt, float* ck, size_t ck_stride, int nck) {
