@@ -5,8 +5,11 @@
 #include <map>
 #include <vector>
 
-#define IT_MAXT 256   // activation rows per pass: the prompt chunk of prefill_chunks (src/vk/mod.rs:130-134 uses 64; the chunk size changes no result,
-                      // and with 256 rows the tile kernels pay their per-block cost once per 128 rows and the row-parallel kernels fill the GPU)
+#define IT_MAXT 1024  // activation rows per pass: the prompt chunk of prefill_chunks (src/vk/mod.rs:130-134 uses 64; the chunk size changes no result).
+                      // The tile kernel has one CTA per SM and tiles of 128 x 128: at 256 rows a 5120-row matrix is 80 tiles for 148 SMs, at 1024
+                      // it is 320 (2.2 waves), at 7 x 128 rows 280 (1.9).  4 layers of the 27B shape, 777 tokens: 7987 us in 256-row passes, 6284 in
+                      // one; 4096 tokens: 47.7 ms and 40.8
+#define IT_HIDDEN_ROWS 256  // it_engine_hidden_read counts rows of a pass from its last multiple of this many
 #define IT_MAXLOGIT 8 // rows of a pass that can get logits and a greedy pick (verification passes)
 #define IT_MAXCK 3    // recurrent-state checkpoints per pass (rows 0..2 of a verification pass)
 
@@ -58,6 +61,7 @@ struct it_engine {
     std::vector<void*> owned;                        // plain device allocations to free
     int pos, mpos;                                   // trunk position; next MTP position (src/vk/mod.rs: pos, mpos)
     size_t hp_off; int hp_n;                         // pending h rows for the next draft (arena offset, count)
+    int pass_rows;                                   // rows of the trunk's last pass (it_engine_hidden_read)
     int last_rows;                                   // rows of the last verification pass (it_engine_mtp_rollback)
     it_graph* step_graph;                            // recorded single-token greedy step
     uint32_t* host_pin;                              // pinned staging, laid out like toks_dev, plus the position at [2*IT_MAXT]

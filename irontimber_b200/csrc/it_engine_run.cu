@@ -3,8 +3,8 @@
 // The schedule of one pass is the reference's run_chunk_v (src/vk/mod.rs:763-892): per layer norm -> Hadamard ->
 // grouped ternary matvecs -> delta-rule or attention block -> Hadamard -> output matvec (accumulating into the residual)
 // -> norm -> Hadamard -> gate / up -> silu*mul -> Hadamard -> down (accumulating).  Differences: the Hadamard is fused
-// with q8k quantisation (the CPU numerics), embeddings are gathered on the device, and a pass takes up to IT_MAXT rows (four
-// times the reference's prompt chunk; the chunk size changes no result): passes of more than eight rows run their ternary
+// with q8k quantisation (the CPU numerics), embeddings are gathered on the device, and a pass takes up to IT_MAXT rows (the
+// reference's prompt chunk is 64; the chunk size changes no result): passes of more than eight rows run their ternary
 // products on the tile kernels.
 #include "it_engine.h"
 #include "it_support.h"
@@ -134,7 +134,7 @@ int it_engine_run_chunk(it_engine* e, const uint32_t* toks, int nt, int logit_ro
     IT_TRY(it_sup_rmsnorm_wide(cx, A + L.x, e_, e->output_norm, e_, c.eps, A + L.hrow, e_, nt));
     if (logit_rows == 2) IT_TRY(logits_and_argmax(e, L.hrow, nt));
     else if (logit_rows == 1) IT_TRY(logits_and_argmax(e, L.hrow + (size_t)(nt - 1) * e_, 1));
-    if (!from_dev) e->pos += nt;
+    if (!from_dev) { e->pos += nt; e->pass_rows = nt; }
     return IT_OK;
 }
 
@@ -228,7 +228,7 @@ int trunk_pass(it_engine* e, const uint32_t* toks, int nt, int logit_rows, int n
     IT_CUDA(cudaMemcpyAsync(e->pos_dev, slot + 8, sizeof(uint32_t), cudaMemcpyHostToDevice, cx->stream));
     IT_TRY(replay_pass(e, 1ull << 60 | (uint64_t)nt | (uint64_t)logit_rows << 8 | (uint64_t)nck << 16,
                        [&]() { return it_engine_run_chunk(e, nullptr, nt, logit_rows, nck, true); }));
-    e->pos += nt;
+    e->pos += nt; e->pass_rows = nt;
     return IT_OK;
 }
 int head_pass(it_engine* e, const uint32_t* toks, int nt, int pos0, size_t hoff, bool predict) {
@@ -295,6 +295,7 @@ namespace {
 // one pass with the position read on the device, pick -> token slot and position + 1.
 int begin_device_decode(it_engine* e) {
     it_ctx* cx = e->ctx;
+    e->pass_rows = 1;
     uint32_t* pin = pin_block(e) + 2 * IT_MAXT;
     *pin = (uint32_t)e->pos;
     IT_CUDA(cudaMemcpyAsync(e->pos_dev, pin, 4, cudaMemcpyHostToDevice, cx->stream));
