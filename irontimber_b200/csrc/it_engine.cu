@@ -242,6 +242,15 @@ int it_engine_build(int device, const it_model_config* cfg, uint64_t seed, int w
         E_TRY(dev_alloc(e, (void**)&e->mkc, (size_t)c.ctx_len * kvd * 4, true)); E_TRY(dev_alloc(e, (void**)&e->mvc, (size_t)c.ctx_len * kvd * 4, true));
     }
     E_TRY(it_q8_create(e->ctx, (size_t)std::max(std::max(e_, ff), std::max(inner, nh * hd)), IT_MAXT, &e->q8));
+    {
+        std::vector<it_state_ptrs> sp;
+        for (const it_layer& l : e->layers) if (l.recurrent) sp.push_back({ l.conv_st, l.ssm_st, l.ck_conv, l.ck_ssm });
+        e->n_recurrent = (int)sp.size(); e->state_ptrs = nullptr;
+        if (!sp.empty()) {
+            E_TRY(dev_alloc(e, (void**)&e->state_ptrs, sp.size() * sizeof(it_state_ptrs), false));
+            if (cudaMemcpy(e->state_ptrs, sp.data(), sp.size() * sizeof(it_state_ptrs), cudaMemcpyHostToDevice) != cudaSuccess) return fail(it_fail(IT_ECUDA, "engine: state table upload failed"));
+        }
+    }
     e->att_scratch_floats = std::min(IT_ATT_SCRATCH_FLOATS, (size_t)IT_MAXT * nh * (((size_t)c.ctx_len + 127) / 128 * 128));
     E_TRY(dev_alloc(e, (void**)&e->att_scratch, e->att_scratch_floats * sizeof(float), false));
     E_TRY(dev_alloc(e, (void**)&e->toks_dev, (2 * IT_MAXT + 8) * sizeof(uint32_t), true));

@@ -35,6 +35,9 @@ struct it_arena_layout {   // element offsets into the context's f32 arena; ever
     size_t big1_stride, big2_stride, o_stride, logits_stride;
 };
 
+// State buffers of one delta-net layer and their checkpoints, for the kernel that restores all layers at once
+struct it_state_ptrs { float *conv_st, *ssm_st; const float *ck_conv, *ck_ssm; };
+
 struct it_step_state;   // geometry and device tables of the persistent decode-step kernel (it_step.cu)
 
 struct it_engine {
@@ -57,6 +60,7 @@ struct it_engine {
     int* pos_dev;                                    // position read by the recorded decode step
     it_arena_layout lay;
     float theta_scale;
+    it_state_ptrs* state_ptrs; int n_recurrent;      // device table of the delta-net layers' state (restore_checkpoint); null when there is none
     float* att_scratch; size_t att_scratch_floats;   // attention scores of a block of prompt rows (it_sup_attention_tiled)
     std::vector<void*> owned;                        // plain device allocations to free
     int pos, mpos;                                   // trunk position; next MTP position (src/vk/mod.rs: pos, mpos)
