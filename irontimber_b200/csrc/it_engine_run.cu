@@ -97,14 +97,9 @@ int it_engine_run_chunk(it_engine* e, const uint32_t* toks, int nt, int logit_ro
             if (gr < 0) return gr;
             if (gr == 0) IT_TRY(it_sup_norm_head(cx, A + L.o, sd, inner, A + L.o, sd, inner, sd, nv, l.ssm_norm, 1, c.eps, A + L.big1 + cd, sd, s_gdn, nt));
             else if (sd == 128) {
-                // [delta rule | gated norm] in one launch, for any number of rows (the state stays in shared memory across the rows)
-                // (the kernel stages up to IT_GDN_MAXROWS rows at a time; the state carries over from one launch to the next)
-                for (int t0 = 0; t0 < nt; t0 += IT_GDN_MAXROWS) {
-                    const int n0 = std::min(IT_GDN_MAXROWS, nt - t0);
-                    IT_TRY(it_sup_gdn_norm(cx, A + L.conv + (size_t)t0 * cd, cd, A + L.beta + (size_t)t0 * nv, A + L.alpha + (size_t)t0 * nv, nv, l.dt, l.a, l.ssm_st,
-                                           A + L.o + (size_t)t0 * inner, inner, nv, nk, sd, qk, n0, l.ck_ssm, ssz, t0 ? 0 : nck,
-                                           l.ssm_norm, c.eps, A + L.big1 + cd + (size_t)t0 * s_gdn, s_gdn));
-                }
+                // [delta rule | gated norm] in one launch (the state stays in shared memory across the rows)
+                IT_TRY(it_sup_gdn_norm(cx, A + L.conv, cd, A + L.beta, A + L.alpha, nv, l.dt, l.a, l.ssm_st, A + L.o, inner, nv, nk, sd, qk, nt, l.ck_ssm, ssz, nck,
+                                       l.ssm_norm, c.eps, A + L.big1 + cd, s_gdn));
             } else {
                 IT_TRY(it_sup_gdn(cx, A + L.conv, cd, A + L.beta, A + L.alpha, nv, l.dt, l.a, l.ssm_st, A + L.o, inner, nv, nk, sd, qk, nt, l.ck_ssm, ssz, nck));
                 IT_TRY(it_sup_norm_head(cx, A + L.o, sd, inner, A + L.o, sd, inner, sd, nv, l.ssm_norm, 1, c.eps, A + L.big1 + cd, sd, s_gdn, nt));
