@@ -13,7 +13,7 @@
 //            code - 1 in the same K-major 128-byte-swizzled layout (row r at 128 r, 16-byte piece p at (p ^ (r & 7)) * 16), so that
 //            the accumulator is S - sum128 at once, and the f16 block scales of the 128 rows into f32
 //   warp 17  one thread issues eight tcgen05.mma (M 128, K 32, s8 x s8 -> s32) per step into the step's two accumulators in tensor
-//            memory and commits them to one mbarrier (accumulators ready; tiles and boxes free again)
+//            memory and commits them to two mbarriers (accumulators ready and tiles free again; boxes free again)
 //   warp 19  fetches the next tile's activation scales
 //   warps 0-7 epilogue: reads the accumulators (a thread gets four rows x every fourth column), forms
 //            (d_w * d_x) * float(S - sum128) for each and adds it to an f32 accumulator it keeps in registers for the
@@ -67,7 +67,7 @@ template <int NH> __host__ __device__ inline TcSmem tc_layout(int nb, int wstage
     L.w = o; o += wstages * TC_W_BYTES;
     L.dx = o; L.dx_bytes = (nb / 2) * Tc<NH>::TOK * 4; o += dxbufs * L.dx_bytes;
     L.dw = o; o += Tc<NH>::NDW * TC_ROWS * 4;
-    L.bars = o; o += (2 * wstages + xsteps + TC_NA + 2 * Tc<NH>::ND + 4) * 8;
+    L.bars = o; o += (2 * wstages + 2 * xsteps + TC_NA + 2 * Tc<NH>::ND + 4) * 8;
     o = (o + 15) & ~15;
     L.tmem = o; o += 16;
     L.flag = o; o += 16;
@@ -137,11 +137,13 @@ k_matmul_tc(const __grid_constant__ CUtensorMap xmap, const uint8_t* __restrict_
     volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + L.flag);
     unsigned* tmem_slot = reinterpret_cast<unsigned*>(smem + L.tmem);
     const unsigned bars = smem_u32(smem + L.bars);
-    // barrier addresses: weight stages (full / empty), activation boxes of a step landed, tiles of a step expanded, accumulators of a
-    // step (full / empty), activation scales (full / empty).  "Accumulators d full" is the one commit of a step: it also tells the
-    // expanders and the activation producer that the tiles and boxes the step read may be reused.
-    const unsigned wfull0 = bars, wempty0 = wfull0 + 8 * wstages, xfull0 = wempty0 + 8 * wstages,
-                   afull0 = xfull0 + 8 * xsteps, dfull0 = afull0 + 8 * TC_NA, dempty0 = dfull0 + 8 * TC_ND, sfull0 = dempty0 + 8 * TC_ND, sempty0 = sfull0 + 16;
+    // barrier addresses: weight stages (full / empty), activation boxes of a step (landed / free), tiles of a step expanded, accumulators of
+    // a step (full / empty), activation scales (full / empty).  "Accumulators d full" also tells the expanders that the tiles the step
+    // read may be reused: the next phase of that barrier needs their next tiles.  The boxes have barriers of their own, one per slot:
+    // with two accumulators and three slots the box of step n - 1 is in place while the producer waits for step n - 3, and
+    // both commit to one "accumulators full", whose parity could flip twice before the producer looks.
+    const unsigned wfull0 = bars, wempty0 = wfull0 + 8 * wstages, xfull0 = wempty0 + 8 * wstages, xempty0 = xfull0 + 8 * xsteps,
+                   afull0 = xempty0 + 8 * xsteps, dfull0 = afull0 + 8 * TC_NA, dempty0 = dfull0 + 8 * TC_ND, sfull0 = dempty0 + 8 * TC_ND, sempty0 = sfull0 + 16;
     // The CTA's tiles: blockIdx.x, + gridDim.x, ...; the activation tiles of one group of matrix rows are neighbours.  Every role walks
     // the same tiles with its ring positions running on, so the next tile's weights, boxes and products are under way while
     // the epilogue still stores the last one's results.
@@ -150,7 +152,7 @@ k_matmul_tc(const __grid_constant__ CUtensorMap xmap, const uint8_t* __restrict_
     if (tid == 0) {
         *abort_flag = 0;
         for (int s = 0; s < wstages; s++) { mbar_init(wfull0 + 8 * s, 1); mbar_init(wempty0 + 8 * s, 8); }
-        for (int s = 0; s < xsteps; s++) mbar_init(xfull0 + 8 * s, 1);
+        for (int s = 0; s < xsteps; s++) { mbar_init(xfull0 + 8 * s, 1); mbar_init(xempty0 + 8 * s, 1); }
         for (int a = 0; a < TC_NA; a++) mbar_init(afull0 + 8 * a, 4);
         for (int d = 0; d < TC_ND; d++) { mbar_init(dfull0 + 8 * d, 1); mbar_init(dempty0 + 8 * d, TC_EPI_WARPS); }
         for (int k = 0; k < 2; k++) { mbar_init(sfull0 + 8 * k, 1); mbar_init(sempty0 + 8 * k, TC_EPI_WARPS); }
@@ -198,21 +200,17 @@ k_matmul_tc(const __grid_constant__ CUtensorMap xmap, const uint8_t* __restrict_
         // ---------------- activation producer: the rows come from the kernel before this one
         if (lane == 0) {
             asm volatile("griddepcontrol.wait;" ::: "memory");
-            int s = 0, issued = 0, dp = 0; unsigned dpp = 0; bool ok = true;
+            int s = 0, issued = 0; unsigned ph = 0; bool ok = true;
             for (int tile = tile0; ok && tile < ntiles; tile += tstep) {
                 const int tok0 = tile % tok_tiles * TC_TOK;
                 for (int p = 0; p < np; p++) {
-                    // the slot was last read xsteps steps ago: wait for that step's commit
-                    if (issued >= xsteps) {
-                        if (!mbar_wait(dfull0 + 8 * dp, dpp, abort_flag, error_flag, 19)) { ok = false; break; }
-                        if (++dp == TC_ND) { dp = 0; dpp ^= 1u; }
-                    }
+                    if (!mbar_wait(xempty0 + 8 * s, ph ^ 1u, abort_flag, error_flag, 19)) { ok = false; break; }   // the step that last read the slot has committed
                     mbar_expect_tx(xfull0 + 8 * s, (unsigned)(2 * TC_X_BYTES));
 #pragma unroll
                     for (int k = 0; k < 2 * NH; k++)     // 64 rows per box; the boxes of a block lie one under the other like one box of TOK rows
                         tma_load_2d(smem_u32(smem + L.x + s * 2 * TC_X_BYTES + k * 64 * 128), &xmap, (2 * p + k / NH) * 128, tok0 + 64 * (k % NH), xfull0 + 8 * s);
                     issued++;
-                    if (++s == xsteps) s = 0;
+                    if (++s == xsteps) { s = 0; ph ^= 1u; }
                 }
             }
             if (*abort_flag) {
@@ -226,7 +224,7 @@ k_matmul_tc(const __grid_constant__ CUtensorMap xmap, const uint8_t* __restrict_
     } else if (warp == TC_EPI_WARPS + TC_EXP_WARPS + 1) {
         // ---------------- MMA issuer
         if (lane == 0) {
-            int s = 0, a = 0, d = 0; unsigned xph = 0, aph = 0, dph = 0; bool ok = true;
+            int s = 0, a = 0, d = 0; unsigned xph = 0, aph = 0, dph = 0, last = 0, last_ph = 0; bool ok = true;
             const unsigned long long adesc0 = tc_smem_desc(smem_u32(smem + L.a)), bdesc0 = tc_smem_desc(smem_u32(smem + L.x));
             for (int tile = tile0; ok && tile < ntiles; tile += tstep)
             for (int p = 0; p < np; p++) {
@@ -244,11 +242,16 @@ k_matmul_tc(const __grid_constant__ CUtensorMap xmap, const uint8_t* __restrict_
                     tc_mma<true>(dt, ad + 4, bd + 4, Tc<NH>::IDESC);
                     tc_mma<true>(dt, ad + 6, bd + 6, Tc<NH>::IDESC);
                 }
-                tc_commit(dfull0 + 8 * d);        // accumulators complete; tiles and boxes of this step may be reused
+                tc_commit(dfull0 + 8 * d);        // accumulators complete; the tiles of this step may be reused
+                tc_commit(xempty0 + 8 * s);       // its boxes too
+                last = xempty0 + 8 * s; last_ph = xph;
                 if (++s == xsteps) { s = 0; xph ^= 1u; }
                 if (++a == TC_NA) { a = 0; aph ^= 1u; }
                 if (++d == TC_ND) { d = 0; dph ^= 1u; }
             }
+            // the last commit's arrival must find the CTA's shared memory still its own (bounded)
+            const long long t0 = clock64();
+            while (last && !mbar_test(last, last_ph) && clock64() - t0 < WAIT_CLOCKS) { }
         }
     } else if (warp == TC_EPI_WARPS + TC_EXP_WARPS + 3) {
         // ---------------- activation scales of every tile but the first (which the epilogue warps fetch together), one tile ahead

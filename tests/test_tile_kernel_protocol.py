@@ -1,0 +1,65 @@
+"""The hand-over protocol of the tensor-memory tile kernel (it_matmul_tc.cu), without a GPU.
+
+A wait on an mbarrier sees one bit, the parity of the phase: a role that has not yet seen phase q complete must be sure that phase
+q + 1 of the same barrier cannot complete first, or it waits for good.  The model below has the kernel's roles as step counters and
+walks every order in which they can proceed; which barrier the activation producer waits for is read from the source.
+"""
+import os
+import re
+
+import pytest
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "irontimber_b200", "csrc")
+STEPS = 14
+
+
+def source(name):
+    with open(os.path.join(CSRC, name)) as f:
+        return f.read()
+
+
+def producer_ring():
+    """The ring of barriers on which the activation producer waits before it fills a slot again."""
+    role = source("it_matmul_tc.cu").split("---------------- activation producer", 1)[1].split("} else if (warp", 1)[0]
+    return re.search(r"mbar_wait\((\w+)0 \+ 8 \*", role).group(1)
+
+
+def overtaken(acc, boxes, ring):
+    """(role, step) of a wait whose barrier can be two phases on; None when there is no such order.  acc: accumulator barriers, boxes:
+    slots of the activation ring, ring: "dfull" or "xempty" (one barrier per accumulator or per slot)."""
+    lag = acc if ring == "dfull" else boxes         # commits between two phases of one barrier the producer waits for
+    seen, todo = set(), [(0, 0, 0, 0, 0, 0)]
+    while todo:
+        st = todo.pop()
+        if st in seen:
+            continue
+        seen.add(st)
+        x, e0, e1, m, c, p = st                     # boxes issued, steps expanded by either set, MMAs issued, committed, steps folded
+        for role, q, per in (("producer", x - boxes, lag), ("expanders 0", 2 * e0 - 2, acc), ("expanders 1", 2 * e1 - 1, acc), ("epilogue", p, acc)):
+            if q >= 0 and c > q + per:
+                return role, q
+        if x < STEPS and (x < boxes or c > x - boxes):
+            todo.append((x + 1, e0, e1, m, c, p))
+        if 2 * e0 < STEPS and c > 2 * e0 - 2:
+            todo.append((x, e0 + 1, e1, m, c, p))
+        if 2 * e1 + 1 < STEPS and c > 2 * e1 - 1:
+            todo.append((x, e0, e1 + 1, m, c, p))
+        if m < x and (e1 if m & 1 else e0) > m // 2 and p > m - acc:
+            todo.append((x, e0, e1, m + 1, c, p))
+        if c < m:
+            todo.append((x, e0, e1, m, c + 1, p))
+        if p < c:
+            todo.append((x, e0, e1, m, c, p + 1))
+    assert (STEPS, STEPS // 2, STEPS // 2, STEPS, STEPS, STEPS) in seen           # the model can run to its end
+    return None
+
+
+@pytest.mark.parametrize("acc,boxes", [(4, 2), (4, 3), (2, 2), (2, 3)])      # 64- and 128-row tiles, with two and three steps of boxes
+def test_no_wait_can_be_overtaken(acc, boxes):
+    assert overtaken(acc, boxes, producer_ring()) is None
+
+
+def test_the_model_sees_an_overtaken_wait():
+    """Three slots freed by the commits of two accumulators: box n - 1 is in place while the producer waits for step n - 3, and both commit
+    to one barrier."""
+    assert overtaken(2, 3, "dfull") == ("producer", 0)
