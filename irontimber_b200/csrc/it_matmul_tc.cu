@@ -260,8 +260,7 @@ k_matmul_tc(const __grid_constant__ CUtensorMap xmap, const uint8_t* __restrict_
         for (int tile = tile0 + tstep; tile < ntiles; tile += tstep, j++) {
             const int k = j & 1;
             const int tok0 = tile % tok_tiles * TC_TOK, ntv = min(TC_TOK, ntok - tok0);
-            const bool ok = mbar_wait(sempty0 + 8 * k, ((unsigned)(j >> 1) & 1u) ^ 1u, abort_flag, error_flag, 20);     // tile j - 2 is done with it
-            if (!__all_sync(0xffffffffu, ok)) break;
+            if (!mbar_wait_warp(sempty0 + 8 * k, ((unsigned)(j >> 1) & 1u) ^ 1u, abort_flag, error_flag, 20)) break;     // tile j - 2 is done with it
             float* dxs = reinterpret_cast<float*>(smem + L.dx + k * L.dx_bytes);
             for (int m = lane; m < TC_TOK; m += 32) {
                 const float* src = xd + (size_t)(tok0 + m) * (x_stride / 256);
@@ -286,10 +285,10 @@ k_matmul_tc(const __grid_constant__ CUtensorMap xmap, const uint8_t* __restrict_
         for (int p = 0; p < np; p++, gp++) {
             const bool last = (p & 1) || p + 1 == np;         // last step of the weight stage
             if ((gp & 1) == eset) {
-                if (!mbar_wait(wfull0 + 8 * s, sph, abort_flag, error_flag, 15)) { ok = false; break; }
+                if (!mbar_wait_warp(wfull0 + 8 * s, sph, abort_flag, error_flag, 15)) { ok = false; break; }
                 // the tile pair was last read two steps ago: wait for that step's commit
                 if (gp >= 2) {
-                    if (!mbar_wait(dfull0 + 8 * dp, dpp, abort_flag, error_flag, 16)) { ok = false; break; }
+                    if (!mbar_wait_warp(dfull0 + 8 * dp, dpp, abort_flag, error_flag, 16)) { ok = false; break; }
                     dp += 2;
                     if (dp >= TC_ND) { dp -= TC_ND; dpp ^= 1u; }
                 }
@@ -350,7 +349,7 @@ k_matmul_tc(const __grid_constant__ CUtensorMap xmap, const uint8_t* __restrict_
             const int k = j & 1;
             const int rg0 = tile / tok_tiles * 4, tok0 = tile % tok_tiles * TC_TOK, ntv = min(TC_TOK, ntok - tok0);
             const bool active = m0 < ntv;              // groups past the last activation row only release the accumulators
-            if (j > 0 && !mbar_wait(sfull0 + 8 * k, (unsigned)((j - 1) >> 1) & 1u, abort_flag, error_flag, 18)) break;
+            if (j > 0 && !mbar_wait_warp(sfull0 + 8 * k, (unsigned)((j - 1) >> 1) & 1u, abort_flag, error_flag, 18)) break;
             const float4* dxs = reinterpret_cast<const float4*>(smem + L.dx + k * L.dx_bytes) + m0 / 4 + t;
             f32x2 acc[2][8 * CC];                      // rows g + 16 hf and g + 8 + 16 hf of column 4 c + t
 #pragma unroll
@@ -358,8 +357,7 @@ k_matmul_tc(const __grid_constant__ CUtensorMap xmap, const uint8_t* __restrict_
 #pragma unroll
                 for (int c = 0; c < 8 * CC; c++) acc[hf][c] = 0ull;
             for (int p = 0; p < np; p++) {             // two blocks at a time: they share the activation scale, the wait and the release
-                if (!mbar_wait(dfull0 + 8 * d, dph, abort_flag, error_flag, 17)) { ok = false; break; }
-                __syncwarp();
+                if (!mbar_wait_warp(dfull0 + 8 * d, dph, abort_flag, error_flag, 17)) { ok = false; break; }
                 if (active) {
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     // chunks of 32 columns of one block; the next one is on its way while one is folded
@@ -397,7 +395,7 @@ k_matmul_tc(const __grid_constant__ CUtensorMap xmap, const uint8_t* __restrict_
                 if (++d == TC_ND) { d = 0; dph ^= 1u; }
                 r = r + 2 == NDW ? 0 : r + 2;
             }
-            if (!ok || *abort_flag) break;
+            if (!ok || __any_sync(0xffffffffu, *abort_flag)) break;
             __syncwarp();
             if (lane == 0) mbar_arrive(sempty0 + 8 * k);          // the tile's activation scales have been read
             if (!active) continue;

@@ -54,6 +54,11 @@ __device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned parity, volatil
     if (mbar_test(bar, parity)) return true;
     return mbar_wait_retry(bar, parity, abort_flag, error_flag, site);
 }
+// For a warp that goes on as one: true in every lane or in none.  A lane that gave up by itself would leave its siblings at the next
+// warp-wide instruction, without a limit.
+__device__ __forceinline__ bool mbar_wait_warp(unsigned bar, unsigned parity, volatile int* abort_flag, int* error_flag, int site = 1) {
+    return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, error_flag, site));
+}
 __device__ __forceinline__ void bulk_load(unsigned dst, const void* src, unsigned bytes, unsigned bar) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                  :: "r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");

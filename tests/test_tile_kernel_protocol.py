@@ -63,3 +63,27 @@ def test_the_model_sees_an_overtaken_wait():
     """Three slots freed by the commits of two accumulators: box n - 1 is in place while the producer waits for step n - 3, and both commit
     to one barrier."""
     assert overtaken(2, 3, "dfull") == ("producer", 0)
+
+
+def warp_statements(src, pattern):
+    """Statements of `src` in which `pattern` occurs and that no enclosing condition gives to one lane."""
+    out, scopes = [], []
+    for m in re.finditer(r"[{}]|" + pattern, src):
+        head = re.split(r"[;{}]", src[:m.start()])[-1]
+        if m.group() == "{":
+            scopes.append(head)
+        elif m.group() == "}":
+            scopes.pop()
+        elif not any("lane == 0" in s or "tid == 0" in s for s in scopes + [head]):
+            out.append(head + re.split(r"[;{}]", src[m.start():])[0])
+    return out
+
+
+def test_a_warp_gives_up_as_one():
+    """The roles of whole warps go on to warp-wide instructions: a lane that leaves alone after a wait that ran out, or after a look of its
+    own at the abort flag, leaves its siblings there without a limit."""
+    src = re.sub(r'//[^\n]*|"[^"\n]*"', "", source("it_matmul_tc.cu"))
+    kernel = src[src.index("k_matmul_tc("):src.index("it_shard_finish")]
+    assert warp_statements(kernel, r"mbar_wait\(") == []
+    assert [s for s in warp_statements(kernel, r"\*abort_flag\b") if "__any_sync" not in s and "lane == 0" not in s and "volatile int* abort_flag" not in s] == []
+    assert len(warp_statements(kernel, r"mbar_wait_warp\(")) == 5          # expanders (two), scales, epilogue (two)
