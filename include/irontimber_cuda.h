@@ -233,7 +233,10 @@ int it_engine_tensor_read(it_engine* e, int layer, int tensor, void* host);
 int it_engine_signs_read(it_engine* e, size_t width, float* host);
 /* which: 0 conv state, 1 ssm state, 2 K cache, 3 V cache (active positions, decoded to f32), 4 MTP K, 5 MTP V. */
 int it_engine_state_read(it_engine* e, int layer, int which, float* host, size_t max_floats, size_t* n_floats);
-int it_engine_hidden_read(it_engine* e, size_t row, float* host);   /* output-normed hidden row of the last pass (h_nextn) */
+/* Output-normed hidden row (h_nextn), row < 256.  Rows count as if every call ran its tokens in passes of 256, whatever passes the library
+ * runs: after n tokens given at once row r is token (n - 1) / 256 * 256 + r of them, the last token row (n - 1) % 256; a row that
+ * the last such pass did not reach is the one an earlier pass left there. */
+int it_engine_hidden_read(it_engine* e, size_t row, float* host);
 int it_engine_position(it_engine* e);
 
 /* Engine trait (src/engine.rs:8-15).  eval: feed tokens, optionally return the last token's logits (n_vocab floats).

@@ -179,7 +179,8 @@ int it_engine_build(int device, const it_model_config* cfg, uint64_t seed, int w
     e->ctx = nullptr; e->step = nullptr; e->pin_next = 0; e->cfg = c; e->seed = seed; e->has_mtp = with_mtp != 0; e->rank = rank; e->world = world; e->output = nullptr; e->tok_embd = e->m_tok_embd = nullptr; e->q8 = nullptr; e->step_graph = nullptr; e->host_pin = nullptr; e->small_pin = nullptr; e->small_next = 0;
     { const char* v = getenv("IT_PASS_GRAPHS"); e->record_passes = !v || atoi(v) != 0; }
     e->m_eh = e->m_q = e->m_k = e->m_v = e->m_o = e->m_gate = e->m_up = e->m_down = nullptr;
-    e->pos = 0; e->mpos = 1; e->hp_off = 0; e->hp_n = 0; e->last_rows = 0; e->pass_rows = 1;
+    e->pos = 0; e->mpos = 1; e->hp_off = 0; e->hp_n = 0; e->last_rows = 0;
+    for (int r = 0; r < IT_HIDDEN_ROWS; r++) e->hidden_at[r] = (uint16_t)r;
     // arena layout
     it_arena_layout& L = e->lay; size_t o = 0;
     auto take = [&](size_t& field, size_t n) { field = o; o += up64(n); };
@@ -374,8 +375,5 @@ IT_API int it_engine_state_read(it_engine* e, int layer, int which, float* host,
 }
 IT_API int it_engine_hidden_read(it_engine* e, size_t row, float* host) {
     IT_CHECK_ARG(e && host && row < IT_HIDDEN_ROWS, "it_engine_hidden_read: bad argument");
-    // rows [first, pass_rows) are counted from 0; rows past them are what the rows before them left
-    const size_t first = (size_t)(e->pass_rows - 1) / IT_HIDDEN_ROWS * IT_HIDDEN_ROWS;
-    const size_t at = first + row < (size_t)e->pass_rows || first == 0 ? first + row : first - IT_HIDDEN_ROWS + row;
-    return it_arena_read(e->ctx, e->lay.hrow + at * e->cfg.n_embd, host, e->cfg.n_embd);
+    return it_arena_read(e->ctx, e->lay.hrow + (size_t)e->hidden_at[row] * e->cfg.n_embd, host, e->cfg.n_embd);
 }

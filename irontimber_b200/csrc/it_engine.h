@@ -9,7 +9,7 @@
                       // The tile kernel has one CTA per SM and tiles of 128 x 128: at 256 rows a 5120-row matrix is 80 tiles for 148 SMs, at 1024
                       // it is 320 (2.2 waves), at 7 x 128 rows 280 (1.9).  4 layers of the 27B shape, 777 tokens: 7987 us in 256-row passes, 6284 in
                       // one; 4096 tokens: 47.7 ms and 40.8
-#define IT_HIDDEN_ROWS 256  // it_engine_hidden_read counts rows of a pass from its last multiple of this many
+#define IT_HIDDEN_ROWS 256  // rows it_engine_hidden_read can be asked for: they count as if prompts ran in passes of this many
 #define IT_MAXLOGIT 8 // rows of a pass that can get logits and a greedy pick (verification passes)
 #define IT_MAXCK 3    // recurrent-state checkpoints per pass (rows 0..2 of a verification pass)
 
@@ -65,7 +65,7 @@ struct it_engine {
     std::vector<void*> owned;                        // plain device allocations to free
     int pos, mpos;                                   // trunk position; next MTP position (src/vk/mod.rs: pos, mpos)
     size_t hp_off; int hp_n;                         // pending h rows for the next draft (arena offset, count)
-    int pass_rows;                                   // rows of the trunk's last pass (it_engine_hidden_read)
+    uint16_t hidden_at[IT_HIDDEN_ROWS];              // where in the arena's hrow the rows of it_engine_hidden_read lie (it_engine_note_rows)
     int last_rows;                                   // rows of the last verification pass (it_engine_mtp_rollback)
     it_graph* step_graph;                            // recorded single-token greedy step
     uint32_t* host_pin;                              // pinned staging, laid out like toks_dev, plus the position at [2*IT_MAXT]
@@ -110,6 +110,12 @@ static inline int it_cfg_conv_dim(const it_model_config& c) { return 2 * it_cfg_
 static inline bool it_cfg_recurrent(const it_model_config& c, int il) { return (il + 1) % c.full_attn_interval != 0; }
 
 #define IT_TRY(expr) do { int r__ = (expr); if (r__) return r__; } while (0)
+
+// After a pass of nt rows: a buffer that a prompt goes through IT_HIDDEN_ROWS rows at a time would hold, at row r, the pass's last row that is r
+// modulo IT_HIDDEN_ROWS, and past its end what earlier passes left (a pass of fewer rows never overwrites those in the arena either).
+static inline void it_engine_note_rows(it_engine* e, int nt) {
+    for (int r = 0; r < IT_HIDDEN_ROWS && r < nt; r++) e->hidden_at[r] = (uint16_t)(r + (nt - 1 - r) / IT_HIDDEN_ROWS * IT_HIDDEN_ROWS);
+}
 
 // Runs one pass over nt <= IT_MAXT tokens (run_chunk_v, src/vk/mod.rs:763-892).  logit_rows: 0 none, 1 last row, 2 every
 // row; nck: recurrent-state checkpoints to take (after rows 0..nck-1); from_dev: token ids are already in toks_dev and the

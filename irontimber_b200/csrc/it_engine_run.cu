@@ -140,7 +140,7 @@ int it_engine_run_chunk(it_engine* e, const uint32_t* toks, int nt, int logit_ro
     IT_TRY(it_sup_rmsnorm_wide(cx, A + L.x, e_, e->output_norm, e_, c.eps, A + L.hrow, e_, nt));
     if (logit_rows == 2) IT_TRY(logits_and_argmax(e, L.hrow, nt));
     else if (logit_rows == 1) IT_TRY(logits_and_argmax(e, L.hrow + (size_t)(nt - 1) * e_, 1));
-    if (!from_dev) { e->pos += nt; e->pass_rows = nt; }
+    if (!from_dev) { e->pos += nt; it_engine_note_rows(e, nt); }
     return IT_OK;
 }
 
@@ -234,7 +234,7 @@ int trunk_pass(it_engine* e, const uint32_t* toks, int nt, int logit_rows, int n
     IT_CUDA(cudaMemcpyAsync(e->pos_dev, slot + 8, sizeof(uint32_t), cudaMemcpyHostToDevice, cx->stream));
     IT_TRY(replay_pass(e, 1ull << 60 | (uint64_t)nt | (uint64_t)logit_rows << 8 | (uint64_t)nck << 16,
                        [&]() { return it_engine_run_chunk(e, nullptr, nt, logit_rows, nck, true); }));
-    e->pos += nt; e->pass_rows = nt;
+    e->pos += nt; it_engine_note_rows(e, nt);
     return IT_OK;
 }
 int head_pass(it_engine* e, const uint32_t* toks, int nt, int pos0, size_t hoff, bool predict) {
@@ -297,7 +297,6 @@ namespace {
 // one pass with the position read on the device, pick -> token slot and position + 1.
 int begin_device_decode(it_engine* e) {
     it_ctx* cx = e->ctx;
-    e->pass_rows = 1;
     uint32_t* pin = pin_block(e) + 2 * IT_MAXT;
     *pin = (uint32_t)e->pos;
     IT_CUDA(cudaMemcpyAsync(e->pos_dev, pin, 4, cudaMemcpyHostToDevice, cx->stream));
@@ -332,7 +331,7 @@ IT_API int it_engine_generate(it_engine* e, const uint32_t* prompt, size_t n_pro
     IT_TRY(begin_device_decode(e));
     while (*n_out < n_predict) {
         IT_TRY(it_graph_launch(e->ctx, e->step_graph));
-        e->pos += 1;
+        e->pos += 1; it_engine_note_rows(e, 1);
         IT_TRY(read_pick(e, 0, &t));
         out[(*n_out)++] = t;
         if (t == eos) break;
@@ -347,7 +346,7 @@ IT_API int it_engine_decode_steps(it_engine* e, size_t n, uint32_t* last_pick) {
     if (e->pos < 1) return it_fail(IT_ESTATE, "it_engine_decode_steps: nothing has been evaluated yet");
     if (e->pos + (long long)n > e->cfg.ctx_len) return it_fail(IT_ESTATE, "it_engine_decode_steps: context full");
     IT_TRY(begin_device_decode(e));
-    for (size_t i = 0; i < n; i++) { IT_TRY(it_graph_launch(e->ctx, e->step_graph)); e->pos += 1; }
+    for (size_t i = 0; i < n; i++) { IT_TRY(it_graph_launch(e->ctx, e->step_graph)); e->pos += 1; it_engine_note_rows(e, 1); }
     if (last_pick) return read_pick(e, 0, last_pick);
     return IT_OK;
 }

@@ -231,6 +231,7 @@ class CudaEngine:
         return out
 
     def hidden(self, row=0):
+        """Output-normed hidden row, row < 256; rows count as in passes of 256 tokens (it_engine_hidden_read)."""
         out = np.empty(self.cfg.n_embd, np.float32)
         _lib.check(self.L.it_engine_hidden_read(self.h, row, _p(out)))
         return out

@@ -277,6 +277,54 @@ def test_prompt_of_several_full_passes_bit_exact(orc):
         m.close(); eng.close()
 
 
+def test_hidden_rows_count_as_in_passes_of_256(orc):
+    """it_engine_hidden_read's row rule (include/irontimber_cuda.h) whatever passes the engine runs: every row that a buffer of 256 rows
+    would hold after a prompt in several passes, a single token, a ragged prompt, decode steps and a verification pass."""
+    from irontimber_b200 import _lib
+    from irontimber_b200.engine import CudaEngine, ModelConfig
+    eng = CudaEngine(tiny_config(ModelConfig, ctx_len=1536), seed=47, with_mtp=True)
+    m = oracle_model_from_engine(orc, eng, with_mtp=True)
+    try:
+        toks = [int(t) for t in np.random.default_rng(5).integers(0, eng.cfg.n_vocab, 1100 + 1 + 300 + 9)]
+        st, h = m.new_state(), []
+
+        def follow(ts):
+            for t in ts:
+                lg = m.forward_token(st, t, True, orc.DEVICE_ORDER)
+                h.append(bits(m.state_h(st)).copy())
+            return orc.argmax(lg)
+        held = {}
+
+        def passes(n):                              # n tokens given at once
+            for s in range(0, n, 256):
+                for r in range(min(256, n - s)):
+                    held[r] = len(h) - n + s + r
+
+        def check():
+            for r in (0, 1, 2, 8, 9, 43, 44, 75, 76, 200, 255):
+                assert np.array_equal(bits(eng.hidden(r)), h[held[r]]), f"row {r}: token {held[r]}"
+        done = 0
+        for n in (1100, 1, 300, 9):
+            part = toks[done:done + n]
+            pick = follow(part)
+            assert eng.eval_argmax(part) == pick
+            passes(n); done += n
+            check()
+        eng.step_kernels()                          # records the step, runs none
+        check()
+        for _ in range(2):
+            pick = follow([pick]); passes(1)
+        assert eng.decode_steps(2) == pick
+        check()
+        a = eng.mtp_verify(pick, 7)
+        follow([pick, 7]); passes(2)
+        check()
+        with pytest.raises(_lib.IronTimberError):
+            eng.hidden(256)
+    finally:
+        m.close(); eng.close()
+
+
 def test_step_kernel_matches_the_per_op_schedule_at_long_positions(monkeypatch):
     """Decode steps after a 330-token prompt: the attention block of the step kernel then walks more K tiles and V chunks
     than its ring holds and crosses a 32-position tile boundary.  Picks, logits and caches equal the per-op schedule's."""
