@@ -19,6 +19,7 @@
 // waits (again bounded) for its copies in flight and the CTA leaves.
 #include "it_internal.h"
 #include "it_pipe.cuh"
+#include "it_route.h"
 
 namespace {
 
@@ -206,22 +207,16 @@ int mm_launch(it_ctx* c, const it_mat* w, int ntok, const it_q8* x, float* y, si
 
 }  // namespace
 
-// Tile policy: 128-row tiles with sixteen consumer warps when that still gives the grid at least 0.6 CTAs per SM, else
-// 64-row tiles (eight warps, two CTAs per SM), else 32-row tiles.
+// Tile policy: it_mm_groups and it_mm_takes_tc (it_route.h).
 int it_matmul_t2_launch(it_ctx* c, const it_mat* w, int ntok, const it_q8* x, float* y, size_t y_stride, int accum) {
-    const long tok_tiles = (ntok + MM_TOK - 1) / MM_TOK;
-    const long want = (long)c->sm_count * 6 / 10;
-    const long rg = (long)w->row_groups;
-    const int wr = (rg + 3) / 4 * tok_tiles >= want ? 4 : (rg + 1) / 2 * tok_tiles >= want ? 2 : 1;
+    const int wr = it_mm_groups((long)w->row_groups, ntok, c->sm_count);
     if (mm_layout(wr, (int)(w->cols / 128), 2).total + 1024 > MM_SMEM_MAX)
         return it_fail(IT_EINVAL, "it_matvec_t2: rows of width %zu exceed the shared-memory budget of the tile kernel", w->cols);
-    // The tensor-memory kernel (it_matmul_tc.cu) works on 128-row tiles: it takes the shapes that give such tiles to
-    // most SMs; smaller matrices keep the finer tiles of the kernel in this file.  IT_MATMUL=legacy / tc forces one.
+    // The tensor-memory kernel (it_matmul_tc.cu) works on 128-row tiles; smaller matrices keep the finer tiles of the kernel in this
+    // file.  IT_MATMUL=legacy / tc forces one.
     const char* fv = getenv("IT_MATMUL");      // read on every call so that a test can exercise both kernels on one shape
     const int force = !fv ? 0 : !strcmp(fv, "legacy") ? 1 : !strcmp(fv, "tc") ? 2 : 0;
-    // 5120-row matrices at 33 to 64 activation rows too: their 160 row groups are one wave and twelve CTAs of 32-row tiles here
-    // (5120 x 17408 x 64: 67.6 us, 57.6 there; x 40: 58.9 and 57.3; x 12: 44.3 and 50.0; 2560 rows x 64, K 5120: 14.8 and 19.9)
-    if (force != 1 && (force == 2 || wr == 4 || (rg > c->sm_count && ntok > MM_TOK / 2))) {
+    if (force != 1 && (force == 2 || it_mm_takes_tc((long)w->row_groups, ntok, c->sm_count))) {
         const int r = it_matmul_tc_launch(c, w, ntok, x, y, y_stride, accum); if (r <= 0) return r;
     }
     if (wr == 4) return mm_launch<4, 4>(c, w, ntok, x, y, y_stride, accum);
