@@ -12,13 +12,11 @@
 // ascending position order, then * sigmoid(gate).  Results are bit-identical to k_attention's.
 #include "it_math.h"
 #include "it_support.h"
+#include "it_route.h"
 
 namespace {
 
-constexpr int AP_THREADS = 1024;
-constexpr int AP_CHUNK_POS = 64;                    // positions per V chunk (two cache tiles)
-constexpr int AP_RING = 2;                          // V chunks in flight
-constexpr int AP_SMEM = 220 * 1024;
+constexpr int AP_THREADS = IT_ATTN_THREADS, AP_CHUNK_POS = IT_ATTN_CHUNK_POS, AP_RING = IT_ATTN_RING;
 
 // HD: the head dimension as a compile-time constant (0: taken from the argument): with it every shared-memory address of the
 // score loop is an immediate offset, which removes a third of the kernel's instructions (it is bound by instruction issue).
@@ -166,10 +164,9 @@ __global__ void __launch_bounds__(AP_THREADS, 1) k_attention_group(const float* 
 template <int G, int RW, int HD>
 int launch_group_hd(it_ctx* c, const float* q, size_t q_hs, size_t q_ts, const float* gate, const __half* kc, const __half* vc, int hd, int nh, int nkv, int slot0, int nt, float* out, size_t o_ts) {
     const int npad = (slot0 + nt + 3) / 4 * 4;
-    const size_t smem = ((size_t)G * RW * npad + (size_t)G * RW * hd) * sizeof(float) + (size_t)AP_RING * AP_CHUNK_POS * hd * sizeof(__half);
-    if (smem > AP_SMEM) return 1;
+    const size_t smem = it_attn_group_smem(it_attn_group{ G, RW }, hd, slot0 + nt);
     static bool set[16] = {};       // the attribute is per device
-    if (!set[c->device & 15]) { IT_CUDA(cudaFuncSetAttribute(k_attention_group<G, RW, HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, AP_SMEM)); set[c->device & 15] = true; }
+    if (!set[c->device & 15]) { IT_CUDA(cudaFuncSetAttribute(k_attention_group<G, RW, HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)IT_ATTN_SMEM)); set[c->device & 15] = true; }
     it_pdl(k_attention_group<G, RW, HD>, dim3(nh / G, (nt + RW - 1) / RW), dim3(AP_THREADS), smem, c->stream, q, q_hs, q_ts, gate, kc, vc, hd, nh, nkv, slot0, nt, npad, out, o_ts);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return it_fail(IT_ECUDA, "launch attention_group: %s", cudaGetErrorString(e));
@@ -188,19 +185,12 @@ int launch_group(it_ctx* c, const float* q, size_t q_hs, size_t q_ts, const floa
 // the shared memory; the caller then uses it_sup_attention.
 int it_sup_attention_prefill(it_ctx* c, const float* q, size_t q_hs, size_t q_ts, const float* gate, const void* kc, const void* vc, int hd, int nh, int nkv, int slot0,
                              float* out, size_t o_ts, int nt) {
-    if (hd % 8 || nh % nkv) return 1;
-    const int rep = nh / nkv;
     const __half* k = (const __half*)kc; const __half* v = (const __half*)vc;
+    const it_attn_group g = it_attn_grouping(hd, nh, nkv, slot0 + nt);
+    if (g.rows == 0) return 1;
     it_note_op(c);
-    int r = 1;
-    if (rep % 3 == 0 && 3 * hd <= AP_THREADS) {
-        r = launch_group<3, 2>(c, q, q_hs, q_ts, gate, k, v, hd, nh, nkv, slot0, nt, out, o_ts);
-        if (r == 1) r = launch_group<3, 1>(c, q, q_hs, q_ts, gate, k, v, hd, nh, nkv, slot0, nt, out, o_ts);
-    } else if (rep % 2 == 0 && 2 * hd <= AP_THREADS) {
-        r = launch_group<2, 2>(c, q, q_hs, q_ts, gate, k, v, hd, nh, nkv, slot0, nt, out, o_ts);
-        if (r == 1) r = launch_group<2, 1>(c, q, q_hs, q_ts, gate, k, v, hd, nh, nkv, slot0, nt, out, o_ts);
-    } else if (hd <= AP_THREADS) {
-        r = launch_group<1, 2>(c, q, q_hs, q_ts, gate, k, v, hd, nh, nkv, slot0, nt, out, o_ts);
-    }
-    return r;
+#define IT_AP_LAUNCH(G, RW) if (g.heads == G && g.rows == RW) return launch_group<G, RW>(c, q, q_hs, q_ts, gate, k, v, hd, nh, nkv, slot0, nt, out, o_ts)
+    IT_AP_LAUNCH(3, 2); IT_AP_LAUNCH(3, 1); IT_AP_LAUNCH(2, 2); IT_AP_LAUNCH(2, 1); IT_AP_LAUNCH(1, 2);
+#undef IT_AP_LAUNCH
+    return 1;
 }

@@ -15,6 +15,7 @@
 // rows spans few positions of the causal diagonal.
 #include "it_math.h"
 #include "it_support.h"
+#include "it_route.h"
 
 namespace {
 
@@ -221,14 +222,12 @@ __global__ void __launch_bounds__(128, 3) k_attn_values(const float* __restrict_
 // Same results as it_sup_attention for the rows of one pass at known positions.  scratch: scores of a block of rows; rows are taken in blocks
 // that fit it.  Returns 1 (nothing launched) when the shape or the scratch does not suit: the caller then uses it_sup_attention_prefill.
 int it_sup_attention_tiled(it_ctx* c, const float* q, size_t q_hs, size_t q_ts, const float* gate, const void* kc, const void* vc, int hd, int nh, int nkv, int slot0,
-                           float* out, size_t o_ts, int nt, float* scratch, size_t scratch_floats) {
-    if (hd % 64 || nh % nkv || ((q_hs | q_ts | o_ts) & 3) || ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(gate) | reinterpret_cast<uintptr_t>(out)) & 15)) return 1;
+                           float* out, size_t o_ts, int nt, float* scratch, size_t scratch_floats, int choice) {
+    if (choice == 0 || hd % 64 || nh % nkv || ((q_hs | q_ts | o_ts) & 3) || ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(gate) | reinterpret_cast<uintptr_t>(out)) & 15)) return 1;
     const int rep = nh / nkv, npad = (slot0 + nt + AT_N - 1) / AT_N * AT_N;
     const size_t fit = scratch_floats / ((size_t)nh * npad);
     const int blk = (int)(fit < (size_t)nt ? fit : (size_t)nt);
-    // enough tiles for the GPU: a short prompt has too few rows x positions, and the kernel with a CTA per few rows is quicker
-    const long tiles = (long)((blk * rep + AT_M - 1) / AT_M) * ((slot0 + nt + AT_N - 1) / AT_N) * nkv;
-    if (blk < 1 || tiles < c->sm_count) return 1;
+    if (blk < 1 || (choice < 0 && !it_attn_takes_tiled(hd, nh, nkv, slot0, nt, blk, c->sm_count))) return 1;
     it_note_op(c);
     const int nblk = (nt + blk - 1) / blk, per = (nt + nblk - 1) / nblk;       // blocks of equal size
     for (int t0 = 0; t0 < nt; t0 += per) {

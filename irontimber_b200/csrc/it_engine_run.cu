@@ -69,6 +69,8 @@ int it_engine_run_chunk(it_engine* e, const uint32_t* toks, int nt, int logit_ro
         for (int t = 0; t < nt; t++) pin[t] = toks[t];
         IT_CUDA(cudaMemcpyAsync(e->toks_dev, pin, nt * sizeof(uint32_t), cudaMemcpyHostToDevice, cx->stream));
     }
+    const char* tv = getenv("IT_ATTN_TILED");      // read on every pass so that a test can run one prompt through both kernels
+    const int tiled = tv ? atoi(tv) != 0 : -1;
     IT_TRY(it_sup_embed(cx, e->toks_dev, e->tok_embd, e_, nt, A + L.x));
     // rmsnorm fused into the Hadamard + q8k kernel; the normed f32 row is kept only where a dense f32 op needs it
     auto norm_had = [&](const float* w, float* xn_out) {
@@ -119,11 +121,11 @@ int it_engine_run_chunk(it_engine* e, const uint32_t* toks, int nt, int logit_ro
                 IT_TRY(it_sup_rope(cx, k, hd, s_att, nkv, nt, pos0, pos_ptr, c.n_rot, e->theta_scale, c.rope_sections));
                 IT_TRY(it_sup_kv_store(cx, k, v, s_att, l.kc, l.vc, kvd, hd, pos0, pos_ptr, nt, 1));
             }
-            // prompt passes: one CTA per group of query heads and pair of rows that share their K / V reads; else one per (head, row)
+            // prompt passes: tiled products, or one CTA per group of query heads and rows that share their K / V reads (it_attn_takes_tiled); else one per (head, row)
             int ar = 1;
             static const bool grouped = []{ const char* v = getenv("IT_ATTN_GROUPED"); return !v || atoi(v) != 0; }();
             if (grouped && nt > 8 && !pos_ptr) {
-                ar = it_sup_attention_tiled(cx, q, 2 * hd, s_att, q + hd, l.kc, l.vc, hd, nh, nkv, pos0, A + L.o, (size_t)nh * hd, nt, e->att_scratch, e->att_scratch_floats);
+                ar = it_sup_attention_tiled(cx, q, 2 * hd, s_att, q + hd, l.kc, l.vc, hd, nh, nkv, pos0, A + L.o, (size_t)nh * hd, nt, e->att_scratch, e->att_scratch_floats, tiled);
                 if (ar == 1) ar = it_sup_attention_prefill(cx, q, 2 * hd, s_att, q + hd, l.kc, l.vc, hd, nh, nkv, pos0, A + L.o, (size_t)nh * hd, nt);
                 if (ar < 0) return ar;
             }

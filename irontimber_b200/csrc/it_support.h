@@ -53,9 +53,10 @@ int it_sup_attention_prefill(it_ctx* c, const float* q, size_t q_hs, size_t q_ts
                              float* out, size_t o_ts, int nt);
 
 // The same for long prompt passes (it_attention_tiled.cu): scores go through `scratch` a block of rows at a time.  Returns 1 when the shape
-// or the scratch does not suit or the pass is too small for it (nothing launched), a negative code on error.
+// or the scratch does not suit or the pass is too small for it (nothing launched), a negative code on error.  choice: 1 takes small passes too,
+// 0 takes none, -1 decides by size.
 int it_sup_attention_tiled(it_ctx* c, const float* q, size_t q_hs, size_t q_ts, const float* gate, const void* kc, const void* vc, int hd, int nh, int nkv, int slot0,
-                           float* out, size_t o_ts, int nt, float* scratch, size_t scratch_floats);
+                           float* out, size_t o_ts, int nt, float* scratch, size_t scratch_floats, int choice);
 
 // The delta rule alone over the rows of a prompt pass (it_gdn_prefill.cu); returns 1 when the shape does not suit it (nothing launched).
 int it_sup_gdn_rows(it_ctx* c, const float* co, size_t co_ts, const float* beta, const float* alpha, size_t ba_ts, const float* dt, const float* a, float* state, float* o, size_t o_ts,

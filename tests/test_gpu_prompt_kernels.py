@@ -1,8 +1,8 @@
 """Prompt passes against passes of eight rows at the 27B model's widths (4 layers, reduced vocabulary).
 
 Passes of up to eight rows run the kernels that the oracle tests pin (one attention CTA per head and row, delta rule and gated
-norm in one launch, the small-M product); longer ones run the prompt kernels: tiled attention once there are enough tiles,
-grouped attention before that, the delta rule spread over the GPU, the tile products.  The chunk size changes no result, so
+norm in one launch, the small-M product); longer ones run the prompt kernels: tiled or grouped attention, by size,
+the delta rule spread over the GPU, the tile products.  The chunk size changes no result, so
 logits, recurrent state and caches must agree bit for bit.
 """
 import numpy as np
@@ -27,8 +27,8 @@ def states(eng):
     return [bits(eng.state(il, k)).copy() for il in range(eng.cfg.n_layer) for k in ((0, 1) if eng.cfg.is_recurrent(il) else (2, 3))]
 
 
-# 9: shortest prompt pass; 17 / 49: one row into the next stage of tokens; 127, 300: grouped attention; 700: tiled attention with ragged
-# tiles of rows, positions and elements behind the diagonal; 2250: several passes, a block of rows at a time
+# 9: shortest prompt pass; 17 / 49: one row into the next stage of tokens; 127: grouped attention, as in the two uneven calls of 300; 300, 700:
+# tiled attention with ragged tiles of rows, positions and elements behind the diagonal; 2250: several passes, a block of rows at a time
 @pytest.mark.parametrize("n", [9, 17, 49, 127, 300, 700, 2250])
 def test_prompt_pass_equals_eight_row_passes(eng, n):
     prompt = np.random.default_rng(n).integers(0, N_VOCAB, n).astype(np.uint32)
@@ -48,3 +48,19 @@ def test_prompt_pass_equals_eight_row_passes(eng, n):
     if k < n:
         assert np.array_equal(bits(eng.eval(prompt[k:])), want)
         assert all(np.array_equal(a, b) for a, b in zip(states(eng), want_states))
+
+
+# rows at a position: on either side of a tile of rows (21 x 6 = 126, 22 x 6 = 132) and of positions, one row, and a few rows far into a context
+@pytest.mark.parametrize("at,n", [(0, 9), (0, 21), (0, 22), (0, 127), (0, 129), (0, 257), (100, 28), (1500, 24), (1500, 128)])
+def test_both_attention_kernels_take_the_same_pass(eng, monkeypatch, at, n):
+    """The rule by sizes gives a pass to one kernel; either one must give the same bits on any pass that it accepts."""
+    toks = np.random.default_rng(at + n).integers(0, N_VOCAB, at + n).astype(np.uint32)
+    got = {}
+    for tiled in ("0", "1"):
+        eng.reset()
+        if at:
+            monkeypatch.delenv("IT_ATTN_TILED", raising=False)
+            eng.eval(toks[:at], want_logits=False)
+        monkeypatch.setenv("IT_ATTN_TILED", tiled)
+        got[tiled] = [bits(eng.eval(toks[at:])).copy()] + states(eng)
+    assert all(np.array_equal(a, b) for a, b in zip(got["0"], got["1"]))

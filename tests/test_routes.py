@@ -14,7 +14,9 @@ def routes(tmp_path_factory):
     d = tmp_path_factory.mktemp("routes")
     src, lib = d / "routes.cpp", d / "routes.so"
     src.write_text('#include "it_route.h"\n'
-                   'extern "C" int takes_tc(long rg, long ntok, int sm) { return it_mm_takes_tc(rg, ntok, sm); }\n')
+                   'extern "C" int takes_tc(long rg, long ntok, int sm) { return it_mm_takes_tc(rg, ntok, sm); }\n'
+                   'extern "C" int attn_tiled(int slot0, int nt, int blk, int sm) { return it_attn_takes_tiled(256, 24, 4, slot0, nt, blk, sm); }\n'
+                   'extern "C" int attn_group(int hd, int nh, int nkv, int npos) { auto g = it_attn_grouping(hd, nh, nkv, npos); return 10 * g.heads + g.rows; }\n')
     subprocess.run(["g++", "-std=c++17", "-Wall", "-Werror", "-Wno-unused-function", "-shared", "-fPIC", "-I", CSRC, str(src), "-o", str(lib)], check=True)
     return C.CDLL(str(lib))
 
@@ -26,3 +28,23 @@ def routes(tmp_path_factory):
     (11137, 9, 1), (34816, 9, 1), (2689, 256, 1), (2688, 256, 0)])                                  # 128-row tiles for 0.6 of the SMs
 def test_tile_kernel_of_a_product(routes, rows, ntok, tc):
     assert routes.takes_tc(C.c_long((rows + 31) // 32), C.c_long(ntok), SM) == tc
+
+
+# passes at the 27B shape measured both ways (24 heads over 4 of dimension 256), where the sides differ by more than 2 %: a prompt from
+# position 0, a few new tokens far into a context, passes in several blocks of rows
+@pytest.mark.parametrize("slot0,nt,tiled", [
+    (0, 9, 0), (0, 128, 0), (0, 257, 0), (0, 384, 1), (0, 512, 1), (0, 777, 1),
+    (500, 32, 0), (500, 96, 0), (500, 192, 1), (1024, 9, 0), (1024, 96, 0), (1024, 128, 1), (2048, 32, 0), (2048, 96, 0), (2048, 128, 1),
+    (4096, 24, 0), (4096, 64, 0), (4096, 96, 0), (4096, 128, 1), (4096, 256, 1), (7000, 9, 0), (7000, 64, 0), (7000, 96, 1), (7000, 192, 1),
+    (11200, 192, 0), (12400, 256, 0), (13900, 9, 0), (14000, 32, 1), (14300, 64, 1), (19500, 256, 1)])
+def test_attention_of_a_prompt_pass(routes, slot0, nt, tiled):
+    npad = (slot0 + nt + 127) // 128 * 128
+    assert routes.attn_tiled(slot0, nt, min(nt, (32 << 20) // (24 * npad)), SM) == tiled
+
+
+@pytest.mark.parametrize("hd,nh,nkv,npos,heads,rows", [
+    (256, 24, 4, 6400, 3, 2), (256, 24, 4, 6402, 3, 1), (256, 24, 4, 13056, 3, 1), (256, 24, 4, 13057, 3, 0), (256, 4, 2, 100, 2, 2), (256, 4, 4, 100, 1, 2),
+    (256, 4, 4, 19713, 1, 0), (64, 32, 1, 100, 2, 2), (100, 24, 4, 100, 0, 0)])
+def test_grouping_of_attention_heads(routes, hd, nh, nkv, npos, heads, rows):
+    """One head a CTA keeps two rows or gives way."""
+    assert routes.attn_group(hd, nh, nkv, npos) == 10 * heads + rows
