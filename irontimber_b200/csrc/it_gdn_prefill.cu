@@ -13,6 +13,7 @@
 #include "it_math.h"
 #include "it_support.h"
 #include "it_pipe.cuh"
+#include "it_route.h"
 
 namespace {
 
@@ -187,7 +188,8 @@ __global__ void __launch_bounds__(160) k_gdn_rows(const float* co, size_t co_ts,
 // Delta rule of nt rows without the norm behind it.  Returns 1 (nothing launched) when the shape does not suit this kernel.
 int it_sup_gdn_rows(it_ctx* c, const float* co, size_t co_ts, const float* beta, const float* alpha, size_t ba_ts, const float* dt, const float* a, float* state, float* o, size_t o_ts,
                     int nv, int nk, int sd, int qk, int nt) {
-    if (sd != GP_SD || nt < 1 || (reinterpret_cast<uintptr_t>(co) & 15) || co_ts % 4 || qk % 4) return 1;
+    static_assert(GP_SD == 128, "it_gdn_rows_takes");
+    if (!it_gdn_rows_takes(sd, nt) || ((reinterpret_cast<uintptr_t>(co) | reinterpret_cast<uintptr_t>(state)) & 15) || co_ts % 4 || qk % 4) return 1;
     it_note_op(c);
     const size_t smem = GP_RING * sizeof(GpStage);
     static bool set[16] = {};       // the attribute is per device

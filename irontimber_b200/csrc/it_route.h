@@ -64,3 +64,8 @@ static inline bool it_attn_takes_tiled(int hd, int nh, int nkv, int slot0, int n
     const double tiled = 200.0 * blocks + (scores > 1e8 ? 0.95 : 0.7) * width * nt;
     return other * p > tiled * p + 40000;
 }
+
+// ---- delta rule of a prompt pass --------------------------------------------------------------------------------------------
+// k_gdn_rows (it_gdn_prefill.cu) is built for a state size of 128 and for three tokens or more: the warp that stores a state row first waits for
+// the other warp's read of it at the third token.
+static inline bool it_gdn_rows_takes(int sd, int nt) { return sd == 128 && nt >= 3; }

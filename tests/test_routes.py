@@ -16,7 +16,8 @@ def routes(tmp_path_factory):
     src.write_text('#include "it_route.h"\n'
                    'extern "C" int takes_tc(long rg, long ntok, int sm) { return it_mm_takes_tc(rg, ntok, sm); }\n'
                    'extern "C" int attn_tiled(int slot0, int nt, int blk, int sm) { return it_attn_takes_tiled(256, 24, 4, slot0, nt, blk, sm); }\n'
-                   'extern "C" int attn_group(int hd, int nh, int nkv, int npos) { auto g = it_attn_grouping(hd, nh, nkv, npos); return 10 * g.heads + g.rows; }\n')
+                   'extern "C" int attn_group(int hd, int nh, int nkv, int npos) { auto g = it_attn_grouping(hd, nh, nkv, npos); return 10 * g.heads + g.rows; }\n'
+                   'extern "C" int gdn_rows(int sd, int nt) { return it_gdn_rows_takes(sd, nt); }\n')
     subprocess.run(["g++", "-std=c++17", "-Wall", "-Werror", "-Wno-unused-function", "-shared", "-fPIC", "-I", CSRC, str(src), "-o", str(lib)], check=True)
     return C.CDLL(str(lib))
 
@@ -48,3 +49,9 @@ def test_attention_of_a_prompt_pass(routes, slot0, nt, tiled):
 def test_grouping_of_attention_heads(routes, hd, nh, nkv, npos, heads, rows):
     """One head a CTA keeps two rows or gives way."""
     assert routes.attn_group(hd, nh, nkv, npos) == 10 * heads + rows
+
+
+@pytest.mark.parametrize("sd,nt,takes", [(128, 1, 0), (128, 2, 0), (128, 3, 1), (128, 9, 1), (64, 9, 0), (256, 9, 0)])
+def test_prompt_delta_rule(routes, sd, nt, takes):
+    """One or two tokens are refused: one warp would store a state row that the other may not have read yet."""
+    assert routes.gdn_rows(sd, nt) == takes
