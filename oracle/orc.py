@@ -321,6 +321,12 @@ class Model:
     def new_mtp_state(self):
         return C.c_void_p(lib().orc_mtp_state_new())
 
+    def mtp_state_read(self, ms, which):
+        n = int(lib().orc_mtp_state_read(ms, C.c_int(which), None))
+        out = np.empty(n, np.float32)
+        lib().orc_mtp_state_read(ms, C.c_int(which), _p(out))
+        return out
+
     def mtp_step(self, ms, h, tok, pos, mode=REFERENCE_ORDER):
         """cpu_step (src/mtp.rs:100)."""
         h = _c(h, np.float32)

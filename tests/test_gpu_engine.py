@@ -106,9 +106,8 @@ def test_speculative_decode_equals_plain_greedy_with_oracle_counts(orc, pair):
 
 
 def test_long_prompt_in_several_passes_bit_exact(orc):
-    """A 300-token prompt runs as one pass of 256 rows and one of 44 (prefill_chunks, src/vk/mod.rs:130-134, with a larger
-    chunk): logits, the greedy continuation and the speculative loop with its head catch-up across passes equal the
-    token-by-token oracle."""
+    """A 300-token prompt, five of the reference's chunks (prefill_chunks, src/vk/mod.rs:130-134), in one pass and in two: logits, state, the
+    greedy continuation and the speculative loop with its head catch-up equal the token-by-token oracle."""
     from irontimber_b200.engine import CudaEngine, ModelConfig
     eng = CudaEngine(tiny_config(ModelConfig, ctx_len=352), seed=23, with_mtp=True)
     m = oracle_model_from_engine(orc, eng, with_mtp=True)
@@ -123,12 +122,64 @@ def test_long_prompt_in_several_passes_bit_exact(orc):
             kinds = (0, 1) if eng.cfg.is_recurrent(il) else (2, 3)
             for kind in kinds:
                 assert np.array_equal(bits(eng.state(il, kind)), bits(m.state_read(st, il, kind))), f"state {kind} of layer {il}"
+        eng.reset()
+        eng.eval(prompt[:256], want_logits=False)
+        assert np.array_equal(bits(eng.eval(prompt[256:])), bits(want))
         plain = orc.generate_greedy(m, prompt, 10, orc.DEVICE_ORDER)
         eng.reset()
         assert eng.generate(prompt, 10) == plain
         want_out, want_stats = orc.greedy_mtp(orc.CpuMtp(m, orc.DEVICE_ORDER), prompt, 10)
         out, stats = eng.generate_mtp(prompt, 10)
         assert out == plain == want_out and stats == want_stats
+    finally:
+        m.close(); eng.close()
+
+
+def test_speculative_prefill_of_two_passes_bit_exact(orc):
+    """A prompt of more rows than a pass takes: the head catches up pass by pass, the second time with the last hidden row of the pass
+    before.  Its KV cache, the draft it makes next and the loop that follows equal the oracle's."""
+    from irontimber_b200.engine import CudaEngine, ModelConfig
+    eng = CudaEngine(tiny_config(ModelConfig, ctx_len=1152), seed=29, with_mtp=True)
+    m = oracle_model_from_engine(orc, eng, with_mtp=True)
+
+    class Ready(orc.CpuMtp):                        # prefilled once, drafts kept
+        def mtp_prefill(self, prompt): return x
+        def mtp_draft(self, toks): drafts.append(super().mtp_draft(toks)); return drafts[-1]
+    try:
+        prompt = [int(t) for t in np.random.default_rng(1100).integers(0, eng.cfg.n_vocab, 1100)]
+        cpu, drafts = Ready(m, orc.DEVICE_ORDER), []
+        x = orc.CpuMtp.mtp_prefill(cpu, prompt)
+        assert eng.mtp_prefill(prompt) == x
+        for which in (4, 5):
+            assert np.array_equal(bits(eng.state(0, which)), bits(m.mtp_state_read(cpu.ms, which - 4)))
+        first = eng.mtp_draft([x])
+        want = orc.greedy_mtp(cpu, prompt, 8)
+        assert first == drafts[0]
+        assert eng.generate_mtp(prompt, 8) == want
+    finally:
+        m.close(); eng.close()
+
+
+@pytest.mark.parametrize("conv_k", [2, 3, 9])
+def test_conv_kernel_sizes_bit_exact(orc, conv_k):
+    """Other sizes of the causal conv than the 27B model's four: a prompt pass, a three-row pass and single tokens equal the oracle."""
+    from irontimber_b200.engine import CudaEngine, ModelConfig
+    cfg = tiny_config(ModelConfig)
+    cfg.conv_k = conv_k
+    eng = CudaEngine(cfg, seed=37)
+    m = oracle_model_from_engine(orc, eng, with_mtp=False)
+    try:
+        toks = [int(t) for t in np.random.default_rng(conv_k).integers(0, eng.cfg.n_vocab, 37)]
+        st, done = m.new_state(), 0
+        for n in (10, 3, 21, 1, 1, 1):              # 10: no more rows than a state of eight inputs and two; 21: two groups of rows
+            lg = eng.eval(toks[done:done + n])
+            for t in toks[done:done + n]:
+                want = m.forward_token(st, t, True, orc.DEVICE_ORDER)
+            done += n
+            assert np.array_equal(bits(lg), bits(want)), f"{done} tokens"
+            for il in range(cfg.n_layer):
+                if cfg.is_recurrent(il):
+                    assert np.array_equal(bits(eng.state(il, 0)), bits(m.state_read(st, il, 0))), f"conv state of layer {il}"
     finally:
         m.close(); eng.close()
 
@@ -253,9 +304,10 @@ def test_step_kernel_and_per_op_schedule_agree(orc, monkeypatch):
 
 
 def test_prompt_of_several_full_passes_bit_exact(orc):
-    """A 1100-token prompt is four 256-row passes and one of 76 rows, enqueued back to back while the device still works on
-    the first: every pass must see its own token ids (the host stages them in a ring of pinned blocks).  Logits, state and
-    the continuation (attention over more K / V tiles than the step kernel's ring holds) equal the token-by-token oracle."""
+    """A 1100-token prompt is a pass of 1024 rows and one of 76, the second enqueued while the device still works on the first; the same
+    tokens in twelve calls without logits are twelve passes in flight, more than the ring of pinned blocks that stages their token ids
+    has slots.  Logits, state and the continuation (attention over more K / V tiles than the step kernel's ring holds) equal
+    the token-by-token oracle."""
     from irontimber_b200.engine import CudaEngine, ModelConfig
     eng = CudaEngine(tiny_config(ModelConfig, ctx_len=1152), seed=43, with_mtp=False)
     m = oracle_model_from_engine(orc, eng, with_mtp=False)
@@ -271,6 +323,11 @@ def test_prompt_of_several_full_passes_bit_exact(orc):
             for il in range(eng.cfg.n_layer):
                 for kind in ((0, 1) if eng.cfg.is_recurrent(il) else (2, 3)):
                     assert np.array_equal(bits(eng.state(il, kind)), bits(m.state_read(st, il, kind))), f"state {kind} of layer {il}"
+        for _ in range(3):
+            eng.reset()
+            for s in range(0, 1056, 96):
+                eng.eval(prompt[s:s + 96], want_logits=False)
+            assert np.array_equal(bits(eng.eval(prompt[1056:])), bits(want))
         eng.reset()
         assert eng.generate(prompt, 12) == orc.generate_greedy(m, prompt, 12, orc.DEVICE_ORDER)
     finally:

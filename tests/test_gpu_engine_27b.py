@@ -27,8 +27,8 @@ def pair(orc):
 
 
 PROMPT = [int(t) for t in np.random.default_rng(27).integers(0, N_VOCAB, 70)]     # one ragged pass of 70 rows
-LONG_PROMPT = [int(t) for t in np.random.default_rng(28).integers(0, N_VOCAB, 262)]  # one pass of 256 rows + a ragged one of 6
-ROWS_PER_PASS = 256
+LONG_PROMPT = [int(t) for t in np.random.default_rng(28).integers(0, N_VOCAB, 262)]  # a pass of 262 rows, or one of 256 and a ragged one of 6
+ROWS_PER_PASS = 256                                                                # as hidden rows count (it_engine_hidden_read)
 
 
 def test_prompt_passes_logits_state_and_hidden_bit_exact(orc, pair):
@@ -53,19 +53,22 @@ def test_prompt_passes_logits_state_and_hidden_bit_exact(orc, pair):
 
 
 def test_two_prompt_passes_logits_and_state_bit_exact(orc, pair):
-    """262 tokens: a full pass of 256 rows (the tile kernels' 128-row CTAs, four launches of the delta-rule kernel) and a
-    ragged pass of 6 rows that continues from its state."""
+    """262 tokens at once (the tile kernels' 128-row CTAs, the last with six rows), then as a pass of 256 rows and a ragged pass of 6
+    that continues from its state."""
     eng, m = pair
-    eng.reset()
-    lg = eng.eval(LONG_PROMPT)
     st = m.new_state()
     for i, t in enumerate(LONG_PROMPT):
         want = m.forward_token(st, t, i + 1 == len(LONG_PROMPT), orc.DEVICE_ORDER)
-    assert np.array_equal(bits(lg), bits(want))
-    assert np.array_equal(bits(eng.hidden((len(LONG_PROMPT) - 1) % ROWS_PER_PASS)), bits(m.state_h(st)))
-    for il in range(eng.cfg.n_layer):
-        for kind in ((0, 1) if eng.cfg.is_recurrent(il) else (2, 3)):
-            assert np.array_equal(bits(eng.state(il, kind)), bits(m.state_read(st, il, kind))), f"state {kind} of layer {il}"
+    for cut in (0, 256):
+        eng.reset()
+        if cut:
+            eng.eval(LONG_PROMPT[:cut], want_logits=False)
+        lg = eng.eval(LONG_PROMPT[cut:])
+        assert np.array_equal(bits(lg), bits(want))
+        assert np.array_equal(bits(eng.hidden((len(LONG_PROMPT) - 1) % ROWS_PER_PASS)), bits(m.state_h(st)))
+        for il in range(eng.cfg.n_layer):
+            for kind in ((0, 1) if eng.cfg.is_recurrent(il) else (2, 3)):
+                assert np.array_equal(bits(eng.state(il, kind)), bits(m.state_read(st, il, kind))), f"state {kind} of layer {il}"
     m.free_state(st)
 
 

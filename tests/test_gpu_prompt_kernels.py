@@ -64,3 +64,30 @@ def test_both_attention_kernels_take_the_same_pass(eng, monkeypatch, at, n):
         monkeypatch.setenv("IT_ATTN_TILED", tiled)
         got[tiled] = [bits(eng.eval(toks[at:])).copy()] + states(eng)
     assert all(np.array_equal(a, b) for a, b in zip(got["0"], got["1"]))
+
+
+@pytest.mark.parametrize("n", [1025, 1034])      # a last pass of one row (recorded) and of ten
+def test_speculative_prefill_of_two_passes_equals_forced_steps(n):
+    """The head's catch-up across two prompt passes, against a prompt of one pass followed by verification passes of two rows that are fed
+    the rest of the prompt: the same caches of trunk and head, the same next draft."""
+    from irontimber_b200.engine import CudaEngine, config_27b
+    eng = CudaEngine(config_27b(n_layer=4, ctx_len=1056, n_vocab=N_VOCAB), seed=13, with_mtp=True)
+    try:
+        prompt = [int(t) for t in np.random.default_rng(n).integers(0, N_VOCAB, n)]
+        x = eng.mtp_prefill(prompt)
+        want = states(eng) + [bits(eng.state(0, k)).copy() for k in (4, 5)] + [eng.mtp_draft([x])]
+        at = n - 6
+        eng.mtp_prefill(prompt[:at])
+        pending = [prompt[at]]
+        for i in range(at, n, 2):
+            eng.mtp_draft(pending)
+            picks = eng.mtp_verify(prompt[i], prompt[i + 1])
+            pending = [prompt[i + 1], prompt[i + 2] if i + 2 < n else x]
+        assert picks[1] == x
+        got = states(eng)
+        draft = eng.mtp_draft(pending)              # adds the pairs (h, last token) and (h, x) to the head's cache
+        kvd = eng.cfg.n_head_kv * eng.cfg.head_dim
+        got += [bits(eng.state(0, k))[:(n - 1) * kvd] for k in (4, 5)] + [draft]
+        assert all(np.array_equal(a, b) for a, b in zip(got, want))
+    finally:
+        eng.close()
