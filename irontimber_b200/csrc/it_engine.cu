@@ -181,15 +181,17 @@ int it_engine_build(int device, const it_model_config* cfg, uint64_t seed, int w
     e->m_eh = e->m_q = e->m_k = e->m_v = e->m_o = e->m_gate = e->m_up = e->m_down = nullptr;
     e->pos = 0; e->mpos = 1; e->hp_off = 0; e->hp_n = 0; e->last_rows = 0;
     for (int r = 0; r < IT_HIDDEN_ROWS; r++) e->hidden_at[r] = (uint16_t)r;
-    // arena layout
+    // arena layout.  No pass has more rows than the context has positions, so a short context keeps short row buffers (0.47 MB a row at
+    // the 27B widths); it_engine_hidden_read's rows are always there.
+    const int rows = std::min(IT_MAXT, std::max(IT_HIDDEN_ROWS, c.ctx_len));
     it_arena_layout& L = e->lay; size_t o = 0;
     auto take = [&](size_t& field, size_t n) { field = o; o += up64(n); };
     L.big1_stride = (size_t)std::max(std::max(cd + inner, qf + 2 * kvd), 2 * ff); L.big2_stride = (size_t)std::max(inner, ff);
     L.o_stride = (size_t)std::max(inner, nh * hd); L.logits_stride = up64((size_t)c.n_vocab) + 64;
-    take(L.x, (size_t)IT_MAXT * e_); take(L.xn, (size_t)IT_MAXT * e_); take(L.big1, IT_MAXT * L.big1_stride); take(L.big2, IT_MAXT * L.big2_stride);
-    take(L.conv, (size_t)IT_MAXT * cd); take(L.kcur, (size_t)IT_MAXT * kvd); take(L.vcur, (size_t)IT_MAXT * kvd); take(L.o, IT_MAXT * L.o_stride);
-    take(L.beta, (size_t)IT_MAXT * nv); take(L.alpha, (size_t)IT_MAXT * nv); take(L.hrow, (size_t)IT_MAXT * e_); take(L.hprev, (size_t)e_);
-    take(L.mh, (size_t)(IT_MAXT + 1) * e_); take(L.me, (size_t)IT_MAXT * e_); take(L.mcat, (size_t)IT_MAXT * 2 * e_); take(L.mx, (size_t)IT_MAXT * e_);
+    take(L.x, (size_t)rows * e_); take(L.xn, (size_t)rows * e_); take(L.big1, rows * L.big1_stride); take(L.big2, rows * L.big2_stride);
+    take(L.conv, (size_t)rows * cd); take(L.kcur, (size_t)rows * kvd); take(L.vcur, (size_t)rows * kvd); take(L.o, rows * L.o_stride);
+    take(L.beta, (size_t)rows * nv); take(L.alpha, (size_t)rows * nv); take(L.hrow, (size_t)rows * e_); take(L.hprev, (size_t)e_);
+    take(L.mh, (size_t)(rows + 1) * e_); take(L.me, (size_t)rows * e_); take(L.mcat, (size_t)rows * 2 * e_); take(L.mx, (size_t)rows * e_);
     take(L.logits, IT_MAXLOGIT * L.logits_stride); take(L.amx, 64); L.total = o;
     int r = it_ctx_create(device, L.total, &e->ctx);
     if (r) { delete e; return r; }
@@ -242,7 +244,7 @@ int it_engine_build(int device, const it_model_config* cfg, uint64_t seed, int w
         e->m_tok_embd = e->tok_embd; E_TRY(src->mtp_embd(e, &e->m_tok_embd));
         E_TRY(dev_alloc(e, (void**)&e->mkc, (size_t)c.ctx_len * kvd * 4, true)); E_TRY(dev_alloc(e, (void**)&e->mvc, (size_t)c.ctx_len * kvd * 4, true));
     }
-    E_TRY(it_q8_create(e->ctx, (size_t)std::max(std::max(e_, ff), std::max(inner, nh * hd)), IT_MAXT, &e->q8));
+    E_TRY(it_q8_create(e->ctx, (size_t)std::max(std::max(e_, ff), std::max(inner, nh * hd)), rows, &e->q8));
     {
         std::vector<it_state_ptrs> sp;
         for (const it_layer& l : e->layers) if (l.recurrent) sp.push_back({ l.conv_st, l.ssm_st, l.ck_conv, l.ck_ssm });
@@ -252,7 +254,7 @@ int it_engine_build(int device, const it_model_config* cfg, uint64_t seed, int w
             if (cudaMemcpy(e->state_ptrs, sp.data(), sp.size() * sizeof(it_state_ptrs), cudaMemcpyHostToDevice) != cudaSuccess) return fail(it_fail(IT_ECUDA, "engine: state table upload failed"));
         }
     }
-    e->att_scratch_floats = std::min(IT_ATT_SCRATCH_FLOATS, (size_t)IT_MAXT * nh * (((size_t)c.ctx_len + 127) / 128 * 128));
+    e->att_scratch_floats = std::min(IT_ATT_SCRATCH_FLOATS, (size_t)rows * nh * (((size_t)c.ctx_len + 127) / 128 * 128));
     E_TRY(dev_alloc(e, (void**)&e->att_scratch, e->att_scratch_floats * sizeof(float), false));
     E_TRY(dev_alloc(e, (void**)&e->toks_dev, (2 * IT_MAXT + 8) * sizeof(uint32_t), true));
     E_TRY(dev_alloc(e, (void**)&e->pos_dev, 64, true));

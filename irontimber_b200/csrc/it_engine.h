@@ -30,7 +30,7 @@ struct it_layer {
     __half *kc, *vc;                                 // [ctx_len][n_head_kv * head_dim]
 };
 
-struct it_arena_layout {   // element offsets into the context's f32 arena; every row buffer holds IT_MAXT rows
+struct it_arena_layout {   // element offsets into the context's f32 arena; every row buffer holds min(IT_MAXT, max(256, ctx_len)) rows
     size_t x, xn, big1, big2, conv, kcur, vcur, o, beta, alpha, hrow, hprev, mh, me, mcat, mx, logits, amx, total;
     size_t big1_stride, big2_stride, o_stride, logits_stride;
 };

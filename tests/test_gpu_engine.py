@@ -382,6 +382,22 @@ def test_hidden_rows_count_as_in_passes_of_256(orc):
         m.close(); eng.close()
 
 
+def test_a_short_context_keeps_short_row_buffers():
+    """Device memory of an engine beside its weights follows the context: at most 1024 rows a pass, never more than there are positions."""
+    import torch
+    from irontimber_b200.engine import CudaEngine, ModelConfig
+    held = {}
+    for ctx in (256, 1024, 256, 1024):              # the first two also load what the process keeps
+        torch.cuda.synchronize()
+        before = torch.cuda.mem_get_info()[0]
+        eng = CudaEngine(tiny_config(ModelConfig, ctx_len=ctx), seed=3, with_mtp=True)
+        held[ctx] = before - torch.cuda.mem_get_info()[0]
+        eng.close()
+    # 768 rows of: six of n_embd, one of two n_embd, [gate | up], max(inner, n_ff), conv, k, v, o
+    rows = 768 * 4 * (6 * 1024 + 2 * 1024 + 2 * 2048 + 2048 + 1536 + 512 + 512 + 1024)
+    assert held[1024] - held[256] > rows, (held, rows)
+
+
 def test_step_kernel_matches_the_per_op_schedule_at_long_positions(monkeypatch):
     """Decode steps after a 330-token prompt: the attention block of the step kernel then walks more K tiles and V chunks
     than its ring holds and crosses a 32-position tile boundary.  Picks, logits and caches equal the per-op schedule's."""
