@@ -417,8 +417,8 @@ __global__ void __launch_bounds__(256) k_conv_l2_dense(const float* mixed, size_
     if (tid < sd) for (int t = 0; t < nt; t++) out[t * o_ts + ch] = it_mul(vals[t][tid], scs[t]);
 }
 
-// Gated delta rule (src/cpu.rs:215-232) and the gated per-head norm that follows it (:233-237) in one launch: one CTA
-// per head.  Warps 0..SD/32-1 own one state row per thread and walk the tokens; four extra warps take turns to norm the
+// Gated delta rule (src/cpu.rs:215-232) and the gated per-head norm that follows it (:233-237) of a pass of up to eight rows in one
+// launch: one CTA per head.  Warps 0..SD/32-1 own one state row per thread and walk the tokens; four extra warps take turns to norm the
 // outputs of a row (squares added by one lane in index order), weight them and multiply by silu(z) while the row owners
 // are already on the next rows (one output buffer per norm warp).  State layout [head][j][i] as on the CPU.
 // The head's SD x SD state sits in shared memory for the whole launch, rows unpadded, the 16-byte pieces of row j
@@ -759,9 +759,10 @@ int it_sup_gdn_norm(it_ctx* c, const float* co, size_t co_ts, const float* beta,
     if (sd != 128) return it_fail(IT_EINVAL, "gdn_norm: the fused kernel is built for a state size of 128");
     it_note_op(c);
     if (nt > IT_GDN_MAXROWS || (reinterpret_cast<uintptr_t>(co) & 15) || co_ts % 4 || qk % 4) return it_fail(IT_EINVAL, "gdn_norm: %d rows or an unaligned conv output", nt);
-    const size_t smem = ((size_t)sd * sd + GN_NW * sd + 2 * IT_GDN_MAXROWS + (size_t)nt * 3 * sd) * sizeof(float);
+    auto bytes = [&](int rows) { return ((size_t)sd * sd + GN_NW * sd + 2 * IT_GDN_MAXROWS + (size_t)rows * 3 * sd) * sizeof(float); };
+    const size_t smem = bytes(nt), most = bytes(IT_GDN_MAXROWS);
     static bool set[16] = {};       // the attribute is per device
-    if (!set[c->device & 15]) { IT_CUDA(cudaFuncSetAttribute(k_gdn_norm<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024)); set[c->device & 15] = true; }
+    if (!set[c->device & 15]) { IT_CUDA(cudaFuncSetAttribute(k_gdn_norm<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most)); set[c->device & 15] = true; }
     it_pdl(k_gdn_norm<128>, dim3(dim3(nv)), dim3(128 + 32 * GN_NW), smem, c->stream, co, co_ts, beta, alpha, ba_ts, dt, a, state, o, o_ts, nk, qk, nt, ck, ck_stride, nck, nw, eps, z, z_ts);
     KCHK("gdn_norm"); return IT_OK;
 }

@@ -19,7 +19,7 @@ __host__ __device__ static inline size_t it_vc_index(size_t pos, int kh, int j, 
     return ((((pos >> 5) * (size_t)nkv + kh) * ns + (size_t)(j / vs)) * 32 + (pos & 31)) * (size_t)vs + (size_t)(j % vs);
 }
 
-#define IT_GDN_MAXROWS 64    // rows of one pass the fused delta-rule kernel stages in shared memory (it_sup_gdn_norm)
+#define IT_GDN_MAXROWS 8     // rows the fused delta-rule kernel takes: decode and verification passes (it_sup_gdn_norm); longer ones run it_sup_gdn_rows
 
 // Work done on the way into the Hadamard + q8k kernel.  mode 0: nothing.  mode 1: input = silu(x) * b (b is a device
 // pointer, rows b_stride apart).  mode 2: input = rmsnorm(x) over the whole row of width n with weight w and eps; when
