@@ -15,7 +15,7 @@ host memory and reads every pick back to the host (4 bytes per token), timed on 
 as a sweep over 12 distinct weight matrices (285 MB), against the measured HBM copy bandwidth.
 `cpu_baseline` / `--impl reference`: the reference's CPU path (C++ port of src/cpu.rs forward_token, reference
 order, every host thread the process may use) on a truncated stack, extrapolated to the full depth; the sample is stated.
-`prefill_lengths` (config 4): prompts of 64 / 2048 / 4096 / 7168 tokens in 64-row passes.  `mtp` (config 3): 256 tokens
+`prefill_lengths` (config 4): prompts of 64 / 2048 / 4096 / 7168 tokens in passes of up to 1024 rows.  `mtp` (config 3): 256 tokens
 after prompts of 128 and 2048 tokens with draft lengths 1..3, random head and scripted right drafts.
 With N > 1 (one process per GPU, torchrun) `value` is ONE sequence on the row-sharded engine (strong scaling): every
 trunk matrix and the LM head split by output rows over the ranks, each rank's matvec kernels push their result slices
