@@ -13,7 +13,7 @@
 //            code - 1 in the same K-major 128-byte-swizzled layout (row r at 128 r, 16-byte piece p at (p ^ (r & 7)) * 16), so that
 //            the accumulator is S - sum128 at once, and the f16 block scales of the 128 rows into f32
 //   warp 17  one thread issues eight tcgen05.mma (M 128, K 32, s8 x s8 -> s32) per step into the step's two accumulators in tensor
-//            memory and commits them to two mbarriers (accumulators ready and tiles free again; boxes free again)
+//            memory and commits them to one mbarrier (accumulators ready; tiles and boxes free again)
 //   warp 19  fetches the next tile's activation scales
 //   warps 0-7 epilogue: reads the accumulators (a thread gets four rows x every fourth column), forms
 //            (d_w * d_x) * float(S - sum128) for each and adds it to an f32 accumulator it keeps in registers for the
@@ -40,6 +40,7 @@ constexpr int TC_KB = 4;                         // blocks per weight stage: one
                                                  // thread some 250 cycles, so four small copies per block made the producer the bottleneck)
 constexpr int TC_W_BYTES = 4 * TC_KB * IT_TILE_BYTES;   // four row groups x TC_KB consecutive tiles
 constexpr int TC_NA = 2;                         // steps of expanded tiles in flight
+constexpr int TC_NC = 4;                         // barriers the steps commit to in turn; at least the steps of boxes in flight, see the barrier list
 constexpr int TC_SMEM_MAX = 226 * 1024;
 constexpr unsigned TC_TMEM_COLS = 512;           // all of it: 2 * ND accumulators x TOK columns
 constexpr int TC_EPI_WARPS = 8, TC_EXP_WARPS = 8, TC_THREADS = (TC_EPI_WARPS + TC_EXP_WARPS + 4) * 32;
@@ -67,7 +68,7 @@ template <int NH> __host__ __device__ inline TcSmem tc_layout(int nb, int wstage
     L.w = o; o += wstages * TC_W_BYTES;
     L.dx = o; L.dx_bytes = (nb / 2) * Tc<NH>::TOK * 4; o += dxbufs * L.dx_bytes;
     L.dw = o; o += Tc<NH>::NDW * TC_ROWS * 4;
-    L.bars = o; o += (2 * wstages + 2 * xsteps + TC_NA + 2 * Tc<NH>::ND + 4) * 8;
+    L.bars = o; o += (2 * wstages + xsteps + TC_NA + TC_NC + Tc<NH>::ND + 4) * 8;
     o = (o + 15) & ~15;
     L.tmem = o; o += 16;
     L.flag = o; o += 16;
@@ -137,13 +138,13 @@ k_matmul_tc(const __grid_constant__ CUtensorMap xmap, const uint8_t* __restrict_
     volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + L.flag);
     unsigned* tmem_slot = reinterpret_cast<unsigned*>(smem + L.tmem);
     const unsigned bars = smem_u32(smem + L.bars);
-    // barrier addresses: weight stages (full / empty), activation boxes of a step (landed / free), tiles of a step expanded, accumulators of
-    // a step (full / empty), activation scales (full / empty).  "Accumulators d full" also tells the expanders that the tiles the step
-    // read may be reused: the next phase of that barrier needs their next tiles.  The boxes have barriers of their own, one per slot:
-    // with two accumulators and three slots the box of step n - 1 is in place while the producer waits for step n - 3, and
-    // both commit to one "accumulators full", whose parity could flip twice before the producer looks.
-    const unsigned wfull0 = bars, wempty0 = wfull0 + 8 * wstages, xfull0 = wempty0 + 8 * wstages, xempty0 = xfull0 + 8 * xsteps,
-                   afull0 = xempty0 + 8 * xsteps, dfull0 = afull0 + 8 * TC_NA, dempty0 = dfull0 + 8 * TC_ND, sfull0 = dempty0 + 8 * TC_ND, sempty0 = sfull0 + 16;
+    // barrier addresses: weight stages (full / empty), activation boxes of a step landed, tiles of a step expanded, steps committed, accumulators
+    // of a step empty, activation scales (full / empty).  "Committed" is the one commit of a step: accumulators full, and the
+    // tiles and boxes that the step read may be reused.  TC_NC barriers take turns whatever the number of accumulators: a wait sees
+    // one bit, and with a barrier per accumulator (two) and three steps of boxes the box of step n - 1 is in place while the producer
+    // waits for step n - 3 on the barrier that n - 1 commits to as well, so that the parity could flip twice before it looks.
+    const unsigned wfull0 = bars, wempty0 = wfull0 + 8 * wstages, xfull0 = wempty0 + 8 * wstages,
+                   afull0 = xfull0 + 8 * xsteps, dfull0 = afull0 + 8 * TC_NA, dempty0 = dfull0 + 8 * TC_NC, sfull0 = dempty0 + 8 * TC_ND, sempty0 = sfull0 + 16;
     // The CTA's tiles: blockIdx.x, + gridDim.x, ...; the activation tiles of one group of matrix rows are neighbours.  Every role walks
     // the same tiles with its ring positions running on, so the next tile's weights, boxes and products are under way while
     // the epilogue still stores the last one's results.
@@ -152,9 +153,10 @@ k_matmul_tc(const __grid_constant__ CUtensorMap xmap, const uint8_t* __restrict_
     if (tid == 0) {
         *abort_flag = 0;
         for (int s = 0; s < wstages; s++) { mbar_init(wfull0 + 8 * s, 1); mbar_init(wempty0 + 8 * s, 8); }
-        for (int s = 0; s < xsteps; s++) { mbar_init(xfull0 + 8 * s, 1); mbar_init(xempty0 + 8 * s, 1); }
+        for (int s = 0; s < xsteps; s++) mbar_init(xfull0 + 8 * s, 1);
         for (int a = 0; a < TC_NA; a++) mbar_init(afull0 + 8 * a, 4);
-        for (int d = 0; d < TC_ND; d++) { mbar_init(dfull0 + 8 * d, 1); mbar_init(dempty0 + 8 * d, TC_EPI_WARPS); }
+        for (int k = 0; k < TC_NC; k++) mbar_init(dfull0 + 8 * k, 1);
+        for (int d = 0; d < TC_ND; d++) mbar_init(dempty0 + 8 * d, TC_EPI_WARPS);
         for (int k = 0; k < 2; k++) { mbar_init(sfull0 + 8 * k, 1); mbar_init(sempty0 + 8 * k, TC_EPI_WARPS); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -200,17 +202,21 @@ k_matmul_tc(const __grid_constant__ CUtensorMap xmap, const uint8_t* __restrict_
         // ---------------- activation producer: the rows come from the kernel before this one
         if (lane == 0) {
             asm volatile("griddepcontrol.wait;" ::: "memory");
-            int s = 0, issued = 0; unsigned ph = 0; bool ok = true;
+            int s = 0, issued = 0, k0 = 0; unsigned kph = 0; bool ok = true;
             for (int tile = tile0; ok && tile < ntiles; tile += tstep) {
                 const int tok0 = tile % tok_tiles * TC_TOK;
                 for (int p = 0; p < np; p++) {
-                    if (!mbar_wait(xempty0 + 8 * s, ph ^ 1u, abort_flag, error_flag, 19)) { ok = false; break; }   // the step that last read the slot has committed
+                    // the slot was last read xsteps steps ago: wait for that step's commit
+                    if (issued >= xsteps) {
+                        if (!mbar_wait(dfull0 + 8 * k0, kph, abort_flag, error_flag, 19)) { ok = false; break; }
+                        if (++k0 == TC_NC) { k0 = 0; kph ^= 1u; }
+                    }
                     mbar_expect_tx(xfull0 + 8 * s, (unsigned)(2 * TC_X_BYTES));
 #pragma unroll
                     for (int k = 0; k < 2 * NH; k++)     // 64 rows per box; the boxes of a block lie one under the other like one box of TOK rows
                         tma_load_2d(smem_u32(smem + L.x + s * 2 * TC_X_BYTES + k * 64 * 128), &xmap, (2 * p + k / NH) * 128, tok0 + 64 * (k % NH), xfull0 + 8 * s);
                     issued++;
-                    if (++s == xsteps) { s = 0; ph ^= 1u; }
+                    if (++s == xsteps) s = 0;
                 }
             }
             if (*abort_flag) {
@@ -224,7 +230,7 @@ k_matmul_tc(const __grid_constant__ CUtensorMap xmap, const uint8_t* __restrict_
     } else if (warp == TC_EPI_WARPS + TC_EXP_WARPS + 1) {
         // ---------------- MMA issuer
         if (lane == 0) {
-            int s = 0, a = 0, d = 0; unsigned xph = 0, aph = 0, dph = 0, last = 0, last_ph = 0; bool ok = true;
+            int s = 0, a = 0, d = 0, k = 0; unsigned xph = 0, aph = 0, dph = 0, kph = 0, last = 0, last_ph = 0; bool ok = true;
             const unsigned long long adesc0 = tc_smem_desc(smem_u32(smem + L.a)), bdesc0 = tc_smem_desc(smem_u32(smem + L.x));
             for (int tile = tile0; ok && tile < ntiles; tile += tstep)
             for (int p = 0; p < np; p++) {
@@ -242,9 +248,9 @@ k_matmul_tc(const __grid_constant__ CUtensorMap xmap, const uint8_t* __restrict_
                     tc_mma<true>(dt, ad + 4, bd + 4, Tc<NH>::IDESC);
                     tc_mma<true>(dt, ad + 6, bd + 6, Tc<NH>::IDESC);
                 }
-                tc_commit(dfull0 + 8 * d);        // accumulators complete; the tiles of this step may be reused
-                tc_commit(xempty0 + 8 * s);       // its boxes too
-                last = xempty0 + 8 * s; last_ph = xph;
+                tc_commit(dfull0 + 8 * k);        // accumulators complete; tiles and boxes of this step may be reused
+                last = dfull0 + 8 * k; last_ph = kph;
+                if (++k == TC_NC) { k = 0; kph ^= 1u; }
                 if (++s == xsteps) { s = 0; xph ^= 1u; }
                 if (++a == TC_NA) { a = 0; aph ^= 1u; }
                 if (++d == TC_ND) { d = 0; dph ^= 1u; }
@@ -273,7 +279,7 @@ k_matmul_tc(const __grid_constant__ CUtensorMap xmap, const uint8_t* __restrict_
         }
     } else if (warp >= TC_EPI_WARPS) {
         // ---------------- expanders: warp 8 + 4 e + i expands row group i of the steps with number % 2 == e into tile pair e
-        static_assert(TC_NA == 2 && TC_EXP_WARPS == 8, "set e fills tile pair e");
+        static_assert(TC_NA == 2 && TC_EXP_WARPS == 8 && TC_NC % 2 == 0, "set e fills tile pair e and waits for every other commit");
         const int eset = (warp - TC_EPI_WARPS) >> 2, rgl = (warp - TC_EPI_WARPS) & 3, g = lane >> 2, t = lane & 3;
         unsigned char* const at = smem + L.a + 2 * eset * TC_A_BYTES + (rgl * 32 + g) * 128;
         unsigned char* const plo = at + (((2 * t) ^ g) << 4);          // columns 32 t .. 32 t + 15 of row g; the other rows 1024 bytes apart
@@ -290,7 +296,7 @@ k_matmul_tc(const __grid_constant__ CUtensorMap xmap, const uint8_t* __restrict_
                 if (gp >= 2) {
                     if (!mbar_wait_warp(dfull0 + 8 * dp, dpp, abort_flag, error_flag, 16)) { ok = false; break; }
                     dp += 2;
-                    if (dp >= TC_ND) { dp -= TC_ND; dpp ^= 1u; }
+                    if (dp >= TC_NC) { dp -= TC_NC; dpp ^= 1u; }
                 }
 #pragma unroll
                 for (int h = 0; h < 2; h++) {
@@ -343,7 +349,7 @@ k_matmul_tc(const __grid_constant__ CUtensorMap xmap, const uint8_t* __restrict_
             asm volatile("bar.sync 1, %0;" :: "n"(NEPI) : "memory");
         }
         const f32x2 mz = pkf(minus_zero, minus_zero);
-        int d = 0, r = 0, j = 0; unsigned dph = 0;
+        int d = 0, r = 0, j = 0, kc = 0; unsigned kph = 0;
         bool ok = true;
         for (int tile = tile0; tile < ntiles; tile += tstep, j++) {
             const int k = j & 1;
@@ -357,7 +363,7 @@ k_matmul_tc(const __grid_constant__ CUtensorMap xmap, const uint8_t* __restrict_
 #pragma unroll
                 for (int c = 0; c < 8 * CC; c++) acc[hf][c] = 0ull;
             for (int p = 0; p < np; p++) {             // two blocks at a time: they share the activation scale, the wait and the release
-                if (!mbar_wait_warp(dfull0 + 8 * d, dph, abort_flag, error_flag, 17)) { ok = false; break; }
+                if (!mbar_wait_warp(dfull0 + 8 * kc, kph, abort_flag, error_flag, 17)) { ok = false; break; }
                 if (active) {
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     // chunks of 32 columns of one block; the next one is on its way while one is folded
@@ -392,7 +398,8 @@ k_matmul_tc(const __grid_constant__ CUtensorMap xmap, const uint8_t* __restrict_
                     }
                 } else if (lane == 0) mbar_arrive(dempty0 + 8 * d);
                 dxs += TC_TOK / 4;
-                if (++d == TC_ND) { d = 0; dph ^= 1u; }
+                if (++kc == TC_NC) { kc = 0; kph ^= 1u; }
+                if (++d == TC_ND) d = 0;
                 r = r + 2 == NDW ? 0 : r + 2;
             }
             if (!ok || __any_sync(0xffffffffu, *abort_flag)) break;
@@ -448,7 +455,7 @@ static int tc_launch(it_ctx* c, const it_mat* w, int ntok, const it_q8* x, float
     if (!fits(2, 2)) { grid = ntiles; dxbufs = 1; }
     if (!fits(2, 2)) return 1;
     // Activation boxes three steps deep where they fit (two left the MMA waiting 375 cycles a step), then weight stages of TC_KB blocks
-    const int xsteps = fits(2, 3) ? 3 : 2;
+    const int xsteps = fits(2, 3) ? 3 : 2;       // no more than TC_NC
     int stages = 5;
     while (!fits(stages, xsteps)) stages--;
     const TcSmem L = tc_layout<NH>(nb, stages, dxbufs, xsteps);

@@ -2,7 +2,7 @@
 
 A wait on an mbarrier sees one bit, the parity of the phase: a role that has not yet seen phase q complete must be sure that phase
 q + 1 of the same barrier cannot complete first, or it waits for good.  The model below has the kernel's roles as step counters and
-walks every order in which they can proceed; which barrier the activation producer waits for is read from the source.
+walks every order in which they can proceed; how many barriers the steps commit to in turn is read from the source.
 """
 import os
 import re
@@ -18,16 +18,17 @@ def source(name):
         return f.read()
 
 
-def producer_ring():
-    """The ring of barriers on which the activation producer waits before it fills a slot again."""
-    role = source("it_matmul_tc.cu").split("---------------- activation producer", 1)[1].split("} else if (warp", 1)[0]
-    return re.search(r"mbar_wait\((\w+)0 \+ 8 \*", role).group(1)
+def commit_barriers(acc):
+    """Barriers the steps commit to in turn: every wait for a step's commit goes through the same ring."""
+    src = source("it_matmul_tc.cu")
+    rings = set(re.findall(r"if \(\+\+(?:k0|k|kc) == (\w+)\)", src)) | set(re.findall(r"if \(dp >= (\w+)\)", src)) | set(re.findall(r"k < (\w+); k\+\+\) mbar_init\(dfull0", src))
+    assert len(rings) == 1, rings                  # the one ring of issuer, producer, expanders, epilogue and set-up
+    return acc if rings == {"TC_ND"} else int(re.search(rings.pop() + r" = (\d+)", src).group(1))
 
 
-def overtaken(acc, boxes, ring):
-    """(role, step) of a wait whose barrier can be two phases on; None when there is no such order.  acc: accumulator barriers, boxes:
-    slots of the activation ring, ring: "dfull" or "xempty" (one barrier per accumulator or per slot)."""
-    lag = acc if ring == "dfull" else boxes         # commits between two phases of one barrier the producer waits for
+def overtaken(acc, boxes, commits):
+    """(role, step) of a wait whose barrier can be two phases on; None when there is no such order.  acc: steps of accumulators, boxes:
+    slots of the activation ring, commits: barriers the steps commit to in turn."""
     seen, todo = set(), [(0, 0, 0, 0, 0, 0)]
     while todo:
         st = todo.pop()
@@ -35,8 +36,8 @@ def overtaken(acc, boxes, ring):
             continue
         seen.add(st)
         x, e0, e1, m, c, p = st                     # boxes issued, steps expanded by either set, MMAs issued, committed, steps folded
-        for role, q, per in (("producer", x - boxes, lag), ("expanders 0", 2 * e0 - 2, acc), ("expanders 1", 2 * e1 - 1, acc), ("epilogue", p, acc)):
-            if q >= 0 and c > q + per:
+        for role, q in (("producer", x - boxes), ("expanders 0", 2 * e0 - 2), ("expanders 1", 2 * e1 - 1), ("epilogue", p)):
+            if q >= 0 and c > q + commits:
                 return role, q
         if x < STEPS and (x < boxes or c > x - boxes):
             todo.append((x + 1, e0, e1, m, c, p))
@@ -56,13 +57,13 @@ def overtaken(acc, boxes, ring):
 
 @pytest.mark.parametrize("acc,boxes", [(4, 2), (4, 3), (2, 2), (2, 3)])      # 64- and 128-row tiles, with two and three steps of boxes
 def test_no_wait_can_be_overtaken(acc, boxes):
-    assert overtaken(acc, boxes, producer_ring()) is None
+    assert overtaken(acc, boxes, commit_barriers(acc)) is None
 
 
 def test_the_model_sees_an_overtaken_wait():
-    """Three slots freed by the commits of two accumulators: box n - 1 is in place while the producer waits for step n - 3, and both commit
-    to one barrier."""
-    assert overtaken(2, 3, "dfull") == ("producer", 0)
+    """A barrier per accumulator, two of them, and three slots of boxes: box n - 1 is in place while the producer waits for step n - 3, and
+    both commit to one barrier."""
+    assert overtaken(2, 3, 2) == ("producer", 0)
 
 
 def warp_statements(src, pattern):
