@@ -28,7 +28,8 @@
 // Integer block sums are exact whatever the hardware's summation order, so only the f32 epilogue decides the bits.
 //
 // Every wait is bounded; when one runs out the CTA raises the context's error flag (IT_ETIMEOUT), every role leaves
-// its loop, the producer waits (bounded) for its copies in flight, and the tensor memory is released before the CTA exits.
+// its loop (expanders and epilogue by going on without waits or arrivals, the epilogue to the end of its tile and without storing
+// it: a lane that left alone would leave the rest of its warp in a warp-wide instruction), the producer waits (bounded) for its copies in flight, and the tensor memory is released before the CTA exits.
 #include "it_internal.h"
 #include "it_pipe.cuh"
 
@@ -287,14 +288,14 @@ k_matmul_tc(const __grid_constant__ CUtensorMap xmap, const uint8_t* __restrict_
         float* const dws = reinterpret_cast<float*>(smem + L.dw) + rgl * 32 + 4 * g;
         const unsigned char* const src0 = smem + L.w + rgl * TC_KB * IT_TILE_BYTES;
         int s = 0, dp = eset, r = 0, gp = 0; unsigned sph = 0, dpp = 0; bool ok = true;
-        for (int tile = tile0; ok && tile < ntiles; tile += tstep)
+        for (int tile = tile0; tile < ntiles; tile += tstep)
         for (int p = 0; p < np; p++, gp++) {
             const bool last = (p & 1) || p + 1 == np;         // last step of the weight stage
             if ((gp & 1) == eset) {
-                if (!mbar_wait_warp(wfull0 + 8 * s, sph, abort_flag, error_flag, 15)) { ok = false; break; }
+                ok = ok && mbar_wait(wfull0 + 8 * s, sph, abort_flag, error_flag, 15);
                 // the tile pair was last read two steps ago: wait for that step's commit
                 if (gp >= 2) {
-                    if (!mbar_wait_warp(dfull0 + 8 * dp, dpp, abort_flag, error_flag, 16)) { ok = false; break; }
+                    ok = ok && mbar_wait(dfull0 + 8 * dp, dpp, abort_flag, error_flag, 16);
                     dp += 2;
                     if (dp >= TC_NC) { dp -= TC_NC; dpp ^= 1u; }
                 }
@@ -318,7 +319,7 @@ k_matmul_tc(const __grid_constant__ CUtensorMap xmap, const uint8_t* __restrict_
                 }
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");     // generic-proxy stores before the MMA's async-proxy reads
                 __syncwarp();
-                if (lane == 0) {
+                if (lane == 0 && ok) {
                     mbar_arrive(afull0 + 8 * eset);
                     mbar_arrive_n(wempty0 + 8 * s, last && !(p & 1) ? 2u : 1u);  // read its tiles; a stage of one step counts them twice
                 }
@@ -355,7 +356,7 @@ k_matmul_tc(const __grid_constant__ CUtensorMap xmap, const uint8_t* __restrict_
             const int k = j & 1;
             const int rg0 = tile / tok_tiles * 4, tok0 = tile % tok_tiles * TC_TOK, ntv = min(TC_TOK, ntok - tok0);
             const bool active = m0 < ntv;              // groups past the last activation row only release the accumulators
-            if (j > 0 && !mbar_wait_warp(sfull0 + 8 * k, (unsigned)((j - 1) >> 1) & 1u, abort_flag, error_flag, 18)) break;
+            if (j > 0) ok = ok && mbar_wait(sfull0 + 8 * k, (unsigned)((j - 1) >> 1) & 1u, abort_flag, error_flag, 18);
             const float4* dxs = reinterpret_cast<const float4*>(smem + L.dx + k * L.dx_bytes) + m0 / 4 + t;
             f32x2 acc[2][8 * CC];                      // rows g + 16 hf and g + 8 + 16 hf of column 4 c + t
 #pragma unroll
@@ -363,7 +364,8 @@ k_matmul_tc(const __grid_constant__ CUtensorMap xmap, const uint8_t* __restrict_
 #pragma unroll
                 for (int c = 0; c < 8 * CC; c++) acc[hf][c] = 0ull;
             for (int p = 0; p < np; p++) {             // two blocks at a time: they share the activation scale, the wait and the release
-                if (!mbar_wait_warp(dfull0 + 8 * kc, kph, abort_flag, error_flag, 17)) { ok = false; break; }
+                ok = ok && mbar_wait(dfull0 + 8 * kc, kph, abort_flag, error_flag, 17);
+                __syncwarp();
                 if (active) {
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     // chunks of 32 columns of one block; the next one is on its way while one is folded
@@ -387,7 +389,7 @@ k_matmul_tc(const __grid_constant__ CUtensorMap xmap, const uint8_t* __restrict_
                         else {
                             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                             __syncwarp();
-                            if (lane == 0) mbar_arrive(dempty0 + 8 * d);      // the MMAs of step p + ND may use the accumulators
+                            if (lane == 0 && ok) mbar_arrive(dempty0 + 8 * d);      // the MMAs of step p + ND may use the accumulators
                         }
 #pragma unroll
                         for (int c = 0; c < 8; c++) {
@@ -396,13 +398,13 @@ k_matmul_tc(const __grid_constant__ CUtensorMap xmap, const uint8_t* __restrict_
                             acc[1][cc] = add2(acc[1][cc], mul2_rounded(mul2(dwb[ch & 1].y, dx[c]), pkf((float)v[16 + 2 * c], (float)v[16 + 2 * c + 1]), mz));
                         }
                     }
-                } else if (lane == 0) mbar_arrive(dempty0 + 8 * d);
+                } else if (lane == 0 && ok) mbar_arrive(dempty0 + 8 * d);
                 dxs += TC_TOK / 4;
                 if (++kc == TC_NC) { kc = 0; kph ^= 1u; }
                 if (++d == TC_ND) d = 0;
                 r = r + 2 == NDW ? 0 : r + 2;
             }
-            if (!ok || __any_sync(0xffffffffu, *abort_flag)) break;
+            if (!__all_sync(0xffffffffu, ok && !*abort_flag)) break;
             __syncwarp();
             if (lane == 0) mbar_arrive(sempty0 + 8 * k);          // the tile's activation scales have been read
             if (!active) continue;
