@@ -264,8 +264,14 @@ int it_check_device_error(it_ctx* c, const char* who) {
     if (c->error_flag_host && *(volatile int*)c->error_flag_host) {
         const int code = *(volatile int*)c->error_flag_host;
         *(volatile int*)c->error_flag_host = 0;
-        // a persistent kernel that gave up leaves its barrier words inconsistent and the abort word set
-        if (c->grid_sync && !c->capturing) { cudaMemsetAsync(c->grid_sync, 0, 256, c->stream); cudaStreamSynchronize(c->stream); }
+        // a persistent kernel that gave up leaves its barrier words inconsistent and the abort word set.  The tags of
+        // values handed between CTAs go on from where no tag of the abandoned launch reaches.
+        if (c->grid_sync && !c->capturing) {
+            unsigned w[4] = { 0, 0, 0, 0 };
+            cudaMemcpyAsync(w, c->grid_sync, sizeof w, cudaMemcpyDeviceToHost, c->stream); cudaStreamSynchronize(c->stream);
+            w[1] = w[0]; w[2] = 0; w[3] += 1u << 20;
+            cudaMemcpyAsync(c->grid_sync, w, sizeof w, cudaMemcpyHostToDevice, c->stream); cudaStreamSynchronize(c->stream);
+        }
         return it_fail(IT_ETIMEOUT, "%s: a kernel gave up on a bounded wait (site %d); its results are not valid", who, code);
     }
     return IT_OK;
@@ -345,8 +351,11 @@ IT_API int it_signs_set(it_ctx* c, size_t n, const float* signs) {
     for (size_t i = 0; i < n; i++) IT_CHECK_ARG(signs[i] == 1.0f || signs[i] == -1.0f, "it_signs_set: sign %zu is %g, not +-1", i, (double)signs[i]);
     IT_CUDA(cudaSetDevice(c->device));
     float*& d = c->signs[n];
-    if (!d) IT_CUDA(cudaMalloc(&d, n * 4));
+    if (!d) IT_CUDA(cudaMalloc(&d, n * 4 + n / 8));
+    std::vector<uint32_t> bits(n / 32);
+    for (size_t i = 0; i < n; i++) if (signs[i] < 0.f) bits[i / 32] |= 1u << (i % 32);
     IT_CUDA(cudaMemcpyAsync(d, signs, n * 4, cudaMemcpyHostToDevice, c->stream));
+    IT_CUDA(cudaMemcpyAsync(d + n, bits.data(), n / 8, cudaMemcpyHostToDevice, c->stream));
     IT_CUDA(cudaStreamSynchronize(c->stream)); return IT_OK;
 }
 

@@ -103,7 +103,7 @@ struct it_ctx {
     cudaStream_t stream;
     float* arena;
     size_t arena_floats;
-    std::map<size_t, float*> signs;   // width -> device sign vector
+    std::map<size_t, float*> signs;   // width n -> device sign vector [n], then the same as n / 32 words of bits (1: -1), for kernels that keep it in shared memory
     // argmax scratch: per-block partial (value, index) pairs + a completion counter
     unsigned long long* argmax_partials;
     unsigned int* argmax_counter;
@@ -113,8 +113,8 @@ struct it_ctx {
     // costs nothing on the normal path
     int* error_flag_host;
     int* error_flag_dev;
-    // words of the grid-wide barrier of persistent kernels: [0] arrivals so far, [1] arrivals at the end of the last
-    // launch, [2] abort word (set by a CTA whose wait ran out; cleared by the host together with the error flag)
+    // words of a persistent kernel that hands values from CTA to CTA: [0] its counter, [1] the counter at the end of the last
+    // launch, [2] abort word (set by a CTA whose wait ran out; cleared by the host together with the error flag), [3] tag of the next launch
     unsigned* grid_sync;
     // Programmatic-dependent-launch bookkeeping: the q8 buffer whose contents are known to be complete by the
     // time the most recently enqueued kernel lets its dependents start (null after any op that is not a matvec).

@@ -77,7 +77,7 @@ IT_HD uint32_t it_float_to_bits(float f) {
 }
 
 // exp(x).  n = round(x / ln 2), r = x - n ln 2 in two pieces, degree-6 polynomial, exact scaling by 2^n.
-IT_HD_BIG float it_expf(float x) {
+IT_HD float it_expf_inline(float x) {
     if (!(x == x)) return x;
     if (x > 88.72283935546875f) return it_bits_to_float(0x7f800000u);
     if (x < -103.97208404541015625f) return 0.0f;
@@ -96,6 +96,7 @@ IT_HD_BIG float it_expf(float x) {
     const float s1 = it_bits_to_float((uint32_t)(n1 + 127) << 23), s2 = it_bits_to_float((uint32_t)(n2 + 127) << 23);
     return it_mul(it_mul(p, s1), s2);
 }
+IT_HD_BIG float it_expf(float x) { return it_expf_inline(x); }
 
 // log(x) for finite x > 0 (normal numbers): x = m 2^e with m in [sqrt(1/2), sqrt(2)), polynomial in m - 1.
 IT_HD_BIG float it_logf(float x) {

@@ -3,57 +3,74 @@
 // The per-op schedule of a pass (it_engine_run.cu; the reference's run_chunk_v, src/vk/mod.rs:763-892) is a chain of about
 // ten dependent kernels per layer.  At one activation row every kernel is a few microseconds long, so most of a step is
 // spent draining and refilling the GPU at kernel boundaries, not streaming weights.  This kernel runs the whole step with
-// one CTA per SM that stays resident: the ops of the schedule become phases separated by a barrier over the grid, and a
-// producer warp per CTA streams the CTA's share of every ternary matrix of the step, in schedule order, into a ring in
-// shared memory.  Weights never depend on activations, so the producer is only ever held back by the ring being full:
-// while the CTAs sit in a short phase (Hadamard, delta rule, attention) or in a barrier, the ring already holds the first
-// 150 KB per SM of the next matrix, and the HBM stream does not drain at op boundaries.
+// one CTA per SM that stays resident: the ops of the schedule become phases, and a producer warp per CTA streams the CTA's share of
+// every ternary matrix of the step, in schedule order, into a ring in shared memory.  Weights never depend on activations, so the
+// producer is only ever held back by the ring being full: while the CTAs wait for a phase's input, the ring already holds the
+// first 136 KB per SM of the next matrix, and the HBM stream does not drain at op boundaries.
 //
 // Arithmetic: every phase performs, per output element, the operations of the kernel it replaces in the same order (the
 // kernels of it_support.cu, it_hadamard.cuh, it_matvec_t2.cu), so logits, state and picks are bit-identical to the per-op
 // schedule; tests run both and compare.  What changes is only which thread does the work and where intermediate values live.
 //
-// Phases of a delta-net layer (attention layer in brackets), one grid barrier after each:
-//   A  rmsnorm -> Hadamard -> q8k of the residual row                         5 CTAs (one per 1024-block)
-//   B  [qkv | gate] ([q | k | v]) ternary matvec                              all CTAs
-//   C  conv + l2norm + dense beta/alpha rows + delta rule + gated norm        one CTA per value head
-//      (q/k norms + rope + KV store + attention                               one CTA per head)
-//   D  permuted Hadamard -> q8k of the block output                           6 CTAs
-//   E  output projection, accumulating into the residual                      all CTAs
-//   F  rmsnorm -> Hadamard -> q8k                                             5 CTAs
-//   G  [gate | up] matvec                                                     all CTAs
-//   H  silu(gate) * up -> Hadamard -> q8k                                     17 CTAs
-//   I  down projection, accumulating into the residual                        all CTAs
+// Phases of a layer:
+//   A  rmsnorm -> Hadamard -> q8k of the residual row: one CTA per block of 1024; the dense beta / alpha rows of a delta-net layer
+//      from the same normed row: one CTA per row
+//   B  everyone: the input projection.  The lane that has added up a row finishes it: conv + SiLU or SiLU (delta-net), or as it is
+//   C  delta-net: l2norms + delta rule + gated norm, one CTA per value head; attention: four CTAs per head
+//   D  Hadamard -> q8k of the block's output row
+//   E  everyone: the output projection, into the residual
+//   F  as A, with the layer's other norm
+//   G  everyone: gate / up, silu(gate) * up by the lane that has both
+//   H  Hadamard -> q8k of the activation row
+//   I  everyone: the down projection, into the residual
 // then output norm + Hadamard + q8k, the LM head with the greedy pick folded into its epilogue, and the pick's hand-over
 // to the next step (token slot, position + 1).
 //
-// Every wait (mbarrier, grid barrier) is bounded; when one runs out the CTA raises the context's error flag and an abort
-// word that makes every other CTA leave at its next barrier, drains its copies and returns (IT_ETIMEOUT on the host).
+// What bounds it.  One row leaves 15.5 us of weight stream a layer; a delta-net layer of the 27B shape takes 44 us (61 with a grid
+// barrier after each phase), the rest is latency: a value takes about 0.5 us from one SM to another, a block's transform 1.5,
+// the first round of tiles 0.6, a row's last terms 0.4 and its tail, the delta rule 3.5.  What follows from that: values travel
+// with tags instead of behind barriers (granules, below); a matrix is cut into equal runs of chunks whatever row groups they
+// start in; transforms are as parallel as their blocks and no phase is repeated by everyone (every CTA transforming the whole
+// row cost 2.3 us where the owners' way costs 1.4 and one more hop).  Code is kept small: measured on this GPU, straight-line code
+// runs at one instruction per cycle and scheduler while it fits 32 KB, at half that up to about 100 KB, at a sixth beyond 128 KB.
+//
+// Every wait (mbarrier, counter, tag) is bounded; when one runs out the CTA raises the context's error flag and an abort word
+// that makes every other CTA leave at its next wait, drains its copies and returns (IT_ETIMEOUT on the host).
 #define IT_PIPE_OUTLINE_WAIT  // one copy of the retry loop of bounded waits
 #define IT_MATH_OUTLINE      // one copy of division, square root and the elementary functions: this kernel's code size is its speed
 #include "it_math.h"
 #include "it_engine.h"
 #include "it_support.h"
 #include "it_pipe.cuh"
-#include "it_hadamard.cuh"
 #include <algorithm>
 #include <vector>
 
 namespace {
 
 constexpr int ST_CW = 4;                               // warps per consumer group
-constexpr int ST_NG = 3;                               // consumer groups; group j takes the chunks k of the CTA's stream with k % ST_NG == j
-constexpr int ST_TPW = 2;                              // tiles a warp takes from a chunk (computed side by side)
-constexpr int ST_TPC = ST_CW * ST_TPW;                 // tiles per chunk = per ring slot
+constexpr int ST_NG = 3;                               // consumer groups; group j takes the chunks i of a phase with i % ST_NG == j
+constexpr int ST_TPC = 8;                              // tiles per chunk = per ring slot: two per warp of a group, computed side by side (widths are multiples of 1024, eight tiles)
 constexpr int ST_NCONS = ST_CW * ST_NG;                // consumer warps
 constexpr int ST_CT = ST_NCONS * 32;                   // consumer threads
-constexpr int ST_NSUM = 2;                             // warps that only add the per-block terms of finished row groups in block order
-constexpr int ST_TB = 3;                               // terms buffers (row groups in flight between the consumer warps and the sum warps)
+constexpr int ST_NSUM = 2;                             // warps that only add the per-block terms in block order
 constexpr int ST_THREADS = ST_CT + (ST_NSUM + 1) * 32; // + the sum warps + the producer warp
 constexpr int ST_CHUNK = ST_TPC * IT_TILE_BYTES;       // bytes of one ring slot
+constexpr int ST_TERMS = ST_TPC * 32;                  // terms of one chunk (floats)
 constexpr int ST_SMEM = 227 * 1024;                    // dynamic shared memory of the CTA
-constexpr int ST_BARS = 1024;                          // bytes reserved for mbarriers and flags
+constexpr int ST_BARS = 1024;                          // bytes reserved for mbarriers, flags, layer descriptions and spans
 constexpr int ST_SD = 128;                             // delta-rule state size this kernel is built for
+constexpr int ST_HB = ST_NCONS / 2;                    // Hadamard blocks of 1024 transformed at a time, two warps each
+constexpr int ST_HPITCH = 1344;                        // floats of a block in the transform's exchange area: 64 runs of 16, padded
+constexpr int ST_RED = 384;                            // bytes: the dense row's eight f64 warp sums, then the transform's [8] sums of squares and [ST_HB][4][2] group maxima
+
+// A CTA's share of one ternary matrix.  The matrix is a sequence of chunks (eight 32 x 128 tiles of one row group, row
+// groups in order); every CTA gets an equal run of it, whatever row group the run starts or ends in (5120 rows are 160 row
+// groups: whole ones would leave most of 148 CTAs with one and some with two).  A cut row group is finished by the later
+// CTA: the earlier one adds its first blocks and hands the running sums over, which is the same order of additions.  It does
+// that part first and the later CTA does its own last, so that nobody waits.  Order of a CTA's chunks: hl of the row group it
+// starts but does not finish, whole row groups, tl of the row group begun by the CTA before.
+struct StepSpan { int n, hl, tl, lead, uh, uf, ut, nb, cpr, parts, units; unsigned magic; };     // uh, uf, ut: row groups of the three parts
+enum { SP_IN_GDN, SP_IN_ATT, SP_OUT_GDN, SP_OUT_ATT, SP_GATE_UP, SP_DOWN, SP_HEAD, SP_KINDS };
 
 struct StepLayer {
     const uint8_t *in_proj, *out_proj, *gate_up, *down;
@@ -65,24 +82,36 @@ struct StepLayer {
     int recurrent, in_rows;
 };
 
+// Values that one CTA hands to others travel as granules: 16 bytes written and read by single 128-bit accesses, three values and
+// the tag of the phase that made them (32 rows of a row group: eleven granules).  A reader that finds the tag has the values; no
+// fence is involved.  Why: one value crosses between two SMs in about 960 cycles whatever else the memory system does, but a
+// release or acquire-release fence takes 840 cycles on an idle GPU and 1900 while weights stream in, on every CTA's way into
+// every barrier.  Tags grow from phase to phase and launch to launch, so no granule needs to be cleared.
+typedef uint4 granule;
+constexpr int ST_GPU = 11;                             // granules of a row group (32 rows)
+constexpr int ST_COPIES = 4;                           // copies of the quantised row: all SMs read it at once, and its few lines would crowd a few L2 slices
+
 struct StepParams {
-    const StepLayer* layers; int n_layer;
-    int e, ff, hd, nh, nkv, cd, inner, nv, nk, qk, conv_k, n_rot, n_vocab;
+    const StepLayer* layers; const StepSpan* spans; int n_layer;
+    int e, ff, widest, hd, nh, nkv, cd, inner, nv, nk, qk, conv_k, n_rot, n_vocab;
     float eps, theta_scale; int sec[4]; int v_grouped;
-    float* arena; size_t x, xn, big1, o, hrow, logits, amx;
-    int8_t* qs; float* qd; int32_t* qsum; size_t q_stride;
-    const float *sg_e, *sg_inner, *sg_att, *sg_ff;
+    float* arena; size_t hrow, logits, amx;
+    granule *xe, *xi, *rows, *o, *act; // residual row after the output / down projection; input projection's rows; block output; silu(gate) * up
+    granule* codes; int codes_half;    // the quantised row: 128 granules a block of 1024, ST_COPIES copies; codes_half granules further: the activation row's
+    unsigned long long* gate;          // per value head beta, then decay: value and tag
+    granule* prefix;                   // [grid][32] running sums of a cut row group (two matrices' worth) and the tag
+    granule* partials;                 // one greedy-pick partial per sum warp: value, row, tag
+    unsigned long long* att_sc; int att_stride; unsigned* att_cnt;   // per head: the scores its CTAs exchange [nh][att_stride] (value and tag), their arrival counter [nh]
+    const uint32_t* sg[4]; int sg_off[4], sg_words[4];   // sign bits of the four widths (n_embd, ssm_inner, attention output, n_ff): words, and where they start in shared memory
     const float *tok_embd, *output_norm; const uint8_t* output;
     uint32_t* toks; int* pos;
     unsigned* sync;                    // [0] arrivals, [1] arrivals at the end of the last launch, [2] abort word
-    unsigned long long* partials;      // one greedy-pick partial per CTA
     int* error_flag;
-    unsigned long long* trace;         // optional: clock readings of CTA 0 and of the last CTA at every grid barrier (arrive, leave)
-    int slots, scratch;                // ring slots; bytes of the phase scratch that follows the ring
+    unsigned long long* trace;         // optional: clock readings of CTA 0 and of the last CTA at the waits in front of matrix phases (arrive, leave)
+    int slots, scratch, w_off;         // ring slots; bytes of the phase scratch that follows the ring; where a norm's weights lie in it (a dense row in front of them)
     int attn_g;                        // CTAs that share an attention head
-    float* att_sc; int att_stride; unsigned* att_cnt;   // per head: the scores its CTAs exchange [nh][att_stride], their arrival counter [nh]
-    int had_base, attn_base;           // first CTA of the Hadamard blocks / of the attention heads (value heads start at CTA 0): roles on
-                                       // different CTAs keep each CTA's instruction footprint small
+    int attn_base;                     // first CTA of the attention heads (value heads start at CTA 0; dense rows count down from the last CTA)
+    int had_step;                      // the CTAs that transform the activation row's blocks are this far apart
     int gdn_off;                       // where the delta-net block keeps its state tile inside the scratch (clear of the input projection's buffers)
     int flags;                         // bit 0: the token is the previous pick (amx) instead of toks[0]; bit 1: hand the pick over (toks[0], pos + 1); bit 2: logits wanted
 };
@@ -93,20 +122,23 @@ __device__ __forceinline__ Pick pick_better(Pick a, Pick b) { return (b.v > a.v 
 // Per-thread view of the CTA's state that every phase needs.
 struct Cta {
     unsigned char* smem; unsigned char* scratch; unsigned bars; volatile int* abort_flag;
+    volatile int* verdict;             // thread 0's answer after a wait, so that all consumer warps leave or stay together
     int tid, warp, lane;
-    unsigned q;                        // chunks of the CTA's stream the consumers have passed (slot = q % slots, phase = (q / slots) & 1; slots is a power of two)
-    unsigned nseq;                     // row groups this CTA has started in all matvec phases so far (terms buffer = nseq % ST_TB)
-    unsigned mph;                      // matvec phases finished so far
-    unsigned tf, te, pd, ps;           // mbarriers: terms full [ST_TB], terms empty [ST_TB], phase done, phase started
+    unsigned q;                        // chunks of the CTA's stream passed so far (slot = q % slots, phase = (q / slots) & 1; slots is a power of two)
+    unsigned tf, ps, pd, dn;           // mbarriers: terms of a slot's chunk in place [slots], phase started, phase summed, dense row's warp sums in place
+    unsigned mph;                      // matrix phases so far
     unsigned at;                       // mbarriers of the attention block: K full / free, V full / free, eight of each
     const StepLayer* lay;              // the two shared-memory copies of layer descriptions (layer il at lay[il & 1])
-    unsigned target;                   // arrivals the next grid barrier waits for
-    int nsync;                         // grid barriers passed so far (index into the trace)
-    unsigned att_seq;                  // attention blocks this CTA has run in this launch
+    const StepSpan* sp;                // this CTA's spans, by matrix kind
+    const uint32_t* sg;                // sign bits of the four widths (P.sg_off)
+    unsigned base, target;             // tags of this launch start here; what the counter reaches when the transforms so far have begun
+    int nsync;                         // waits in front of matrix phases passed so far (index into the trace)
+    unsigned att_seq;                  // attention blocks this CTA has run in this launch (a sum warp: dense rows)
+    unsigned att_base;                 // the head's arrival counter at the start of the launch (thread 0)
     float inv_sqrt_sd, inv_sqrt_hd;    // 1 / sqrt(state size), 1 / sqrt(head dimension): formed once per launch
     int evt_on, evt_base;              // diagnostics: this thread records fine-grained events into slots evt_base ..
 };
-constexpr int ST_TRACE_MAX = 1024;     // barriers recorded per traced CTA
+constexpr int ST_TRACE_MAX = 1024;     // waits recorded per traced CTA
 constexpr int ST_EVT_MAX = 2048;       // fine-grained events (diagnostics)
 // Diagnostics: slot `id` of the event area receives the nanosecond clock when the chosen thread passes (one store, no read).
 // fine-grained events are compiled in only with -DIT_STEP_EVENTS: their two dozen sites cost 2.8 KB of code, about 1 % of a step
@@ -119,138 +151,421 @@ constexpr int ST_EVT_MAX = 2048;       // fine-grained events (diagnostics)
 __device__ __forceinline__ void cons_sync() { consumer_barrier<ST_CT>(); }
 // four u8 x s8 products added to c
 __device__ __forceinline__ int dp4a_us(unsigned a, int b, int c) { int d; asm("dp4a.u32.s32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c)); return d; }
+__device__ __forceinline__ granule ld_granule(const granule* p) {
+    unsigned long long a, b;
+    asm volatile("{\n.reg .b128 q;\nld.relaxed.gpu.global.b128 q, [%2];\nmov.b128 {%0, %1}, q;\n}" : "=l"(a), "=l"(b) : "l"(p) : "memory");
+    return make_uint4((unsigned)a, (unsigned)(a >> 32), (unsigned)b, (unsigned)(b >> 32));
+}
+__device__ __forceinline__ void st_granule(granule* p, unsigned x, unsigned y, unsigned z, unsigned tag) {
+    const unsigned long long a = (unsigned long long)y << 32 | x, b = (unsigned long long)tag << 32 | z;
+    asm volatile("{\n.reg .b128 q;\nmov.b128 q, {%1, %2};\nst.relaxed.gpu.global.b128 [%0], q;\n}" :: "l"(p), "l"(a), "l"(b) : "memory");
+}
+// A wait for tagged values has gone round `it` times: true when it has to end without them (the abort flag is up).
+__device__ __noinline__ bool tag_late(unsigned it, long long t0, volatile int* abort_flag, int* error_flag, int site) {
+    if (it & 31u) return false;
+    if (*abort_flag) return true;
+    if (clock64() - t0 > WAIT_CLOCKS) { atomicExch(error_flag, site); *abort_flag = 1; return true; }
+    return false;
+}
+__device__ __noinline__ granule wait_granule(const granule* p, unsigned tag, volatile int* abort_flag, int* error_flag, int site) {
+    const long long t0 = clock64();
+    granule v;
+#pragma unroll 1
+    for (unsigned it = 1;; it++) { v = ld_granule(p); if (v.w == tag || tag_late(it, t0, abort_flag, error_flag, site)) return v; }
+}
+// Granules p, p + stride, ... (n of them, n <= N; the last one again in the places behind it): all requested, then all again until
+// each has its tag.  Bounded by a count of round trips (at least 500 cycles each); no call, so that nothing is spilled around it.
+constexpr unsigned ST_POLLS = 1u << 22;
+template <int N> __device__ __forceinline__ void read_granules(granule (&g)[N], const granule* p, int stride, int n, unsigned tag, const Cta& c, int* error_flag, int site) {
+#pragma unroll 1
+    for (unsigned it = 0;; it++) {
+#pragma unroll
+        for (int u = 0; u < N; u++) g[u] = ld_granule(p + min(u, n - 1) * stride);
+        unsigned miss = 0;
+#pragma unroll
+        for (int u = 0; u < N; u++) miss |= g[u].w ^ tag;
+        if (miss == 0) return;
+        if (*c.abort_flag) return;
+        if (it == ST_POLLS) { atomicExch(error_flag, site); *c.abort_flag = 1; return; }
+    }
+}
+// value and tag in one 8-byte word
+__device__ __forceinline__ void st_tagged(unsigned long long* p, float v, unsigned tag) { asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" :: "l"(p), "l"((unsigned long long)tag << 32 | __float_as_uint(v)) : "memory"); }
+__device__ __noinline__ float ld_tagged(const unsigned long long* p, unsigned tag, volatile int* abort_flag, int* error_flag, int site) {
+    const long long t0 = clock64();
+#pragma unroll 1
+    for (unsigned it = 1;; it++) {
+        unsigned long long v; asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+        if ((unsigned)(v >> 32) == tag || tag_late(it, t0, abort_flag, error_flag, site)) return __uint_as_float((unsigned)v);
+    }
+}
+// One value per lane of a warp (32 consecutive rows) as the granules of row group u.
+__device__ __forceinline__ void publish(granule* dst, int u, int lane, float v, unsigned tag) {
+    const float b = __shfl_down_sync(0xffffffffu, v, ST_GPU), d = __shfl_down_sync(0xffffffffu, v, 2 * ST_GPU);
+    if (lane < ST_GPU) st_granule(dst + (size_t)u * ST_GPU + lane, __float_as_uint(v), __float_as_uint(b), __float_as_uint(d), tag);
+}
+// Granule i of a run of row groups holds rows r, r + 11 and (unless it is the last of its row group) r + 22.
+__device__ __forceinline__ int granule_row(int i, bool& two) { const int u = i / ST_GPU, l = i - u * ST_GPU; two = l == ST_GPU - 1; return u * 32 + l; }
+enum { PH_A, PH_B, PH_C, PH_D, PH_E, PH_F, PH_G, PH_H, PH_I, ST_SUBS };       // phases of a layer
+__device__ __forceinline__ unsigned tag_of(unsigned base, int il, int sub) { return base + 1u + (unsigned)(ST_SUBS * il + sub); }
+// Scratch of a matrix phase of nb blocks a row: ST_RED bytes of sums, the q8k row with its scales (a float per 256) and block sums
+// (an int per 128), then the transform's exchange area and, after it, the terms [slots][ST_TPC][32] of the ring's chunks.
+__host__ __device__ __forceinline__ int terms_at(int nb) { return ST_RED + ((nb * 134 + 127) & ~127); }
 
-// Barrier over the grid (consumer threads only; the producer warp never takes part).  Writes made by any CTA before the
-// barrier are visible to every CTA after it: thread 0 announces the CTA with a release add and waits with acquire loads
-// until every CTA of this round has arrived (the adds form one chain on the counter, so the load that sees the last of
-// them is ordered after every CTA's writes).  Returns false when the step
-// has been given up (by this CTA's own timeout or by another CTA's).
-__device__ __forceinline__ bool grid_sync(const StepParams& P, Cta& c, int site) {
-    cons_sync();
-    if (c.tid == 0 && *c.abort_flag) atomicExch(P.sync + 2, 1u);      // a wait of this CTA ran out: tell the others
-    if (c.tid == 0 && !*c.abort_flag) {
-        const bool traced = P.trace && (blockIdx.x == 0 || blockIdx.x == gridDim.x - 1) && c.nsync < ST_TRACE_MAX;
-        unsigned long long* rec = traced ? P.trace + ((size_t)(blockIdx.x ? 1 : 0) * ST_TRACE_MAX + c.nsync) * 2 : nullptr;
-        if (rec) { unsigned long long t; asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t)); rec[0] = t; }
-        c.target += gridDim.x;
-        // release: the CTA's writes (ordered before this thread by the barrier above) become visible before the arrival
-        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" :: "l"(P.sync) : "memory");
+// Nothing waits for everyone: a phase starts where its granules are, and polls them.  All CTAs polling a row through the whole of
+// the phases that lead to it would take bandwidth from the weights, so they wait on a counter until the owners of the row's
+// blocks have begun to transform them (a hint: it orders nothing and needs no fence), about 1500 cycles before the codes come.
+// A barrier instead costs 3800 cycles from the last arrival with release adds while weights stream in, 1400 with relaxed ones, and
+// another round trip for the row behind it.
+__device__ __forceinline__ void count_up(unsigned* counter) { asm volatile("red.relaxed.gpu.global.add.u32 [%0], 1;" :: "l"(counter) : "memory"); }
+__device__ __forceinline__ void grid_arrive(const StepParams& P) { count_up(P.sync); }
+__device__ __noinline__ void trace_clock(unsigned long long* trace, int nsync, int side) {
+    if ((blockIdx.x == 0 || blockIdx.x == gridDim.x - 1) && nsync < ST_TRACE_MAX) {
+        unsigned long long t; asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+        trace[((size_t)(blockIdx.x ? 1 : 0) * ST_TRACE_MAX + nsync) * 2 + side] = t;
+    }
+}
+// Consumer threads only: thread 0 waits until `counter` has reached `target`.  Returns false when the step has been given up (by
+// this CTA's own timeout or by another CTA's).
+__device__ __forceinline__ bool count_wait(const StepParams& P, Cta& c, const unsigned* counter, unsigned target, int site, bool traced = true) {
+    if (c.tid == 0) {
+        if (P.trace && traced) trace_clock(P.trace, c.nsync, 0);
         const long long t0 = clock64();
+#pragma unroll 1
         for (unsigned it = 0;; it++) {
-            unsigned v; asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(P.sync) : "memory");
-            if ((int)(v - c.target) >= 0) break;
+            unsigned v; asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(counter) : "memory");
+            if ((int)(v - target) >= 0) break;
             if ((it & 63u) == 63u) {
+                if (*c.abort_flag) { atomicExch(P.sync + 2, 1u); break; }                       // a wait of this CTA ran out: tell the others
                 if (*reinterpret_cast<volatile unsigned*>(P.sync + 2)) { *c.abort_flag = 1; break; }
                 if (clock64() - t0 > WAIT_CLOCKS) { atomicExch(P.error_flag, 100 + site); atomicExch(P.sync + 2, 1u); *c.abort_flag = 1; break; }
             }
         }
-        if (rec) { unsigned long long t; asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t)); rec[1] = t; }
-        c.nsync++;
+        *c.verdict = *c.abort_flag;
+        if (P.trace && traced) trace_clock(P.trace, c.nsync++, 1);
     }
     cons_sync();
-    return !*c.abort_flag;
+    return !*c.verdict;
 }
 
 // The ternary matvecs of a step in order: four per layer (input projection, output projection, gate/up, down), then the
-// LM head.  Every role of the CTA (producer, consumers, sum warps) walks this list with ONE copy of its loop in the code:
-// the kernel is executed once per step, front to back, so its size is what the instruction cache sees.
-struct MatDesc { const uint8_t* tiles; int nb, rows, accum, pick; size_t y_off; };
-__device__ __forceinline__ MatDesc mat_desc(const StepParams& P, int mp) {
-    MatDesc d; d.pick = 0;
-    const int il = mp >> 2, sub = mp & 3;
-    if (il >= P.n_layer) { d.tiles = P.output; d.nb = P.e / 128; d.rows = P.n_vocab; d.accum = 0; d.y_off = P.logits; d.pick = 1; return d; }
-    const StepLayer& L = P.layers[il];
-    if (sub == 0) { d.tiles = L.in_proj; d.nb = P.e / 128; d.rows = L.in_rows; d.accum = 0; d.y_off = P.big1; }
-    else if (sub == 1) { d.tiles = L.out_proj; d.nb = (L.recurrent ? P.inner : P.nh * P.hd) / 128; d.rows = P.e; d.accum = 1; d.y_off = P.x; }
-    else if (sub == 2) { d.tiles = L.gate_up; d.nb = P.e / 128; d.rows = 2 * P.ff; d.accum = 0; d.y_off = P.big1; }
-    else { d.tiles = L.down; d.nb = P.ff / 128; d.rows = P.e; d.accum = 1; d.y_off = P.x; }
-    return d;
-}
+// LM head.  Every role of the CTA (producer, consumers, sum warps) walks this list with ONE copy of its loop in the code.
 __device__ __forceinline__ int mat_count(const StepParams& P) { return 4 * P.n_layer + ((P.flags & 4) ? 1 : 0); }
+__device__ __forceinline__ int span_kind(int sub, int recurrent) { return sub == 0 ? (recurrent ? SP_IN_GDN : SP_IN_ATT) : sub == 1 ? (recurrent ? SP_OUT_GDN : SP_OUT_ATT) : sub == 2 ? SP_GATE_UP : SP_DOWN; }
 
 // ---------------------------------------------------------------- producer
-struct Ring { int s; unsigned ph; int issued; };
-__device__ __forceinline__ bool produce_matrix(const StepParams& P, const Cta& c, Ring& r, const uint8_t* tiles, int nb, int rows, int* error_flag) {
-    const int rgs = (rows + 31) / 32, cpr = (nb + ST_TPC - 1) / ST_TPC;
-    for (int rg = blockIdx.x; rg < rgs; rg += gridDim.x) {
-        const uint8_t* src = tiles + (size_t)rg * nb * IT_TILE_BYTES;
-        for (int cq = 0; cq < cpr; cq++) {
-            if (!mbar_wait(c.bars + 8 * (P.slots + r.s), r.ph ^ 1u, c.abort_flag, error_flag, 2)) return false;
-            const int ntile = min(ST_TPC, nb - cq * ST_TPC);
-            const unsigned bytes = (unsigned)ntile * IT_TILE_BYTES;
-            mbar_expect_tx(c.bars + 8 * r.s, bytes);
-            bulk_load(smem_u32(c.smem + r.s * ST_CHUNK), src + (size_t)cq * ST_CHUNK, bytes, c.bars + 8 * r.s);
-            r.issued++;
-            if (++r.s == P.slots) { r.s = 0; r.ph ^= 1u; }
-        }
-    }
-    return true;
-}
 __device__ __forceinline__ void producer(const StepParams& P, const Cta& c) {
-    Ring r{0, 0u, 0};
+    int s = 0, issued = 0; unsigned ph = 0u;
     bool ok = true;
     const int nmat = mat_count(P);
-    for (int mp = 0; mp < nmat && ok; mp++) { const MatDesc d = mat_desc(P, mp); ok = produce_matrix(P, c, r, d.tiles, d.nb, d.rows, P.error_flag); }
+#pragma unroll 1
+    for (int mp = 0; mp < nmat && ok; mp++) {
+        const int il = mp >> 2, sub = mp & 3;
+        const uint8_t* tiles = P.output; int kind = SP_HEAD;
+        if (il < P.n_layer) { const StepLayer& L = P.layers[il]; kind = span_kind(sub, L.recurrent); tiles = sub == 0 ? L.in_proj : sub == 1 ? L.out_proj : sub == 2 ? L.gate_up : L.down; }
+        const StepSpan sp = c.sp[kind];
+        const int cpu = sp.cpr * sp.parts;
+        int unit = sp.uh, cq = 0;
+#pragma unroll 1
+        for (int i = 0; i < sp.n; i++) {
+            if (i == sp.hl) { unit = sp.uf; cq = 0; }
+            if (i == sp.n - sp.tl) { unit = sp.ut; cq = sp.lead; }
+            if (!mbar_wait(c.bars + 8 * (P.slots + s), ph ^ 1u, c.abort_flag, P.error_flag, 2)) { ok = false; break; }
+            const bool second = cq >= sp.cpr;
+            mbar_expect_tx(c.bars + 8 * s, ST_CHUNK);
+            bulk_load(smem_u32(c.smem + s * ST_CHUNK), tiles + ((size_t)(second ? unit + sp.units : unit) * sp.cpr + (second ? cq - sp.cpr : cq)) * ST_CHUNK, ST_CHUNK, c.bars + 8 * s);
+            issued++;
+            if (++s == P.slots) { s = 0; ph ^= 1u; }
+            if (++cq == cpu) { cq = 0; unit++; }
+        }
+    }
     if (!ok || *c.abort_flag) {
         // leave only after every copy this thread started has landed (each wait bounded by the clock limit)
-        const int first = r.issued > P.slots ? r.issued - P.slots : 0;
-        for (int k = first; k < r.issued; k++) {
+        const int first = issued > P.slots ? issued - P.slots : 0;
+        for (int k = first; k < issued; k++) {
             const long long t0 = clock64();
             while (!mbar_test(c.bars + 8 * (k % P.slots), (unsigned)(k / P.slots) & 1u) && clock64() - t0 < WAIT_CLOCKS) { }
         }
     }
 }
 
-// ---------------------------------------------------------------- ternary matvec phase (one activation row)
-// Same arithmetic as k_matvec_t2<1> (it_matvec_t2.cu): per 32 x 128 tile the exact integer block sums, the per-block terms
-// (d_w * d_x) * float(S - sum128), and per row group one warp that adds the terms in ascending block order.  The sixteen
-// consumer warps only form terms; two sum warps add them, a row group at a time, out of ST_TB buffers handed over through
-// mbarriers, so that the consumers never stop at a row-group boundary.
-struct MvSmem { int x, dx, s128, terms, plane, total; };
-__host__ __device__ inline MvSmem mv_layout(int nb) {
-    MvSmem L; int o = 0;
-    L.plane = nb * 32;
-    L.x = o; o += nb * 128 + 16;
-    L.dx = o; o += (nb / 2) * 4;
-    L.s128 = o; o += nb * 4;
-    o = (o + 127) & ~127;
-    L.terms = o; o += ST_TB * L.plane * 4;
-    L.total = o;
-    return L;
+// Vectors that a later phase reads once: on their way into L2 while the weight stream would make them wait (lines of 128 bytes, a thread each).
+__device__ __forceinline__ void warm_l2(const void* p, int bytes, int i) {
+    if (i >= 0 && i * 128 < bytes) asm volatile("prefetch.global.L2 [%0];" :: "l"(reinterpret_cast<const char*>(p) + (size_t)i * 128));
+}
+// The next layer's (or, behind the last layer, the output norm's): by the last CTA; the conv taps and state of a CTA's own rows by that CTA.
+__device__ __forceinline__ void warm_layer(const StepParams& P, const Cta& c, const StepLayer& N, int drow) {
+    const int tid = c.tid;
+    if (blockIdx.x == gridDim.x - 1) {
+        warm_l2(N.attn_norm, P.e * 4, tid); warm_l2(N.post_norm, P.e * 4, tid);
+        if (N.recurrent) { warm_l2(N.ssm_norm, ST_SD * 4, tid); warm_l2(N.dt, P.nv * 4, tid - 32); warm_l2(N.a, P.nv * 4, tid - 64); }
+        else { warm_l2(N.q_norm, P.hd * 4, tid); warm_l2(N.k_norm, P.hd * 4, tid - 32); }
+    }
+    if (!N.recurrent) return;
+    if (drow < 2 * P.nv) warm_l2((drow < P.nv ? N.beta : N.alpha - (size_t)P.nv * P.e) + (size_t)drow * P.e, P.e * 4, tid);
+    const StepSpan& sp = c.sp[SP_IN_GDN];
+    const int u = (sp.tl ? sp.ut : sp.uf) + (tid >> 4), k = tid & 15, row = u * 32;      // sixteen threads a row group: conv_k - 1 state rows, conv_k lines of taps
+    if (row < P.cd && (tid >> 4) * sp.cpr < sp.n + sp.cpr) {
+        if (k < P.conv_k - 1) warm_l2(N.conv_st + (size_t)k * P.cd + row, 128, 0);
+        else warm_l2(N.conv_w + (size_t)row * P.conv_k, 128 * P.conv_k, k - (P.conv_k - 1));
+    }
 }
 
-// prefetch_layer: when set, the delta-net block's state tile of that layer is requested right after the activation row has
-// been staged (asynchronous copies for the phase after this one)
-__device__ __forceinline__ void gdn_prefetch(const StepParams& P, const StepLayer& L, const Cta& c, int h);
-__device__ __forceinline__ void attn_prefetch(const StepParams& P, const StepLayer& L, const Cta& c, int h);
-__device__ __forceinline__ void matvec_phase(const StepParams& P, Cta& c, int nb, int rows, const StepLayer* prefetch_layer) {
-    const MvSmem L = mv_layout(nb);
-    int8_t* xs = reinterpret_cast<int8_t*>(c.scratch + L.x);
-    float* dxs = reinterpret_cast<float*>(c.scratch + L.dx);
-    int* sss = reinterpret_cast<int*>(c.scratch + L.s128);
-    const int tid = c.tid, warp = c.warp, lane = c.lane;
-    ST_EV(P, c, c.evt_base + 0);
-    if (lane == 0) mbar_arrive(c.ps);                                // the sum warps may enter this phase (they never run ahead of the consumers)
-    {   // the q8k row, its scales and block sums, once per CTA (written by other CTAs before the last barrier: read through L2)
-        for (int ch = tid; ch < nb * 8; ch += ST_CT) cp_async16(xs + 16 * ch, P.qs + 16 * ch);
-        for (int i = tid; i < nb / 2; i += ST_CT) dxs[i] = __ldcg(P.qd + i);
-        for (int i = tid; i < nb; i += ST_CT) sss[i] = __ldcg(P.qsum + i);
-        cp_async_wait_all();
-        if (prefetch_layer) { if (prefetch_layer->recurrent) gdn_prefetch(P, *prefetch_layer, c, (int)blockIdx.x); else attn_prefetch(P, *prefetch_layer, c, (int)blockIdx.x - P.attn_base); }
-        cons_sync();
+// ---------------------------------------------------------------- row transform
+// [rmsnorm ->] signs -> Hadamard over blocks of 1024 -> q8k of one row of nblk blocks, from global memory into this CTA's
+// scratch, in the operation order of it_hadamard_block (it_hadamard.cuh).  Two warps take a block, six blocks run at a time.
+// A thread holds 16 values through three layouts: 16 consecutive ones (strides 1..8), every 16th of a run of 256 (16..128),
+// a run of four from each of the block's four q8k groups (256, 512); the row comes in through cp.async into the padded layout
+// that makes the first read and both changes of layout free of bank conflicts.  (Read straight into registers, 64 bytes a thread,
+// 24 KB cost 2000 cycles with all SMs at it; the same 16-byte pieces in lane order cost 560.)  The norm's weights and the dense
+// row do not depend on the step and are in shared memory before the barrier in front of the phase opens.
+struct RowIn {
+    const granule* x; unsigned tag; const float* plain;      // the row (norm) or its block, as granules of a phase, or (plain) as floats
+    const uint32_t* signs; float* normed;                    // normed: where the normed row goes, or null
+    granule* codes; unsigned code_tag; int codes_copy;       // where the quantised block goes (copies codes_copy granules apart), or null
+    int nblk, blk; bool norm, dense;                         // blocks brought in, the one to transform; dense: multiply the normed row with this CTA's dense row
+};
+__device__ __forceinline__ bool ieee_negative_zero(float x) { return __float_as_uint(x) == 0x80000000u; }
+__device__ __forceinline__ void pair_sync() { asm volatile("bar.sync 5, 64;" ::: "memory"); }
+__device__ __forceinline__ int ex_at(int e) { return e + 4 * (e >> 4) + 16 * (e >> 8); }      // element e of a row in the padded layout: 1344 floats a block, 336 a run of 256, 20 a run of 16
+// nblk blocks of 1024 rows (32 row groups, 352 granules: a thread each) from `x` into the padded layout at `ex`
+constexpr int ST_GPB = 32 * ST_GPU;
+static_assert(ST_GPB <= ST_CT, "a granule of every block per thread");
+__device__ __forceinline__ void row_place(const StepParams& P, const Cta& c, float* ex, const granule* x, int nblk, unsigned tag) {
+    constexpr int N = 6;
+    if (c.tid >= ST_GPB) return;
+    bool two; const int r = granule_row(c.tid, two);
+    float *p0 = ex + ex_at(r), *p1 = ex + ex_at(r + ST_GPU), *p2 = two ? p1 : ex + ex_at(r + 2 * ST_GPU);
+#pragma unroll 1
+    for (int b = 0; b < nblk; b += N, p0 += N * ST_HPITCH, p1 += N * ST_HPITCH, p2 += N * ST_HPITCH) {
+        granule g[N];
+        const int m = min(N, nblk - b);
+        read_granules(g, x + b * ST_GPB + c.tid, ST_GPB, m, tag, c, P.error_flag, 14);
+#pragma unroll
+        for (int u = 0; u < N; u++) {
+            const int o = min(u, m - 1) * ST_HPITCH;
+            p2[o] = __uint_as_float(two ? g[u].y : g[u].z); p0[o] = __uint_as_float(g[u].x); p1[o] = __uint_as_float(g[u].y);
+        }
     }
-    ST_EV(P, c, c.evt_base + 1);
-    const int t = lane & 3;
-    const int group = warp / ST_CW, wi = warp % ST_CW;
-    const int rgs = (rows + 31) / 32, cpr = (nb + ST_TPC - 1) / ST_TPC;
+}
+// Requests a norm's weights (padded layout, at shared-memory address wb) and, for a CTA that has one, a dense row (natural order,
+// in front of them); one group per thread.
+__device__ __noinline__ void norm_request(float* wb, const float* w, const float* dense, int e) {
+    const int tid = threadIdx.x;
+#pragma unroll 1
+    for (int i = 4 * tid; i < e; i += 4 * ST_CT) {
+        cp_async16(wb + (i >> 10) * ST_HPITCH + ex_at(i & 1023), w + i);
+        if (dense) cp_async16(wb - e + i, dense + i);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+}
+__device__ __forceinline__ void block_transform(const StepParams& P, const Cta& c, const RowIn in) {
+    const int tid = c.tid, warp = c.warp, lane = c.lane, half = warp & 1, j = tid & 63;
+    const int n = in.nblk * 1024;
+    float* ex0 = reinterpret_cast<float*>(c.scratch + ST_RED);
+    float* red = reinterpret_cast<float*>(c.scratch + 64);   // [8] warp sums of squares, [4][2] group maxima
+    const float* wb = reinterpret_cast<const float*>(c.scratch + P.w_off);
+    cons_sync();                                             // the scratch is nobody's any more (the block before may still have been writing state)
+    if (in.plain) {
+#pragma unroll 1
+        for (int i = 4 * tid; i < n; i += 4 * ST_CT) *reinterpret_cast<float4*>(ex0 + ex_at(i)) = *reinterpret_cast<const float4*>(in.plain + i);
+    } else row_place(P, c, ex0, in.x, in.nblk, in.tag);
+    asm volatile("cp.async.wait_group 0;" ::: "memory");             // the norm's weights
+    cons_sync();
+    if (tid == 0 && in.codes) grid_arrive(P);                        // the codes will follow
+    float sc = 0.f;
+    if (in.norm) {
+        // rmsnorm of the whole row in the order of k_rmsnorm_wide: thread i of 256 adds x[i]^2, x[i + 256]^2, ...; warp
+        // butterflies; eight warp sums in ascending order
+        if (tid < 256) {
+            const float* xp = ex0 + ex_at(tid);
+            float s = 0.f, a[4];
+#pragma unroll
+            for (int u = 0; u < 4; u++) a[u] = xp[336 * u];
+#pragma unroll 1
+            for (int k = 1; k <= in.nblk; k++) {                     // the next block's four elements are requested before this one's are added
+                float b[4];
+                xp += k < in.nblk ? ST_HPITCH : 0;
+#pragma unroll
+                for (int u = 0; u < 4; u++) b[u] = xp[336 * u];
+#pragma unroll
+                for (int u = 0; u < 4; u++) { s = it_add(s, it_mul(a[u], a[u])); a[u] = b[u]; }
+            }
+#pragma unroll
+            for (int m = 16; m >= 1; m >>= 1) s = it_add(s, __shfl_xor_sync(0xffffffffu, s, m));
+            if (lane == 0) red[warp] = s;
+        }
+        cons_sync();
+        float tot = red[0];
+#pragma unroll
+        for (int k = 1; k < 8; k++) tot = it_add(tot, red[k]);
+        sc = __fdiv_rn(1.0f, __fsqrt_rn(it_add(__fdiv_rn(tot, (float)n), P.eps)));
+        if (in.normed) {
+#pragma unroll 1
+            for (int i = tid; i < n; i += ST_CT) { const int o = (i >> 10) * ST_HPITCH + ex_at(i & 1023); in.normed[i] = it_mul(it_mul(ex0[o], sc), wb[o]); }
+            cons_sync();
+        }
+        if (in.dense) {
+            if (tid < 256) {
+                // one row of the beta / alpha matrices times the normed row, in the order of k_dense_rows: thread i adds the
+                // products i, i + 256, ... in f64, warp butterflies, eight warp sums in ascending order (by sum warp 1)
+                const float* xp = ex0 + ex_at(tid); const float* wp = wb + ex_at(tid); const float* dp = wb - P.e + tid;
+                double d = 0.0;
+#pragma unroll 2
+                for (int k = 0; k < in.nblk * 4; k++) d += (double)it_mul(dp[256 * k], it_mul(it_mul(xp[336 * k], sc), wp[336 * k]));
+#pragma unroll
+                for (int m = 16; m >= 1; m >>= 1) d += __shfl_xor_sync(0xffffffffu, d, m);
+                if (lane == 0) { reinterpret_cast<double*>(c.scratch)[warp] = d; mbar_arrive(c.dn); }
+            }
+            cons_sync();                                     // the row is about to be overwritten
+        }
+    }
+    if (warp < 2 && in.codes) {
+        float* ex = ex0 + in.blk * ST_HPITCH;
+        {
+            float v[16];
+            float* p1 = ex + ex_at(16 * j);
+#pragma unroll
+            for (int u = 0; u < 4; u++) { const float4 t = *reinterpret_cast<const float4*>(p1 + 4 * u); v[4 * u] = t.x; v[4 * u + 1] = t.y; v[4 * u + 2] = t.z; v[4 * u + 3] = t.w; }
+            if (in.norm) {
+                const float* wp = wb + in.blk * ST_HPITCH + ex_at(16 * j);
+#pragma unroll
+                for (int u = 0; u < 4; u++) {
+                    const float4 w = *reinterpret_cast<const float4*>(wp + 4 * u);
+                    v[4 * u] = it_mul(it_mul(v[4 * u], sc), w.x); v[4 * u + 1] = it_mul(it_mul(v[4 * u + 1], sc), w.y);
+                    v[4 * u + 2] = it_mul(it_mul(v[4 * u + 2], sc), w.z); v[4 * u + 3] = it_mul(it_mul(v[4 * u + 3], sc), w.w);
+                }
+            }
+            const unsigned m16 = reinterpret_cast<const unsigned short*>(in.signs)[j];
+#pragma unroll
+            for (int i = 0; i < 16; i++) v[i] = __uint_as_float(__float_as_uint(v[i]) ^ ((m16 << (31 - i)) & 0x80000000u));     // times +-1
+            auto stage = [&](int h) {
+#pragma unroll
+                for (int i = 0; i < 16; i++) if (!(i & h)) { const float a = v[i], b = v[i | h]; v[i] = it_add(a, b); v[i | h] = it_sub(a, b); }
+            };
+            stage(1); stage(2); stage(4); stage(8);
+#pragma unroll
+            for (int u = 0; u < 4; u++) *reinterpret_cast<float4*>(p1 + 4 * u) = make_float4(v[4 * u], v[4 * u + 1], v[4 * u + 2], v[4 * u + 3]);
+            pair_sync();
+            float* p2 = ex + 336 * ((lane >> 4) + 2 * half) + (lane & 15);
+#pragma unroll
+            for (int i = 0; i < 16; i++) v[i] = p2[20 * i];
+            stage(1); stage(2); stage(4); stage(8);
+#pragma unroll
+            for (int i = 0; i < 16; i++) p2[20 * i] = v[i];
+            pair_sync();
+            const float* p3 = ex + ex_at(4 * j);                         // group g (of 256): values 4 g .. 4 g + 3
+#pragma unroll
+            for (int g = 0; g < 4; g++) { const float4 t = *reinterpret_cast<const float4*>(p3 + 336 * g); v[4 * g] = t.x; v[4 * g + 1] = t.y; v[4 * g + 2] = t.z; v[4 * g + 3] = t.w; }
+            stage(4); stage(8);
+            // q8k: the first element of maximum magnitude of each group sets its scale
+            float* mx = red + 8;
+            float any = 0.f, best[4];
+#pragma unroll
+            for (int i = 0; i < 16; i++) { v[i] = it_mul(v[i], 0.03125f); any += v[i]; }
+            // the first element of largest magnitude; b stands for higher indices than a, a NaN is never taken
+            auto larger = [](float a, float b, bool tie) { return fabsf(b) > fabsf(a) || (tie && fabsf(b) == fabsf(a)) ? b : a; };
+#pragma unroll
+            for (int g = 0; g < 4; g++) { best[g] = 0.f; for (int u = 0; u < 4; u++) best[g] = larger(best[g], v[4 * g + u], false); }
+            const bool odd = __any_sync(0xffffffffu, !(fabsf(any) <= 3.4e38f));
+            // lanes in ranges that double: the first two steps also share the groups out, lane l keeps group 2 (l & 1) + (l >> 1 & 1)
+            float k0 = lane & 1 ? best[2] : best[0], k1 = lane & 1 ? best[3] : best[1];
+            const float g0 = __shfl_xor_sync(0xffffffffu, lane & 1 ? best[0] : best[2], 1), g1 = __shfl_xor_sync(0xffffffffu, lane & 1 ? best[1] : best[3], 1);
+            k0 = larger(k0, g0, lane & 1); k1 = larger(k1, g1, lane & 1);
+            const float g2 = __shfl_xor_sync(0xffffffffu, lane & 2 ? k0 : k1, 2);
+            k0 = larger(lane & 2 ? k1 : k0, g2, lane & 2);
+#pragma unroll
+            for (int m = 4; m <= 16; m <<= 1) k0 = larger(k0, __shfl_xor_sync(0xffffffffu, k0, m), lane & m);
+            if (lane < 4) mx[2 * (2 * (lane & 1) + (lane >> 1)) + half] = k0;
+            pair_sync();
+            float isc = 0.f;
+            {   // lane g (and g + 4, ...): group g's scale
+                const float2 ab = *reinterpret_cast<const float2*>(mx + 2 * (lane & 3));
+                const float val = fabsf(ab.y) > fabsf(ab.x) ? ab.y : ab.x;       // equal magnitudes: the lower index
+                if (val != 0.f) isc = __fdiv_rn(-127.0f, val);       // a group of zeros keeps 0, and so codes of 0
+            }
+            // codes: round to nearest even by adding 1.5 * 2^23 (|is * v| <= 127, and a conversion takes eight cycles of the sub-core where an
+            // addition takes one); a scale that overflowed (a group below 4e-37) and values that are not finite go through the conversion
+            // and its saturation
+            // (1 / scale by a Newton step and a corrected quotient in f64, rounded once: exact to more than twice f32's digits, so the
+            // rounding is the division's; branch-free, it overlaps the codes)
+            float dk;
+            { float r; asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(isc)); const double b = isc, r0 = r, r1 = fma(r0, fma(-b, r0, 1.0), r0); dk = __double2float_rn(fma(fma(-b, r1, 1.0), r1, r1)); }
+            if (!(fabsf(isc) >= 3.7e-37f && fabsf(isc) < 1e37f)) dk = isc != 0.f || ieee_negative_zero(isc) ? __fdiv_rn(1.0f, isc) : 0.f;
+            const bool odd_scale = odd || __any_sync(0xffffffffu, fabsf(isc) > 3.4e38f);
+            uint32_t packed[4];
+#pragma unroll
+            for (int g = 0; g < 4; g++) {
+                const float is = __shfl_sync(0xffffffffu, isc, g);
+                unsigned q[4];
+#pragma unroll
+                for (int u = 0; u < 4; u++) q[u] = __float_as_uint(__fadd_rn(it_mul(is, v[4 * g + u]), 12582912.0f));
+                if (odd_scale) {
+#pragma unroll
+                    for (int u = 0; u < 4; u++) q[u] = (unsigned)min(__float2int_rn(it_mul(is, v[4 * g + u])), 127);
+                }
+                packed[g] = __byte_perm(__byte_perm(q[0], q[1], 0x0040), __byte_perm(q[2], q[3], 0x0040), 0x5410);
+                if (is == 0.f) packed[g] = 0;                        // a group of zeros, or one whose maximum is infinite
+            }
+            const int t0 = __reduce_add_sync(0xffffffffu, __dp4a((int)packed[0], 0x01010101, __dp4a((int)packed[1], 0x01010101, 0) << 16));   // two groups' code sums
+            const int t1 = __reduce_add_sync(0xffffffffu, __dp4a((int)packed[2], 0x01010101, __dp4a((int)packed[3], 0x01010101, 0) << 16));   // (at most 128 * 127 in magnitude) to a word
+            const int t = lane & 2 ? t1 : t0, lo = (short)t, sum = lane & 1 ? (t - lo) >> 16 : lo;
+            // thread j: its four words of codes; threads 0..3 of each half also the group's scale and the half's sum
+#pragma unroll 1
+            for (int k = 0; k < ST_COPIES; k++) {
+                granule* to = in.codes + k * in.codes_copy + j;
+                st_granule(to, packed[0], packed[1], packed[2], in.code_tag);
+                st_granule(to + 64, packed[3], __float_as_uint(dk), (unsigned)sum, in.code_tag);
+            }
+        }
+    }
+}
+
+// The quantised row of nblk blocks that other CTAs have published, into this CTA's scratch.
+__device__ __forceinline__ void codes_place(const StepParams& P, const Cta& c, const granule* codes, int nblk, unsigned tag) {
+    constexpr int N = 6, BPT = ST_CT / 128;                          // blocks a turn of all threads covers
+    const int n = nblk * 1024, j = c.tid & 63, blk = c.tid >> 7; const bool odd = c.tid & 64;
+    int8_t* xs = reinterpret_cast<int8_t*>(c.scratch + ST_RED);
+    float* dxs = reinterpret_cast<float*>(xs + n) + blk * 4 + (j & 3);
+    int* sss = reinterpret_cast<int*>(xs + n + n / 64) + blk * 8 + 2 * (j & 3) + (j >> 5);
+    uint32_t* at = reinterpret_cast<uint32_t*>(xs + blk * 1024 + 4 * j) + (odd ? 192 : 0);
+    const granule* src = codes + (blockIdx.x % ST_COPIES) * nblk * 128 + c.tid;
+#pragma unroll 1
+    for (int b = 0; b < nblk - blk; b += N * BPT, at += N * BPT * 256, dxs += N * BPT * 4, sss += N * BPT * 8, src += N * ST_CT) {
+        const int m = min(N, (nblk - blk - b + BPT - 1) / BPT);
+        granule g[N];
+        read_granules(g, src, ST_CT, m, tag, c, P.error_flag, 15);
+#pragma unroll
+        for (int u = 0; u < N; u++) {
+            const int o = min(u, m - 1) * BPT;
+            at[o * 256] = g[u].x;
+            if (!odd) { at[o * 256 + 64] = g[u].y; at[o * 256 + 128] = g[u].z; }
+            else if ((j & 31) < 4) { if (j < 4) dxs[o * 4] = __uint_as_float(g[u].y); sss[o * 8] = (int)g[u].z; }
+        }
+    }
+    cons_sync();
+}
+
+// ---------------------------------------------------------------- ternary matvec phase (one activation row)
+// Same arithmetic as k_matvec_t2<1> (it_matvec_t2.cu): per 32 x 128 tile the exact integer block sums, then the per-block
+// terms (d_w * d_x) * float(S - sum128), which the sum warps add in ascending block order.  A chunk passes through one ring
+// slot: producer -> consumers (a group of four warps) -> sum warp (terms of the slot), whose arrival frees the slot and its
+// terms together.
+__device__ __forceinline__ void matvec_phase(const StepParams& P, Cta& c, const StepSpan& sp) {
+    const int warp = c.warp, lane = c.lane, nb = sp.nb, n = sp.n, hl = sp.hl, whole = sp.n - sp.tl, lead = sp.lead - whole, cpr = sp.cpr;   // in registers: stores to the terms would make the compiler fetch the span again
+    const unsigned magic = sp.magic;
+    const int8_t* xs = reinterpret_cast<const int8_t*>(c.scratch + ST_RED);
+    const float* dxs = reinterpret_cast<const float*>(xs + nb * 128);
+    const int* sss = reinterpret_cast<const int*>(xs + nb * 130);
+    float* terms = reinterpret_cast<float*>(c.scratch + terms_at(nb));
+    const int t = lane & 3, wi = warp % ST_CW;
     const int trow = (lane >> 2) + 8 * t;                            // the matrix row of a tile whose term this lane forms: g + 8 t
     const unsigned smask = (unsigned)P.slots - 1u; const int sshift = 31 - __clz(P.slots);
     // One activation row: integer dot products on the SIMT pipe (dp4a, u8 x s8).  Lane 4 g + t owns the 32 columns
     // 32 t .. 32 t + 31 of a tile and, per 32-bit word, the four matrix rows g, g + 8, g + 16, g + 24 (bit pairs 0..3 of
-    // every byte): masking a word with 0x03030303 << 2 i leaves row g + 8 i's four codes scaled by 4^i.  The four lanes of a
-    // row group g then add their sums (exact integers) in a reduce-scatter that leaves row g + 8 t with lane t, which forms
-    // that row's term.  (At eight activation columns the tensor-core path of it_matvec_t2.cu does this work; at one column
-    // its dependent mma chain costs more latency than these short instructions, and this kernel has 16 warps per SM.)
+    // every byte).  Masks that keep everything up to a bit pair need three operations a word where isolating the pairs needs four;
+    // the differences of the four sums are the rows' sums scaled by 1, 4, 16, 64.  The four lanes of a row group g then add
+    // their sums (exact integers) in a reduce-scatter that leaves row g + 8 t with lane t, which forms that row's term.
     auto dots = [&](const unsigned char* tile, int b, int (&a)[4]) {
         const uint4 wa = *reinterpret_cast<const uint4*>(tile + 16 * lane);
         const uint4 wb = *reinterpret_cast<const uint4*>(tile + 512 + 16 * lane);
@@ -262,12 +577,13 @@ __device__ __forceinline__ void matvec_phase(const StepParams& P, Cta& c, int nb
 #pragma unroll
         for (int k = 0; k < 8; k++) {
             a[0] = dp4a_us(w[k] & 0x03030303u, xb[k], a[0]);
-            a[1] = dp4a_us(w[k] & 0x0c0c0c0cu, xb[k], a[1]);
-            a[2] = dp4a_us(w[k] & 0x30303030u, xb[k], a[2]);
-            a[3] = dp4a_us(w[k] & 0xc0c0c0c0u, xb[k], a[3]);
+            a[1] = dp4a_us(w[k] & 0x0f0f0f0fu, xb[k], a[1]);
+            a[2] = dp4a_us(w[k] & 0x3f3f3f3fu, xb[k], a[2]);
+            a[3] = dp4a_us(w[k], xb[k], a[3]);
         }
+        a[3] -= a[2]; a[2] -= a[1]; a[1] -= a[0];
     };
-    auto term = [&](const unsigned char* tile, int b, const int (&a)[4], float* tbuf) {
+    auto term = [&](const unsigned char* tile, int b, const int (&a)[4]) {
         const bool hi2 = t & 2, hi1 = t & 1;
         int k0 = hi2 ? a[2] : a[0], k1 = hi2 ? a[3] : a[1];
         const int s0 = hi2 ? a[0] : a[2], s1 = hi2 ? a[1] : a[3];
@@ -275,267 +591,309 @@ __device__ __forceinline__ void matvec_phase(const StepParams& P, Cta& c, int nb
         int S = hi1 ? k1 : k0;
         S += __shfl_xor_sync(0xffffffffu, hi1 ? k0 : k1, 1);
         const __half dwh = *reinterpret_cast<const __half*>(tile + 1024 + 2 * lane);   // scale of row g + 8 t: half 4 g + t
-        tbuf[b * 32 + trow] = __fmul_rn(__fmul_rn(__half2float(dwh), dxs[b >> 1]), (float)((S >> (2 * t)) - sss[b]));
+        return __fmul_rn(__fmul_rn(__half2float(dwh), dxs[b >> 1]), (float)((S >> (2 * t)) - sss[b]));
     };
-    unsigned n = c.nseq;
-    for (int rg = blockIdx.x; rg < rgs; rg += gridDim.x, n++) {
-        const unsigned k = n % ST_TB, u = n / ST_TB;
-        float* tbuf = reinterpret_cast<float*>(c.scratch + L.terms) + k * L.plane;
-        // the buffer's previous row group has been added up (the sum warp's arrival number u - 1)
-        if (u && !mbar_wait(c.te + 8 * k, (u - 1) & 1u, c.abort_flag, P.error_flag, 4)) break;
-        for (int cq = (int)((unsigned)(group + ST_NG) - c.q % ST_NG) % ST_NG; cq < cpr; cq += ST_NG) {      // the chunks of this row group that fall to this group
-            const unsigned q = c.q + (unsigned)cq;
-            const int cs = (int)(q & smask); const unsigned cph = (q >> sshift) & 1u;
-            const int b0 = cq * ST_TPC + wi, b1 = b0 + ST_CW;
-            const bool ready = mbar_wait(c.bars + 8 * cs, cph, c.abort_flag, P.error_flag, 3);
-            if (ready && b0 < nb) {
-                const unsigned char* tile0 = c.smem + cs * ST_CHUNK + wi * IT_TILE_BYTES;
-                const unsigned char* tile1 = tile0 + ST_CW * IT_TILE_BYTES;
-                int a0[4], a1[4];
-                if (b1 < nb) {          // warp-uniform
-                    dots(tile0, b0, a0); dots(tile1, b1, a1);
-                    term(tile0, b0, a0, tbuf); term(tile1, b1, a1, tbuf);
-                } else {
-                    dots(tile0, b0, a0); term(tile0, b0, a0, tbuf);
-                }
-            }
-            __syncwarp();
-            if (lane == 0) mbar_arrive(c.bars + 8 * (P.slots + cs));     // the slot may be refilled
-        }
-        c.q += (unsigned)cpr;
+    bool ok = true;                                                  // a lane whose wait ran out goes on without waits and arrivals; the CTA leaves at its next wait
+#pragma unroll 1
+    for (int i = warp / ST_CW; i < n; i += ST_NG) {
+        const unsigned q = c.q + (unsigned)i;
+        const int cs = (int)(q & smask);
+        const unsigned r = (unsigned)(i < hl ? i : i < whole ? i - hl : i + lead);
+        const int b0 = (cpr == 1 ? 0 : (int)(r - __umulhi(r, magic) * (unsigned)cpr)) * ST_TPC + wi, b1 = b0 + ST_CW;      // r modulo cpr: the chunk's index within its row of blocks
+        if (ok) ok = mbar_wait(c.bars + 8 * cs, (q >> sshift) & 1u, c.abort_flag, P.error_flag, 3);
+        const unsigned char *tile0 = c.smem + cs * ST_CHUNK + wi * IT_TILE_BYTES, *tile1 = tile0 + ST_CW * IT_TILE_BYTES;
+        int a0[4], a1[4];
+        dots(tile0, b0, a0); dots(tile1, b1, a1);
+        const float t0 = term(tile0, b0, a0), t1 = term(tile1, b1, a1);
+        float* tb = terms + cs * ST_TERMS + wi * 32 + trow;
+        tb[0] = t0; tb[ST_CW * 32] = t1;
         __syncwarp();
-        if (lane == 0) mbar_arrive(c.tf + 8 * k);                        // this warp's terms of the row group are in place
+        if (lane == 0 && ok) mbar_arrive(c.tf + 8 * cs);
     }
-    c.nseq = n;
-    ST_EV(P, c, c.evt_base + 2);
-    // the phase is over when the sum warps have stored its last results
-    mbar_wait(c.pd, c.mph & 1u, c.abort_flag, P.error_flag, 5);
-    c.mph++;
-    ST_EV(P, c, c.evt_base + 3);
+    c.q += (unsigned)n;
 }
 
-// The sum warps' side of a matvec phase: warp j adds the row groups whose sequence number is j modulo ST_NSUM.
+// The sum warps' side: warp j takes every second row group (in the order of the CTA's chunks), adds its terms in block order
+// and finishes the row: into the residual, through conv and SiLU, through silu(gate) * up, or plainly.
 __device__ __forceinline__ void sum_warps(const StepParams& P, Cta& c) {
-    const int j = c.warp - ST_NCONS, lane = c.lane;
-    float* arena = P.arena;
+    const int jw = c.warp - ST_NCONS, lane = c.lane;
+    float* A = P.arena;
     Pick best{ -INFINITY, 0xffffffffu };
     const int nmat = mat_count(P);
-    unsigned n = 0;
+    const unsigned smask = (unsigned)P.slots - 1u; const int sshift = 31 - __clz(P.slots);
+    const float* xsrc;
+    { const uint32_t tok = (P.flags & 1) ? __float_as_uint(*reinterpret_cast<volatile float*>(A + P.amx)) : *reinterpret_cast<volatile uint32_t*>(P.toks); xsrc = P.tok_embd + (size_t)tok * P.e; }
+    const unsigned base = *reinterpret_cast<volatile unsigned*>(P.sync + 3);
     bool ok = true;
+#pragma unroll 1
     for (int mp = 0; mp < nmat && ok; mp++) {
-        const MatDesc d = mat_desc(P, mp);
-        const MvSmem L = mv_layout(d.nb);
-        const int rgs = (d.rows + 31) / 32;
-        // not before the consumers have entered the phase: a CTA without row groups in a phase would otherwise run through
-        // its phase-done arrivals and leave the consumers waiting on a parity that has come round again
-        if (!mbar_wait(c.ps, (unsigned)mp & 1u, c.abort_flag, P.error_flag, 7)) break;
-        for (int rg = blockIdx.x; rg < rgs; rg += gridDim.x, n++) {
-            if ((int)(n % ST_NSUM) != j) continue;
-            const unsigned k = n % ST_TB, u = n / ST_TB;
-            const int row = rg * 32 + lane;
-            const float old = (d.accum && row < d.rows) ? __ldcg(arena + d.y_off + row) : 0.f;   // on its way while the terms are still being formed
-            if (!mbar_wait(c.tf + 8 * k, u & 1u, c.abort_flag, P.error_flag, 6)) { ok = false; break; }
-            if (row < d.rows) {
-                const float* tcol = reinterpret_cast<const float*>(c.scratch + L.terms) + k * L.plane + lane;
-                float sum = 0.f;
-#pragma unroll 8
-                for (int b = 0; b < d.nb; b++) sum = __fadd_rn(sum, tcol[b * 32]);
-                if (d.accum) sum = __fadd_rn(old, sum);
-                __stcg(arena + d.y_off + row, sum);
-                if (d.pick) best = pick_better(best, Pick{ sum, (unsigned)row });
+        const int il = mp >> 2, sub = mp & 3;
+        const bool head = il >= P.n_layer;
+        const StepLayer& L = P.layers[head ? 0 : il];
+        const StepSpan sp = c.sp[head ? SP_HEAD : span_kind(sub, L.recurrent)];
+        const int rows = head ? P.n_vocab : sub == 0 ? L.in_rows : sub == 2 ? P.ff : P.e;
+        const int n = sp.n, cpu = sp.cpr * sp.parts;
+        const float* terms = reinterpret_cast<const float*>(c.scratch + terms_at(sp.nb));
+        const bool gdn_in = !head && sub == 0 && L.recurrent, accum = !head && (sub & 1);
+        const int ph = head || sub == 0 ? PH_B : sub == 1 ? PH_E : sub == 2 ? PH_G : PH_I;
+        const unsigned tag = tag_of(base, il, ph);
+        granule* y = sub == 0 ? P.rows : sub == 1 ? P.xe : sub == 2 ? P.act : P.xi;
+        // where the residual row comes from: the down projection of the layer before, or this layer's output projection
+        const granule* yo = sub == 1 ? P.xi : P.xe; const unsigned old_tag = sub == 1 ? tag_of(base, il - 1, PH_I) : tag_of(base, il, PH_E);
+        // not before the consumers have passed the barrier in front of this phase: an arrival of a warp without row groups
+        // would count for the wrong barrier
+        if (!mbar_wait_warp(c.ps, (unsigned)mp & 1u, c.abort_flag, P.error_flag, 7)) break;
+        const int drow = (int)gridDim.x - 1 - (int)blockIdx.x;
+        if (gdn_in && jw == 1 && drow < 2 * P.nv) {
+            // the dense row of this CTA: beta (sigmoid) or alpha (decay) gate of a value head
+            if (!mbar_wait_warp(c.dn, (unsigned)(c.att_seq++) & 1u, c.abort_flag, P.error_flag, 12)) break;
+            if (lane == 0) {
+                const double* ws = reinterpret_cast<const double*>(c.scratch);
+                double tt = ws[0];
+                for (int k = 1; k < 8; k++) tt += ws[k];
+                const float tf = (float)tt;
+                const int h = drow % P.nv;
+                st_tagged(P.gate + drow, drow < P.nv ? it_sigmoid(tf) : it_expf(it_mul(it_softplus(it_add(tf, L.dt[h])), L.a[h])), tag);
             }
             __syncwarp();
-            if (lane == 0) mbar_arrive(c.te + 8 * k);
         }
-        if (d.pick) {       // greedy pick (first index of the maximum) over this warp's rows, left behind the layer descriptions
+        int unit = sp.uf;
+#pragma unroll 1
+        for (int i = 0, ord = 0, len; i < n; i += len, ord++) {
+            const bool first = i < sp.hl, last = !first && i >= n - sp.tl;       // begun here and finished by the next CTA / the other way round
+            len = first ? sp.hl : last ? sp.tl : cpu;
+            const int u = first ? sp.uh : last ? sp.ut : unit++;
+            if ((ord & 1) != jw) continue;
+            const int row = u * 32 + lane;
+            const bool live = row < rows;
+            float s = 0.f, sg = 0.f, old = 0.f;
+            float st[3]; float4 cw;                                  // the usual conv size, four taps: operands on their way while the terms are added
+            const bool conv = gdn_in && row < P.cd && !first;
+            if (accum && live && !first) {
+                if (sub == 1 && il == 0) old = xsrc[row];
+                else { const int k = lane / ST_GPU; const granule og = wait_granule(yo + (size_t)u * ST_GPU + lane - k * ST_GPU, old_tag, c.abort_flag, P.error_flag, 16); old = __uint_as_float(k == 0 ? og.x : k == 1 ? og.y : og.z); }
+            }
+            if (conv && P.conv_k == 4) {
+#pragma unroll
+                for (int k = 0; k < 3; k++) st[k] = L.conv_st[(size_t)k * P.cd + row];
+                cw = *reinterpret_cast<const float4*>(L.conv_w + (size_t)row * 4);
+            }
+            const int turn = last ? sp.cpr - sp.lead : sp.cpr;       // never reached when there is one matrix
+            if (last) {
+                // running sums of the blocks the CTA before has added (it does them first)
+                const granule a = wait_granule(P.prefix + (size_t)(blockIdx.x - 1) * 32 + lane, tag, c.abort_flag, P.error_flag, 13);
+                s = __uint_as_float(a.x); sg = __uint_as_float(a.y);
+            }
+            // a lane whose wait ran out goes on without waits; the warp leaves by a vote after the row group
+            unsigned q = c.q + (unsigned)i;
+#pragma unroll 1
+            for (int k = 0; k < len; k += 2, q += 2) {               // two chunks a turn: this warp has one issue slot in four, and half a turn is overhead
+                const int c0 = (int)(q & smask), c1 = (int)((q + 1) & smask);
+                const bool two = k + 1 < len;
+                if (ok) ok = mbar_wait(c.tf + 8 * c0, (q >> sshift) & 1u, c.abort_flag, P.error_flag, 6);
+                if (ok && two) ok = mbar_wait(c.tf + 8 * c1, ((q + 1) >> sshift) & 1u, c.abort_flag, P.error_flag, 6);
+                const float *t0 = terms + c0 * ST_TERMS + lane, *t1 = terms + c1 * ST_TERMS + lane;
+                float ta[ST_TPC], tb[ST_TPC];
+#pragma unroll
+                for (int b = 0; b < ST_TPC; b++) ta[b] = t0[32 * b];
+#pragma unroll
+                for (int b = 0; b < ST_TPC; b++) tb[b] = two ? t1[32 * b] : 0.f;      // + 0 changes no sum
+                if (k == turn) { sg = s; s = 0.f; }                  // second matrix of the pair
+#pragma unroll
+                for (int b = 0; b < ST_TPC; b++) s = __fadd_rn(s, ta[b]);
+                if (k + 1 == turn && two) { sg = s; s = 0.f; }
+#pragma unroll
+                for (int b = 0; b < ST_TPC; b++) s = __fadd_rn(s, tb[b]);
+                __syncwarp();
+                if (lane < (two ? 2 : 1) && ok) mbar_arrive(c.bars + 8 * (P.slots + (lane ? c1 : c0)));     // the slots may be refilled, their terms overwritten
+            }
+            ok = __all_sync(0xffffffffu, ok);
+            if (!ok) break;
+            if (first) {
+                st_granule(P.prefix + (size_t)blockIdx.x * 32 + lane, __float_as_uint(s), __float_as_uint(sg), 0u, tag);
+                continue;
+            }
+            if (accum) {
+                s = __fadd_rn(old, s);
+            } else if (sp.parts == 2 || gdn_in) {
+                if (conv) {
+                    // conv over the row's last inputs (taps in order) and the state's shift by one input
+                    const float mx = s;
+                    if (P.conv_k == 4) {
+                        s = it_add(it_add(it_add(it_add(0.f, it_mul(st[0], cw.x)), it_mul(st[1], cw.y)), it_mul(st[2], cw.z)), it_mul(mx, cw.w));
+                        L.conv_st[row] = st[1]; L.conv_st[(size_t)P.cd + row] = st[2]; L.conv_st[2 * (size_t)P.cd + row] = mx;
+                    } else {
+                        s = 0.f;
+#pragma unroll 1
+                        for (int k = 0; k < P.conv_k; k++) {
+                            float* at = L.conv_st + (size_t)k * P.cd + row;
+                            const float x = k < P.conv_k - 1 ? *at : mx;
+                            s = it_add(s, it_mul(x, L.conv_w[(size_t)row * P.conv_k + k]));
+                            if (k) at[-(ptrdiff_t)P.cd] = x;
+                        }
+                    }
+                }
+                // silu(gate) * up; silu of a conv channel, or of a gate row behind them
+                const float a = sp.parts == 2 ? sg : s, sl = __fdiv_rn(a, it_add(1.0f, it_expf_inline(-a)));
+                s = sp.parts == 2 ? it_mul(sl, s) : sl;
+            }
+            if (head) { if (live) { __stcg(A + P.logits + row, s); best = pick_better(best, Pick{ s, (unsigned)row }); } }
+            else {
+                publish(y, u, lane, s, tag);
+            }
+        }
+        c.q += (unsigned)n;
+        if (!ok) break;
+        if (head) {         // greedy pick (first index of the maximum) over this warp's rows
 #pragma unroll
             for (unsigned mm = 16; mm > 0; mm >>= 1) { Pick o{ __shfl_xor_sync(0xffffffffu, best.v, mm), __shfl_xor_sync(0xffffffffu, best.i, mm) }; best = pick_better(best, o); }
-            if (lane == 0) reinterpret_cast<Pick*>(const_cast<StepLayer*>(c.lay) + 2)[j] = best;
+            if (lane == 0) st_granule(P.partials + blockIdx.x * ST_NSUM + jw, __float_as_uint(best.v), best.i, 0u, tag);
         }
         __syncwarp();
-        if (lane == 0) mbar_arrive(c.pd);
+        if (lane == 0) mbar_arrive(c.pd);                            // this phase's terms have been read
     }
+    if (ok && lane == 0) grid_arrive(P);
 }
 
 // ---------------------------------------------------------------- delta-net block of one value head
-// conv + SiLU (+ l2norm of the q and k runs), the dense beta / alpha rows, the delta rule and the gated norm for head
-// blockIdx.x, in the operation order of k_conv_l2_dense and k_gdn_norm (it_support.cu; src/cpu.rs:199-237).  The q / k
-// runs of a key group are recomputed by each of the value heads that share it.  The new conv state of the runs this CTA
-// is responsible for (its own v run; the q and k runs when it is the first head of the group) is returned in `keep`
-// and stored after the next grid barrier, when no CTA reads the old state any more.
-struct ConvKeep { int ch; float mx; };    // a conv channel whose state this thread shifts after the next barrier, and this step's input of that channel
+// l2norm of q and k, the delta rule and the gated norm for head blockIdx.x, in the operation order of k_conv_l2_dense and
+// k_gdn_norm (it_support.cu; src/cpu.rs:199-237); conv, SiLU and the gates come from the input projection's phase.
 // Issued by the CTA of value head blockIdx.x while the input projection runs: the head's state tile (64 KB, it does not
-// depend on this step's activations) into its place in shared memory, and the head's beta / alpha rows into L2.
+// depend on this step's activations) into its place in shared memory.
 __device__ __forceinline__ void gdn_prefetch(const StepParams& P, const StepLayer& L, const Cta& c, int h) {
     constexpr int SD = ST_SD, PPR = SD / 4;
-    const int tid = c.tid;
     float* tile = reinterpret_cast<float*>(c.scratch + P.gdn_off);
     const float4* m = reinterpret_cast<const float4*>(L.ssm_st + (size_t)h * SD * SD);
-    for (int f = tid; f < SD * PPR; f += ST_CT) { const int j = f / PPR, cc = f % PPR; cp_async16(tile + j * SD + ((cc ^ (j & 7)) << 2), m + f); }
+#pragma unroll 1
+    for (int f = c.tid; f < SD * PPR; f += ST_CT) { const int j = f / PPR, cc = f % PPR; cp_async16(tile + j * SD + ((cc ^ (j & 7)) << 2), m + f); }
     asm volatile("cp.async.commit_group;" ::: "memory");
-    const int lines = P.e * 4 / 128;
-    for (int i = tid; i < 2 * lines; i += ST_CT) {
-        const float* row = (i < lines ? L.beta : L.alpha) + (size_t)h * P.e + (size_t)(i % lines) * 32;
-        asm volatile("prefetch.global.L2 [%0];" :: "l"(row));
-    }
 }
-__device__ __forceinline__ void gdn_phase(const StepParams& P, const StepLayer& L, const Cta& c, ConvKeep& keep, int h) {
+// sum of a[i] * b[i] in index order (one lane); n a multiple of 16, both 16-byte aligned
+__device__ __noinline__ float chain_dot(const float* a, const float* b, int n) {
+    float s = 0.f;
+    float4 x[4], y[4];
+#pragma unroll
+    for (int u = 0; u < 4; u++) { x[u] = *reinterpret_cast<const float4*>(a + 4 * u); y[u] = *reinterpret_cast<const float4*>(b + 4 * u); }
+#pragma unroll 1
+    for (int i = 16; i <= n; i += 16) {
+        float p[16];                                             // this run's products; the next run on its way while they are added
+#pragma unroll
+        for (int u = 0; u < 4; u++) { p[4 * u] = it_mul(x[u].x, y[u].x); p[4 * u + 1] = it_mul(x[u].y, y[u].y); p[4 * u + 2] = it_mul(x[u].z, y[u].z); p[4 * u + 3] = it_mul(x[u].w, y[u].w); }
+        const int at = i < n ? i : 0;
+#pragma unroll
+        for (int u = 0; u < 4; u++) { x[u] = *reinterpret_cast<const float4*>(a + at + 4 * u); y[u] = *reinterpret_cast<const float4*>(b + at + 4 * u); }
+#pragma unroll
+        for (int u = 0; u < 16; u++) s = it_add(s, p[u]);
+    }
+    return s;
+}
+__device__ __forceinline__ void gdn_phase(const StepParams& P, const StepLayer& L, const Cta& c, int h, int il) {
     constexpr int SD = ST_SD, PPR = SD / 4;
-    const int tid = c.tid, warp = c.warp, lane = c.lane, kh = h % P.nk, kk = P.conv_k, cd = P.cd;
+    const int tid = c.tid, warp = c.warp, lane = c.lane, kh = h % P.nk;
     float* tile = reinterpret_cast<float*>(c.scratch + P.gdn_off);   // [SD][SD], 16-byte pieces of row j stored at piece index ^ (j & 7); requested by gdn_prefetch
-    float* vals = tile + SD * SD;                                    // [3][SD]: q, k, v runs after conv + SiLU
-    float* os = vals + 3 * SD;                                       // [SD] delta-rule outputs
-    float* scs = os + SD;                                            // [2] l2norm scales, [2] beta, alpha, [2] sigmoid(beta), exp(decay)
-    double* wsum = reinterpret_cast<double*>(scs + 8);               // [16] warp sums of the two dense rows
-    float* gzs = reinterpret_cast<float*>(wsum + 16);                // [SD] silu of the head's gate row
-    const float* A = P.arena;
+    float* qs = reinterpret_cast<float*>(c.scratch);                 // [SD] q, [SD] k
+    float* ks = qs + SD;
+    float* dl = ks + SD;                                             // [SD] deltas
+    float* os = dl + SD;                                             // [SD] delta-rule outputs
+    float* scs = os + SD;                                            // [2] l2norm scales, [2] beta, decay
+    float* raw = scs + 4;                                            // [4][SD] the head's q, k, v and gate rows
     auto piece = [&](int j, int cc) { return reinterpret_cast<float4*>(tile + j * SD + ((cc ^ (j & 7)) << 2)); };
     float* m = L.ssm_st + (size_t)h * SD * SD;
-    keep.ch = -1;
-    // dense rows: warps 0-7 beta row h, warps 8-15 alpha row h, in the order of k_dense_rows (thread i of 256 adds the products
-    // i, i + 256, ... in f64).  The first sixteen products' operands are requested before anything else so that their
-    // latency overlaps the conv; the gate values the norm needs at the very end are requested here too.
-    // sixteen virtual warps (0-7: beta row h, 8-15: alpha row h) on the CTA's consumer warps; virtual thread i of a row's
-    // 256 adds the products i, i + 256, ... in f64 (the order of k_dense_rows)
-    const float* xr = A + P.xn;
-    float wv[16], xv[16];
-    {
-        const int t8 = (warp & 7) * 32 + lane; const float* wr = (warp >= 8 ? L.alpha : L.beta) + (size_t)h * P.e;
-#pragma unroll
-        for (int k = 0; k < 16; k++) { const int i = t8 + 256 * k; wv[k] = i < P.e ? wr[i] : 0.f; xv[k] = i < P.e ? __ldcg(xr + i) : 0.f; }
-    }
-    // the gate values the norm needs at the very end: warp 0 keeps the norm weights, warp 8 (done early with its share of
-    // the dense rows) forms silu(z) while the other warps are still busy
-    float zr[SD / 32], nwr[SD / 32];
+    const unsigned tag = tag_of(c.base, il, PH_B);
+    constexpr int GH = SD / 32 * ST_GPU;                             // granules of a run of SD rows
+    static_assert(4 * GH <= ST_CT, "one granule a thread");
+    if (tid < 4 * GH) {
+        const int r = tid / GH, first = r == 0 ? kh * SD : r == 1 ? P.qk + kh * SD : r == 2 ? 2 * P.qk + h * SD : P.cd + h * SD;
+        const granule* gp = P.rows + (size_t)(first / 32) * ST_GPU + (tid - r * GH);
+        const granule g = wait_granule(gp, tag, c.abort_flag, P.error_flag, 17);
+        bool two; float* at = raw + r * SD + granule_row(tid - r * GH, two);
+        at[0] = __uint_as_float(g.x); at[ST_GPU] = __uint_as_float(g.y); if (!two) at[2 * ST_GPU] = __uint_as_float(g.z);
+    } else if (tid >= ST_CT - 2) scs[2 + tid - (ST_CT - 2)] = ld_tagged(P.gate + (tid - (ST_CT - 2)) * P.nv + h, tag, c.abort_flag, P.error_flag, 18);
+    float nw[SD / 32];
     if (warp == 0) {
 #pragma unroll
-        for (int i = 0; i < SD / 32; i++) nwr[i] = L.ssm_norm[lane + 32 * i];
+        for (int i = 0; i < SD / 32; i++) nw[i] = L.ssm_norm[lane + 32 * i];
     }
-    if (warp == 8) {
-#pragma unroll
-        for (int i = 0; i < SD / 32; i++) zr[i] = __ldcg(A + P.big1 + cd + h * SD + lane + 32 * i);
-    }
-    if (tid < 3 * SD) {
-        const int r = tid / SD, cc = tid % SD;
-        const int ch = (r == 0 ? kh * SD : r == 1 ? P.qk + kh * SD : 2 * P.qk + h * SD) + cc;
-        float st[8], cw[8];                                          // kk <= 8 taps: fixed-size loops keep these in registers
-#pragma unroll
-        for (int i = 0; i < 8; i++) { st[i] = i < kk - 1 ? L.conv_st[(size_t)i * cd + ch] : 0.f; cw[i] = i < kk ? L.conv_w[ch * kk + i] : 0.f; }
-        const float mx = __ldcg(A + P.big1 + ch);
-        float s = 0.f;
-#pragma unroll
-        for (int i = 0; i < 8; i++) if (i < kk) s = it_add(s, it_mul(i < kk - 1 ? st[i] : mx, cw[i]));
-        vals[r * SD + cc] = it_silu(s);
-        if (r == 2 || h < P.nk) { keep.ch = ch; keep.mx = mx; }
-    }
-    ST_EV(P, c, c.evt_base + 5);
-    for (int vw = warp; vw < 16; vw += ST_NCONS) {
-        const int t8 = (vw & 7) * 32 + lane; const float* wr = (vw >= 8 ? L.alpha : L.beta) + (size_t)h * P.e;
-        double s = 0.0;
-#pragma unroll 1
-        for (int base = 0; base < P.e; base += 16 * 256) {            // one copy of the load and of the add block: the first block of the warp's own row is already in registers
-            if (vw != warp || base) {
-#pragma unroll
-                for (int k = 0; k < 16; k++) { const int i = base + t8 + 256 * k; wv[k] = i < P.e ? wr[i] : 0.f; xv[k] = i < P.e ? __ldcg(xr + i) : 0.f; }
-            }
-#pragma unroll
-            for (int k = 0; k < 16; k++) if (base + t8 + 256 * k < P.e) s += (double)it_mul(wv[k], xv[k]);
-        }
-#pragma unroll
-        for (int mm = 16; mm >= 1; mm >>= 1) s += __shfl_xor_sync(0xffffffffu, s, mm);
-        if (lane == 0) wsum[vw] = s;
-    }
-    ST_EV(P, c, c.evt_base + 6);
-    cons_sync();
-    if (lane == 0 && warp < 2) {                                     // l2norm of the q run (warp 0) and the k run (warp 1): squares in index order
-        const float* v = vals + warp * SD;
-        float s = 0.f;
-#pragma unroll 8
-        for (int i = 0; i < SD; i++) s = it_add(s, it_mul(v[i], v[i]));
-        scs[warp] = it_div(1.0f, fmaxf(it_sqrt(s), P.eps));
-    } else if (lane == 0 && warp < 4) {
-        const double* ws = wsum + (warp - 2) * 8;
-        double tt = ws[0];
-        for (int k = 1; k < 8; k++) tt += ws[k];
-        const float tf = (float)tt;                                  // warp 2: beta, warp 3: alpha; the gates follow at once, off the owners' path
-        scs[warp] = tf;
-        if (warp == 2) scs[4] = it_sigmoid(tf);
-        else scs[5] = it_expf(it_mul(it_softplus(it_add(tf, L.dt[h])), L.a[h]));
-    } else if (warp == 8) {
-#pragma unroll
-        for (int i = 0; i < SD / 32; i++) gzs[lane + 32 * i] = it_silu(zr[i]);
-    }
-    ST_EV(P, c, c.evt_base + 7);
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     cons_sync();
-    ST_EV(P, c, c.evt_base + 8);
+    const float q = raw[tid & (SD - 1)], k = raw[SD + (tid & (SD - 1))], v = raw[2 * SD + (tid & (SD - 1))], bt = scs[2], eg = scs[3];
+    if (warp >= 4 && warp < 6 && lane == 0) { const float* r = raw + (warp - 4) * SD; scs[warp - 4] = __fdiv_rn(1.0f, fmaxf(__fsqrt_rn(chain_dot(r, r, SD)), P.eps)); }
+    if (warp < 6) asm volatile("bar.sync 3, 192;" ::: "memory");
     if (tid < SD) {
-        const float q = it_mul(vals[tid], scs[0]), k = it_mul(vals[SD + tid], scs[1]);
-        asm volatile("bar.sync 3, %0;" :: "n"(SD) : "memory");       // every owner has read the raw q / k values
-        vals[tid] = q; vals[SD + tid] = k;
-        asm volatile("bar.sync 3, %0;" :: "n"(SD) : "memory");
-        const float* qs = vals; const float* ks = vals + SD;
-        const float v = vals[2 * SD + tid];
-        const float bt = scs[4];
-        const float eg = scs[5];
+        qs[tid] = it_mul(q, scs[0]); ks[tid] = it_mul(k, scs[1]);
+        asm volatile("bar.sync 2, 128;" ::: "memory");
         const float scale = c.inv_sqrt_sd;
-        // Two passes over the thread's state row, eight 16-byte pieces at a time (requested together, then used in order).
-        // The first pass only reads: s = sum_i (row[i] * eg) * k[i] in index order.  The second forms row[i] * eg again (the
-        // same rounded product), adds k[i] * delta, stores the new state and accumulates the output in index order.
+        // Two passes over the thread's state row.  The first: s = sum_i (row[i] * eg) * k[i] in index order.  The second forms the new
+        // row, row[i] * eg (the same rounded product) + k[i] * delta, and adds the output in index order.  Four 16-byte pieces at a
+        // time; while their products are added (the chain), the next four and their factors are on their way.  The rows' stores
+        // are the other warps' work (below), after the output: beside the second pass and the norm they cost 2000 cycles.
         float s = 0.f;
+        {
+            float4 r[4], kk[4];
+#pragma unroll
+            for (int u = 0; u < 4; u++) { r[u] = *piece(tid, u); kk[u] = *reinterpret_cast<const float4*>(ks + 4 * u); }
 #pragma unroll 1
-        for (int c0 = 0; c0 < PPR; c0 += 8) {
-            float4 rr[8];
+            for (int c0 = 4; c0 <= PPR; c0 += 4) {
+                float p[16];
 #pragma unroll
-            for (int u = 0; u < 8; u++) rr[u] = *piece(tid, c0 + u);
+                for (int u = 0; u < 4; u++) {
+                    p[4 * u] = it_mul(it_mul(r[u].x, eg), kk[u].x); p[4 * u + 1] = it_mul(it_mul(r[u].y, eg), kk[u].y);
+                    p[4 * u + 2] = it_mul(it_mul(r[u].z, eg), kk[u].z); p[4 * u + 3] = it_mul(it_mul(r[u].w, eg), kk[u].w);
+                }
+                const int at = c0 & (PPR - 1);
 #pragma unroll
-            for (int u = 0; u < 8; u++) {
-                const float4 k4 = *reinterpret_cast<const float4*>(ks + 4 * (c0 + u));
-                s = it_add(s, it_mul(it_mul(rr[u].x, eg), k4.x)); s = it_add(s, it_mul(it_mul(rr[u].y, eg), k4.y));
-                s = it_add(s, it_mul(it_mul(rr[u].z, eg), k4.z)); s = it_add(s, it_mul(it_mul(rr[u].w, eg), k4.w));
+                for (int u = 0; u < 4; u++) { r[u] = *piece(tid, at + u); kk[u] = *reinterpret_cast<const float4*>(ks + 4 * (at + u)); }
+#pragma unroll
+                for (int u = 0; u < 16; u++) s = it_add(s, p[u]);
             }
         }
         const float delta = it_mul(it_sub(v, s), bt);
+        dl[tid] = delta;
         float acc = 0.f;
+        {
+            float4 r[4], kk[4], qq[4];
+#pragma unroll
+            for (int u = 0; u < 4; u++) { r[u] = *piece(tid, u); kk[u] = *reinterpret_cast<const float4*>(ks + 4 * u); qq[u] = *reinterpret_cast<const float4*>(qs + 4 * u); }
 #pragma unroll 1
-        for (int c0 = 0; c0 < PPR; c0 += 8) {
-            float4 rr[8];
+            for (int c0 = 4; c0 <= PPR; c0 += 4) {
+                float p[16];
 #pragma unroll
-            for (int u = 0; u < 8; u++) rr[u] = *piece(tid, c0 + u);
+                for (int u = 0; u < 4; u++) {
+                    p[4 * u] = it_mul(it_add(it_mul(r[u].x, eg), it_mul(kk[u].x, delta)), qq[u].x); p[4 * u + 1] = it_mul(it_add(it_mul(r[u].y, eg), it_mul(kk[u].y, delta)), qq[u].y);
+                    p[4 * u + 2] = it_mul(it_add(it_mul(r[u].z, eg), it_mul(kk[u].z, delta)), qq[u].z); p[4 * u + 3] = it_mul(it_add(it_mul(r[u].w, eg), it_mul(kk[u].w, delta)), qq[u].w);
+                }
+                const int at = c0 & (PPR - 1);
 #pragma unroll
-            for (int u = 0; u < 8; u++) {
-                const float4 k4 = *reinterpret_cast<const float4*>(ks + 4 * (c0 + u)), q4 = *reinterpret_cast<const float4*>(qs + 4 * (c0 + u));
-                float4 r;
-                r.x = it_add(it_mul(rr[u].x, eg), it_mul(k4.x, delta)); r.y = it_add(it_mul(rr[u].y, eg), it_mul(k4.y, delta));
-                r.z = it_add(it_mul(rr[u].z, eg), it_mul(k4.z, delta)); r.w = it_add(it_mul(rr[u].w, eg), it_mul(k4.w, delta));
-                *piece(tid, c0 + u) = r;
-                acc = it_add(acc, it_mul(r.x, q4.x)); acc = it_add(acc, it_mul(r.y, q4.y)); acc = it_add(acc, it_mul(r.z, q4.z)); acc = it_add(acc, it_mul(r.w, q4.w));
+                for (int u = 0; u < 4; u++) { r[u] = *piece(tid, at + u); kk[u] = *reinterpret_cast<const float4*>(ks + 4 * (at + u)); qq[u] = *reinterpret_cast<const float4*>(qs + 4 * (at + u)); }
+#pragma unroll
+                for (int u = 0; u < 16; u++) acc = it_add(acc, p[u]);
             }
         }
         os[tid] = it_mul(acc, scale);
+        asm volatile("bar.sync 2, 128;" ::: "memory");
+        if (warp > 0) asm volatile("bar.arrive 6, 384;" ::: "memory");
+    } else {
+        // the new state to global memory, a 16-byte piece a thread at a time (coalesced), once the head's output is out
+        asm volatile("bar.sync 6, 384;" ::: "memory");
+#pragma unroll 2
+        for (int f = tid - SD; f < SD * PPR; f += ST_CT - SD) {
+            const int j = f / PPR, cc = f % PPR;
+            const float4 o = *piece(j, cc), k4 = *reinterpret_cast<const float4*>(ks + 4 * cc);
+            const float delta = dl[j];
+            reinterpret_cast<float4*>(m)[f] = make_float4(it_add(it_mul(o.x, eg), it_mul(k4.x, delta)), it_add(it_mul(o.y, eg), it_mul(k4.y, delta)), it_add(it_mul(o.z, eg), it_mul(k4.z, delta)), it_add(it_mul(o.w, eg), it_mul(k4.w, delta)));
+        }
     }
-    ST_EV(P, c, c.evt_base + 9);
-    cons_sync();
-    ST_EV(P, c, c.evt_base + 10);
-    // the new state back to global memory (coalesced 16-byte stores by warps 1..15) while warp 0 norms the outputs
-    if (warp > 0) for (int f = tid - 32; f < SD * PPR; f += ST_CT - 32) reinterpret_cast<float4*>(m)[f] = *piece(f / PPR, f % PPR);
     if (warp == 0) {
         float sc = 0.f;
-        if (lane == 0) {
-            float s = 0.f;
-#pragma unroll 8
-            for (int i = 0; i < SD; i++) s = it_add(s, it_mul(os[i], os[i]));
-            sc = it_div(1.0f, it_sqrt(it_add(it_div(s, (float)SD), P.eps)));
-        }
+        if (lane == 0) sc = __fdiv_rn(1.0f, __fsqrt_rn(it_add(__fdiv_rn(chain_dot(os, os, SD), (float)SD), P.eps)));
         sc = __shfl_sync(0xffffffffu, sc, 0);
-        float* o = P.arena + P.o + h * SD;                           // zr: the gate rows, which follow the qkv rows in the stacked output
+        // the output projection's columns may be grouped [rep][key head] where value heads are [key head][rep]
+        const int u0 = (P.v_grouped ? h / P.nk + P.nv / P.nk * kh : h) * (SD / 32);
+        const unsigned otag = tag_of(c.base, il, PH_C);
 #pragma unroll
-        for (int i = 0; i < SD / 32; i++) {
-            const int j = lane + 32 * i;
-            __stcg(o + j, it_mul(it_mul(it_mul(os[j], sc), nwr[i]), gzs[j]));
-        }
+        for (int i = 0; i < SD / 32; i++) { const int j = lane + 32 * i; publish(P.o, u0 + i, lane, it_mul(it_mul(it_mul(os[j], sc), nw[i]), raw[3 * SD + j]), otag); }
+        asm volatile("bar.arrive 6, 384;" ::: "memory");             // the other warps may form the new rows
     }
-    ST_EV(P, c, c.evt_base + 11);
 }
 
 // ---------------------------------------------------------------- attention block of one head
@@ -560,14 +918,14 @@ __device__ __forceinline__ void attn_prefetch(const StepParams& P, const StepLay
         asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" :: "l"(L.vc + it_vc_index((size_t)i * 32, kh, 0, P.nkv, P.hd)), "r"(bytes) : "memory");
 }
 constexpr int ST_AT_MAXS = 8, ST_AT_LOADER = ST_NCONS - 1, ST_AT_T = (ST_NCONS - 1) * 32;
-// the block's own barrier: every consumer warp but the loader, which runs ahead and only joins the grid barrier
+// the block's own barrier: every consumer warp but the loader, which runs ahead and only joins the next phase
 __device__ __forceinline__ void at_sync() { asm volatile("bar.sync 4, %0;" :: "n"(ST_AT_T) : "memory"); }
 // G = P.attn_g CTAs share a head (hg = G h + g).  Each forms q and the new position's k and v for itself, scores the K
 // tiles i with i % G == g, publishes those scores, meets the head's other CTAs at a counter of their own, reads their
 // scores, runs the softmax for itself (one thread adds the exponentials in position order) and accumulates the
 // head_dim / G output elements [g head_dim / G, ...) over all positions from row slices of the V tiles.  A single SM can
 // keep only so many bytes in flight, so a head's cache traffic is spread over G SMs.
-__device__ __forceinline__ void attn_phase(const StepParams& P, const StepLayer& L, Cta& c, int hg) {
+__device__ __forceinline__ void attn_phase(const StepParams& P, const StepLayer& L, Cta& c, int hg, int il) {
     const int tid = c.tid, warp = c.warp, lane = c.lane, hd = P.hd, nkv = P.nkv, kvd = nkv * hd;
     const int G = P.attn_g, h = hg / G, g = hg % G, epc = hd / G;   // elements of the output this CTA owns
     const int vs = it_vc_slice(hd);                                  // elements per V slice: epc is a multiple of it
@@ -582,7 +940,8 @@ __device__ __forceinline__ void attn_phase(const StepParams& P, const StepLayer&
     float* qs = sc + ((n + 3) & ~3);                                 // [hd] q head after norm + rope
     float* kl = qs + hd;                                             // [hd] k row of the new position as the cache holds it
     float* vl = kl + hd;                                             // [hd] v row of the new position as the cache holds it
-    float* red = vl + hd;                                            // [32] + the sum
+    float* gs = vl + hd;                                             // [hd] gate row of the head
+    float* red = gs + hd;                                            // [32] + the sum
     unsigned char* ring = reinterpret_cast<unsigned char*>(red + 48) + ((128u - (smem_u32(red + 48) & 127u)) & 127u);
     const int room = (int)((c.scratch + P.scratch) - ring);
     // K: tile j of this CTA goes to slot j % S and is scored by warp j % S, so every slot is filled and emptied by the same two
@@ -599,10 +958,18 @@ __device__ __forceinline__ void attn_phase(const StepParams& P, const StepLayer&
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     ST_EV(P, c, c.evt_base + 4);
+    {   // the head's q and gate rows (adjacent in the stacked output, and here with k, v between them) and the KV head's k and v rows
+        const unsigned tag = tag_of(c.base, il, PH_B);
+        const int gh = hd / 32 * ST_GPU, r = tid / gh;                // granules of hd rows; hd <= 256: four parts of at most 88
+        if (r < 4) {
+            const int first = r < 2 ? (2 * h + r) * hd : P.nh * 2 * hd + (r - 2) * kvd + kh * hd;
+            const granule g = wait_granule(P.rows + (size_t)(first / 32) * ST_GPU + (tid - r * gh), tag, c.abort_flag, P.error_flag, 17);
+            bool two; float* at = (r == 0 ? qs : r == 1 ? gs : r == 2 ? kl : vl) + granule_row(tid - r * gh, two);
+            at[0] = __uint_as_float(g.x); at[ST_GPU] = __uint_as_float(g.y); if (!two) at[2 * ST_GPU] = __uint_as_float(g.z);
+        }
+    }
     cons_sync();                                                     // all twelve warps, the loader included
     ST_EV(P, c, c.evt_base + 5);
-    const float* row = P.arena + P.big1;
-    const float* qh = row + (size_t)h * 2 * hd; const float* gate = qh + hd;
     const __half* kc = L.kc; const __half* vc = L.vc;
 
     if (warp == ST_AT_LOADER) {
@@ -630,23 +997,17 @@ __device__ __forceinline__ void attn_phase(const StepParams& P, const StepLayer&
                 bulk_load(smem_u32(ring + sl * vslot_bytes), vc + it_vc_index((size_t)i * 32, kh, g * epc, nkv, hd), (unsigned)vslot_bytes, vf + 8 * sl);
             }
         }
-        return;                                                      // the loader meets the others at the grid barrier
+        return;                                                      // the loader meets the others at the next phase
     }
     if (warp < 2) {
         // warp 0: q head; warp 1: k head.  rmsnorm with the squares added by one lane in index order, weight, rope.
         float* buf = warp == 0 ? qs : kl;
-        const float* x = warp == 0 ? qh : row + (size_t)P.nh * 2 * hd + kh * hd;
         const float* w = warp == 0 ? L.q_norm : L.k_norm;
         float wr[8];                                                  // hd <= 256: the norm weights are requested before the sum needs time
 #pragma unroll
         for (int k = 0; k < 8; k++) wr[k] = lane + 32 * k < hd ? w[lane + 32 * k] : 0.f;
-        for (int i = lane; i < hd; i += 32) buf[i] = __ldcg(x + i);
-        __syncwarp();
         float s = 0.f;
-        if (lane == 0) {
-#pragma unroll 16
-            for (int i = 0; i < hd; i++) s = it_add(s, it_mul(buf[i], buf[i]));
-        }
+        if (lane == 0) s = chain_dot(buf, buf, hd);
         s = __shfl_sync(0xffffffffu, s, 0);
         const float scl = it_div(1.0f, it_sqrt(it_add(it_div(s, (float)hd), P.eps)));
 #pragma unroll
@@ -671,9 +1032,8 @@ __device__ __forceinline__ void attn_phase(const StepParams& P, const StepLayer&
             buf[i] = __half2float(hv);
         }
     } else if (warp == 2) {
-        const float* v = row + (size_t)P.nh * 2 * hd + kvd + kh * hd;
         for (int i = lane; i < hd; i += 32) {
-            const __half hv = __float2half_rn(__ldcg(v + i));
+            const __half hv = __float2half_rn(vl[i]);
             if (writer) const_cast<__half*>(vc)[it_vc_index(pos, kh, i, nkv, hd)] = hv;
             vl[i] = __half2float(hv);
         }
@@ -682,7 +1042,8 @@ __device__ __forceinline__ void attn_phase(const StepParams& P, const StepLayer&
     ST_EV(P, c, c.evt_base + 6);
     const float scale = c.inv_sqrt_hd;
     const int nvec = hd / 8;
-    float* shared_sc = P.att_sc + (size_t)h * P.att_stride;          // the head's scores, where its CTAs leave theirs for one another
+    unsigned long long* shared_sc = P.att_sc + (size_t)h * P.att_stride;      // the head's scores, where its CTAs leave theirs for one another
+    const unsigned sc_tag = tag_of(c.base, il, PH_C);
     if (warp < S) {
         // ---- scores: this CTA's tile j by warp j % S, position 32 (g + G j) + lane; piece v of the tile's 32 positions is contiguous
         for (int j = warp; j < my_tiles; j += S) {
@@ -703,16 +1064,13 @@ __device__ __forceinline__ void attn_phase(const StepParams& P, const StepLayer&
                     f = __half22float2(hh[3]); s = it_add(s, it_mul(qb.z, f.x)); s = it_add(s, it_mul(qb.w, f.y));
                 }
                 s = it_mul(s, scale); sc[p] = s;
-                if (G > 1) __stcg(shared_sc + p, s);
+                if (G > 1) st_tagged(shared_sc + p, s, sc_tag);
             }
             __syncwarp();
             if (lane == 0) mbar_arrive(ke + 8 * sl);
         }
     } else if (warp == ST_AT_MAXS && lane == 0) {
-        float s = 0.f;                                               // the new position, from its row in shared memory (every CTA of the head for itself)
-#pragma unroll 16
-        for (int j = 0; j < hd; j++) s = it_add(s, it_mul(qs[j], kl[j]));
-        sc[nold] = it_mul(s, scale);
+        sc[nold] = it_mul(chain_dot(qs, kl, hd), scale);             // the new position, from its row in shared memory (every CTA of the head for itself)
     }
     ST_EV(P, c, c.evt_base + 7);
     if (G > 1) {
@@ -720,11 +1078,11 @@ __device__ __forceinline__ void attn_phase(const StepParams& P, const StepLayer&
         at_sync();
         if (tid == 0) {
             unsigned* cnt = P.att_cnt + h;
-            const unsigned target = (unsigned)G * c.att_seq;
-            asm volatile("red.release.gpu.global.add.u32 [%0], 1;" :: "l"(cnt) : "memory");
+            const unsigned target = c.att_base + (unsigned)G * c.att_seq;
+            count_up(cnt);
             const long long t0 = clock64();
             for (unsigned it = 0;; it++) {
-                unsigned v; asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(cnt) : "memory");
+                unsigned v; asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(cnt) : "memory");
                 if ((int)(v - target) >= 0) break;
                 if ((it & 63u) == 63u) {
                     if (*reinterpret_cast<volatile unsigned*>(P.sync + 2)) { *c.abort_flag = 1; break; }
@@ -738,7 +1096,7 @@ __device__ __forceinline__ void attn_phase(const StepParams& P, const StepLayer&
             for (int i = 0; i < ntiles; i++) {
                 if (i % G == g) continue;
                 const int p = i * 32 + (tid & 31);
-                if ((tid >> 5) == (i % (ST_NCONS - 1)) && p < nold) sc[p] = __ldcg(shared_sc + p);
+                if ((tid >> 5) == (i % (ST_NCONS - 1)) && p < nold) sc[p] = ld_tagged(shared_sc + p, sc_tag, c.abort_flag, P.error_flag, 19);
             }
         }
         at_sync();
@@ -802,10 +1160,16 @@ __device__ __forceinline__ void attn_phase(const StepParams& P, const StepLayer&
         if (live) {
             const int e0 = g * epc + tid;
             acc = it_add(acc, it_mul(sc[nold], vl[e0]));
-            __stcg(P.arena + P.o + (size_t)h * hd + e0, it_mul(acc, it_sigmoid(__ldcg(gate + e0))));
+            acc = it_mul(acc, it_sigmoid(gs[e0]));
         }
+        publish(P.o, (h * hd + g * epc) / 32 + warp, lane, acc, sc_tag);      // epc is a multiple of 32
     }
     ST_EV(P, c, c.evt_base + 10);
+}
+
+// Dense row `drow` (beta rows, then alpha rows) of a delta-net layer, or null.
+__device__ __forceinline__ const float* dense_row(const StepParams& P, const StepLayer& L, int drow) {
+    return L.recurrent && drow < 2 * P.nv ? (drow < P.nv ? L.beta : L.alpha - (size_t)P.nv * P.e) + (size_t)drow * P.e : nullptr;
 }
 
 // ---------------------------------------------------------------- the step
@@ -814,130 +1178,135 @@ __global__ void __launch_bounds__(ST_THREADS, 1) k_decode_step(const __grid_cons
     Cta c;
     c.smem = smem; c.scratch = smem + P.slots * ST_CHUNK;
     unsigned char* tail = c.scratch + P.scratch;
-    c.bars = smem_u32(tail);                                         // full[s] at bars + 8 s, empty[s] at bars + 8 (slots + s)
-    c.abort_flag = reinterpret_cast<volatile int*>(tail + ST_BARS - 16);
+    c.bars = smem_u32(tail);                                         // full[s] at bars + 8 s, empty[s] at bars + 8 (slots + s), terms full[s] at tf + 8 s
+    c.tf = c.bars + 16 * P.slots; c.ps = c.tf + 8 * P.slots; c.pd = c.ps + 8; c.dn = c.pd + 8; c.at = c.dn + 8;
+    c.lay = reinterpret_cast<const StepLayer*>(tail + 704);         // two layer descriptions
+    c.abort_flag = reinterpret_cast<volatile int*>(tail + ST_BARS - 16); c.verdict = c.abort_flag + 1;
+    c.sp = reinterpret_cast<const StepSpan*>(tail + ST_BARS);
+    c.sg = reinterpret_cast<const uint32_t*>(tail + ST_BARS + SP_KINDS * sizeof(StepSpan));
     c.tid = threadIdx.x; c.warp = c.tid >> 5; c.lane = c.tid & 31;
-    c.q = 0u; c.nseq = 0u; c.mph = 0u; c.nsync = 0; c.evt_on = 0; c.att_seq = 0u;
-    c.tf = c.bars + 8 * (2 * P.slots); c.te = c.tf + 8 * ST_TB; c.pd = c.te + 8 * ST_TB; c.ps = c.pd + 8; c.at = c.bars + 704;
-    c.lay = reinterpret_cast<const StepLayer*>(tail + 384);         // two layer descriptions, then the sum warps' greedy picks
+    c.q = 0u; c.nsync = 0; c.evt_on = 0; c.att_seq = 0u; c.mph = 0u;
     if (c.tid == 0) {
         *c.abort_flag = *reinterpret_cast<volatile unsigned*>(P.sync + 2) ? 1 : 0;      // a step that was given up earlier: nothing runs until the host has cleared the words
-        for (int s = 0; s < P.slots; s++) { mbar_init(c.bars + 8 * s, 1); mbar_init(c.bars + 8 * (P.slots + s), ST_CW); }
-        for (int k = 0; k < ST_TB; k++) { mbar_init(c.tf + 8 * k, ST_NCONS); mbar_init(c.te + 8 * k, 1); }
-        mbar_init(c.pd, ST_NSUM); mbar_init(c.ps, ST_NCONS);
+        for (int s = 0; s < P.slots; s++) { mbar_init(c.bars + 8 * s, 1); mbar_init(c.bars + 8 * (P.slots + s), 1); mbar_init(c.tf + 8 * s, ST_CW); }
+        mbar_init(c.ps, 1); mbar_init(c.pd, ST_NSUM); mbar_init(c.dn, 8);
         for (int k = 0; k < 4 * ST_AT_MAXS; k++) mbar_init(c.at + 8 * k, 1);     // set up again, with their counts, by every attention block
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    {   // the first layer's description into shared memory (later ones are copied a layer ahead)
-        constexpr int words = (int)(sizeof(StepLayer) / 4);
-        if (c.tid < words) reinterpret_cast<uint32_t*>(tail + 384)[c.tid] = reinterpret_cast<const uint32_t*>(P.layers)[c.tid];
+    {   // the first layer's description and this CTA's spans into shared memory (later layers are copied a layer ahead)
+        constexpr int words = (int)(sizeof(StepLayer) / 4), sw = (int)(SP_KINDS * sizeof(StepSpan) / 4);
+        if (c.tid < words) reinterpret_cast<uint32_t*>(tail + 704)[c.tid] = reinterpret_cast<const uint32_t*>(P.layers)[c.tid];
+        if (c.tid < sw) reinterpret_cast<uint32_t*>(tail + ST_BARS)[c.tid] = reinterpret_cast<const uint32_t*>(P.spans + (size_t)blockIdx.x * SP_KINDS)[c.tid];
+#pragma unroll 1
+        for (int k = 0; k < 4; k++) for (int i = c.tid; i < P.sg_words[k]; i += ST_THREADS) const_cast<uint32_t*>(c.sg)[P.sg_off[k] + i] = P.sg[k][i];
     }
     __syncthreads();
     if (*c.abort_flag) return;
     if (c.warp == ST_NCONS + ST_NSUM) { if (c.lane == 0) producer(P, c); return; }
     if (c.warp >= ST_NCONS) { sum_warps(P, c); return; }
 
-    c.target = *reinterpret_cast<volatile unsigned*>(P.sync + 1);
-    if (c.tid == 0 && (int)blockIdx.x < P.nh) __stcg(P.att_cnt + blockIdx.x, 0u);       // the heads' arrival counters start every launch at zero (grid barriers precede their first use)
+    c.base = *reinterpret_cast<volatile unsigned*>(P.sync + 3); c.target = *reinterpret_cast<volatile unsigned*>(P.sync + 1);
     c.inv_sqrt_sd = it_div(1.0f, it_sqrt((float)ST_SD)); c.inv_sqrt_hd = it_div(1.0f, it_sqrt((float)P.hd));
-    if (P.trace && blockIdx.x == 0 && c.tid == 32) P.trace[4 * ST_TRACE_MAX] = 0;
-    const int e = P.e, nb_e = e / 128;
     float* A = P.arena;
+    const int cta = (int)blockIdx.x, grid = (int)gridDim.x, drow = grid - 1 - cta, ah = cta - P.attn_base;
+    const int hb = cta % P.had_step == 0 && cta / P.had_step < P.widest / 1024 ? cta / P.had_step : -1;      // the block this CTA transforms, of every row that has as many
+    // the heads' arrival counters only grow; nobody counts before this CTA has taken part in the first layer
+    c.att_base = c.tid == 0 && ah >= 0 && ah < P.nh * P.attn_g ? *reinterpret_cast<volatile unsigned*>(P.att_cnt + ah / P.attn_g) : 0u;
     const uint32_t tok = (P.flags & 1) ? __float_as_uint(*reinterpret_cast<volatile float*>(A + P.amx)) : *reinterpret_cast<volatile uint32_t*>(P.toks);
-    const float* xsrc = P.tok_embd + (size_t)tok * e;               // the residual row of layer 0 is the embedding row (Model::embed, src/cpu.rs:118-122)
-    ConvKeep keep; keep.ch = -1; keep.mx = 0.f;
-    // Phases: nine per layer (0 norm+Hadamard, 1 input projection, 2 delta-net / attention block, 3 Hadamard of its output,
-    // 4 output projection, 5 norm+Hadamard, 6 gate/up, 7 silu*mul+Hadamard, 8 down), then the output norm (+ Hadamard), the LM
-    // head and the pick.  One loop, one copy of each kind of phase: the kernel runs front to back once per step, so its code
-    // size, not its loop structure, is what the instruction cache sees.
+    float* wb = reinterpret_cast<float*>(c.scratch + P.w_off);
+    // the norms' weights are wanted where a block of a normed row is transformed and where a dense row is multiplied
+    auto want_norm = [&](const float* w, const float* dense) { if (dense || (hb >= 0 && hb * 1024 < P.e)) norm_request(wb, w, dense, P.e); };
+    want_norm(c.lay->attn_norm, dense_row(P, *c.lay, drow));
+    // Nine phases a layer, then the output norm with the LM head.  One loop, one copy of each kind of phase: transforms (A D F H: the
+    // owners of the row's blocks, in A also the owners of dense rows), matrices (B E G I: everyone), the block in between (C).
     const bool logits = (P.flags & 4) != 0;
-    const int nphase = 9 * P.n_layer + (logits ? 3 : 1);
-    for (int ph = 0; ph < nphase; ph++) {
-        const int il = ph / 9, sub = ph - 9 * il;
-        const bool tail = il >= P.n_layer;
+    int il = 0, ph = PH_A;
+#pragma unroll 1
+    for (;;) {
+        const bool tail_ph = il >= P.n_layer;
         const StepLayer& L = c.lay[il & 1];
-        if (!tail && sub == 0 && il + 1 < P.n_layer && c.warp == ST_NCONS - 1) {          // the next layer's description, long before it is needed
-            constexpr int words = (int)(sizeof(StepLayer) / 4);
-            uint32_t* dst = reinterpret_cast<uint32_t*>(const_cast<StepLayer*>(c.lay + ((il + 1) & 1)));
-            for (int i = c.lane; i < words; i += 32) dst[i] = reinterpret_cast<const uint32_t*>(P.layers + il + 1)[i];
-        }
-        c.evt_on = (il == 1 || il == 3) && c.warp == 0 && ((sub == 2) ? ((int)blockIdx.x == (il == 1 ? 0 : P.attn_base)) : (blockIdx.x == gridDim.x - 1)); c.evt_base = (il == 1 ? 0 : 256) + 16 * sub;
-        const int kind = tail ? (sub == 0 ? 0 : sub == 1 ? 1 : 3) : (sub == 2 ? 2 : sub < 2 ? sub : ((sub & 1) ? 0 : 1));   // 0 Hadamard, 1 matvec, 2 block, 3 pick
-        if (kind == 0) {
-            it_had_prologue p; const float* in = A + P.x; const float* signs = P.sg_e; int nblocks = nb_e / 8; unsigned ph_hd = 0, ph_nk = 0, ph_rep = 0;
-            float shift[6]; const bool shifting = !tail && sub == 3 && keep.ch >= 0;
-            if (tail || sub == 0 || sub == 5) {
-                // rmsnorm -> Hadamard -> q8k of the residual row; the normed row is kept where a later op reads it in f32
-                p.mode = 2; p.w = tail ? P.output_norm : sub == 0 ? L.attn_norm : L.post_norm; p.eps = P.eps; p.n = (unsigned)e; p.xn_stride = e;
-                p.xn_out = tail ? A + P.hrow : (sub == 0 && L.recurrent) ? A + P.xn : nullptr;
-                if (!tail && sub == 0 && il == 0) {
-                    in = xsrc;
-                    const int vb0 = (int)blockIdx.x - P.had_base;
-                    if (vb0 >= 0 && vb0 < nblocks && c.tid < 256)
-                        *reinterpret_cast<float4*>(A + P.x + vb0 * 1024 + 4 * c.tid) = *reinterpret_cast<const float4*>(xsrc + vb0 * 1024 + 4 * c.tid);
+        c.evt_on = (il == 1 || il == 3) && c.warp == 0 && (ph == PH_C ? (cta == (il == 1 ? 0 : P.attn_base)) : (ph & 1) == 0 && ph < PH_C || ph == PH_D || ph == PH_F || ph == PH_H ? cta == 0 : (cta == grid - 1)); c.evt_base = (il == 1 ? 0 : 256) + 16 * ph;
+        const int row_blocks = (ph < PH_C || ph == PH_F || ph == PH_G ? P.e : ph < PH_F ? (L.recurrent ? P.inner : P.nh * P.hd) : P.ff) / 1024;      // of the row that the phase transforms or reads
+        if (ph == PH_C) {
+            const int heads = L.recurrent ? P.nv : P.nh * P.attn_g;
+            if (L.recurrent) { if (cta < P.nv) { cons_sync(); gdn_phase(P, L, c, cta, il); } }
+            else if (ah >= 0 && ah < heads) { cons_sync(); attn_phase(P, L, c, ah, il); }
+        } else if (ph == PH_A || ph == PH_D || ph == PH_F || ph == PH_H) {
+            RowIn in; in.normed = nullptr; in.plain = nullptr; in.norm = ph == PH_A || ph == PH_F; in.dense = ph == PH_A && !tail_ph && L.recurrent && drow < 2 * P.nv;
+            const bool owner = hb >= 0 && hb < row_blocks && (!tail_ph || logits || cta == 0);
+            if (owner || in.dense) {
+                in.codes = owner && (!tail_ph || logits) ? P.codes + (ph == PH_H ? P.codes_half : 0) + hb * 128 : nullptr; in.codes_copy = row_blocks * 128; in.code_tag = tag_of(c.base, il, ph);
+                in.nblk = row_blocks; in.blk = hb;
+                in.signs = c.sg + (hb >= 0 ? 32 * hb : 0) + P.sg_off[ph == PH_D ? (L.recurrent ? 1 : 2) : ph == PH_H ? 3 : 0];
+                if (ph == PH_A) {
+                    in.x = P.xi; in.tag = tag_of(c.base, il - 1, PH_I);
+                    if (il == 0) in.plain = P.tok_embd + (size_t)tok * P.e;      // the residual row of layer 0 is the embedding row (Model::embed, src/cpu.rs:118-122)
+                    if (tail_ph && cta == 0) in.normed = A + P.hrow;
+                } else if (ph == PH_F) { in.x = P.xe; in.tag = tag_of(c.base, il, PH_E); }
+                else {
+                    in.x = (ph == PH_D ? P.o : P.act) + (size_t)hb * ST_GPB; in.tag = tag_of(c.base, il, ph == PH_D ? PH_C : PH_G); in.nblk = 1; in.blk = 0;
                 }
-            } else if (sub == 3) {
-                // the block's output row (delta-net: with the value-head permutation).  The conv state of the channels this
-                // thread owns moves on by one input now that no CTA reads the old one: loads here, stores after the transform
-                if (shifting) {
-#pragma unroll
-                    for (int i = 0; i < 6; i++) shift[i] = i < P.conv_k - 2 ? L.conv_st[(size_t)(i + 1) * P.cd + keep.ch] : 0.f;
-                }
-                const bool perm = L.recurrent && P.v_grouped;
-                in = A + P.o; signs = L.recurrent ? P.sg_inner : P.sg_att; nblocks = (L.recurrent ? P.inner : P.nh * P.hd) / 1024;
-                if (perm) { ph_hd = ST_SD; ph_nk = (unsigned)P.nk; ph_rep = (unsigned)(P.nv / P.nk); }
-            } else {
-                p.mode = 1; p.b = A + P.big1 + P.ff; p.b_stride = 2 * (size_t)P.ff;        // silu(gate) * up on the way in
-                in = A + P.big1; signs = P.sg_ff; nblocks = P.ff / 1024;
+                if (!owner && !count_wait(P, c, P.sync, c.target + (unsigned)row_blocks, 1 + ph, false)) return;      // a dense row's owner follows the blocks' owners
+                ST_EV(P, c, c.evt_base + 0);
+                block_transform(P, c, in);
+                ST_EV(P, c, c.evt_base + 1);
             }
-            const int vb = (int)blockIdx.x - P.had_base;
-            if (vb >= 0 && vb < nblocks && c.tid < 256) {
-                it_had_smem& sm = *reinterpret_cast<it_had_smem*>(c.scratch);
-                it_hadamard_block<true>(sm, (unsigned)c.tid, (unsigned)vb, 0, in, 0, 0, nullptr, 0, 0, signs, 1, 0, ph_hd, ph_nk, ph_rep, P.qs, P.qd, P.qsum, P.q_stride, p);
-            }
-            if (shifting) {
-#pragma unroll
-                for (int i = 0; i < 6; i++) if (i < P.conv_k - 2) L.conv_st[(size_t)i * P.cd + keep.ch] = shift[i];
-                L.conv_st[(size_t)(P.conv_k - 2) * P.cd + keep.ch] = keep.mx;
-                keep.ch = -1;
-            }
-        } else if (kind == 1) {
-            int nb, rows;
-            if (tail) { nb = nb_e; rows = P.n_vocab; }
-            else if (sub == 1) { nb = nb_e; rows = L.in_rows; }
-            else if (sub == 4) { nb = (L.recurrent ? P.inner : P.nh * P.hd) / 128; rows = e; }
-            else if (sub == 6) { nb = nb_e; rows = 2 * P.ff; }
-            else { nb = P.ff / 128; rows = e; }
-            const bool block_cta = L.recurrent ? (int)blockIdx.x < P.nv : ((int)blockIdx.x >= P.attn_base && (int)blockIdx.x < P.attn_base + P.nh * P.attn_g);
-            matvec_phase(P, c, nb, rows, (!tail && sub == 1 && block_cta) ? &L : nullptr);
-            if (tail && c.warp == 0 && c.lane == 0) {
-                // greedy pick (first index of the maximum): each sum warp has left the best of its rows behind the layer descriptions
-                const Pick* pk = reinterpret_cast<const Pick*>(c.lay + 2);
-                Pick pbest = pk[0];
-                for (int j = 1; j < ST_NSUM; j++) pbest = pick_better(pbest, pk[j]);
-                P.partials[blockIdx.x] = ((unsigned long long)__float_as_uint(pbest.v) << 32) | pbest.i;
-            }
-        } else if (kind == 2) {
-            const int ah = (int)blockIdx.x - P.attn_base;
-            if (L.recurrent) { if ((int)blockIdx.x < P.nv) gdn_phase(P, L, c, keep, (int)blockIdx.x); }
-            else if (ah >= 0 && ah < P.nh * P.attn_g) attn_phase(P, L, c, ah);
+            if (tail_ph && !logits) { if (cta != 0) return; break; }
+            c.target += (unsigned)row_blocks;
         } else {
-            if (blockIdx.x == 0 && c.warp == 0) {
-                Pick q{ -INFINITY, 0xffffffffu };
-                for (unsigned b = c.lane; b < gridDim.x; b += 32) { const unsigned long long u = __ldcg(P.partials + b); q = pick_better(q, Pick{ __uint_as_float((unsigned)(u >> 32)), (unsigned)u }); }
-#pragma unroll
-                for (unsigned mm = 16; mm > 0; mm >>= 1) { Pick o{ __shfl_xor_sync(0xffffffffu, q.v, mm), __shfl_xor_sync(0xffffffffu, q.i, mm) }; q = pick_better(q, o); }
-                if (c.lane == 0) {
-                    const unsigned pick = q.i == 0xffffffffu ? 0u : q.i;
-                    A[P.amx] = __uint_as_float(pick);
-                    if (P.flags & 2) { P.toks[0] = pick; *P.pos += 1; }
+            const int sub = ph == PH_B ? 0 : ph == PH_E ? 1 : ph == PH_G ? 2 : 3;
+            const int kind = tail_ph ? SP_HEAD : span_kind(sub, L.recurrent);
+            if (!count_wait(P, c, P.sync, c.target, 1 + ph)) return;
+            ST_EV(P, c, c.evt_base + 0);
+            if (c.tid == 0) mbar_arrive(c.ps);                       // the sum warps may enter this phase
+            // (a CTA without row groups does not read the codes: nothing would keep them for it)
+            if (c.sp[kind].n) codes_place(P, c, P.codes + (ph == PH_I ? P.codes_half : 0), row_blocks, tag_of(c.base, il, ph - 1));
+            ST_EV(P, c, c.evt_base + 1);
+            if (ph == PH_B && !tail_ph) {
+                if (il + 1 < P.n_layer && c.warp == ST_NCONS - 1) {          // the next layer's description, long before it is needed
+                    constexpr int words = (int)(sizeof(StepLayer) / 4);
+                    uint32_t* dst = reinterpret_cast<uint32_t*>(const_cast<StepLayer*>(c.lay + ((il + 1) & 1)));
+#pragma unroll 1
+                    for (int i = c.lane; i < words; i += 32) dst[i] = reinterpret_cast<const uint32_t*>(P.layers + il + 1)[i];
                 }
+                if (L.recurrent) { if (cta < P.nv) gdn_prefetch(P, L, c, cta); }
+                else attn_prefetch(P, L, c, ah);
             }
-            break;                                                   // nothing follows the pick
+            if (ph == PH_G) { if (il + 1 < P.n_layer) warm_layer(P, c, c.lay[(il + 1) & 1], drow); else if (cta == grid - 1) warm_l2(P.output_norm, P.e * 4, c.tid); }
+            matvec_phase(P, c, c.sp[kind]);
+            ST_EV(P, c, c.evt_base + 2);
+            // the next norm's weights (and dense row) while the other CTAs finish
+            if (ph == PH_E) want_norm(L.post_norm, nullptr);
+            if (ph == PH_I) {
+                const bool more = il + 1 < P.n_layer; const StepLayer& N = c.lay[(il + 1) & 1];
+                want_norm(more ? N.attn_norm : P.output_norm, more ? dense_row(P, N, drow) : nullptr);
+            }
+            if (tail_ph) { if (cta != 0) return; break; }
+            // the scratch is the next phase's once this CTA's sum warps are through (they are before anything the next phase needs has arrived)
+            mbar_wait(c.pd, c.mph & 1u, c.abort_flag, P.error_flag, 5);
+            c.mph++;
         }
-        if (!grid_sync(P, c, 1 + sub + (tail ? 9 : 0))) return;
+        if (++ph == ST_SUBS) { ph = PH_A; il++; }
     }
-    if (blockIdx.x == 0 && c.tid == 0) P.sync[1] = c.target;        // every CTA has read the old value before its first arrival
+    // every sum warp counts when it is through: nobody is left who could still read the words written below
+    c.target += ST_NSUM * (unsigned)grid;
+    if (!count_wait(P, c, P.sync, c.target, 10, false)) return;
+    if (logits && c.warp == 0) {
+        Pick q{ -INFINITY, 0xffffffffu };
+#pragma unroll 1
+        for (unsigned b = c.lane; b < gridDim.x * ST_NSUM; b += 32) {
+            const granule u = wait_granule(P.partials + b, tag_of(c.base, P.n_layer, PH_B), c.abort_flag, P.error_flag, 20);
+            q = pick_better(q, Pick{ __uint_as_float(u.x), u.y });
+        }
+#pragma unroll
+        for (unsigned mm = 16; mm > 0; mm >>= 1) { Pick o{ __shfl_xor_sync(0xffffffffu, q.v, mm), __shfl_xor_sync(0xffffffffu, q.i, mm) }; q = pick_better(q, o); }
+        if (c.lane == 0) {
+            const unsigned pick = q.i == 0xffffffffu ? 0u : q.i;
+            A[P.amx] = __uint_as_float(pick);
+            if (P.flags & 2) { P.toks[0] = pick; *P.pos += 1; }
+        }
+    }
+    if (c.tid == 0) { P.sync[1] = c.target; P.sync[3] = c.base + (unsigned)(ST_SUBS * (P.n_layer + 1) + 1); }
 }
 
 }  // namespace
@@ -945,21 +1314,67 @@ __global__ void __launch_bounds__(ST_THREADS, 1) k_decode_step(const __grid_cons
 // ---------------------------------------------------------------- host side
 struct it_step_state {
     StepLayer* layers_dev;
+    StepSpan* spans_dev;
     unsigned long long* trace;
-    unsigned long long* partials;
-    int grid, slots, scratch, gdn_off, had_base, attn_base, attn_g, att_stride;
-    float* att_sc; unsigned* att_cnt;
+    granule *xe, *xi, *rows, *o, *act, *codes, *prefix, *partials;
+    unsigned long long* gate;
+    int had_step;
+    int grid, slots, scratch, gdn_off, attn_base, attn_g, att_stride;
+    unsigned long long* att_sc; unsigned* att_cnt;
     bool cooperative;
 };
 
-static size_t step_gdn_off(const it_model_config& c) { return ((size_t)mv_layout(c.n_embd / 128).total + 127) / 128 * 128; }
-static size_t step_scratch_bytes(const it_model_config& c) {
-    const int widest = std::max(std::max(c.n_embd, c.n_ff), std::max(c.ssm_inner, c.n_head * c.head_dim));
-    size_t s = (size_t)mv_layout(widest / 128).total;
-    s = std::max(s, sizeof(it_had_smem));
-    s = std::max(s, step_gdn_off(c) + (size_t)(ST_SD * ST_SD + 5 * ST_SD + 8) * 4 + 16 * 8 + 64);
-    s = std::max(s, ((size_t)c.ctx_len + 4 + 3 * c.head_dim + 48) * 4 + 128 + 3 * (size_t)c.head_dim * 64);
+static int step_widest(const it_model_config& c) { return std::max(std::max(c.n_embd, c.n_ff), std::max(c.ssm_inner, c.n_head * c.head_dim)); }
+// the state tile of the delta-net block comes in while the input projection's chunks run: behind their terms
+static size_t step_gdn_off(const it_model_config& c, int slots) { return (size_t)terms_at(c.n_embd / 128) + (size_t)slots * ST_TERMS * 4; }
+static size_t step_w_bytes(const it_model_config& c) { return (size_t)(c.n_embd / 1024) * ST_HPITCH * 4; }
+static size_t step_scratch_bytes(const it_model_config& c, int slots) {
+    size_t s = (size_t)terms_at(step_widest(c) / 128) + (size_t)slots * ST_TERMS * 4;
+    s = std::max(s, (size_t)ST_RED + (size_t)(c.n_embd / 1024) * ST_HPITCH * 4 + (size_t)c.n_embd * 4 + step_w_bytes(c));      // a normed row, a dense row, the norm's weights
+    s = std::max(s, step_gdn_off(c, slots) + (size_t)ST_SD * ST_SD * 4);
+    // a norm's weights and a dense row come in while the widest matrix's chunks run, and stay while their row is transformed
+    const size_t below = std::max((size_t)terms_at(step_widest(c) / 128) + (size_t)slots * ST_TERMS * 4, (size_t)terms_at(c.n_embd / 128) + (size_t)(c.n_embd / 1024) * ST_HPITCH * 4);
+    s = std::max(s, below + (size_t)c.n_embd * 4 + step_w_bytes(c));
+    s = std::max(s, ((size_t)c.ctx_len + 4 + 4 * c.head_dim + 48) * 4 + 128 + 3 * (size_t)c.head_dim * 64);
     return (s + 127) / 128 * 128;
+}
+// where the sign bits of the four widths start (words): a width that occurs twice is kept once
+static int step_sign_words(const it_model_config& c, int (&off)[4], int (&words)[4]) {
+    const int n[4] = { c.n_embd, c.ssm_inner, c.n_head * c.head_dim, c.n_ff };
+    int o = 0;
+    for (int k = 0; k < 4; k++) {
+        int same = -1;
+        for (int j = 0; j < k; j++) if (n[j] == n[k]) same = j;
+        off[k] = same >= 0 ? off[same] : o; words[k] = same >= 0 ? 0 : n[k] / 32; o += words[k];
+    }
+    return o;
+}
+static size_t step_smem_bytes(const it_model_config& c, int slots) {
+    int off[4], words[4];
+    return (size_t)slots * ST_CHUNK + step_scratch_bytes(c, slots) + ST_BARS + SP_KINDS * sizeof(StepSpan) + 4 * (size_t)step_sign_words(c, off, words);
+}
+
+// The chunks [c0, c1) of a matrix of `units` row groups (pairs of row groups when parts == 2), in the order a CTA takes them.
+static StepSpan step_span(long long c0, long long c1, int nb, int parts, int units) {
+    StepSpan s; memset(&s, 0, sizeof s);
+    s.nb = nb; s.cpr = nb / ST_TPC; s.parts = parts; s.units = units; s.magic = 0xffffffffu / (unsigned)s.cpr + 1u;
+    const long long cpu = (long long)s.cpr * parts;
+    s.n = (int)(c1 - c0); s.lead = (int)(c0 % cpu);
+    if (s.n == 0) { s.lead = 0; return s; }
+    s.tl = s.lead ? (int)(cpu - s.lead) : 0; s.hl = (int)(c1 % cpu);
+    s.ut = (int)(c0 / cpu); s.uf = (int)((c0 + s.tl) / cpu); s.uh = (int)(c1 / cpu);
+    return s;
+}
+// Equal runs of chunks when every CTA gets at least one whole row group's worth (then a row group is cut at most once), else whole
+// row groups.
+static void step_spans(std::vector<StepSpan>& out, int kind, int grid, int rows, int cols, int parts) {
+    const int nb = cols / 128, units = (rows / parts + 31) / 32; const long long cpu = (long long)(nb / ST_TPC) * parts, total = units * cpu;
+    for (int b = 0; b < grid; b++) {
+        long long c0, c1;
+        if (units >= grid) { c0 = total * b / grid; c1 = total * (b + 1) / grid; }
+        else { c0 = (long long)units * b / grid * cpu; c1 = (long long)units * (b + 1) / grid * cpu; }
+        out[(size_t)b * SP_KINDS + kind] = step_span(c0, c1, nb, parts, units);
+    }
 }
 
 // Whether this engine's decode step can run as the persistent kernel, and with which geometry.
@@ -968,31 +1383,26 @@ int it_step_prepare(it_engine* e) {
     e->step = nullptr;
     { const char* v = getenv("IT_STEP_KERNEL"); if (v && atoi(v) == 0) return IT_OK; }
     if (e->world != 1) return IT_OK;                                  // row shards exchange results inside the per-op kernels
-    if (c.ssm_state != ST_SD || c.conv_k > 8 || c.head_dim > 256 || c.head_dim % 8 || c.n_embd > 8192 || c.n_ff % 1024 || c.ssm_inner % 1024 || (c.n_head * c.head_dim) % 1024) return IT_OK;
-    if (c.ssm_vheads > cx->sm_count || c.n_head > cx->sm_count || c.n_ff / 1024 > cx->sm_count || c.ssm_vheads % c.ssm_groups) return IT_OK;
-    const size_t scratch = step_scratch_bytes(c);
-    const long long ring = (long long)ST_SMEM - (long long)scratch - ST_BARS;
-    int slots = 1;
-    while (2 * slots <= 16 && (long long)(2 * slots) * ST_CHUNK <= ring) slots *= 2;   // a power of two: slot = chunk index & (slots - 1); at most 16 (the mbarriers share 384 reserved bytes)
+    if (c.ssm_state != ST_SD || c.conv_k > 8 || c.head_dim > 256 || c.head_dim % 32 || c.n_embd > 8192 || c.n_embd % 1024 || c.n_ff % 1024 || c.ssm_inner % 1024 || (c.n_head * c.head_dim) % 1024) return IT_OK;
+    if (2 * c.ssm_vheads > cx->sm_count || c.n_head > cx->sm_count || step_widest(c) / 1024 > cx->sm_count || c.n_embd % 32 || c.ssm_vheads % c.ssm_groups) return IT_OK;
+    int slots = 16;                                                   // a power of two: slot = chunk index & (slots - 1)
+    while (slots > 2 && step_smem_bytes(c, slots) > (size_t)ST_SMEM) slots /= 2;
     if (slots < 4) return IT_OK;
     IT_CUDA(cudaSetDevice(cx->device));
     static bool attr_set[16] = {};
     if (!attr_set[cx->device & 15]) { IT_CUDA(cudaFuncSetAttribute(k_decode_step, cudaFuncAttributeMaxDynamicSharedMemorySize, ST_SMEM)); attr_set[cx->device & 15] = true; }
     int per_sm = 0;
-    IT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_decode_step, ST_THREADS, (size_t)slots * ST_CHUNK + scratch + ST_BARS));
+    IT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_decode_step, ST_THREADS, step_smem_bytes(c, slots)));
     if (per_sm < 1) return IT_OK;
     it_step_state* st = new it_step_state();
-    st->grid = cx->sm_count; st->slots = slots; st->scratch = (int)scratch; st->gdn_off = (int)step_gdn_off(c);
-    {   // Hadamard blocks on the last CTAs, attention heads behind the value heads when they all fit side by side
-        const int widest = std::max(std::max(c.n_embd, c.n_ff), std::max(c.ssm_inner, c.n_head * c.head_dim)) / 1024;
-        st->had_base = st->grid - widest;
-        // several CTAs per attention head when the grid has them: each takes a share of the K tiles and of the output elements
-        st->attn_g = 1;
-        for (int g = 4; g > 1; g /= 2) if (c.head_dim % g == 0 && (c.head_dim / g) % it_vc_slice(c.head_dim) == 0 && g * c.n_head <= st->grid) { st->attn_g = g; break; }
-        { const char* v = getenv("IT_STEP_ATTN_G"); if (v && (atoi(v) == 1 || atoi(v) == 2) && atoi(v) < st->attn_g) st->attn_g = atoi(v); }
-        st->attn_base = (c.ssm_vheads + st->attn_g * c.n_head <= st->grid) ? c.ssm_vheads : 0;
-    }
-    st->layers_dev = nullptr; st->partials = nullptr; st->trace = nullptr; st->att_sc = nullptr; st->att_cnt = nullptr;
+    st->grid = cx->sm_count; st->slots = slots; st->scratch = (int)step_scratch_bytes(c, slots); st->gdn_off = (int)step_gdn_off(c, slots);
+    // several CTAs per attention head when the grid has them: each takes a share of the K tiles and of the output elements;
+    // attention heads sit behind the value heads when they all fit side by side
+    st->attn_g = 1;
+    for (int g = 4; g > 1; g /= 2) if (c.head_dim % (32 * g) == 0 && (c.head_dim / g) % it_vc_slice(c.head_dim) == 0 && g * c.n_head <= st->grid) { st->attn_g = g; break; }
+    { const char* v = getenv("IT_STEP_ATTN_G"); if (v && (atoi(v) == 1 || atoi(v) == 2) && atoi(v) < st->attn_g) st->attn_g = atoi(v); }
+    st->attn_base = (c.ssm_vheads + st->attn_g * c.n_head <= st->grid) ? c.ssm_vheads : 0;
+    st->layers_dev = nullptr; st->spans_dev = nullptr; st->partials = nullptr; st->gate = nullptr; st->trace = nullptr; st->had_step = st->grid / (step_widest(c) / 1024); st->att_sc = nullptr; st->att_cnt = nullptr;
     st->att_stride = (c.ctx_len + 32 + 3) / 4 * 4;
     { const char* v = getenv("IT_STEP_COOP"); st->cooperative = !v || atoi(v) != 0; }
     std::vector<StepLayer> hl(c.n_layer);
@@ -1004,13 +1414,28 @@ int it_step_prepare(it_engine* e) {
         s.conv_w = l.conv_w; s.dt = l.dt; s.a = l.a; s.beta = l.beta; s.alpha = l.alpha; s.ssm_norm = l.ssm_norm; s.conv_st = l.conv_st; s.ssm_st = l.ssm_st;
         s.q_norm = l.q_norm; s.k_norm = l.k_norm; s.kc = l.kc; s.vc = l.vc;
     }
+    std::vector<StepSpan> sp((size_t)st->grid * SP_KINDS);
+    step_spans(sp, SP_IN_GDN, st->grid, it_cfg_conv_dim(c) + c.ssm_inner, c.n_embd, 1);
+    step_spans(sp, SP_IN_ATT, st->grid, (2 * c.n_head + 2 * c.n_head_kv) * c.head_dim, c.n_embd, 1);
+    step_spans(sp, SP_OUT_GDN, st->grid, c.n_embd, c.ssm_inner, 1);
+    step_spans(sp, SP_OUT_ATT, st->grid, c.n_embd, c.n_head * c.head_dim, 1);
+    step_spans(sp, SP_GATE_UP, st->grid, 2 * c.n_ff, c.n_embd, 2);
+    step_spans(sp, SP_DOWN, st->grid, c.n_embd, c.n_ff, 1);
+    step_spans(sp, SP_HEAD, st->grid, c.n_vocab, c.n_embd, 1);
     int r = it_engine_dev_alloc(e, (void**)&st->layers_dev, hl.size() * sizeof(StepLayer), false);
-    if (r == IT_OK) r = it_engine_dev_alloc(e, (void**)&st->partials, (size_t)st->grid * sizeof(unsigned long long), true);
-    if (r == IT_OK) r = it_engine_dev_alloc(e, (void**)&st->att_sc, (size_t)c.n_head * st->att_stride * sizeof(float), true);
+    if (r == IT_OK) r = it_engine_dev_alloc(e, (void**)&st->spans_dev, sp.size() * sizeof(StepSpan), false);
+    auto granules = [&](granule** p, size_t n) { if (r == IT_OK) r = it_engine_dev_alloc(e, (void**)p, n * sizeof(granule), true); };
+    auto row_of = [&](granule** p, size_t rows) { granules(p, (rows + 31) / 32 * ST_GPU); };
+    row_of(&st->xe, c.n_embd); row_of(&st->xi, c.n_embd); row_of(&st->rows, std::max((size_t)it_cfg_conv_dim(c) + c.ssm_inner, (size_t)(2 * c.n_head + 2 * c.n_head_kv) * c.head_dim));
+    row_of(&st->o, std::max(c.ssm_inner, c.n_head * c.head_dim)); row_of(&st->act, c.n_ff);
+    granules(&st->codes, (size_t)(step_widest(c) / 1024) * 128 * ST_COPIES * 2); granules(&st->prefix, (size_t)st->grid * 32); granules(&st->partials, (size_t)st->grid * ST_NSUM);
+    if (r == IT_OK) r = it_engine_dev_alloc(e, (void**)&st->gate, 2 * (size_t)c.ssm_vheads * sizeof(unsigned long long), true);
+    if (r == IT_OK) r = it_engine_dev_alloc(e, (void**)&st->att_sc, (size_t)c.n_head * st->att_stride * sizeof(unsigned long long), true);
     if (r == IT_OK) r = it_engine_dev_alloc(e, (void**)&st->att_cnt, (size_t)c.n_head * sizeof(unsigned), true);
     { const char* v = getenv("IT_STEP_TRACE"); if (r == IT_OK && v && atoi(v) != 0) r = it_engine_dev_alloc(e, (void**)&st->trace, (2 * ST_TRACE_MAX * 2 + ST_EVT_MAX) * sizeof(unsigned long long), true); }
     if (r) { delete st; return r; }
     IT_CUDA(cudaMemcpyAsync(st->layers_dev, hl.data(), hl.size() * sizeof(StepLayer), cudaMemcpyHostToDevice, cx->stream));
+    IT_CUDA(cudaMemcpyAsync(st->spans_dev, sp.data(), sp.size() * sizeof(StepSpan), cudaMemcpyHostToDevice, cx->stream));
     IT_CUDA(cudaStreamSynchronize(cx->stream));
     e->step = st;
     return IT_OK;
@@ -1021,30 +1446,29 @@ void it_step_release(it_engine* e) { delete e->step; e->step = nullptr; }
 int it_step_launch(it_engine* e, int flags) {
     it_step_state* st = e->step; it_ctx* cx = e->ctx; const it_model_config& c = e->cfg; const it_arena_layout& L = e->lay;
     StepParams P; memset(&P, 0, sizeof P);
-    P.layers = st->layers_dev; P.n_layer = c.n_layer;
-    P.e = c.n_embd; P.ff = c.n_ff; P.hd = c.head_dim; P.nh = c.n_head; P.nkv = c.n_head_kv; P.cd = it_cfg_conv_dim(c); P.inner = c.ssm_inner; P.nv = c.ssm_vheads;
+    P.layers = st->layers_dev; P.spans = st->spans_dev; P.n_layer = c.n_layer;
+    P.e = c.n_embd; P.ff = c.n_ff; P.widest = step_widest(c); P.hd = c.head_dim; P.nh = c.n_head; P.nkv = c.n_head_kv; P.cd = it_cfg_conv_dim(c); P.inner = c.ssm_inner; P.nv = c.ssm_vheads;
     P.nk = c.ssm_groups; P.qk = it_cfg_qk(c); P.conv_k = c.conv_k; P.n_rot = c.n_rot; P.n_vocab = c.n_vocab;
     P.eps = c.eps; P.theta_scale = e->theta_scale; for (int i = 0; i < 4; i++) P.sec[i] = c.rope_sections[i]; P.v_grouped = c.gdn_v_grouped;
-    P.arena = cx->arena; P.x = L.x; P.xn = L.xn; P.big1 = L.big1; P.o = L.o; P.hrow = L.hrow; P.logits = L.logits; P.amx = L.amx;
-    P.qs = e->q8->qs; P.qd = e->q8->d; P.qsum = e->q8->sum128; P.q_stride = e->q8->max_n;
-    P.sg_e = cx->signs[(size_t)c.n_embd]; P.sg_inner = cx->signs[(size_t)c.ssm_inner]; P.sg_att = cx->signs[(size_t)c.n_head * c.head_dim]; P.sg_ff = cx->signs[(size_t)c.n_ff];
+    P.arena = cx->arena; P.xe = st->xe; P.xi = st->xi; P.rows = st->rows; P.o = st->o; P.act = st->act; P.codes = st->codes; P.codes_half = step_widest(c) / 1024 * 128 * ST_COPIES; P.prefix = st->prefix; P.had_step = st->had_step; P.hrow = L.hrow; P.logits = L.logits; P.amx = L.amx; P.gate = st->gate;
+    { const size_t w[4] = { (size_t)c.n_embd, (size_t)c.ssm_inner, (size_t)c.n_head * c.head_dim, (size_t)c.n_ff }; for (int k = 0; k < 4; k++) P.sg[k] = reinterpret_cast<const uint32_t*>(cx->signs[w[k]] + w[k]); }
+    step_sign_words(c, P.sg_off, P.sg_words);
     P.tok_embd = e->tok_embd; P.output_norm = e->output_norm; P.output = e->output->tiles;
     P.toks = e->toks_dev; P.pos = e->pos_dev;
     P.sync = cx->grid_sync; P.partials = st->partials; P.error_flag = cx->error_flag_dev;
-    P.slots = st->slots; P.scratch = st->scratch; P.flags = flags; P.trace = st->trace; P.gdn_off = st->gdn_off; P.had_base = st->had_base; P.attn_base = st->attn_base; P.attn_g = st->attn_g; P.att_sc = st->att_sc; P.att_stride = st->att_stride; P.att_cnt = st->att_cnt;
+    P.slots = st->slots; P.scratch = st->scratch; P.w_off = st->scratch - (int)step_w_bytes(c); P.flags = flags; P.trace = st->trace; P.gdn_off = st->gdn_off; P.attn_base = st->attn_base; P.attn_g = st->attn_g; P.att_sc = st->att_sc; P.att_stride = st->att_stride; P.att_cnt = st->att_cnt;
     it_note_op(cx);
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)st->grid); cfg.blockDim = dim3(ST_THREADS); cfg.dynamicSmemBytes = (size_t)st->slots * ST_CHUNK + st->scratch + ST_BARS; cfg.stream = cx->stream;
+    cfg.gridDim = dim3((unsigned)st->grid); cfg.blockDim = dim3(ST_THREADS); cfg.dynamicSmemBytes = step_smem_bytes(c, st->slots); cfg.stream = cx->stream;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeCooperative; attr[0].val.cooperative = 1;
     cfg.attrs = attr; cfg.numAttrs = st->cooperative ? 1 : 0;
     IT_CUDA(cudaLaunchKernelEx(&cfg, k_decode_step, P));
-    e->q8->n = (size_t)c.n_embd;
     return IT_OK;
 }
 
 // Diagnostics (IT_STEP_TRACE=1 when the engine is built): the nanosecond clock of CTA 0 and of the last CTA when they arrive
-// at and leave each grid barrier of the most recent step: out[(cta * max + barrier) * 2 + {0, 1}], cta in {0, 1}.
+// at and leave each wait in front of a matrix phase of the most recent step: out[(cta * max + barrier) * 2 + {0, 1}], cta in {0, 1}.
 IT_API int it_engine_step_trace(it_engine* e, uint64_t* out, size_t max_barriers) {
     IT_CHECK_ARG(e && out, "it_engine_step_trace: null argument");
     if (!e->step || !e->step->trace) return it_fail(IT_ESTATE, "it_engine_step_trace: the engine was not built with IT_STEP_TRACE=1, or does not run the step kernel");

@@ -398,6 +398,36 @@ def test_a_short_context_keeps_short_row_buffers():
     assert held[1024] - held[256] > rows, (held, rows)
 
 
+@pytest.mark.parametrize("over", [
+    dict(n_embd=3072, n_ff=5120, ssm_vheads=16, ssm_groups=4, ssm_inner=2048, n_head=8, head_dim=128, conv_k=3, gdn_v_grouped=0, n_vocab=5000),   # gate/up and head cut across CTAs, general conv
+    dict(n_embd=2048, n_ff=5120, ssm_vheads=24, ssm_groups=8, ssm_inner=3072, n_head=16, n_head_kv=4, head_dim=64, n_vocab=4767, conv_k=2),      # 149 row groups of the head, the last one short
+    dict(n_embd=5120, n_ff=1024, ssm_vheads=48, ssm_groups=16, ssm_inner=6144, full_attn_interval=2, n_vocab=64),                                # 160 row groups for the residual, CTAs without any of the head
+    dict(n_embd=8192, n_ff=2048, n_vocab=200)])                                                                                                  # widest norm row: fewer ring slots
+def test_step_kernel_geometries(monkeypatch, over):
+    """Matrices that cut a row group between two CTAs, leave CTAs without work, or leave the ring fewer slots: logits, picks and
+    state of the persistent kernel equal the per-op schedule's bit for bit."""
+    from irontimber_b200.engine import CudaEngine, ModelConfig
+    results = []
+    for flag in ("1", "0"):
+        monkeypatch.setenv("IT_STEP_KERNEL", flag)
+        cfg = tiny_config(ModelConfig)
+        for k, v in over.items():
+            setattr(cfg, k, v)
+        eng = CudaEngine(cfg, seed=47, with_mtp=False)
+        try:
+            prompt = [t % cfg.n_vocab for t in PROMPT]
+            hist = eng.generate(prompt, 24)
+            lg = bits(eng.eval(hist[-1:])).copy()
+            states = [bits(eng.state(il, k)).copy() for il in range(cfg.n_layer) for k in ((0, 1) if cfg.is_recurrent(il) else (2, 3))]
+            results.append((hist, lg, states, eng.step_kernels()))
+        finally:
+            eng.close()
+    a, b = results
+    assert a[3] == 1 and b[3] > 10
+    assert a[0] == b[0] and np.array_equal(a[1], b[1])
+    assert all(np.array_equal(x, y) for x, y in zip(a[2], b[2]))
+
+
 def test_step_kernel_matches_the_per_op_schedule_at_long_positions(monkeypatch):
     """Decode steps after a 330-token prompt: the attention block of the step kernel then walks more K tiles and V chunks
     than its ring holds and crosses a 32-position tile boundary.  Picks, logits and caches equal the per-op schedule's."""
