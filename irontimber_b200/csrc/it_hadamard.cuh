@@ -137,4 +137,109 @@ __device__ __forceinline__ void it_hadamard_block(it_had_smem& sm, const unsigne
     if ((tid & 63) == 0) qd[tok * (q_stride / 256) + blk * 4 + (tid >> 6)] = d;
 }
 
+// ---- the same transform, 64 threads a block and 16 values a thread ---------------------------------------------------------
+// Bit-identical to it_hadamard_block (the same pairs in the same stage order).  Thread j (0..63, two warps) passes through three
+// layouts: elements 16 j .. (strides 1..8), every 16th of a run of 256 (16..128), four neighbours of each of the block's four
+// q8k groups (256, 512).  Between them the block goes through shared memory in a padded layout: a run of 16 is 20 floats apart
+// from the next, a run of 256 336 floats, so that neither the 16-byte accesses of the first and last layout nor the 4-byte
+// ones of the second meet in a bank.  About 430 instructions a thread and three barriers of 64 threads; the 256-thread form
+// has 150 and eleven barriers of 256, i.e. 1.4 times the instructions a block.
+constexpr int IT_HAD_PITCH = 1344;                     // floats of a block in the padded layout
+__device__ __forceinline__ int it_had_at(int e) { return e + 4 * (e >> 4) + 16 * (e >> 8); }
+__device__ __forceinline__ void it_had16_stage(float (&v)[16], int h) {
+#pragma unroll
+    for (int i = 0; i < 16; i++) if (!(i & h)) { const float a = v[i], b = v[i | h]; v[i] = it_add(a, b); v[i | h] = it_sub(a, b); }
+}
+// v: elements 16 j + i in, element 256 g + 4 j + u at 4 g + u out, scaled by 1/32.  ex: the block's IT_HAD_PITCH floats; `sync`
+// joins the block's 64 threads.
+template <typename Sync> __device__ __forceinline__ void it_had16_rotate(float (&v)[16], float* ex, int j, Sync&& sync) {
+    const int lane = j & 31;
+    it_had16_stage(v, 1); it_had16_stage(v, 2); it_had16_stage(v, 4); it_had16_stage(v, 8);
+    float* p1 = ex + it_had_at(16 * j);
+#pragma unroll
+    for (int u = 0; u < 4; u++) *reinterpret_cast<float4*>(p1 + 4 * u) = make_float4(v[4 * u], v[4 * u + 1], v[4 * u + 2], v[4 * u + 3]);
+    sync();
+    float* p2 = ex + 336 * ((lane >> 4) + 2 * (j >> 5)) + (lane & 15);
+#pragma unroll
+    for (int i = 0; i < 16; i++) v[i] = p2[20 * i];
+    it_had16_stage(v, 1); it_had16_stage(v, 2); it_had16_stage(v, 4); it_had16_stage(v, 8);
+#pragma unroll
+    for (int i = 0; i < 16; i++) p2[20 * i] = v[i];
+    sync();
+    const float* p3 = ex + it_had_at(4 * j);
+#pragma unroll
+    for (int g = 0; g < 4; g++) { const float4 t = *reinterpret_cast<const float4*>(p3 + 336 * g); v[4 * g] = t.x; v[4 * g + 1] = t.y; v[4 * g + 2] = t.z; v[4 * g + 3] = t.w; }
+    it_had16_stage(v, 4); it_had16_stage(v, 8);
+#pragma unroll
+    for (int i = 0; i < 16; i++) v[i] = it_mul(v[i], 0.03125f);
+}
+// q8k codes of v (element 256 g + 4 j + u at 4 g + u): word g holds the thread's four codes of group g; in lane l < 4, d is the
+// scale of group l and sum the sum of group l's codes over the lane's warp (128 elements).  mx: 8 floats of shared memory.
+struct it_had16_codes { uint32_t packed[4]; float d; int sum; };
+template <typename Sync> __device__ __forceinline__ it_had16_codes it_had16_quantise(const float (&v)[16], float* mx, int j, Sync&& sync) {
+    const int lane = j & 31;
+    it_had16_codes r;
+    // the first element of largest magnitude of each group; b stands for higher indices than a, a NaN is never taken
+    auto larger = [](float a, float b, bool tie) { return fabsf(b) > fabsf(a) || (tie && fabsf(b) == fabsf(a)) ? b : a; };
+    float any = 0.f, best[4];
+#pragma unroll
+    for (int i = 0; i < 16; i++) any += v[i];
+#pragma unroll
+    for (int g = 0; g < 4; g++) {
+        best[g] = 0.f;
+#pragma unroll
+        for (int u = 0; u < 4; u++) best[g] = larger(best[g], v[4 * g + u], false);
+    }
+    const bool odd = __any_sync(0xffffffffu, !(fabsf(any) <= 3.4e38f));
+    // lanes in ranges that double; the first two steps also share the groups out: lane l keeps group 2 (l & 1) + (l >> 1 & 1)
+    float k0 = lane & 1 ? best[2] : best[0], k1 = lane & 1 ? best[3] : best[1];
+    const float g0 = __shfl_xor_sync(0xffffffffu, lane & 1 ? best[0] : best[2], 1), g1 = __shfl_xor_sync(0xffffffffu, lane & 1 ? best[1] : best[3], 1);
+    k0 = larger(k0, g0, lane & 1); k1 = larger(k1, g1, lane & 1);
+    const float g2 = __shfl_xor_sync(0xffffffffu, lane & 2 ? k0 : k1, 2);
+    k0 = larger(lane & 2 ? k1 : k0, g2, lane & 2);
+#pragma unroll
+    for (int m = 4; m <= 16; m <<= 1) k0 = larger(k0, __shfl_xor_sync(0xffffffffu, k0, m), lane & m);
+    if (lane < 4) mx[2 * (2 * (lane & 1) + (lane >> 1)) + (j >> 5)] = k0;
+    sync();
+    const float2 ab = *reinterpret_cast<const float2*>(mx + 2 * (lane & 3));     // lane g (and g + 4, ...): group g's two halves
+    const float val = fabsf(ab.y) > fabsf(ab.x) ? ab.y : ab.x;           // equal magnitudes: the lower index
+    const float isc = val != 0.f ? __fdiv_rn(-127.0f, val) : 0.f;        // a group of zeros keeps 0, and so codes of 0
+    // 1 / scale by a Newton step and a corrected quotient in f64, rounded once: exact to more than twice f32's digits, so the
+    // rounding is the division's; without branches, it overlaps the codes
+    {
+        float r0f; asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r0f) : "f"(isc));
+        const double b = isc, r0 = r0f, r1 = fma(r0, fma(-b, r0, 1.0), r0);
+        r.d = __double2float_rn(fma(fma(-b, r1, 1.0), r1, r1));
+    }
+    if (!(fabsf(isc) >= 3.7e-37f && fabsf(isc) < 1e37f)) r.d = val != 0.f ? __fdiv_rn(1.0f, isc) : 0.f;
+    // codes: round to nearest even by adding 1.5 * 2^23 (|is * v| <= 127, and a conversion takes eight cycles of the sub-core where
+    // an addition takes one); a scale that overflowed (a group below 4e-37) and values that are not finite go through the
+    // conversion and its saturation
+    const bool convert = odd || __any_sync(0xffffffffu, fabsf(isc) > 3.4e38f);
+    int total[4];
+#pragma unroll
+    for (int g = 0; g < 4; g++) {
+        const float is = __shfl_sync(0xffffffffu, isc, g);
+        unsigned q[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) q[u] = __float_as_uint(__fadd_rn(it_mul(is, v[4 * g + u]), 12582912.0f));
+        if (convert) {
+#pragma unroll
+            for (int u = 0; u < 4; u++) q[u] = is == 0.f ? 0u : (unsigned)min(__float2int_rn(it_mul(is, v[4 * g + u])), 127);
+            total[g] = (int)(q[0] + q[1] + q[2] + q[3]);             // saturated below, a code is its low byte and still counts whole
+        }
+        r.packed[g] = __byte_perm(__byte_perm(q[0], q[1], 0x0040), __byte_perm(q[2], q[3], 0x0040), 0x5410);
+        if (is == 0.f) r.packed[g] = 0;                              // a group of zeros, or one whose maximum is infinite
+    }
+    const int t0 = __reduce_add_sync(0xffffffffu, __dp4a((int)r.packed[0], 0x01010101, __dp4a((int)r.packed[1], 0x01010101, 0) << 16));   // two groups' sums
+    const int t1 = __reduce_add_sync(0xffffffffu, __dp4a((int)r.packed[2], 0x01010101, __dp4a((int)r.packed[3], 0x01010101, 0) << 16));   // (below 2^15) to a word
+    const int t = lane & 2 ? t1 : t0, lo = (short)t;
+    r.sum = lane & 1 ? (t - lo) >> 16 : lo;
+    if (convert) {
+#pragma unroll
+        for (int g = 0; g < 4; g++) { const int t4 = __reduce_add_sync(0xffffffffu, total[g]); if (lane == g) r.sum = t4; }
+    }
+    return r;
+}
+
 }  // namespace

@@ -77,11 +77,11 @@ IT_HD uint32_t it_float_to_bits(float f) {
 }
 
 // exp(x).  n = round(x / ln 2), r = x - n ln 2 in two pieces, degree-6 polynomial, exact scaling by 2^n.
+// (The rounding goes through an addition of 1.5 * 2^23, whose low bits are the integer: a conversion takes eight times as long as an
+// addition on the device.  What lies outside the range is computed like the rest and replaced at the end, so that several calls
+// overlap.)
 IT_HD float it_expf_inline(float x) {
-    if (!(x == x)) return x;
-    if (x > 88.72283935546875f) return it_bits_to_float(0x7f800000u);
-    if (x < -103.97208404541015625f) return 0.0f;
-    const float n = rintf(it_mul(x, 1.44269502162933349609375f));
+    const float t = it_add(it_mul(x, 1.44269502162933349609375f), 12582912.0f), n = it_sub(t, 12582912.0f);
     float r = it_fma(n, -0.693145751953125f, x);
     r = it_fma(n, -1.42860682030941723212e-6f, r);
     float p = 1.9875691500e-4f;
@@ -92,9 +92,11 @@ IT_HD float it_expf_inline(float x) {
     p = it_fma(p, r, 5.0000001201e-1f);
     p = it_fma(it_mul(p, r), r, r);
     p = it_add(p, 1.0f);
-    const int ni = (int)n, n1 = ni / 2, n2 = ni - n1;    // two exact power-of-two factors keep subnormal results right
-    const float s1 = it_bits_to_float((uint32_t)(n1 + 127) << 23), s2 = it_bits_to_float((uint32_t)(n2 + 127) << 23);
-    return it_mul(it_mul(p, s1), s2);
+    const int ni = (int)(it_float_to_bits(t) - 0x4b400000u), n1 = ni / 2, n2 = (int)((uint32_t)ni - (uint32_t)n1);    // two exact power-of-two factors keep subnormal results right
+    const float s1 = it_bits_to_float((uint32_t)(n1 + 127) << 23), s2 = it_bits_to_float(((uint32_t)n2 + 127u) << 23);
+    p = it_mul(it_mul(p, s1), s2);
+    p = x > 88.72283935546875f ? it_bits_to_float(0x7f800000u) : x < -103.97208404541015625f ? 0.0f : p;
+    return x == x ? p : x;
 }
 IT_HD_BIG float it_expf(float x) { return it_expf_inline(x); }
 

@@ -42,6 +42,7 @@
 #include "it_engine.h"
 #include "it_support.h"
 #include "it_pipe.cuh"
+#include "it_hadamard.cuh"
 #include <algorithm>
 #include <vector>
 
@@ -59,9 +60,7 @@ constexpr int ST_TERMS = ST_TPC * 32;                  // terms of one chunk (fl
 constexpr int ST_SMEM = 227 * 1024;                    // dynamic shared memory of the CTA
 constexpr int ST_BARS = 1024;                          // bytes reserved for mbarriers, flags, layer descriptions and spans
 constexpr int ST_SD = 128;                             // delta-rule state size this kernel is built for
-constexpr int ST_HB = ST_NCONS / 2;                    // Hadamard blocks of 1024 transformed at a time, two warps each
-constexpr int ST_HPITCH = 1344;                        // floats of a block in the transform's exchange area: 64 runs of 16, padded
-constexpr int ST_RED = 384;                            // bytes: the dense row's eight f64 warp sums, then the transform's [8] sums of squares and [ST_HB][4][2] group maxima
+constexpr int ST_RED = 384;                            // bytes: the dense row's eight f64 warp sums, then the transform's [8] sums of squares and [4][2] group maxima
 
 // A CTA's share of one ternary matrix.  The matrix is a sequence of chunks (eight 32 x 128 tiles of one row group, row
 // groups in order); every CTA gets an equal run of it, whatever row group the run starts or ends in (5120 rows are 160 row
@@ -312,22 +311,18 @@ __device__ __forceinline__ void warm_layer(const StepParams& P, const Cta& c, co
 }
 
 // ---------------------------------------------------------------- row transform
-// [rmsnorm ->] signs -> Hadamard over blocks of 1024 -> q8k of one row of nblk blocks, from global memory into this CTA's
-// scratch, in the operation order of it_hadamard_block (it_hadamard.cuh).  Two warps take a block, six blocks run at a time.
-// A thread holds 16 values through three layouts: 16 consecutive ones (strides 1..8), every 16th of a run of 256 (16..128),
-// a run of four from each of the block's four q8k groups (256, 512); the row comes in through cp.async into the padded layout
-// that makes the first read and both changes of layout free of bank conflicts.  (Read straight into registers, 64 bytes a thread,
-// 24 KB cost 2000 cycles with all SMs at it; the same 16-byte pieces in lane order cost 560.)  The norm's weights and the dense
-// row do not depend on the step and are in shared memory before the barrier in front of the phase opens.
+// [rmsnorm ->] signs -> Hadamard -> q8k of one block of 1024 of a row, by the CTA that owns it, in the operation order of
+// it_hadamard_block (it_hadamard.cuh).  All consumer warps bring the row in (a normed one whole, else the block) and form the
+// norm; two of them transform the block, 16 values a thread.  The row is read in lane order and put into the padded layout
+// of the transform (64 bytes a thread straight into registers: 24 KB cost 2000 cycles with all SMs at it, in lane order 560).
+// The norm's weights and the dense row do not depend on the step and are in shared memory before the row is.
 struct RowIn {
     const granule* x; unsigned tag; const float* plain;      // the row (norm) or its block, as granules of a phase, or (plain) as floats
     const uint32_t* signs; float* normed;                    // normed: where the normed row goes, or null
     granule* codes; unsigned code_tag; int codes_copy;       // where the quantised block goes (copies codes_copy granules apart), or null
     int nblk, blk; bool norm, dense;                         // blocks brought in, the one to transform; dense: multiply the normed row with this CTA's dense row
 };
-__device__ __forceinline__ bool ieee_negative_zero(float x) { return __float_as_uint(x) == 0x80000000u; }
 __device__ __forceinline__ void pair_sync() { asm volatile("bar.sync 5, 64;" ::: "memory"); }
-__device__ __forceinline__ int ex_at(int e) { return e + 4 * (e >> 4) + 16 * (e >> 8); }      // element e of a row in the padded layout: 1344 floats a block, 336 a run of 256, 20 a run of 16
 // nblk blocks of 1024 rows (32 row groups, 352 granules: a thread each) from `x` into the padded layout at `ex`
 constexpr int ST_GPB = 32 * ST_GPU;
 static_assert(ST_GPB <= ST_CT, "a granule of every block per thread");
@@ -335,15 +330,15 @@ __device__ __forceinline__ void row_place(const StepParams& P, const Cta& c, flo
     constexpr int N = 6;
     if (c.tid >= ST_GPB) return;
     bool two; const int r = granule_row(c.tid, two);
-    float *p0 = ex + ex_at(r), *p1 = ex + ex_at(r + ST_GPU), *p2 = two ? p1 : ex + ex_at(r + 2 * ST_GPU);
+    float *p0 = ex + it_had_at(r), *p1 = ex + it_had_at(r + ST_GPU), *p2 = two ? p1 : ex + it_had_at(r + 2 * ST_GPU);
 #pragma unroll 1
-    for (int b = 0; b < nblk; b += N, p0 += N * ST_HPITCH, p1 += N * ST_HPITCH, p2 += N * ST_HPITCH) {
+    for (int b = 0; b < nblk; b += N, p0 += N * IT_HAD_PITCH, p1 += N * IT_HAD_PITCH, p2 += N * IT_HAD_PITCH) {
         granule g[N];
         const int m = min(N, nblk - b);
         read_granules(g, x + b * ST_GPB + c.tid, ST_GPB, m, tag, c, P.error_flag, 14);
 #pragma unroll
         for (int u = 0; u < N; u++) {
-            const int o = min(u, m - 1) * ST_HPITCH;
+            const int o = min(u, m - 1) * IT_HAD_PITCH;
             p2[o] = __uint_as_float(two ? g[u].y : g[u].z); p0[o] = __uint_as_float(g[u].x); p1[o] = __uint_as_float(g[u].y);
         }
     }
@@ -354,7 +349,7 @@ __device__ __noinline__ void norm_request(float* wb, const float* w, const float
     const int tid = threadIdx.x;
 #pragma unroll 1
     for (int i = 4 * tid; i < e; i += 4 * ST_CT) {
-        cp_async16(wb + (i >> 10) * ST_HPITCH + ex_at(i & 1023), w + i);
+        cp_async16(wb + (i >> 10) * IT_HAD_PITCH + it_had_at(i & 1023), w + i);
         if (dense) cp_async16(wb - e + i, dense + i);
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
@@ -368,7 +363,7 @@ __device__ __forceinline__ void block_transform(const StepParams& P, const Cta& 
     cons_sync();                                             // the scratch is nobody's any more (the block before may still have been writing state)
     if (in.plain) {
 #pragma unroll 1
-        for (int i = 4 * tid; i < n; i += 4 * ST_CT) *reinterpret_cast<float4*>(ex0 + ex_at(i)) = *reinterpret_cast<const float4*>(in.plain + i);
+        for (int i = 4 * tid; i < n; i += 4 * ST_CT) *reinterpret_cast<float4*>(ex0 + it_had_at(i)) = *reinterpret_cast<const float4*>(in.plain + i);
     } else row_place(P, c, ex0, in.x, in.nblk, in.tag);
     asm volatile("cp.async.wait_group 0;" ::: "memory");             // the norm's weights
     cons_sync();
@@ -378,14 +373,14 @@ __device__ __forceinline__ void block_transform(const StepParams& P, const Cta& 
         // rmsnorm of the whole row in the order of k_rmsnorm_wide: thread i of 256 adds x[i]^2, x[i + 256]^2, ...; warp
         // butterflies; eight warp sums in ascending order
         if (tid < 256) {
-            const float* xp = ex0 + ex_at(tid);
+            const float* xp = ex0 + it_had_at(tid);
             float s = 0.f, a[4];
 #pragma unroll
             for (int u = 0; u < 4; u++) a[u] = xp[336 * u];
 #pragma unroll 1
             for (int k = 1; k <= in.nblk; k++) {                     // the next block's four elements are requested before this one's are added
                 float b[4];
-                xp += k < in.nblk ? ST_HPITCH : 0;
+                xp += k < in.nblk ? IT_HAD_PITCH : 0;
 #pragma unroll
                 for (int u = 0; u < 4; u++) b[u] = xp[336 * u];
 #pragma unroll
@@ -402,14 +397,14 @@ __device__ __forceinline__ void block_transform(const StepParams& P, const Cta& 
         sc = __fdiv_rn(1.0f, __fsqrt_rn(it_add(__fdiv_rn(tot, (float)n), P.eps)));
         if (in.normed) {
 #pragma unroll 1
-            for (int i = tid; i < n; i += ST_CT) { const int o = (i >> 10) * ST_HPITCH + ex_at(i & 1023); in.normed[i] = it_mul(it_mul(ex0[o], sc), wb[o]); }
+            for (int i = tid; i < n; i += ST_CT) { const int o = (i >> 10) * IT_HAD_PITCH + it_had_at(i & 1023); in.normed[i] = it_mul(it_mul(ex0[o], sc), wb[o]); }
             cons_sync();
         }
         if (in.dense) {
             if (tid < 256) {
                 // one row of the beta / alpha matrices times the normed row, in the order of k_dense_rows: thread i adds the
                 // products i, i + 256, ... in f64, warp butterflies, eight warp sums in ascending order (by sum warp 1)
-                const float* xp = ex0 + ex_at(tid); const float* wp = wb + ex_at(tid); const float* dp = wb - P.e + tid;
+                const float* xp = ex0 + it_had_at(tid); const float* wp = wb + it_had_at(tid); const float* dp = wb - P.e + tid;
                 double d = 0.0;
 #pragma unroll 2
                 for (int k = 0; k < in.nblk * 4; k++) d += (double)it_mul(dp[256 * k], it_mul(it_mul(xp[336 * k], sc), wp[336 * k]));
@@ -421,14 +416,14 @@ __device__ __forceinline__ void block_transform(const StepParams& P, const Cta& 
         }
     }
     if (warp < 2 && in.codes) {
-        float* ex = ex0 + in.blk * ST_HPITCH;
+        float* ex = ex0 + in.blk * IT_HAD_PITCH;
         {
             float v[16];
-            float* p1 = ex + ex_at(16 * j);
+            float* p1 = ex + it_had_at(16 * j);
 #pragma unroll
             for (int u = 0; u < 4; u++) { const float4 t = *reinterpret_cast<const float4*>(p1 + 4 * u); v[4 * u] = t.x; v[4 * u + 1] = t.y; v[4 * u + 2] = t.z; v[4 * u + 3] = t.w; }
             if (in.norm) {
-                const float* wp = wb + in.blk * ST_HPITCH + ex_at(16 * j);
+                const float* wp = wb + in.blk * IT_HAD_PITCH + it_had_at(16 * j);
 #pragma unroll
                 for (int u = 0; u < 4; u++) {
                     const float4 w = *reinterpret_cast<const float4*>(wp + 4 * u);
@@ -439,83 +434,14 @@ __device__ __forceinline__ void block_transform(const StepParams& P, const Cta& 
             const unsigned m16 = reinterpret_cast<const unsigned short*>(in.signs)[j];
 #pragma unroll
             for (int i = 0; i < 16; i++) v[i] = __uint_as_float(__float_as_uint(v[i]) ^ ((m16 << (31 - i)) & 0x80000000u));     // times +-1
-            auto stage = [&](int h) {
-#pragma unroll
-                for (int i = 0; i < 16; i++) if (!(i & h)) { const float a = v[i], b = v[i | h]; v[i] = it_add(a, b); v[i | h] = it_sub(a, b); }
-            };
-            stage(1); stage(2); stage(4); stage(8);
-#pragma unroll
-            for (int u = 0; u < 4; u++) *reinterpret_cast<float4*>(p1 + 4 * u) = make_float4(v[4 * u], v[4 * u + 1], v[4 * u + 2], v[4 * u + 3]);
-            pair_sync();
-            float* p2 = ex + 336 * ((lane >> 4) + 2 * half) + (lane & 15);
-#pragma unroll
-            for (int i = 0; i < 16; i++) v[i] = p2[20 * i];
-            stage(1); stage(2); stage(4); stage(8);
-#pragma unroll
-            for (int i = 0; i < 16; i++) p2[20 * i] = v[i];
-            pair_sync();
-            const float* p3 = ex + ex_at(4 * j);                         // group g (of 256): values 4 g .. 4 g + 3
-#pragma unroll
-            for (int g = 0; g < 4; g++) { const float4 t = *reinterpret_cast<const float4*>(p3 + 336 * g); v[4 * g] = t.x; v[4 * g + 1] = t.y; v[4 * g + 2] = t.z; v[4 * g + 3] = t.w; }
-            stage(4); stage(8);
-            // q8k: the first element of maximum magnitude of each group sets its scale
-            float* mx = red + 8;
-            float any = 0.f, best[4];
-#pragma unroll
-            for (int i = 0; i < 16; i++) { v[i] = it_mul(v[i], 0.03125f); any += v[i]; }
-            // the first element of largest magnitude; b stands for higher indices than a, a NaN is never taken
-            auto larger = [](float a, float b, bool tie) { return fabsf(b) > fabsf(a) || (tie && fabsf(b) == fabsf(a)) ? b : a; };
-#pragma unroll
-            for (int g = 0; g < 4; g++) { best[g] = 0.f; for (int u = 0; u < 4; u++) best[g] = larger(best[g], v[4 * g + u], false); }
-            const bool odd = __any_sync(0xffffffffu, !(fabsf(any) <= 3.4e38f));
-            // lanes in ranges that double: the first two steps also share the groups out, lane l keeps group 2 (l & 1) + (l >> 1 & 1)
-            float k0 = lane & 1 ? best[2] : best[0], k1 = lane & 1 ? best[3] : best[1];
-            const float g0 = __shfl_xor_sync(0xffffffffu, lane & 1 ? best[0] : best[2], 1), g1 = __shfl_xor_sync(0xffffffffu, lane & 1 ? best[1] : best[3], 1);
-            k0 = larger(k0, g0, lane & 1); k1 = larger(k1, g1, lane & 1);
-            const float g2 = __shfl_xor_sync(0xffffffffu, lane & 2 ? k0 : k1, 2);
-            k0 = larger(lane & 2 ? k1 : k0, g2, lane & 2);
-#pragma unroll
-            for (int m = 4; m <= 16; m <<= 1) k0 = larger(k0, __shfl_xor_sync(0xffffffffu, k0, m), lane & m);
-            if (lane < 4) mx[2 * (2 * (lane & 1) + (lane >> 1)) + half] = k0;
-            pair_sync();
-            float isc = 0.f;
-            {   // lane g (and g + 4, ...): group g's scale
-                const float2 ab = *reinterpret_cast<const float2*>(mx + 2 * (lane & 3));
-                const float val = fabsf(ab.y) > fabsf(ab.x) ? ab.y : ab.x;       // equal magnitudes: the lower index
-                if (val != 0.f) isc = __fdiv_rn(-127.0f, val);       // a group of zeros keeps 0, and so codes of 0
-            }
-            // codes: round to nearest even by adding 1.5 * 2^23 (|is * v| <= 127, and a conversion takes eight cycles of the sub-core where an
-            // addition takes one); a scale that overflowed (a group below 4e-37) and values that are not finite go through the conversion
-            // and its saturation
-            // (1 / scale by a Newton step and a corrected quotient in f64, rounded once: exact to more than twice f32's digits, so the
-            // rounding is the division's; branch-free, it overlaps the codes)
-            float dk;
-            { float r; asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(isc)); const double b = isc, r0 = r, r1 = fma(r0, fma(-b, r0, 1.0), r0); dk = __double2float_rn(fma(fma(-b, r1, 1.0), r1, r1)); }
-            if (!(fabsf(isc) >= 3.7e-37f && fabsf(isc) < 1e37f)) dk = isc != 0.f || ieee_negative_zero(isc) ? __fdiv_rn(1.0f, isc) : 0.f;
-            const bool odd_scale = odd || __any_sync(0xffffffffu, fabsf(isc) > 3.4e38f);
-            uint32_t packed[4];
-#pragma unroll
-            for (int g = 0; g < 4; g++) {
-                const float is = __shfl_sync(0xffffffffu, isc, g);
-                unsigned q[4];
-#pragma unroll
-                for (int u = 0; u < 4; u++) q[u] = __float_as_uint(__fadd_rn(it_mul(is, v[4 * g + u]), 12582912.0f));
-                if (odd_scale) {
-#pragma unroll
-                    for (int u = 0; u < 4; u++) q[u] = (unsigned)min(__float2int_rn(it_mul(is, v[4 * g + u])), 127);
-                }
-                packed[g] = __byte_perm(__byte_perm(q[0], q[1], 0x0040), __byte_perm(q[2], q[3], 0x0040), 0x5410);
-                if (is == 0.f) packed[g] = 0;                        // a group of zeros, or one whose maximum is infinite
-            }
-            const int t0 = __reduce_add_sync(0xffffffffu, __dp4a((int)packed[0], 0x01010101, __dp4a((int)packed[1], 0x01010101, 0) << 16));   // two groups' code sums
-            const int t1 = __reduce_add_sync(0xffffffffu, __dp4a((int)packed[2], 0x01010101, __dp4a((int)packed[3], 0x01010101, 0) << 16));   // (at most 128 * 127 in magnitude) to a word
-            const int t = lane & 2 ? t1 : t0, lo = (short)t, sum = lane & 1 ? (t - lo) >> 16 : lo;
+            it_had16_rotate(v, ex, j, [] { pair_sync(); });
+            const it_had16_codes q = it_had16_quantise(v, red + 8, j, [] { pair_sync(); });
             // thread j: its four words of codes; threads 0..3 of each half also the group's scale and the half's sum
 #pragma unroll 1
             for (int k = 0; k < ST_COPIES; k++) {
                 granule* to = in.codes + k * in.codes_copy + j;
-                st_granule(to, packed[0], packed[1], packed[2], in.code_tag);
-                st_granule(to + 64, packed[3], __float_as_uint(dk), (unsigned)sum, in.code_tag);
+                st_granule(to, q.packed[0], q.packed[1], q.packed[2], in.code_tag);
+                st_granule(to + 64, q.packed[3], __float_as_uint(q.d), (unsigned)q.sum, in.code_tag);
             }
         }
     }
@@ -1327,13 +1253,13 @@ struct it_step_state {
 static int step_widest(const it_model_config& c) { return std::max(std::max(c.n_embd, c.n_ff), std::max(c.ssm_inner, c.n_head * c.head_dim)); }
 // the state tile of the delta-net block comes in while the input projection's chunks run: behind their terms
 static size_t step_gdn_off(const it_model_config& c, int slots) { return (size_t)terms_at(c.n_embd / 128) + (size_t)slots * ST_TERMS * 4; }
-static size_t step_w_bytes(const it_model_config& c) { return (size_t)(c.n_embd / 1024) * ST_HPITCH * 4; }
+static size_t step_w_bytes(const it_model_config& c) { return (size_t)(c.n_embd / 1024) * IT_HAD_PITCH * 4; }
 static size_t step_scratch_bytes(const it_model_config& c, int slots) {
     size_t s = (size_t)terms_at(step_widest(c) / 128) + (size_t)slots * ST_TERMS * 4;
-    s = std::max(s, (size_t)ST_RED + (size_t)(c.n_embd / 1024) * ST_HPITCH * 4 + (size_t)c.n_embd * 4 + step_w_bytes(c));      // a normed row, a dense row, the norm's weights
+    s = std::max(s, (size_t)ST_RED + (size_t)(c.n_embd / 1024) * IT_HAD_PITCH * 4 + (size_t)c.n_embd * 4 + step_w_bytes(c));      // a normed row, a dense row, the norm's weights
     s = std::max(s, step_gdn_off(c, slots) + (size_t)ST_SD * ST_SD * 4);
     // a norm's weights and a dense row come in while the widest matrix's chunks run, and stay while their row is transformed
-    const size_t below = std::max((size_t)terms_at(step_widest(c) / 128) + (size_t)slots * ST_TERMS * 4, (size_t)terms_at(c.n_embd / 128) + (size_t)(c.n_embd / 1024) * ST_HPITCH * 4);
+    const size_t below = std::max((size_t)terms_at(step_widest(c) / 128) + (size_t)slots * ST_TERMS * 4, (size_t)terms_at(c.n_embd / 128) + (size_t)(c.n_embd / 1024) * IT_HAD_PITCH * 4);
     s = std::max(s, below + (size_t)c.n_embd * 4 + step_w_bytes(c));
     s = std::max(s, ((size_t)c.ctx_len + 4 + 4 * c.head_dim + 48) * 4 + 128 + 3 * (size_t)c.head_dim * 64);
     return (s + 127) / 128 * 128;

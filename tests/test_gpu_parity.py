@@ -110,6 +110,34 @@ def test_hadamard_q8_bit_exact(be, orc, n, ntok, mode):
     q.close()
 
 
+# on either side of two blocks per SM (296), where 64 threads take a block instead of 256
+@pytest.mark.parametrize("n,ntok", [(1024, 295), (1024, 296), (5120, 59), (5120, 60), (6144, 50), (17408, 18)])
+@pytest.mark.parametrize("mode", ["signs", "perm", "perm2", "norotate"])
+def test_hadamard_q8_many_rows_bit_exact(be, orc, n, ntok, mode):
+    rng = np.random.default_rng(n + ntok)
+    X = rng.standard_normal((ntok, n)).astype(np.float32)
+    X[0, :256] = 0.0                       # an all-zero q8k block
+    X[0, 300] = 2.5; X[0, 301] = -2.5      # equal magnitudes: the first one decides the sign of iscale
+    X[1] *= 1e-38; X[2, :1024] *= 1e-37    # scales that overflow
+    X[3] *= 3e37                           # sums that overflow
+    X[4, 7] = np.inf; X[5, 1000] = np.nan
+    signs = None if mode == "norotate" else np.where(rng.integers(0, 2, n) == 1, 1.0, -1.0).astype(np.float32)
+    perm = (128, 4, n // 512) if mode == "perm" else (2, 4, n // 8) if mode == "perm2" else None
+    if signs is not None:
+        be.set_signs(signs)
+    q, q1 = be.q8_rows(n, ntok), be.q8_rows(n, 1)
+    be.upload(0, X)
+    be.had_q8(n, ntok, 0, n, q, perm=perm, signs=signs is not None, rotate=mode != "norotate")
+    for t in (0, 1, 2, 3, 4, 5, 6, ntok // 2, ntok - 1):
+        got = q.read(t)
+        be.had_q8(n, 1, t * n, n, q1, perm=perm, signs=signs is not None, rotate=mode != "norotate")
+        assert all(np.array_equal(bits(a) if a.dtype == np.float32 else a, bits(b) if b.dtype == np.float32 else b) for a, b in zip(got, q1.read(0))), t
+        if t in (0, 6, ntok // 2, ntok - 1):
+            d, qs, s = orc.quantize_q8k(orc.hadamard_forward(X[t], 1024, signs, perm) if mode != "norotate" else X[t])
+            assert np.array_equal(got[1], qs) and np.array_equal(bits(got[0]), bits(d)) and np.array_equal(got[2], s)
+    q.close(); q1.close()
+
+
 @pytest.mark.parametrize("inverse", [False, True])
 def test_hadamard_f32_bit_exact(be, orc, inverse):
     rng = np.random.default_rng(5)
