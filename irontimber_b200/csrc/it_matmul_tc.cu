@@ -20,11 +20,14 @@
 //            whole row of blocks: ascending block order, one thread per (row, activation row) pair - the CPU's order, bit for bit.
 // What bounds it: per block and SM sub-core the epilogue's 64 pairs of values cost about 6.5 cycles each (conversion, two products, one
 // addition, every one rounded; a two-value instruction takes two cycles of the f32 pipe) = 420 cycles, the MMAs 256 plus their
-// operands' share of the shared-memory port; measured 970 cycles a block with everything running (1900 before).  What the steps
+// operands' share of the shared-memory port; with everything running a block takes 740 cycles at 64 activation rows and 970 at 128
+// (the epilogue alone 510 and 810, the expanders alone 530 and 660: the roles share the issue slots of their sub-core).  What the steps
 // gave, 34816 x 5120 x 512 rows: 310 us with a row per epilogue thread (256 broadcast loads of scales a block: 1024 cycles of the
 // shared-memory port); 251 with the fragment layout and two-value arithmetic; 242 with conversions instead of biased accumulators; 217 with
 // CTAs that walk several tiles (7 us of 31 per tile were fill and drain); 202 with two blocks a step and eight epilogue warps; 197 with
-// the 16x128b read-out.
+// the 16x128b read-out; 180 with an issuer whose descriptors stay in uniform registers (elect.sync) and whose three waits a step are one look
+// ahead, taken over from the expanders' loop (5120 x 17408 x 64 rows: 59.6 us before, 52.2 now).  What gave nothing: 16 epilogue warps
+// of half the columns, the next step's accumulators on their way across steps, conversions by addition of 1.5 x 2^23.
 // Integer block sums are exact whatever the hardware's summation order, so only the f32 epilogue decides the bits.
 //
 // Every wait is bounded; when one runs out the CTA raises the context's error flag (IT_ETIMEOUT), every role leaves
@@ -40,7 +43,8 @@ constexpr int TC_A_BYTES = TC_ROWS * 128;        // one expanded weight tile
 constexpr int TC_KB = 4;                         // blocks per weight stage: one bulk copy per row group and stage (issuing a bulk copy costs a
                                                  // thread some 250 cycles, so four small copies per block made the producer the bottleneck)
 constexpr int TC_W_BYTES = 4 * TC_KB * IT_TILE_BYTES;   // four row groups x TC_KB consecutive tiles
-constexpr int TC_NA = 2;                         // steps of expanded tiles in flight
+constexpr int TC_NA_MAX = 3;                     // steps of expanded tiles in flight where they fit, else two: with two, an expander waits for the commit of its
+                                                 // own last step and the chain commit - expand - issue - commit sets the pace (14336 x 5120 x 64: 19.9 us, with three 19.2)
 constexpr int TC_NC = 4;                         // barriers the steps commit to in turn; at least the steps of boxes in flight, see the barrier list
 constexpr int TC_SMEM_MAX = 226 * 1024;
 constexpr unsigned TC_TMEM_COLS = 512;           // all of it: 2 * ND accumulators x TOK columns
@@ -55,21 +59,21 @@ template <int NH> struct Tc {
     static constexpr int ND = 256 / TOK;                 // steps of accumulators in tensor memory
     static constexpr int EPI_TOK = TOK / 2;              // activation rows per epilogue warp
     static constexpr int CC = EPI_TOK / 32;              // 32-column chunks per epilogue warp
-    static constexpr int NDW = 2 * (TC_NA + ND);         // ring of per-block row scales: the expanders run at most NA + ND steps ahead of the epilogue
+    static constexpr int NDW = 2 * (TC_NA_MAX + ND);     // ring of per-block row scales: the expanders run at most NA + ND steps ahead of the epilogue
     // kind::i8 instruction descriptor: D s32, A signed 8 bit, B signed 8 bit, both K-major, N = TOK, M = 128
     static constexpr unsigned IDESC = (2u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(TOK >> 3) << 17) | ((unsigned)(TC_ROWS >> 4) << 24);
 };
 
 // Weight stages and activation boxes have rings of their own: the weights come from HBM, the boxes from L2.
 struct TcSmem { int x, a, w, dx, dx_bytes, dw, bars, tmem, flag, total; };
-template <int NH> __host__ __device__ inline TcSmem tc_layout(int nb, int wstages, int dxbufs, int xsteps) {
+template <int NH> __host__ __device__ inline TcSmem tc_layout(int nb, int wstages, int dxbufs, int xsteps, int na) {
     TcSmem L; int o = 0;
     L.x = o; o += xsteps * 2 * Tc<NH>::X_BYTES;    // 1024-byte aligned (128-byte swizzle)
-    L.a = o; o += TC_NA * 2 * TC_A_BYTES;              // 1024-byte aligned
+    L.a = o; o += na * 2 * TC_A_BYTES;              // 1024-byte aligned
     L.w = o; o += wstages * TC_W_BYTES;
     L.dx = o; L.dx_bytes = (nb / 2) * Tc<NH>::TOK * 4; o += dxbufs * L.dx_bytes;
     L.dw = o; o += Tc<NH>::NDW * TC_ROWS * 4;
-    L.bars = o; o += (2 * wstages + xsteps + TC_NA + TC_NC + Tc<NH>::ND + 4) * 8;
+    L.bars = o; o += (2 * wstages + xsteps + na + TC_NC + Tc<NH>::ND + 4) * 8;
     o = (o + 15) & ~15;
     L.tmem = o; o += 16;
     L.flag = o; o += 16;
@@ -87,6 +91,21 @@ __device__ __forceinline__ void tc_mma(unsigned d_tmem, unsigned long long adesc
     asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
                  "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n}"
                  :: "r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "n"(ACC ? 1 : 0), "r"(0u) : "memory");
+}
+// One lane of the warp, chosen by the hardware's own instruction: the compiler then knows that what follows runs once, and keeps descriptors
+// and barrier addresses in the warp's uniform registers (under `lane == 0` it moved them there for every instruction).
+__device__ __forceinline__ bool tc_elect() {
+    unsigned e;
+    asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}" : "=r"(e));
+    return e != 0;
+}
+// Non-blocking probe of three phases at once: their answers are under way together.
+__device__ __forceinline__ bool mbar_poll3(unsigned a, unsigned pa, unsigned b, unsigned pb, unsigned c, unsigned pc) {
+    unsigned ok;
+    asm volatile("{\n.reg .pred p, q, r;\nmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\nmbarrier.test_wait.parity.shared::cta.b64 q, [%3], %4;\n"
+                 "mbarrier.test_wait.parity.shared::cta.b64 r, [%5], %6;\nand.pred p, p, q;\nand.pred p, p, r;\nselp.u32 %0, 1, 0, p;\n}"
+                 : "=r"(ok) : "r"(a), "r"(pa), "r"(b), "r"(pb), "r"(c), "r"(pc) : "memory");
+    return ok != 0;
 }
 __device__ __forceinline__ void tc_commit(unsigned bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" :: "r"(bar) : "memory");
@@ -128,13 +147,13 @@ template <int N> __device__ __forceinline__ void reg_dec() { asm volatile("setma
 
 template <int NH>
 __global__ void __launch_bounds__(TC_THREADS, 1)
-k_matmul_tc(const __grid_constant__ CUtensorMap xmap, const uint8_t* __restrict__ tiles, int nb, int rows, int row_groups, int wstages, int ntiles, int tok_tiles, int dxbufs, int xsteps,
+k_matmul_tc(const __grid_constant__ CUtensorMap xmap, const uint8_t* __restrict__ tiles, int nb, int rows, int row_groups, int wstages, int ntiles, int tok_tiles, int dxbufs, int xsteps, int na,
             const float* __restrict__ xd, int x_stride, int ntok,
             float* arena, size_t y_off, size_t y_stride, int accum, int* error_flag, const it_peers* peers, const it_rowmap map, float minus_zero) {
     constexpr int TC_TOK = Tc<NH>::TOK, TC_X_BYTES = Tc<NH>::X_BYTES, TC_ND = Tc<NH>::ND, TC_EPI_TOK = Tc<NH>::EPI_TOK, CC = Tc<NH>::CC, NDW = Tc<NH>::NDW;
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
-    const TcSmem L = tc_layout<NH>(nb, wstages, dxbufs, xsteps);
+    const TcSmem L = tc_layout<NH>(nb, wstages, dxbufs, xsteps, na);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, np = nb / 2;      // np: steps (pairs of blocks) of a tile
     volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + L.flag);
     unsigned* tmem_slot = reinterpret_cast<unsigned*>(smem + L.tmem);
@@ -145,7 +164,7 @@ k_matmul_tc(const __grid_constant__ CUtensorMap xmap, const uint8_t* __restrict_
     // one bit, and with a barrier per accumulator (two) and three steps of boxes the box of step n - 1 is in place while the producer
     // waits for step n - 3 on the barrier that n - 1 commits to as well, so that the parity could flip twice before it looks.
     const unsigned wfull0 = bars, wempty0 = wfull0 + 8 * wstages, xfull0 = wempty0 + 8 * wstages,
-                   afull0 = xfull0 + 8 * xsteps, dfull0 = afull0 + 8 * TC_NA, dempty0 = dfull0 + 8 * TC_NC, sfull0 = dempty0 + 8 * TC_ND, sempty0 = sfull0 + 16;
+                   afull0 = xfull0 + 8 * xsteps, dfull0 = afull0 + 8 * na, dempty0 = dfull0 + 8 * TC_NC, sfull0 = dempty0 + 8 * TC_ND, sempty0 = sfull0 + 16;
     // The CTA's tiles: blockIdx.x, + gridDim.x, ...; the activation tiles of one group of matrix rows are neighbours.  Every role walks
     // the same tiles with its ring positions running on, so the next tile's weights, boxes and products are under way while
     // the epilogue still stores the last one's results.
@@ -155,7 +174,7 @@ k_matmul_tc(const __grid_constant__ CUtensorMap xmap, const uint8_t* __restrict_
         *abort_flag = 0;
         for (int s = 0; s < wstages; s++) { mbar_init(wfull0 + 8 * s, 1); mbar_init(wempty0 + 8 * s, 8); }
         for (int s = 0; s < xsteps; s++) mbar_init(xfull0 + 8 * s, 1);
-        for (int a = 0; a < TC_NA; a++) mbar_init(afull0 + 8 * a, 4);
+        for (int a = 0; a < na; a++) mbar_init(afull0 + 8 * a, 4);
         for (int k = 0; k < TC_NC; k++) mbar_init(dfull0 + 8 * k, 1);
         for (int d = 0; d < TC_ND; d++) mbar_init(dempty0 + 8 * d, TC_EPI_WARPS);
         for (int k = 0; k < 2; k++) { mbar_init(sfull0 + 8 * k, 1); mbar_init(sempty0 + 8 * k, TC_EPI_WARPS); }
@@ -230,31 +249,39 @@ k_matmul_tc(const __grid_constant__ CUtensorMap xmap, const uint8_t* __restrict_
         }
     } else if (warp == TC_EPI_WARPS + TC_EXP_WARPS + 1) {
         // ---------------- MMA issuer
-        if (lane == 0) {
-            int s = 0, a = 0, d = 0, k = 0; unsigned xph = 0, aph = 0, dph = 0, kph = 0, last = 0, last_ph = 0; bool ok = true;
+        if (tc_elect()) {
+            int s = 0, a = 0, d = 0, k = 0; unsigned sph = 0, aph = 0, dph = 1, kph = 0, last = 0, last_ph = 0; bool ok = true, ready = false;
             const unsigned long long adesc0 = tc_smem_desc(smem_u32(smem + L.a)), bdesc0 = tc_smem_desc(smem_u32(smem + L.x));
             for (int tile = tile0; ok && tile < ntiles; tile += tstep)
             for (int p = 0; p < np; p++) {
-                // accumulators read out; boxes landed; tiles expanded (the condition that is met last)
-                if (!mbar_wait(dempty0 + 8 * d, dph ^ 1u, abort_flag, error_flag, 14) || !mbar_wait(xfull0 + 8 * s, xph, abort_flag, error_flag, 13) ||
-                    !mbar_wait(afull0 + 8 * a, aph, abort_flag, error_flag, 12)) { ok = false; break; }
+                // A wait costs this thread some 200 cycles even when it is met, and the tensor pipe idles meanwhile (three of them were 640
+                // of a step's 1650 cycles at 64 activation rows): the next step's three are looked at together, while this one's MMAs run.
+                if (!ready) {
+                    ok = ok && mbar_wait(xfull0 + 8 * s, sph, abort_flag, error_flag, 13);
+                    ok = ok && mbar_wait(dempty0 + 8 * d, dph, abort_flag, error_flag, 14);
+                    ok = ok && mbar_wait(afull0 + 8 * a, aph, abort_flag, error_flag, 12);
+                    if (!ok) break;
+                }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const unsigned long long ad0 = adesc0 + (unsigned)(2 * a * (TC_A_BYTES >> 4)), bd0 = bdesc0 + (unsigned)(2 * s * (TC_X_BYTES >> 4));
+                const unsigned dt0 = tmem_base + (unsigned)(2 * d * TC_TOK), commit = dfull0 + 8 * k;
+                last = commit; last_ph = kph;
+                if (++k == TC_NC) { k = 0; kph ^= 1u; }
+                if (++s == xsteps) { s = 0; sph ^= 1u; }
+                if (++a == na) { a = 0; aph ^= 1u; }
+                if (++d == TC_ND) { d = 0; dph ^= 1u; }
                 // descriptors differ from the first tile's only in the start-address field (16-byte units): + tile index, + 2 per K step of 32
 #pragma unroll
                 for (int h = 0; h < 2; h++) {
-                    const unsigned long long ad = adesc0 + (unsigned)((2 * a + h) * (TC_A_BYTES >> 4)), bd = bdesc0 + (unsigned)((2 * s + h) * (TC_X_BYTES >> 4));
-                    const unsigned dt = tmem_base + (unsigned)((2 * d + h) * TC_TOK);
+                    const unsigned long long ad = ad0 + (unsigned)(h * (TC_A_BYTES >> 4)), bd = bd0 + (unsigned)(h * (TC_X_BYTES >> 4));
+                    const unsigned dt = dt0 + (unsigned)(h * TC_TOK);
                     tc_mma<false>(dt, ad, bd, Tc<NH>::IDESC);
                     tc_mma<true>(dt, ad + 2, bd + 2, Tc<NH>::IDESC);
                     tc_mma<true>(dt, ad + 4, bd + 4, Tc<NH>::IDESC);
                     tc_mma<true>(dt, ad + 6, bd + 6, Tc<NH>::IDESC);
                 }
-                tc_commit(dfull0 + 8 * k);        // accumulators complete; tiles and boxes of this step may be reused
-                last = dfull0 + 8 * k; last_ph = kph;
-                if (++k == TC_NC) { k = 0; kph ^= 1u; }
-                if (++s == xsteps) { s = 0; xph ^= 1u; }
-                if (++a == TC_NA) { a = 0; aph ^= 1u; }
-                if (++d == TC_ND) { d = 0; dph ^= 1u; }
+                tc_commit(commit);                // accumulators complete; tiles and boxes of this step may be reused
+                ready = mbar_poll3(xfull0 + 8 * s, sph, dempty0 + 8 * d, dph, afull0 + 8 * a, aph);
             }
             // the last commit's arrival must find the CTA's shared memory still its own (bounded)
             const long long t0 = clock64();
@@ -279,26 +306,23 @@ k_matmul_tc(const __grid_constant__ CUtensorMap xmap, const uint8_t* __restrict_
             if (lane == 0) mbar_arrive(sfull0 + 8 * k);
         }
     } else if (warp >= TC_EPI_WARPS) {
-        // ---------------- expanders: warp 8 + 4 e + i expands row group i of the steps with number % 2 == e into tile pair e
-        static_assert(TC_NA == 2 && TC_EXP_WARPS == 8 && TC_NC % 2 == 0, "set e fills tile pair e and waits for every other commit");
+        // ---------------- expanders: warp 8 + 4 e + i expands row group i of the steps with number % 2 == e; step n goes into tile pair n % na
+        static_assert(TC_NA_MAX <= TC_NC && TC_EXP_WARPS == 8, "step n commits after it is expanded: a wait for step n - na is at most one phase behind");
         const int eset = (warp - TC_EPI_WARPS) >> 2, rgl = (warp - TC_EPI_WARPS) & 3, g = lane >> 2, t = lane & 3;
-        unsigned char* const at = smem + L.a + 2 * eset * TC_A_BYTES + (rgl * 32 + g) * 128;
+        unsigned char* const at = smem + L.a + (rgl * 32 + g) * 128;
         unsigned char* const plo = at + (((2 * t) ^ g) << 4);          // columns 32 t .. 32 t + 15 of row g; the other rows 1024 bytes apart
         unsigned char* const phi = at + (((2 * t + 1) ^ g) << 4);      // columns 32 t + 16 .. 32 t + 31
         float* const dws = reinterpret_cast<float*>(smem + L.dw) + rgl * 32 + 4 * g;
         const unsigned char* const src0 = smem + L.w + rgl * TC_KB * IT_TILE_BYTES;
-        int s = 0, dp = eset, r = 0, gp = 0; unsigned sph = 0, dpp = 0; bool ok = true;
+        int s = 0, dp = TC_NC - na, r = 0, gp = 0, pair = 0; unsigned sph = 0, dpp = 1; bool ok = true;        // dp, dpp: the barrier and parity of step gp - na
         for (int tile = tile0; tile < ntiles; tile += tstep)
         for (int p = 0; p < np; p++, gp++) {
             const bool last = (p & 1) || p + 1 == np;         // last step of the weight stage
             if ((gp & 1) == eset) {
                 ok = ok && mbar_wait(wfull0 + 8 * s, sph, abort_flag, error_flag, 15);
-                // the tile pair was last read two steps ago: wait for that step's commit
-                if (gp >= 2) {
-                    ok = ok && mbar_wait(dfull0 + 8 * dp, dpp, abort_flag, error_flag, 16);
-                    dp += 2;
-                    if (dp >= TC_NC) { dp -= TC_NC; dpp ^= 1u; }
-                }
+                // the tile pair was last read na steps ago: wait for that step's commit
+                if (gp >= na) ok = ok && mbar_wait(dfull0 + 8 * dp, dpp, abort_flag, error_flag, 16);
+                unsigned char *const lo = plo + 2 * pair * TC_A_BYTES, *const hi = phi + 2 * pair * TC_A_BYTES;
 #pragma unroll
                 for (int h = 0; h < 2; h++) {
                     const unsigned char* src = src0 + s * TC_W_BYTES + (2 * (p & 1) + h) * IT_TILE_BYTES;
@@ -307,8 +331,8 @@ k_matmul_tc(const __grid_constant__ CUtensorMap xmap, const uint8_t* __restrict_
 #pragma unroll
                     for (int i = 0; i < 4; i++) {         // bit pair i of every byte: matrix row g + 8 i of the group
                         auto sgn = [&](unsigned w) { return (((w >> (2 * i)) & 0x03030303u) + 0x7f7f7f7fu) ^ 0x80808080u; };   // code - 1 in every byte; no carry crosses a byte
-                        *reinterpret_cast<uint4*>(plo + h * TC_A_BYTES + i * 1024) = make_uint4(sgn(wa.x), sgn(wa.y), sgn(wa.z), sgn(wa.w));
-                        *reinterpret_cast<uint4*>(phi + h * TC_A_BYTES + i * 1024) = make_uint4(sgn(wb.x), sgn(wb.y), sgn(wb.z), sgn(wb.w));
+                        *reinterpret_cast<uint4*>(lo + h * TC_A_BYTES + i * 1024) = make_uint4(sgn(wa.x), sgn(wa.y), sgn(wa.z), sgn(wa.w));
+                        *reinterpret_cast<uint4*>(hi + h * TC_A_BYTES + i * 1024) = make_uint4(sgn(wb.x), sgn(wb.y), sgn(wb.z), sgn(wb.w));
                     }
                     if (t == 0) {
                         const uint2 sc = *reinterpret_cast<const uint2*>(src + 1024 + 8 * g);
@@ -320,11 +344,14 @@ k_matmul_tc(const __grid_constant__ CUtensorMap xmap, const uint8_t* __restrict_
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");     // generic-proxy stores before the MMA's async-proxy reads
                 __syncwarp();
                 if (lane == 0 && ok) {
-                    mbar_arrive(afull0 + 8 * eset);
+                    mbar_arrive(afull0 + 8 * pair);
                     mbar_arrive_n(wempty0 + 8 * s, last && !(p & 1) ? 2u : 1u);  // read its tiles; a stage of one step counts them twice
                 }
             }
             r = r + 2 == NDW ? 0 : r + 2;
+            if (++pair == na) pair = 0;
+            dp++;
+            if (dp >= TC_NC) { dp = 0; dpp ^= 1u; }
             if (last) { if (++s == wstages) { s = 0; sph ^= 1u; } }
         }
     } else {
@@ -453,14 +480,17 @@ static int tc_launch(it_ctx* c, const it_mat* w, int ntok, const it_q8* x, float
     const int tok_tiles = (ntok + Tc<NH>::TOK - 1) / Tc<NH>::TOK, ntiles = (int)((w->row_groups + 3) / 4) * tok_tiles;
     // One CTA per SM walks its tiles, with two buffers of activation scales; where those do not fit (wide rows), a CTA per tile.
     int grid = ntiles < c->sm_count ? ntiles : c->sm_count, dxbufs = ntiles > grid ? 2 : 1;
-    auto fits = [&](int wst, int xst) { return tc_layout<NH>(nb, wst, dxbufs, xst).total + 1024 <= TC_SMEM_MAX; };
+    int na = 2;
+    auto fits = [&](int wst, int xst) { return tc_layout<NH>(nb, wst, dxbufs, xst, na).total + 1024 <= TC_SMEM_MAX; };
     if (!fits(2, 2)) { grid = ntiles; dxbufs = 1; }
     if (!fits(2, 2)) return 1;
+    na = TC_NA_MAX;
+    if (!fits(2, 2)) na = 2;
     // Activation boxes three steps deep where they fit (two left the MMA waiting 375 cycles a step), then weight stages of TC_KB blocks
     const int xsteps = fits(2, 3) ? 3 : 2;       // no more than TC_NC
     int stages = 5;
     while (!fits(stages, xsteps)) stages--;
-    const TcSmem L = tc_layout<NH>(nb, stages, dxbufs, xsteps);
+    const TcSmem L = tc_layout<NH>(nb, stages, dxbufs, xsteps, na);
     static bool attr_set[16] = {};
     if (!attr_set[c->device & 15]) { IT_CUDA(cudaFuncSetAttribute(k_matmul_tc<NH>, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM_MAX)); attr_set[c->device & 15] = true; }
     cudaLaunchConfig_t cfg = {};
@@ -469,7 +499,7 @@ static int tc_launch(it_ctx* c, const it_mat* w, int ntok, const it_q8* x, float
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization; attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr; cfg.numAttrs = 1;
-    IT_CUDA(cudaLaunchKernelEx(&cfg, k_matmul_tc<NH>, x->tmap, (const uint8_t*)w->tiles, nb, (int)w->rows, (int)w->row_groups, stages, ntiles, tok_tiles, dxbufs, xsteps,
+    IT_CUDA(cudaLaunchKernelEx(&cfg, k_matmul_tc<NH>, x->tmap, (const uint8_t*)w->tiles, nb, (int)w->rows, (int)w->row_groups, stages, ntiles, tok_tiles, dxbufs, xsteps, na,
         (const float*)x->d, (int)x->max_n, ntok, c->arena, (size_t)(y - c->arena), y_stride, accum, c->error_flag_dev,
         (const it_peers*)(w->sharded ? c->peers_dev : nullptr), w->map, -0.0f));
     c->pdl_safe_q8 = x;
@@ -477,9 +507,12 @@ static int tc_launch(it_ctx* c, const it_mat* w, int ntok, const it_q8* x, float
 }
 
 // Returns IT_OK after launching, or a positive value when the shape does not suit this kernel (the caller then uses k_matmul_t2).
-// More than 64 activation rows go to the 128-row variant when its buffers fit (rows of up to about 28,000 columns).
+// More than 64 activation rows go to the 128-row variant when its buffers fit (rows of up to about 28,000 columns), unless 64-row tiles fill
+// idle SMs for less: the busiest SM's tiles decide, and a step of 128 rows takes about 1980 cycles against 1480 (5120 x 17408 x 128 rows: 40 tiles
+// of 128 rows 69.5 us, 80 of 64 rows 53; 34816 x 5120 x 128: 272 tiles 48.2 us, 544 tiles 63).
 int it_matmul_tc_launch(it_ctx* c, const it_mat* w, int ntok, const it_q8* x, float* y, size_t y_stride, int accum) {
     static const bool wide = []{ const char* v = getenv("IT_MATMUL_WIDE"); return !v || atoi(v) != 0; }();
-    if (wide && ntok > 64) { const int r = tc_launch<2>(c, w, ntok, x, y, y_stride, accum); if (r != 1) return r; }
+    auto rounds = [&](int tok) { return ((int)((w->row_groups + 3) / 4) * ((ntok + tok - 1) / tok) + c->sm_count - 1) / c->sm_count; };
+    if (wide && ntok > 64 && 4 * rounds(128) < 3 * rounds(64)) { const int r = tc_launch<2>(c, w, ntok, x, y, y_stride, accum); if (r != 1) return r; }
     return tc_launch<1>(c, w, ntok, x, y, y_stride, accum);
 }

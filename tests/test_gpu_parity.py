@@ -213,6 +213,18 @@ def test_matmul_t2_several_tiles_per_cta_bit_exact(be, orc, rows, cols, ntok, ac
     assert np.array_equal(bits(got), bits(want))
 
 
+# 64-row tiles as long as they fill no more rounds of the SMs (9472 rows: 148 tiles of 64, 9504 rows: 150); CTAs of one and of several tiles,
+# whose rings of tile pairs (three) and steps (four a tile) wrap at different places
+@pytest.mark.parametrize("rows,cols,ntok,acc", [(9472, 1024, 65, True), (9504, 1024, 65, False), (9472, 1024, 128, False), (9504, 1024, 129, True), (28500, 1024, 70, True),
+                                               (18950, 1024, 33, False), (300, 1024, 1000, True)])
+def test_tile_shape_by_rounds_bit_exact(be, orc, rows, cols, ntok, acc):
+    rng = np.random.default_rng(rows + cols + ntok)
+    raw = synth_pq2(rows * 3 + cols, rows, cols)
+    X = rng.standard_normal((ntok, cols)).astype(np.float32)
+    got, want = run_mv(be, orc, raw, rows, cols, X, acc=acc)
+    assert np.array_equal(bits(got), bits(want))
+
+
 def test_matvec_t2_integer_accumulators_bit_exact(be, orc):
     rng = np.random.default_rng(77)
     rows, cols, ntok = 333, 2048, 4
