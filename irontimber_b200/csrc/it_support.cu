@@ -190,9 +190,27 @@ __global__ void __launch_bounds__(256) k_dense_rows(const float* __restrict__ w0
 }
 
 // The same for many rows of activations: a CTA forms DR_W x DR_T results, every one with the additions of k_dense_rows in its order, so
-// that a loaded weight or activation serves four or eight products (one result per CTA moves 1 GB through L2 at 256 rows of
-// 96 x 5120: 70 us; here 55, most of it the conversions to f64).
-constexpr int DR_W = 8, DR_T = 4;
+// that a loaded weight or activation serves two or eight products.  What bounds it is the conversions to f64 (some nine cycles of a sub-core
+// for 32 products) and at few rows the latency of a CTA's 20 turns of loads, hence 64 registers and four CTAs an SM.  96 x 5120:
+// 61 rows 20.9 -> 16.8 us, 777 rows 142 -> 130, against 8 x 4 results with a butterfly a sum and no loads ahead (8 x 4 as
+// here: 19.0 and 128; 8 x 8: 24.7 and 176).
+constexpr int DR_W = 8, DR_T = 2;
+// k_dense_rows' butterfly over HAVE sums of every lane, a lane keeping half of them at every step as long as it has two: the additions of
+// one sum are the same (either lane adds the same two numbers), and 16 exchanges do for 16 sums instead of 80, which took a third
+// of the kernel.  The lane's bits, from the highest down, choose the halves.
+template <int M, int HAVE>
+__device__ __forceinline__ void dense_fold(double* s, int tid) {
+    if constexpr (M > 0) {
+        constexpr int H = HAVE > 1 ? HAVE / 2 : 1;
+        const bool up = tid & M;
+#pragma unroll
+        for (int e = 0; e < H; e++) {
+            const double keep = HAVE > 1 && up ? s[e + HAVE / 2] : s[e], give = HAVE > 1 && !up ? s[e + HAVE / 2] : s[e];
+            s[e] = keep + __shfl_xor_sync(0xffffffffu, give, M);
+        }
+        dense_fold<M / 2, H>(s, tid);
+    }
+}
 __global__ void __launch_bounds__(256) k_dense_tile(const float* __restrict__ w0, const float* __restrict__ w1, int rows, int cols, const float* __restrict__ x, size_t x_ts,
                                                     float* y0, float* y1, size_t y_ts, int nt) {
     IT_PDL_TRIGGER(); IT_PDL_WAIT();
@@ -203,31 +221,32 @@ __global__ void __launch_bounds__(256) k_dense_tile(const float* __restrict__ w0
     for (int r = 0; r < DR_W; r++) { const int g = min(r0 + r, 2 * rows - 1); wp[r] = (g < rows ? w0 + (size_t)g * cols : w1 + (size_t)(g - rows) * cols); }
 #pragma unroll
     for (int t = 0; t < DR_T; t++) xp[t] = x + (size_t)min(t0 + t, nt - 1) * x_ts;
-    double s[DR_W][DR_T];
+    double s[DR_W * DR_T];
 #pragma unroll
-    for (int r = 0; r < DR_W; r++)
+    for (int k = 0; k < DR_W * DR_T; k++) s[k] = 0.0;
+    float a[2][DR_W], b[2][DR_T];
+    auto load = [&](int k, int i) {
 #pragma unroll
-        for (int t = 0; t < DR_T; t++) s[r][t] = 0.0;
-    for (int i = tid; i < cols; i += 256) {
-        float a[DR_W], b[DR_T];
+        for (int r = 0; r < DR_W; r++) a[k][r] = wp[r][i];
 #pragma unroll
-        for (int r = 0; r < DR_W; r++) a[r] = wp[r][i];
-#pragma unroll
-        for (int t = 0; t < DR_T; t++) b[t] = xp[t][i];
+        for (int t = 0; t < DR_T; t++) b[k][t] = xp[t][i];
+    };
+    auto add = [&](int k) {
 #pragma unroll
         for (int r = 0; r < DR_W; r++)
 #pragma unroll
-            for (int t = 0; t < DR_T; t++) s[r][t] += (double)it_mul(a[r], b[t]);
+            for (int t = 0; t < DR_T; t++) s[r * DR_T + t] += (double)it_mul(a[k][r], b[k][t]);
+    };
+    if (tid < cols) load(0, tid);
+    for (int i = tid; i < cols; i += 512) {            // the next values are on their way while these are added
+        if (i + 256 < cols) load(1, i + 256);
+        add(0);
+        if (i + 512 < cols) load(0, i + 512);
+        if (i + 256 < cols) add(1);
     }
-#pragma unroll
-    for (int r = 0; r < DR_W; r++)
-#pragma unroll
-        for (int t = 0; t < DR_T; t++) {
-            double v = s[r][t];
-#pragma unroll
-            for (int m = 16; m >= 1; m >>= 1) v += __shfl_xor_sync(0xffffffffu, v, m);
-            if ((tid & 31) == 0) wsum[tid >> 5][r * DR_T + t] = v;
-        }
+    static_assert(DR_W * DR_T == 16, "two lanes end with the same sum");
+    dense_fold<16, DR_W * DR_T>(s, tid);
+    if (!(tid & 1)) wsum[tid >> 5][(tid & 31) >> 1] = s[0];
     __syncthreads();
     if (tid < DR_W * DR_T) {
         const int g = r0 + tid / DR_T, t = t0 + tid % DR_T;
