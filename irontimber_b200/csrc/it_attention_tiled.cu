@@ -87,15 +87,20 @@ __global__ void __launch_bounds__(256, 2) k_attn_scores(const float* q, size_t q
 
 // Softmax of 16 rows of scores in place.  The sum of a row's exponentials is one thread's ordered chain (4 cycles a term): warp 0
 // runs the 16 chains side by side on one chunk of positions while the other seven warps form the exponentials of the next.
-constexpr int SM_ROWS = 16, SM_CHUNK = 256;
+// Bounded by that chain at a few hundred positions and by its passes over the scores behind that.  24 heads of 256, 777 rows: 98 us
+// with two integer divisions an element; 75 with a row's count formed once; 64 with chunks of 128, which let eight CTAs share an SM and
+// 777 rows be one wave (chunks of 256: six CTAs), and the chain's terms loaded eight ahead.
+constexpr int SM_ROWS = 16, SM_CHUNK = 128;
 __global__ void __launch_bounds__(256) k_attn_softmax(float* scores, AtBlock b, int rows) {
     IT_PDL_TRIGGER(); IT_PDL_WAIT();
     __shared__ float e[2][SM_ROWS][SM_CHUNK + 1];
     __shared__ float mxs[SM_ROWS], sums[SM_ROWS];
-    const int r0 = blockIdx.x * SM_ROWS, nr = min(SM_ROWS, rows - r0), tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nm = b.nt * b.rep;
-    auto n_of = [&](int r) { return b.slot0 + (r0 + r) % nm / b.rep + 1; };          // positions row r sees (itself included)
+    __shared__ int ns[SM_ROWS];                    // positions a row sees (itself included); the divisions once a row, not once an element
+    const int r0 = blockIdx.x * SM_ROWS, nr = min(SM_ROWS, rows - r0), tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    if (tid < SM_ROWS) ns[tid] = tid < nr ? b.slot0 + (r0 + tid) % (b.nt * b.rep) / b.rep + 1 : 0;
+    __syncthreads();
     for (int r = warp; r < nr; r += 8) {
-        const float* s = scores + (size_t)(r0 + r) * b.npad; const int n = n_of(r);
+        const float* s = scores + (size_t)(r0 + r) * b.npad; const int n = ns[r];
         float m = -INFINITY;
 #pragma unroll 4
         for (int p = lane; p < n; p += 32) m = fmaxf(m, s[p]);
@@ -105,25 +110,38 @@ __global__ void __launch_bounds__(256) k_attn_softmax(float* scores, AtBlock b, 
     }
     __syncthreads();
     int nmax = 0;
-    for (int r = 0; r < nr; r++) nmax = max(nmax, n_of(r));
-    const int chunks = (nmax + SM_CHUNK - 1) / SM_CHUNK, myn = lane < nr ? n_of(lane) : 0;
+#pragma unroll
+    for (int r = 0; r < SM_ROWS; r++) nmax = max(nmax, ns[r]);
+    const int chunks = (nmax + SM_CHUNK - 1) / SM_CHUNK, myn = ns[lane % SM_ROWS];
     float sum = 0.f;
     for (int c = 0; c <= chunks; c++) {
         if (warp > 0 && c < chunks) {
 #pragma unroll 4
             for (int i = tid - 32; i < SM_ROWS * SM_CHUNK; i += 224) {
                 const int r = i / SM_CHUNK, j = i % SM_CHUNK, p = c * SM_CHUNK + j;
-                if (r < nr && p < n_of(r)) { float* s = scores + (size_t)(r0 + r) * b.npad + p; const float v = it_expf(it_sub(*s, mxs[r])); *s = v; e[c & 1][r][j] = v; }
+                if (p < ns[r]) { float* s = scores + (size_t)(r0 + r) * b.npad + p; const float v = it_expf(it_sub(*s, mxs[r])); *s = v; e[c & 1][r][j] = v; }
             }
         } else if (warp == 0 && c > 0 && lane < nr) {
             const int k = min(SM_CHUNK, myn - (c - 1) * SM_CHUNK); const float* ec = e[(c - 1) & 1][lane];
             int j = 0;
-            for (; j + 8 <= k; j += 8) {
-                float t[8];
+            float t[2][8];                         // the next eight are on their way while eight are added
+            if (k >= 8)
 #pragma unroll
-                for (int u = 0; u < 8; u++) t[u] = ec[j + u];
+                for (int u = 0; u < 8; u++) t[0][u] = ec[u];
+            for (; j + 16 <= k; j += 16) {
 #pragma unroll
-                for (int u = 0; u < 8; u++) sum = it_add(sum, t[u]);
+                for (int u = 0; u < 8; u++) t[1][u] = ec[j + 8 + u];
+#pragma unroll
+                for (int u = 0; u < 8; u++) sum = it_add(sum, t[0][u]);
+#pragma unroll
+                for (int u = 0; u < 8; u++) t[0][u] = ec[min(j + 16, SM_CHUNK - 8) + u];
+#pragma unroll
+                for (int u = 0; u < 8; u++) sum = it_add(sum, t[1][u]);
+            }
+            if (j + 8 <= k) {
+#pragma unroll
+                for (int u = 0; u < 8; u++) sum = it_add(sum, t[0][u]);
+                j += 8;
             }
             for (; j < k; j++) sum = it_add(sum, ec[j]);
         }
@@ -132,7 +150,7 @@ __global__ void __launch_bounds__(256) k_attn_softmax(float* scores, AtBlock b, 
     if (warp == 0 && lane < nr) sums[lane] = sum;
     __syncthreads();
     for (int r = warp; r < nr; r += 8) {
-        float* s = scores + (size_t)(r0 + r) * b.npad; const int n = n_of(r); const float d = sums[r];
+        float* s = scores + (size_t)(r0 + r) * b.npad; const int n = ns[r]; const float d = sums[r];
 #pragma unroll 4
         for (int p = lane; p < n; p += 32) s[p] = it_div(s[p], d);
     }
@@ -140,12 +158,14 @@ __global__ void __launch_bounds__(256) k_attn_softmax(float* scores, AtBlock b, 
 
 // out[t][head][j] = (sum over p of w[p] * v[p][j]) * sigmoid(gate).  128 threads, thread (ty, tx) owns rows ty * 4 + {0..3}, 64 + ..., elements
 // tx * 4 + {0..3}, 32 + ...  Positions every row of the tile sees run unguarded; the few behind them are added row by row.
+// CTAs start in the order of their length over all heads (777 rows: 592 CTAs, three to an SM; with the longest of one KV head after the shortest
+// of another 264 us, now 187; the multiplies and adds alone are 101).
 __global__ void __launch_bounds__(128, 3) k_attn_values(const float* __restrict__ w, const __half* __restrict__ vc, const float* gate, size_t q_hs, size_t q_ts, int hd, int nkv, AtBlock b,
                                                         float* out, size_t o_ts) {
     IT_PDL_TRIGGER(); IT_PDL_WAIT();
     __shared__ __align__(16) float as[2][AT_K][AT_M], bs[2][AT_K][AT_J];
-    const int slice = blockIdx.x, kvh = blockIdx.z, nm = b.nt * b.rep;
-    const int m0 = ((int)gridDim.y - 1 - (int)blockIdx.y) * AT_M;             // the longest rows first
+    const int slices = hd / AT_J, slice = blockIdx.x % slices, kvh = blockIdx.x / slices, nm = b.nt * b.rep;
+    const int m0 = ((int)gridDim.y - 1 - (int)blockIdx.y) * AT_M;             // the longest rows of all heads first
     const int tid = threadIdx.x, ty = tid >> 3, tx = tid & 7;
     const int n_all = b.slot0 + m0 / b.rep + 1, n_any = b.slot0 + min(nm - 1, m0 + AT_M - 1) / b.rep + 1;    // positions seen by every / by some row of the tile
     const float* wp = w + ((size_t)kvh * nm + min(m0 + tid, nm - 1)) * b.npad;
@@ -235,7 +255,7 @@ int it_sup_attention_tiled(it_ctx* c, const float* q, size_t q_hs, size_t q_ts, 
         const int nm = b.nt * rep, mt = (nm + AT_M - 1) / AT_M, pt = (b.slot0 + b.nt + AT_N - 1) / AT_N;
         it_pdl(k_attn_scores, dim3(pt, mt, nkv), dim3(256), 0, c->stream, q + (size_t)t0 * q_ts, q_hs, q_ts, (const __half*)kc, hd, nkv, b, scratch);
         it_pdl(k_attn_softmax, dim3((nm * nkv + SM_ROWS - 1) / SM_ROWS), dim3(256), 0, c->stream, scratch, b, nm * nkv);
-        it_pdl(k_attn_values, dim3(hd / AT_J, mt, nkv), dim3(128), 0, c->stream, scratch, (const __half*)vc, gate + (size_t)t0 * q_ts, q_hs, q_ts, hd, nkv, b, out + (size_t)t0 * o_ts, o_ts);
+        it_pdl(k_attn_values, dim3(hd / AT_J * nkv, mt), dim3(128), 0, c->stream, scratch, (const __half*)vc, gate + (size_t)t0 * q_ts, q_hs, q_ts, hd, nkv, b, out + (size_t)t0 * o_ts, o_ts);
         IT_LAUNCH_CHECK("attention_tiled");
     }
     return IT_OK;

@@ -46,7 +46,8 @@ static inline it_attn_group it_attn_grouping(int hd, int nh, int nkv, int npos) 
 // kernels' ordered sums walk all positions once per block of rows, however few the rows, and they are three launches.  The constants are
 // those of 24 heads over 4 of dimension 256: a wave of grouped CTAs 83 ns a position (3 heads x 2 rows) or 50 (x 1 row), one of
 // k_attention's two CTAs per SM 83; tiled 200 a block and 0.7 a row, 0.95 once the scores of a block are past 100 MB and leave L2, and 40 us.
-// They are scaled with the chains of a CTA and the width of a row.  us a layer of an attention-only stack, other / tiled:
+// They are scaled with the chains of a CTA and the width of a row.  us a layer of an attention-only stack, other / tiled (taken when the tiled
+// kernels' three launches were 540 us at 777 rows from position 0; they are 435 now, so the line errs towards the other side):
 //   at    0:   9 rows 186 / 248, 256 518 / 522, 257 588 / 632, 300 648 / 652, 384 744 / 704, 512 1106 / 966, 777 1776 / 1482
 //   at 1024:  32 rows 276 / 464, 64 404 / 504, 96 556 / 604, 128 665 / 635, 256 1091 / 899
 //   at 4096:  24 rows 515 / 1092, 64 899 / 1184, 96 1299 / 1346, 128 1653 / 1434, 256 2817 / 2086
