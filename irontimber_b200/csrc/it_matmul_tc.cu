@@ -3,8 +3,8 @@
 // (src/cpu.rs:48-63); it takes the place of the 64x64 tile kernels VkEngine::mv selects for prompt chunks
 // (src/vk/mod.rs:655-677).
 //
-// A CTA walks tiles of 128 matrix rows (four 32-row groups) x 64 activation rows (x 128 when the launch has more than 64: one
-// expanded tile and one issue sequence then feed twice the columns); one CTA per SM, a tile's 128-column blocks in order, two
+// A CTA walks tiles of 128 matrix rows (four 32-row groups; two, where that gives idle SMs a tile) x 64 activation rows (x 128 in larger
+// launches: one expanded tile and one issue sequence then feed twice the columns); one CTA per SM, a tile's 128-column blocks in order, two
 // blocks (the 256 columns of a q8k scale) a step.
 //   warp 16  weight producer: per stage four weight tiles of each of the four row groups (bulk copies)
 //   warp 18  activation producer: per step the int8 activations as boxes of a tiled tensor map with the 128-byte swizzle,
@@ -35,14 +35,12 @@
 // it: a lane that left alone would leave the rest of its warp in a warp-wide instruction), the producer waits (bounded) for its copies in flight, and the tensor memory is released before the CTA exits.
 #include "it_internal.h"
 #include "it_pipe.cuh"
+#include "it_route.h"
 
 namespace {
 
-constexpr int TC_ROWS = 128;                     // matrix rows per CTA (M of the MMA)
-constexpr int TC_A_BYTES = TC_ROWS * 128;        // one expanded weight tile
 constexpr int TC_KB = 4;                         // blocks per weight stage: one bulk copy per row group and stage (issuing a bulk copy costs a
                                                  // thread some 250 cycles, so four small copies per block made the producer the bottleneck)
-constexpr int TC_W_BYTES = 4 * TC_KB * IT_TILE_BYTES;   // four row groups x TC_KB consecutive tiles
 constexpr int TC_NA_MAX = 3;                     // steps of expanded tiles in flight where they fit, else two: with two, an expander waits for the commit of its
                                                  // own last step and the chain commit - expand - issue - commit sets the pace (14336 x 5120 x 64: 19.9 us, with three 19.2)
 constexpr int TC_NC = 4;                         // barriers the steps commit to in turn; at least the steps of boxes in flight, see the barrier list
@@ -53,27 +51,33 @@ constexpr int TC_EPI_WARPS = 8, TC_EXP_WARPS = 8, TC_THREADS = (TC_EPI_WARPS + T
 constexpr int TC_EPI_REGS = 168, TC_OTHER_REGS = 48;
 // NH: 64-row halves of the CTA's activation tile.  NH = 1: 64 activation rows per CTA (prompt passes of up to 64 rows).
 // NH = 2: 128 rows: one expanded weight tile and one issue sequence feed twice the columns.
-template <int NH> struct Tc {
+// RG: row groups of the CTA's weight tile.  RG = 4: 128 matrix rows.  RG = 2: 64 rows, where that gives idle SMs a tile: every warp then has
+// half of a step's work (an expander one block of a row group, an epilogue warp 16 rows).
+template <int NH, int RG> struct Tc {
+    static constexpr int ROWS = 32 * RG;                 // matrix rows per CTA (M of the MMA)
+    static constexpr int A_BYTES = ROWS * 128;           // one expanded weight tile
+    static constexpr int W_BYTES = RG * TC_KB * IT_TILE_BYTES;   // RG row groups x TC_KB consecutive tiles
     static constexpr int TOK = 64 * NH;                  // activation rows per CTA (N of the MMA)
     static constexpr int X_BYTES = TOK * 128;            // the activation tile of one block: NH boxes of the tensor map, one under the other
     static constexpr int ND = 256 / TOK;                 // steps of accumulators in tensor memory
     static constexpr int EPI_TOK = TOK / 2;              // activation rows per epilogue warp
     static constexpr int CC = EPI_TOK / 32;              // 32-column chunks per epilogue warp
     static constexpr int NDW = 2 * (TC_NA_MAX + ND);     // ring of per-block row scales: the expanders run at most NA + ND steps ahead of the epilogue
-    // kind::i8 instruction descriptor: D s32, A signed 8 bit, B signed 8 bit, both K-major, N = TOK, M = 128
-    static constexpr unsigned IDESC = (2u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(TOK >> 3) << 17) | ((unsigned)(TC_ROWS >> 4) << 24);
+    // kind::i8 instruction descriptor: D s32, A signed 8 bit, B signed 8 bit, both K-major, N = TOK, M = ROWS
+    static constexpr unsigned IDESC = (2u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(TOK >> 3) << 17) | ((unsigned)(ROWS >> 4) << 24);
 };
 
 // Weight stages and activation boxes have rings of their own: the weights come from HBM, the boxes from L2.
 struct TcSmem { int x, a, w, dx, dx_bytes, dw, bars, tmem, flag, total; };
-template <int NH> __host__ __device__ inline TcSmem tc_layout(int nb, int wstages, int dxbufs, int xsteps, int na) {
+template <int NH, int RG> __host__ __device__ inline TcSmem tc_layout(int nb, int wstages, int dxbufs, int xsteps, int na) {
+    using T = Tc<NH, RG>;
     TcSmem L; int o = 0;
-    L.x = o; o += xsteps * 2 * Tc<NH>::X_BYTES;    // 1024-byte aligned (128-byte swizzle)
-    L.a = o; o += na * 2 * TC_A_BYTES;              // 1024-byte aligned
-    L.w = o; o += wstages * TC_W_BYTES;
-    L.dx = o; L.dx_bytes = (nb / 2) * Tc<NH>::TOK * 4; o += dxbufs * L.dx_bytes;
-    L.dw = o; o += Tc<NH>::NDW * TC_ROWS * 4;
-    L.bars = o; o += (2 * wstages + xsteps + na + TC_NC + Tc<NH>::ND + 4) * 8;
+    L.x = o; o += xsteps * 2 * T::X_BYTES;    // 1024-byte aligned (128-byte swizzle)
+    L.a = o; o += na * 2 * T::A_BYTES;              // 1024-byte aligned
+    L.w = o; o += wstages * T::W_BYTES;
+    L.dx = o; L.dx_bytes = (nb / 2) * T::TOK * 4; o += dxbufs * L.dx_bytes;
+    L.dw = o; o += T::NDW * T::ROWS * 4;
+    L.bars = o; o += (2 * wstages + xsteps + na + TC_NC + T::ND + 4) * 8;
     o = (o + 15) & ~15;
     L.tmem = o; o += 16;
     L.flag = o; o += 16;
@@ -120,7 +124,17 @@ __device__ __forceinline__ void tc_ld_chunk(unsigned taddr, int (&v)[32]) {
                  : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
                  : "r"(taddr), "r"(taddr + (16u << 16)) : "memory");
 }
+// The same of 16 lanes: v[2 c + e]: row g + 8 e.
+__device__ __forceinline__ void tc_ld_chunk(unsigned taddr, int (&v)[16]) {
+    asm volatile("tcgen05.ld.sync.aligned.16x128b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+                 : "r"(taddr) : "memory");
+}
 // Waits for the loads; the values pass through it so that nothing that uses them moves in front.
+__device__ __forceinline__ void tc_ld_wait(int (&v)[16]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7]), "+r"(v[8]), "+r"(v[9]), "+r"(v[10]), "+r"(v[11]), "+r"(v[12]), "+r"(v[13]), "+r"(v[14]), "+r"(v[15]) :: "memory");
+}
 __device__ __forceinline__ void tc_ld_wait(int (&v)[32]) {
     asm volatile("tcgen05.wait::ld.sync.aligned;"
                  : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7]), "+r"(v[8]), "+r"(v[9]), "+r"(v[10]), "+r"(v[11]), "+r"(v[12]), "+r"(v[13]), "+r"(v[14]), "+r"(v[15]), "+r"(v[16]), "+r"(v[17]), "+r"(v[18]), "+r"(v[19]), "+r"(v[20]), "+r"(v[21]), "+r"(v[22]), "+r"(v[23]), "+r"(v[24]), "+r"(v[25]), "+r"(v[26]), "+r"(v[27]), "+r"(v[28]), "+r"(v[29]), "+r"(v[30]), "+r"(v[31]) :: "memory");
@@ -145,15 +159,16 @@ __device__ __forceinline__ int tc_dx_slot(int m) { return (m & ~15) + (m & 3) * 
 template <int N> __device__ __forceinline__ void reg_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" :: "n"(N)); }
 template <int N> __device__ __forceinline__ void reg_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" :: "n"(N)); }
 
-template <int NH>
+template <int NH, int RG>
 __global__ void __launch_bounds__(TC_THREADS, 1)
 k_matmul_tc(const __grid_constant__ CUtensorMap xmap, const uint8_t* __restrict__ tiles, int nb, int rows, int row_groups, int wstages, int ntiles, int tok_tiles, int dxbufs, int xsteps, int na,
             const float* __restrict__ xd, int x_stride, int ntok,
             float* arena, size_t y_off, size_t y_stride, int accum, int* error_flag, const it_peers* peers, const it_rowmap map, float minus_zero) {
-    constexpr int TC_TOK = Tc<NH>::TOK, TC_X_BYTES = Tc<NH>::X_BYTES, TC_ND = Tc<NH>::ND, TC_EPI_TOK = Tc<NH>::EPI_TOK, CC = Tc<NH>::CC, NDW = Tc<NH>::NDW;
+    using T = Tc<NH, RG>;
+    constexpr int TC_TOK = T::TOK, TC_X_BYTES = T::X_BYTES, TC_ND = T::ND, TC_EPI_TOK = T::EPI_TOK, CC = T::CC, NDW = T::NDW, TC_ROWS = T::ROWS, TC_A_BYTES = T::A_BYTES, TC_W_BYTES = T::W_BYTES;
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
-    const TcSmem L = tc_layout<NH>(nb, wstages, dxbufs, xsteps, na);
+    const TcSmem L = tc_layout<NH, RG>(nb, wstages, dxbufs, xsteps, na);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, np = nb / 2;      // np: steps (pairs of blocks) of a tile
     volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + L.flag);
     unsigned* tmem_slot = reinterpret_cast<unsigned*>(smem + L.tmem);
@@ -196,7 +211,7 @@ k_matmul_tc(const __grid_constant__ CUtensorMap xmap, const uint8_t* __restrict_
         const int nst = (nb + TC_KB - 1) / TC_KB;
         int s = 0, issued = 0; unsigned ph = 0; bool ok = true;
         for (int tile = tile0; ok && tile < ntiles; tile += tstep) {
-            const int rg0 = tile / tok_tiles * 4, nrg = min(4, row_groups - rg0);
+            const int rg0 = tile / tok_tiles * RG, nrg = min(RG, row_groups - rg0);
             for (int q = 0; q < nst; q++) {
                 if (lane == 0) ok = mbar_wait(wempty0 + 8 * s, ph ^ 1u, abort_flag, error_flag, 11);
                 ok = __shfl_sync(0xffffffffu, ok, 0);
@@ -275,10 +290,10 @@ k_matmul_tc(const __grid_constant__ CUtensorMap xmap, const uint8_t* __restrict_
                 for (int h = 0; h < 2; h++) {
                     const unsigned long long ad = ad0 + (unsigned)(h * (TC_A_BYTES >> 4)), bd = bd0 + (unsigned)(h * (TC_X_BYTES >> 4));
                     const unsigned dt = dt0 + (unsigned)(h * TC_TOK);
-                    tc_mma<false>(dt, ad, bd, Tc<NH>::IDESC);
-                    tc_mma<true>(dt, ad + 2, bd + 2, Tc<NH>::IDESC);
-                    tc_mma<true>(dt, ad + 4, bd + 4, Tc<NH>::IDESC);
-                    tc_mma<true>(dt, ad + 6, bd + 6, Tc<NH>::IDESC);
+                    tc_mma<false>(dt, ad, bd, T::IDESC);
+                    tc_mma<true>(dt, ad + 2, bd + 2, T::IDESC);
+                    tc_mma<true>(dt, ad + 4, bd + 4, T::IDESC);
+                    tc_mma<true>(dt, ad + 6, bd + 6, T::IDESC);
                 }
                 tc_commit(commit);                // accumulators complete; tiles and boxes of this step may be reused
                 ready = mbar_poll3(xfull0 + 8 * s, sph, dempty0 + 8 * d, dph, afull0 + 8 * a, aph);
@@ -306,9 +321,10 @@ k_matmul_tc(const __grid_constant__ CUtensorMap xmap, const uint8_t* __restrict_
             if (lane == 0) mbar_arrive(sfull0 + 8 * k);
         }
     } else if (warp >= TC_EPI_WARPS) {
-        // ---------------- expanders: warp 8 + 4 e + i expands row group i of the steps with number % 2 == e; step n goes into tile pair n % na
+        // ---------------- expanders: warp 8 + 4 e + i expands row group i of the steps with number % 2 == e (with two row groups: block i / 2 of
+        // group i % 2); step n goes into tile pair n % na
         static_assert(TC_NA_MAX <= TC_NC && TC_EXP_WARPS == 8, "step n commits after it is expanded: a wait for step n - na is at most one phase behind");
-        const int eset = (warp - TC_EPI_WARPS) >> 2, rgl = (warp - TC_EPI_WARPS) & 3, g = lane >> 2, t = lane & 3;
+        const int eset = (warp - TC_EPI_WARPS) >> 2, rgl = (warp - TC_EPI_WARPS) & (RG - 1), h0 = RG == 4 ? 0 : ((warp - TC_EPI_WARPS) >> 1) & 1, g = lane >> 2, t = lane & 3;
         unsigned char* const at = smem + L.a + (rgl * 32 + g) * 128;
         unsigned char* const plo = at + (((2 * t) ^ g) << 4);          // columns 32 t .. 32 t + 15 of row g; the other rows 1024 bytes apart
         unsigned char* const phi = at + (((2 * t + 1) ^ g) << 4);      // columns 32 t + 16 .. 32 t + 31
@@ -324,7 +340,8 @@ k_matmul_tc(const __grid_constant__ CUtensorMap xmap, const uint8_t* __restrict_
                 if (gp >= na) ok = ok && mbar_wait(dfull0 + 8 * dp, dpp, abort_flag, error_flag, 16);
                 unsigned char *const lo = plo + 2 * pair * TC_A_BYTES, *const hi = phi + 2 * pair * TC_A_BYTES;
 #pragma unroll
-                for (int h = 0; h < 2; h++) {
+                for (int hh = 0; hh < RG / 2; hh++) {
+                    const int h = hh + h0;
                     const unsigned char* src = src0 + s * TC_W_BYTES + (2 * (p & 1) + h) * IT_TILE_BYTES;
                     const uint4 wa = *reinterpret_cast<const uint4*>(src + 16 * lane);
                     const uint4 wb = *reinterpret_cast<const uint4*>(src + 512 + 16 * lane);
@@ -356,14 +373,16 @@ k_matmul_tc(const __grid_constant__ CUtensorMap xmap, const uint8_t* __restrict_
         }
     } else {
         // ---------------- epilogue: warp 4 q + i owns row group i x activation rows EPI_TOK q ..; its thread 4 g + t owns rows
-        // g, g + 8, g + 16, g + 24 of the group and every fourth activation row.  One 16-byte load of row scales per block and one of
+        // g, g + 8, g + 16, g + 24 of the group (with two row groups warp 4 q + i half i % 2 of group i / 2, and two rows) and every fourth activation row.  One 16-byte load of row scales per block and one of
         // activation scales per 16 columns and step then serve all of a thread's results: with a row per thread and all columns
         // (one broadcast 16-byte load per four results) the shared-memory read port was what bounded the kernel.
         constexpr int NEPI = TC_EPI_WARPS * 32;
         reg_inc<TC_EPI_REGS>();
-        const int grp = warp >> 2, rgl = warp & 3, g = lane >> 2, t = lane & 3, m0 = grp * TC_EPI_TOK;
-        const unsigned tquad = tmem_base + ((unsigned)(rgl * 32) << 16) + (unsigned)m0;
-        const ulonglong2* const dws = reinterpret_cast<const ulonglong2*>(smem + L.dw) + rgl * 8 + g;
+        constexpr int HF = RG / 2;                     // pairs of rows of a thread
+        const int grp = warp >> 2, quad = warp & 3, row0 = quad * 8 * RG, g = lane >> 2, t = lane & 3, m0 = grp * TC_EPI_TOK;     // row0: this warp's first row of the tile
+        const unsigned tquad = tmem_base + ((unsigned)(quad * 32) << 16) + (unsigned)m0;
+        // scales: four rows of a group side by side (g, g + 8, g + 16, g + 24), two of them this thread's when it has two
+        const f32x2* const dws = reinterpret_cast<const f32x2*>(smem + L.dw) + (row0 & ~31) / 2 + 2 * g + (RG == 2 ? quad & 1 : 0);
         asm volatile("griddepcontrol.wait;" ::: "memory");            // q8 scales and (when accumulating) y come from earlier kernels
         asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
         {
@@ -381,13 +400,13 @@ k_matmul_tc(const __grid_constant__ CUtensorMap xmap, const uint8_t* __restrict_
         bool ok = true;
         for (int tile = tile0; tile < ntiles; tile += tstep, j++) {
             const int k = j & 1;
-            const int rg0 = tile / tok_tiles * 4, tok0 = tile % tok_tiles * TC_TOK, ntv = min(TC_TOK, ntok - tok0);
+            const int rg0 = tile / tok_tiles * RG, tok0 = tile % tok_tiles * TC_TOK, ntv = min(TC_TOK, ntok - tok0);
             const bool active = m0 < ntv;              // groups past the last activation row only release the accumulators
             if (j > 0) ok = ok && mbar_wait(sfull0 + 8 * k, (unsigned)((j - 1) >> 1) & 1u, abort_flag, error_flag, 18);
             const float4* dxs = reinterpret_cast<const float4*>(smem + L.dx + k * L.dx_bytes) + m0 / 4 + t;
-            f32x2 acc[2][8 * CC];                      // rows g + 16 hf and g + 8 + 16 hf of column 4 c + t
+            f32x2 acc[HF][8 * CC];                     // rows g + 16 hf and g + 8 + 16 hf of column 4 c + t
 #pragma unroll
-            for (int hf = 0; hf < 2; hf++)
+            for (int hf = 0; hf < HF; hf++)
 #pragma unroll
                 for (int c = 0; c < 8 * CC; c++) acc[hf][c] = 0ull;
             for (int p = 0; p < np; p++) {             // two blocks at a time: they share the activation scale, the wait and the release
@@ -398,10 +417,16 @@ k_matmul_tc(const __grid_constant__ CUtensorMap xmap, const uint8_t* __restrict_
                     // chunks of 32 columns of one block; the next one is on its way while one is folded
                     const unsigned ta = tquad + (unsigned)(2 * d * TC_TOK);
                     auto chunk = [&](int ch) { return ta + (unsigned)((ch & 1) * TC_TOK + (ch >> 1) * 32); };
-                    int S[2][32];
+                    int S[2][16 * HF];
                     tc_ld_chunk(chunk(0), S[0]);
                     // row scales of both blocks: stored by the expanders before they released the tiles to the MMAs whose completion we just saw
-                    const ulonglong2 dwb[2] = { dws[r * TC_ROWS / 4], dws[(r + 1) * TC_ROWS / 4] };
+                    f32x2 dwb[2][HF];
+#pragma unroll
+                    for (int bk = 0; bk < 2; bk++) {
+                        const f32x2* p = dws + (r + bk) * (TC_ROWS / 2);
+                        if constexpr (HF == 2) { const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(p); dwb[bk][0] = v.x; dwb[bk][HF - 1] = v.y; }
+                        else dwb[bk][0] = *p;
+                    }
                     f32x2 dx[8];
 #pragma unroll
                     for (int ch = 0; ch < 2 * CC; ch++) {
@@ -410,7 +435,7 @@ k_matmul_tc(const __grid_constant__ CUtensorMap xmap, const uint8_t* __restrict_
                             dx[0] = pkf(xa.x, xa.x); dx[1] = pkf(xa.y, xa.y); dx[2] = pkf(xa.z, xa.z); dx[3] = pkf(xa.w, xa.w);
                             dx[4] = pkf(xb.x, xb.x); dx[5] = pkf(xb.y, xb.y); dx[6] = pkf(xb.z, xb.z); dx[7] = pkf(xb.w, xb.w);
                         }
-                        int (&v)[32] = S[ch & 1];
+                        int (&v)[16 * HF] = S[ch & 1];
                         tc_ld_wait(v);
                         if (ch + 1 < 2 * CC) tc_ld_chunk(chunk(ch + 1), S[(ch + 1) & 1]);
                         else {
@@ -421,8 +446,9 @@ k_matmul_tc(const __grid_constant__ CUtensorMap xmap, const uint8_t* __restrict_
 #pragma unroll
                         for (int c = 0; c < 8; c++) {
                             const int cc = (ch >> 1) * 8 + c;
-                            acc[0][cc] = add2(acc[0][cc], mul2_rounded(mul2(dwb[ch & 1].x, dx[c]), pkf((float)v[2 * c], (float)v[2 * c + 1]), mz));
-                            acc[1][cc] = add2(acc[1][cc], mul2_rounded(mul2(dwb[ch & 1].y, dx[c]), pkf((float)v[16 + 2 * c], (float)v[16 + 2 * c + 1]), mz));
+#pragma unroll
+                            for (int hf = 0; hf < HF; hf++)
+                                acc[hf][cc] = add2(acc[hf][cc], mul2_rounded(mul2(dwb[ch & 1][hf], dx[c]), pkf((float)v[16 * hf + 2 * c], (float)v[16 * hf + 2 * c + 1]), mz));
                         }
                     }
                 } else if (lane == 0 && ok) mbar_arrive(dempty0 + 8 * d);
@@ -436,8 +462,8 @@ k_matmul_tc(const __grid_constant__ CUtensorMap xmap, const uint8_t* __restrict_
             if (lane == 0) mbar_arrive(sempty0 + 8 * k);          // the tile's activation scales have been read
             if (!active) continue;
 #pragma unroll
-            for (int i = 0; i < 4; i++) {
-                const int row = (rg0 + rgl) * 32 + g + 8 * i;
+            for (int i = 0; i < 2 * HF; i++) {
+                const int row = rg0 * 32 + row0 + g + 8 * i;
                 if (row >= rows) continue;
                 const int grow = it_map_row(map, row);
                 const size_t off = y_off + (size_t)(tok0 + m0 + t) * y_stride + grow;     // first of this thread's activation rows
@@ -474,14 +500,14 @@ k_matmul_tc(const __grid_constant__ CUtensorMap xmap, const uint8_t* __restrict_
 
 }  // namespace
 
-template <int NH>
+template <int NH, int RG>
 static int tc_launch(it_ctx* c, const it_mat* w, int ntok, const it_q8* x, float* y, size_t y_stride, int accum) {
     const int nb = (int)(w->cols / 128);
-    const int tok_tiles = (ntok + Tc<NH>::TOK - 1) / Tc<NH>::TOK, ntiles = (int)((w->row_groups + 3) / 4) * tok_tiles;
+    const int tok_tiles = (ntok + Tc<NH, RG>::TOK - 1) / Tc<NH, RG>::TOK, ntiles = (int)((w->row_groups + RG - 1) / RG) * tok_tiles;
     // One CTA per SM walks its tiles, with two buffers of activation scales; where those do not fit (wide rows), a CTA per tile.
     int grid = ntiles < c->sm_count ? ntiles : c->sm_count, dxbufs = ntiles > grid ? 2 : 1;
     int na = 2;
-    auto fits = [&](int wst, int xst) { return tc_layout<NH>(nb, wst, dxbufs, xst, na).total + 1024 <= TC_SMEM_MAX; };
+    auto fits = [&](int wst, int xst) { return tc_layout<NH, RG>(nb, wst, dxbufs, xst, na).total + 1024 <= TC_SMEM_MAX; };
     if (!fits(2, 2)) { grid = ntiles; dxbufs = 1; }
     if (!fits(2, 2)) return 1;
     na = TC_NA_MAX;
@@ -490,16 +516,16 @@ static int tc_launch(it_ctx* c, const it_mat* w, int ntok, const it_q8* x, float
     const int xsteps = fits(2, 3) ? 3 : 2;       // no more than TC_NC
     int stages = 5;
     while (!fits(stages, xsteps)) stages--;
-    const TcSmem L = tc_layout<NH>(nb, stages, dxbufs, xsteps, na);
+    const TcSmem L = tc_layout<NH, RG>(nb, stages, dxbufs, xsteps, na);
     static bool attr_set[16] = {};
-    if (!attr_set[c->device & 15]) { IT_CUDA(cudaFuncSetAttribute(k_matmul_tc<NH>, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM_MAX)); attr_set[c->device & 15] = true; }
+    if (!attr_set[c->device & 15]) { IT_CUDA(cudaFuncSetAttribute(k_matmul_tc<NH, RG>, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM_MAX)); attr_set[c->device & 15] = true; }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)grid);
     cfg.blockDim = dim3(TC_THREADS); cfg.dynamicSmemBytes = (size_t)L.total + 1024; cfg.stream = c->stream;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization; attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr; cfg.numAttrs = 1;
-    IT_CUDA(cudaLaunchKernelEx(&cfg, k_matmul_tc<NH>, x->tmap, (const uint8_t*)w->tiles, nb, (int)w->rows, (int)w->row_groups, stages, ntiles, tok_tiles, dxbufs, xsteps, na,
+    IT_CUDA(cudaLaunchKernelEx(&cfg, k_matmul_tc<NH, RG>, x->tmap, (const uint8_t*)w->tiles, nb, (int)w->rows, (int)w->row_groups, stages, ntiles, tok_tiles, dxbufs, xsteps, na,
         (const float*)x->d, (int)x->max_n, ntok, c->arena, (size_t)(y - c->arena), y_stride, accum, c->error_flag_dev,
         (const it_peers*)(w->sharded ? c->peers_dev : nullptr), w->map, -0.0f));
     c->pdl_safe_q8 = x;
@@ -507,12 +533,11 @@ static int tc_launch(it_ctx* c, const it_mat* w, int ntok, const it_q8* x, float
 }
 
 // Returns IT_OK after launching, or a positive value when the shape does not suit this kernel (the caller then uses k_matmul_t2).
-// More than 64 activation rows go to the 128-row variant when its buffers fit (rows of up to about 28,000 columns), unless 64-row tiles fill
-// idle SMs for less: the busiest SM's tiles decide, and a step of 128 rows takes about 1980 cycles against 1480 (5120 x 17408 x 128 rows: 40 tiles
-// of 128 rows 69.5 us, 80 of 64 rows 53; 34816 x 5120 x 128: 272 tiles 48.2 us, 544 tiles 63).
+// Tiles by it_tc_tile (it_route.h); 128 activation rows only when their buffers fit (rows of up to about 28,000 columns).
 int it_matmul_tc_launch(it_ctx* c, const it_mat* w, int ntok, const it_q8* x, float* y, size_t y_stride, int accum) {
     static const bool wide = []{ const char* v = getenv("IT_MATMUL_WIDE"); return !v || atoi(v) != 0; }();
-    auto rounds = [&](int tok) { return ((int)((w->row_groups + 3) / 4) * ((ntok + tok - 1) / tok) + c->sm_count - 1) / c->sm_count; };
-    if (wide && ntok > 64 && 4 * rounds(128) < 3 * rounds(64)) { const int r = tc_launch<2>(c, w, ntok, x, y, y_stride, accum); if (r != 1) return r; }
-    return tc_launch<1>(c, w, ntok, x, y, y_stride, accum);
+    const int best = it_tc_tile((long)w->row_groups, ntok, c->sm_count);
+    if (best == IT_TC_128X128 && wide) { const int r = tc_launch<2, 4>(c, w, ntok, x, y, y_stride, accum); if (r != 1) return r; }
+    if (best == IT_TC_64X64) return tc_launch<1, 2>(c, w, ntok, x, y, y_stride, accum);
+    return tc_launch<1, 4>(c, w, ntok, x, y, y_stride, accum);
 }

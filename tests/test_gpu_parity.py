@@ -213,9 +213,12 @@ def test_matmul_t2_several_tiles_per_cta_bit_exact(be, orc, rows, cols, ntok, ac
     assert np.array_equal(bits(got), bits(want))
 
 
-# 64-row tiles as long as they fill no more rounds of the SMs (9472 rows: 148 tiles of 64, 9504 rows: 150); CTAs of one and of several tiles,
-# whose rings of tile pairs (three) and steps (four a tile) wrap at different places
-@pytest.mark.parametrize("rows,cols,ntok,acc", [(9472, 1024, 65, True), (9504, 1024, 65, False), (9472, 1024, 128, False), (9504, 1024, 129, True), (28500, 1024, 70, True),
+# Tiles of 64 matrix rows up to one round of them (9472 rows: 148, 9473: a 128-row tile's rounds are fewer), one and several tiles of 64 activation
+# rows, ragged either way; tiles of 64 activation rows as long as they fill no more rounds of the SMs (9472 rows: 148, 9504 rows: 150);
+# CTAs of one and of several tiles, whose rings of tile pairs (three) and steps (four a tile) wrap at different places
+@pytest.mark.parametrize("rows,cols,ntok,acc", [(33, 4096, 9, False), (64, 3072, 33, True), (65, 1024, 64, False), (127, 2048, 65, True), (4737, 2048, 31, False),
+                                               (9472, 1024, 40, True), (9473, 1024, 40, False), (2368, 1024, 256, False), (2369, 1024, 255, True),
+                                               (9472, 1024, 65, True), (9504, 1024, 65, False), (9472, 1024, 128, False), (9504, 1024, 129, True), (28500, 1024, 70, True),
                                                (18950, 1024, 33, False), (300, 1024, 1000, True)])
 def test_tile_shape_by_rounds_bit_exact(be, orc, rows, cols, ntok, acc):
     rng = np.random.default_rng(rows + cols + ntok)

@@ -15,6 +15,8 @@ def routes(tmp_path_factory):
     src, lib = d / "routes.cpp", d / "routes.so"
     src.write_text('#include "it_route.h"\n'
                    'extern "C" int takes_tc(long rg, long ntok, int sm) { return it_mm_takes_tc(rg, ntok, sm); }\n'
+                   'extern "C" int takes_tc64(long rg, long cols, long ntok, int sm) { return it_mm_takes_tc64(rg, cols, ntok, sm); }\n'
+                   'extern "C" int tc_tile(long rg, long ntok, int sm) { return it_tc_tile(rg, ntok, sm); }\n'
                    'extern "C" int attn_tiled(int slot0, int nt, int blk, int sm) { return it_attn_takes_tiled(256, 24, 4, slot0, nt, blk, sm); }\n'
                    'extern "C" int attn_group(int hd, int nh, int nkv, int npos) { auto g = it_attn_grouping(hd, nh, nkv, npos); return 10 * g.heads + g.rows; }\n'
                    'extern "C" int gdn_rows(int sd, int nt) { return it_gdn_rows_takes(sd, nt); }\n')
@@ -29,6 +31,18 @@ def routes(tmp_path_factory):
     (11137, 9, 1), (34816, 9, 1), (2689, 256, 1), (2688, 256, 0)])                                  # 128-row tiles for 0.6 of the SMs
 def test_tile_kernel_of_a_product(routes, rows, ntok, tc):
     assert routes.takes_tc(C.c_long((rows + 31) // 32), C.c_long(ntok), SM) == tc
+
+
+@pytest.mark.parametrize("rows,cols,ntok,tc", [
+    (512, 1024, 32, 0), (512, 1024, 33, 1), (5000, 1024, 9, 0), (9000, 1024, 9, 1), (4736, 2048, 32, 0), (4737, 2048, 9, 1), (32, 3072, 9, 1)])
+def test_64_row_tiles_of_a_product(routes, rows, cols, ntok, tc):
+    assert routes.takes_tc64(C.c_long((rows + 31) // 32), C.c_long(cols), C.c_long(ntok), SM) == tc
+
+
+@pytest.mark.parametrize("rows,ntok,tile", [
+    (9472, 64, 2), (9473, 64, 1), (5120, 65, 1), (4736, 128, 2), (4737, 128, 1), (9472, 128, 1), (9473, 128, 0), (18944, 64, 1), (34816, 512, 0), (34816, 64, 1)])
+def test_tiles_by_rounds(routes, rows, ntok, tile):
+    assert routes.tc_tile(C.c_long((rows + 31) // 32), C.c_long(ntok), SM) == tile
 
 
 # passes at the 27B shape measured both ways (24 heads over 4 of dimension 256), where the sides differ by more than 2 %: a prompt from
