@@ -43,6 +43,7 @@
 #include "it_support.h"
 #include "it_pipe.cuh"
 #include "it_hadamard.cuh"
+#include "it_step_plan.h"
 #include <algorithm>
 #include <vector>
 
@@ -50,7 +51,6 @@ namespace {
 
 constexpr int ST_CW = 4;                               // warps per consumer group
 constexpr int ST_NG = 3;                               // consumer groups; group j takes the chunks i of a phase with i % ST_NG == j
-constexpr int ST_TPC = 8;                              // tiles per chunk = per ring slot: two per warp of a group, computed side by side (widths are multiples of 1024, eight tiles)
 constexpr int ST_NCONS = ST_CW * ST_NG;                // consumer warps
 constexpr int ST_CT = ST_NCONS * 32;                   // consumer threads
 constexpr int ST_NSUM = 2;                             // warps that only add the per-block terms in block order
@@ -61,15 +61,6 @@ constexpr int ST_SMEM = 227 * 1024;                    // dynamic shared memory 
 constexpr int ST_BARS = 1024;                          // bytes reserved for mbarriers, flags, layer descriptions and spans
 constexpr int ST_SD = 128;                             // delta-rule state size this kernel is built for
 constexpr int ST_RED = 384;                            // bytes: the dense row's eight f64 warp sums, then the transform's [8] sums of squares and [4][2] group maxima
-
-// A CTA's share of one ternary matrix.  The matrix is a sequence of chunks (eight 32 x 128 tiles of one row group, row
-// groups in order); every CTA gets an equal run of it, whatever row group the run starts or ends in (5120 rows are 160 row
-// groups: whole ones would leave most of 148 CTAs with one and some with two).  A cut row group is finished by the later
-// CTA: the earlier one adds its first blocks and hands the running sums over, which is the same order of additions.  It does
-// that part first and the later CTA does its own last, so that nobody waits.  Order of a CTA's chunks: hl of the row group it
-// starts but does not finish, whole row groups, tl of the row group begun by the CTA before.
-struct StepSpan { int n, hl, tl, lead, uh, uf, ut, nb, cpr, parts, units; unsigned magic; };     // uh, uf, ut: row groups of the three parts
-enum { SP_IN_GDN, SP_IN_ATT, SP_OUT_GDN, SP_OUT_ATT, SP_GATE_UP, SP_DOWN, SP_HEAD, SP_KINDS };
 
 struct StepLayer {
     const uint8_t *in_proj, *out_proj, *gate_up, *down;
@@ -86,6 +77,15 @@ struct StepLayer {
 // fence is involved.  Why: one value crosses between two SMs in about 960 cycles whatever else the memory system does, but a
 // release or acquire-release fence takes 840 cycles on an idle GPU and 1900 while weights stream in, on every CTA's way into
 // every barrier.  Tags grow from phase to phase and launch to launch, so no granule needs to be cleared.
+// What keeps a buffer until its last reader is through, since nobody waits for everyone (a layer's chain: A to I as above):
+//   codes      step_codes_half: A (F) needs every row of I (E), whose CTAs have read what it overwrites; D and H have the other half
+//   rows       the next input projection follows an A that needed the heads' o through E .. I; every row belongs to a head that has read it
+//   o, act     D (H) reads them; the next heads (gate / up) follow an A or F that needed every row behind all of its blocks
+//   xe, xi     read by F (A) and, row by row, by I (E), into whose rows they go; the next E (I) follows a row that needed all of those
+//   gate       a head reads its pair; the next dense rows follow an A that needed that head's o
+//   prefix     the reader finishes a row of the phase, and the next phase's matrix follows a transform that needed all of them
+//   scores     read by the head's CTAs before their o
+// tests/test_step_protocol.py walks all of it with CTAs as late as they like.
 typedef uint4 granule;
 constexpr int ST_GPU = 11;                             // granules of a row group (32 rows)
 constexpr int ST_COPIES = 4;                           // copies of the quantised row: all SMs read it at once, and its few lines would crowd a few L2 slices
@@ -96,7 +96,7 @@ struct StepParams {
     float eps, theta_scale; int sec[4]; int v_grouped;
     float* arena; size_t hrow, logits, amx;
     granule *xe, *xi, *rows, *o, *act; // residual row after the output / down projection; input projection's rows; block output; silu(gate) * up
-    granule* codes; int codes_half;    // the quantised row: 128 granules a block of 1024, ST_COPIES copies; codes_half granules further: the activation row's
+    granule* codes; int codes_half;    // the quantised row: 128 granules a block of 1024, ST_COPIES copies; codes_half granules further: the other half (step_codes_half)
     unsigned long long* gate;          // per value head beta, then decay: value and tag
     granule* prefix;                   // [grid][32] running sums of a cut row group (two matrices' worth) and the tag
     granule* partials;                 // one greedy-pick partial per sum warp: value, row, tag
@@ -205,7 +205,6 @@ __device__ __forceinline__ void publish(granule* dst, int u, int lane, float v, 
 }
 // Granule i of a run of row groups holds rows r, r + 11 and (unless it is the last of its row group) r + 22.
 __device__ __forceinline__ int granule_row(int i, bool& two) { const int u = i / ST_GPU, l = i - u * ST_GPU; two = l == ST_GPU - 1; return u * 32 + l; }
-enum { PH_A, PH_B, PH_C, PH_D, PH_E, PH_F, PH_G, PH_H, PH_I, ST_SUBS };       // phases of a layer
 __device__ __forceinline__ unsigned tag_of(unsigned base, int il, int sub) { return base + 1u + (unsigned)(ST_SUBS * il + sub); }
 // Scratch of a matrix phase of nb blocks a row: ST_RED bytes of sums, the q8k row with its scales (a float per 256) and block sums
 // (an int per 128), then the transform's exchange area and, after it, the terms [slots][ST_TPC][32] of the ring's chunks.
@@ -1161,7 +1160,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) k_decode_step(const __grid_cons
             RowIn in; in.normed = nullptr; in.plain = nullptr; in.norm = ph == PH_A || ph == PH_F; in.dense = ph == PH_A && !tail_ph && L.recurrent && drow < 2 * P.nv;
             const bool owner = hb >= 0 && hb < row_blocks && (!tail_ph || logits || cta == 0);
             if (owner || in.dense) {
-                in.codes = owner && (!tail_ph || logits) ? P.codes + (ph == PH_H ? P.codes_half : 0) + hb * 128 : nullptr; in.codes_copy = row_blocks * 128; in.code_tag = tag_of(c.base, il, ph);
+                in.codes = owner && (!tail_ph || logits) ? P.codes + step_codes_half(ph) * P.codes_half + hb * 128 : nullptr; in.codes_copy = row_blocks * 128; in.code_tag = tag_of(c.base, il, ph);
                 in.nblk = row_blocks; in.blk = hb;
                 in.signs = c.sg + (hb >= 0 ? 32 * hb : 0) + P.sg_off[ph == PH_D ? (L.recurrent ? 1 : 2) : ph == PH_H ? 3 : 0];
                 if (ph == PH_A) {
@@ -1185,8 +1184,8 @@ __global__ void __launch_bounds__(ST_THREADS, 1) k_decode_step(const __grid_cons
             if (!count_wait(P, c, P.sync, c.target, 1 + ph)) return;
             ST_EV(P, c, c.evt_base + 0);
             if (c.tid == 0) mbar_arrive(c.ps);                       // the sum warps may enter this phase
-            // (a CTA without row groups does not read the codes: nothing would keep them for it)
-            if (c.sp[kind].n) codes_place(P, c, P.codes + (ph == PH_I ? P.codes_half : 0), row_blocks, tag_of(c.base, il, ph - 1));
+            // (a CTA without row groups does not read the codes: nobody waits for it, so nothing would keep them)
+            if (c.sp[kind].n) codes_place(P, c, P.codes + step_codes_half(ph) * P.codes_half, row_blocks, tag_of(c.base, il, ph - 1));
             ST_EV(P, c, c.evt_base + 1);
             if (ph == PH_B && !tail_ph) {
                 if (il + 1 < P.n_layer && c.warp == ST_NCONS - 1) {          // the next layer's description, long before it is needed
@@ -1278,29 +1277,6 @@ static int step_sign_words(const it_model_config& c, int (&off)[4], int (&words)
 static size_t step_smem_bytes(const it_model_config& c, int slots) {
     int off[4], words[4];
     return (size_t)slots * ST_CHUNK + step_scratch_bytes(c, slots) + ST_BARS + SP_KINDS * sizeof(StepSpan) + 4 * (size_t)step_sign_words(c, off, words);
-}
-
-// The chunks [c0, c1) of a matrix of `units` row groups (pairs of row groups when parts == 2), in the order a CTA takes them.
-static StepSpan step_span(long long c0, long long c1, int nb, int parts, int units) {
-    StepSpan s; memset(&s, 0, sizeof s);
-    s.nb = nb; s.cpr = nb / ST_TPC; s.parts = parts; s.units = units; s.magic = 0xffffffffu / (unsigned)s.cpr + 1u;
-    const long long cpu = (long long)s.cpr * parts;
-    s.n = (int)(c1 - c0); s.lead = (int)(c0 % cpu);
-    if (s.n == 0) { s.lead = 0; return s; }
-    s.tl = s.lead ? (int)(cpu - s.lead) : 0; s.hl = (int)(c1 % cpu);
-    s.ut = (int)(c0 / cpu); s.uf = (int)((c0 + s.tl) / cpu); s.uh = (int)(c1 / cpu);
-    return s;
-}
-// Equal runs of chunks when every CTA gets at least one whole row group's worth (then a row group is cut at most once), else whole
-// row groups.
-static void step_spans(std::vector<StepSpan>& out, int kind, int grid, int rows, int cols, int parts) {
-    const int nb = cols / 128, units = (rows / parts + 31) / 32; const long long cpu = (long long)(nb / ST_TPC) * parts, total = units * cpu;
-    for (int b = 0; b < grid; b++) {
-        long long c0, c1;
-        if (units >= grid) { c0 = total * b / grid; c1 = total * (b + 1) / grid; }
-        else { c0 = (long long)units * b / grid * cpu; c1 = (long long)units * (b + 1) / grid * cpu; }
-        out[(size_t)b * SP_KINDS + kind] = step_span(c0, c1, nb, parts, units);
-    }
 }
 
 // Whether this engine's decode step can run as the persistent kernel, and with which geometry.
