@@ -35,7 +35,8 @@
 // runs at one instruction per cycle and scheduler while it fits 32 KB, at half that up to about 100 KB, at a sixth beyond 128 KB.
 //
 // Every wait (mbarrier, counter, tag) is bounded; when one runs out the CTA raises the context's error flag and an abort word
-// that makes every other CTA leave at its next wait, drains its copies and returns (IT_ETIMEOUT on the host).
+// that ends every other CTA's waits, publishes nothing more, drains its copies and returns (IT_ETIMEOUT on the host).  What the
+// phases before it wrote (state, caches) stays written; no phase computes from values that did not come.
 #define IT_PIPE_OUTLINE_WAIT  // one copy of the retry loop of bounded waits
 #define IT_MATH_OUTLINE      // one copy of division, square root and the elementary functions: this kernel's code size is its speed
 #include "it_math.h"
@@ -159,23 +160,28 @@ __device__ __forceinline__ void st_granule(granule* p, unsigned x, unsigned y, u
     const unsigned long long a = (unsigned long long)y << 32 | x, b = (unsigned long long)tag << 32 | z;
     asm volatile("{\n.reg .b128 q;\nmov.b128 q, {%1, %2};\nst.relaxed.gpu.global.b128 [%0], q;\n}" :: "l"(p), "l"(a), "l"(b) : "memory");
 }
+// A wait ran out: the host is told, the other CTAs (the abort word) and the other roles of this one.  From then on nothing that this CTA
+// publishes can be relied on, and none of its roles publishes anything more.
+__device__ __noinline__ void give_up(const StepParams& P, volatile int* abort_flag, int site) { atomicExch(P.error_flag, site); atomicExch(P.sync + 2, 1u); *abort_flag = 1; }
 // A wait for tagged values has gone round `it` times: true when it has to end without them (the abort flag is up).
-__device__ __noinline__ bool tag_late(unsigned it, long long t0, volatile int* abort_flag, int* error_flag, int site) {
+__device__ __noinline__ bool tag_late(const StepParams& P, unsigned it, long long t0, volatile int* abort_flag, int site) {
     if (it & 31u) return false;
     if (*abort_flag) return true;
-    if (clock64() - t0 > WAIT_CLOCKS) { atomicExch(error_flag, site); *abort_flag = 1; return true; }
+    if (*reinterpret_cast<volatile unsigned*>(P.sync + 2)) { *abort_flag = 1; return true; }       // another CTA has given up
+    if (clock64() - t0 > WAIT_CLOCKS) { give_up(P, abort_flag, site); return true; }
     return false;
 }
-__device__ __noinline__ granule wait_granule(const granule* p, unsigned tag, volatile int* abort_flag, int* error_flag, int site) {
+// The granule, with another tag when the wait had to end without it.
+__device__ __noinline__ granule wait_granule(const StepParams& P, const granule* p, unsigned tag, volatile int* abort_flag, int site) {
     const long long t0 = clock64();
     granule v;
 #pragma unroll 1
-    for (unsigned it = 1;; it++) { v = ld_granule(p); if (v.w == tag || tag_late(it, t0, abort_flag, error_flag, site)) return v; }
+    for (unsigned it = 1;; it++) { v = ld_granule(p); if (v.w == tag || tag_late(P, it, t0, abort_flag, site)) return v; }
 }
 // Granules p, p + stride, ... (n of them, n <= N; the last one again in the places behind it): all requested, then all again until
 // each has its tag.  Bounded by a count of round trips (at least 500 cycles each); no call, so that nothing is spilled around it.
 constexpr unsigned ST_POLLS = 1u << 22;
-template <int N> __device__ __forceinline__ void read_granules(granule (&g)[N], const granule* p, int stride, int n, unsigned tag, const Cta& c, int* error_flag, int site) {
+template <int N> __device__ __forceinline__ void read_granules(granule (&g)[N], const granule* p, int stride, int n, unsigned tag, const StepParams& P, const Cta& c, int site) {
 #pragma unroll 1
     for (unsigned it = 0;; it++) {
 #pragma unroll
@@ -185,23 +191,24 @@ template <int N> __device__ __forceinline__ void read_granules(granule (&g)[N], 
         for (int u = 0; u < N; u++) miss |= g[u].w ^ tag;
         if (miss == 0) return;
         if (*c.abort_flag) return;
-        if (it == ST_POLLS) { atomicExch(error_flag, site); *c.abort_flag = 1; return; }
+        if ((it & 63u) == 63u && *reinterpret_cast<volatile unsigned*>(P.sync + 2)) { *c.abort_flag = 1; return; }
+        if (it == ST_POLLS) { give_up(P, c.abort_flag, site); return; }
     }
 }
 // value and tag in one 8-byte word
 __device__ __forceinline__ void st_tagged(unsigned long long* p, float v, unsigned tag) { asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" :: "l"(p), "l"((unsigned long long)tag << 32 | __float_as_uint(v)) : "memory"); }
-__device__ __noinline__ float ld_tagged(const unsigned long long* p, unsigned tag, volatile int* abort_flag, int* error_flag, int site) {
+__device__ __noinline__ float ld_tagged(const StepParams& P, const unsigned long long* p, unsigned tag, volatile int* abort_flag, int site) {
     const long long t0 = clock64();
 #pragma unroll 1
     for (unsigned it = 1;; it++) {
         unsigned long long v; asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
-        if ((unsigned)(v >> 32) == tag || tag_late(it, t0, abort_flag, error_flag, site)) return __uint_as_float((unsigned)v);
+        if ((unsigned)(v >> 32) == tag || tag_late(P, it, t0, abort_flag, site)) return __uint_as_float((unsigned)v);
     }
 }
 // One value per lane of a warp (32 consecutive rows) as the granules of row group u.
-__device__ __forceinline__ void publish(granule* dst, int u, int lane, float v, unsigned tag) {
+__device__ __forceinline__ void publish(granule* dst, int u, int lane, float v, unsigned tag, bool lost = false) {
     const float b = __shfl_down_sync(0xffffffffu, v, ST_GPU), d = __shfl_down_sync(0xffffffffu, v, 2 * ST_GPU);
-    if (lane < ST_GPU) st_granule(dst + (size_t)u * ST_GPU + lane, __float_as_uint(v), __float_as_uint(b), __float_as_uint(d), tag);
+    if (lane < ST_GPU && !lost) st_granule(dst + (size_t)u * ST_GPU + lane, __float_as_uint(v), __float_as_uint(b), __float_as_uint(d), tag);
 }
 // Granule i of a run of row groups holds rows r, r + 11 and (unless it is the last of its row group) r + 22.
 __device__ __forceinline__ int granule_row(int i, bool& two) { const int u = i / ST_GPU, l = i - u * ST_GPU; two = l == ST_GPU - 1; return u * 32 + l; }
@@ -234,12 +241,14 @@ __device__ __forceinline__ bool count_wait(const StepParams& P, Cta& c, const un
             unsigned v; asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(counter) : "memory");
             if ((int)(v - target) >= 0) break;
             if ((it & 63u) == 63u) {
-                if (*c.abort_flag) { atomicExch(P.sync + 2, 1u); break; }                       // a wait of this CTA ran out: tell the others
+                if (*c.abort_flag) break;
                 if (*reinterpret_cast<volatile unsigned*>(P.sync + 2)) { *c.abort_flag = 1; break; }
-                if (clock64() - t0 > WAIT_CLOCKS) { atomicExch(P.error_flag, 100 + site); atomicExch(P.sync + 2, 1u); *c.abort_flag = 1; break; }
+                if (clock64() - t0 > WAIT_CLOCKS) { give_up(P, c.abort_flag, 100 + site); break; }
             }
         }
-        *c.verdict = *c.abort_flag;
+        const int gone = *c.abort_flag;
+        if (gone) atomicExch(P.sync + 2, 1u);                        // a wait inside this CTA ran out (mbarriers do not tell the others)
+        *c.verdict = gone;
         if (P.trace && traced) trace_clock(P.trace, c.nsync++, 1);
     }
     cons_sync();
@@ -334,7 +343,7 @@ __device__ __forceinline__ void row_place(const StepParams& P, const Cta& c, flo
     for (int b = 0; b < nblk; b += N, p0 += N * IT_HAD_PITCH, p1 += N * IT_HAD_PITCH, p2 += N * IT_HAD_PITCH) {
         granule g[N];
         const int m = min(N, nblk - b);
-        read_granules(g, x + b * ST_GPB + c.tid, ST_GPB, m, tag, c, P.error_flag, 14);
+        read_granules(g, x + b * ST_GPB + c.tid, ST_GPB, m, tag, P, c, 14);
 #pragma unroll
         for (int u = 0; u < N; u++) {
             const int o = min(u, m - 1) * IT_HAD_PITCH;
@@ -366,7 +375,8 @@ __device__ __forceinline__ void block_transform(const StepParams& P, const Cta& 
     } else row_place(P, c, ex0, in.x, in.nblk, in.tag);
     asm volatile("cp.async.wait_group 0;" ::: "memory");             // the norm's weights
     cons_sync();
-    if (tid == 0 && in.codes) grid_arrive(P);                        // the codes will follow
+    const bool lost = *c.abort_flag;                                 // the row may not have come
+    if (tid == 0 && in.codes && !lost) grid_arrive(P);               // the codes will follow
     float sc = 0.f;
     if (in.norm) {
         // rmsnorm of the whole row in the order of k_rmsnorm_wide: thread i of 256 adds x[i]^2, x[i + 256]^2, ...; warp
@@ -409,7 +419,7 @@ __device__ __forceinline__ void block_transform(const StepParams& P, const Cta& 
                 for (int k = 0; k < in.nblk * 4; k++) d += (double)it_mul(dp[256 * k], it_mul(it_mul(xp[336 * k], sc), wp[336 * k]));
 #pragma unroll
                 for (int m = 16; m >= 1; m >>= 1) d += __shfl_xor_sync(0xffffffffu, d, m);
-                if (lane == 0) { reinterpret_cast<double*>(c.scratch)[warp] = d; mbar_arrive(c.dn); }
+                if (lane == 0 && !lost) { reinterpret_cast<double*>(c.scratch)[warp] = d; mbar_arrive(c.dn); }
             }
             cons_sync();                                     // the row is about to be overwritten
         }
@@ -437,7 +447,7 @@ __device__ __forceinline__ void block_transform(const StepParams& P, const Cta& 
             const it_had16_codes q = it_had16_quantise(v, red + 8, j, [] { pair_sync(); });
             // thread j: its four words of codes; threads 0..3 of each half also the group's scale and the half's sum
 #pragma unroll 1
-            for (int k = 0; k < ST_COPIES; k++) {
+            for (int k = lost ? ST_COPIES : 0; k < ST_COPIES; k++) {
                 granule* to = in.codes + k * in.codes_copy + j;
                 st_granule(to, q.packed[0], q.packed[1], q.packed[2], in.code_tag);
                 st_granule(to + 64, q.packed[3], __float_as_uint(q.d), (unsigned)q.sum, in.code_tag);
@@ -459,7 +469,7 @@ __device__ __forceinline__ void codes_place(const StepParams& P, const Cta& c, c
     for (int b = 0; b < nblk - blk; b += N * BPT, at += N * BPT * 256, dxs += N * BPT * 4, sss += N * BPT * 8, src += N * ST_CT) {
         const int m = min(N, (nblk - blk - b + BPT - 1) / BPT);
         granule g[N];
-        read_granules(g, src, ST_CT, m, tag, c, P.error_flag, 15);
+        read_granules(g, src, ST_CT, m, tag, P, c, 15);
 #pragma unroll
         for (int u = 0; u < N; u++) {
             const int o = min(u, m - 1) * BPT;
@@ -518,7 +528,7 @@ __device__ __forceinline__ void matvec_phase(const StepParams& P, Cta& c, const 
         const __half dwh = *reinterpret_cast<const __half*>(tile + 1024 + 2 * lane);   // scale of row g + 8 t: half 4 g + t
         return __fmul_rn(__fmul_rn(__half2float(dwh), dxs[b >> 1]), (float)((S >> (2 * t)) - sss[b]));
     };
-    bool ok = true;                                                  // a lane whose wait ran out goes on without waits and arrivals; the CTA leaves at its next wait
+    bool ok = !*c.abort_flag;                                        // (the row may not have come) a lane whose wait ran out goes on without waits and arrivals; the CTA leaves at its next wait
 #pragma unroll 1
     for (int i = warp / ST_CW; i < n; i += ST_NG) {
         const unsigned q = c.q + (unsigned)i;
@@ -596,7 +606,7 @@ __device__ __forceinline__ void sum_warps(const StepParams& P, Cta& c) {
             const bool conv = gdn_in && row < P.cd && !first;
             if (accum && live && !first) {
                 if (sub == 1 && il == 0) old = xsrc[row];
-                else { const int k = lane / ST_GPU; const granule og = wait_granule(yo + (size_t)u * ST_GPU + lane - k * ST_GPU, old_tag, c.abort_flag, P.error_flag, 16); old = __uint_as_float(k == 0 ? og.x : k == 1 ? og.y : og.z); }
+                else { const int k = lane / ST_GPU; const granule og = wait_granule(P, yo + (size_t)u * ST_GPU + lane - k * ST_GPU, old_tag, c.abort_flag, 16); ok = ok && og.w == old_tag; old = __uint_as_float(k == 0 ? og.x : k == 1 ? og.y : og.z); }
             }
             if (conv && P.conv_k == 4) {
 #pragma unroll
@@ -606,7 +616,8 @@ __device__ __forceinline__ void sum_warps(const StepParams& P, Cta& c) {
             const int turn = last ? sp.cpr - sp.lead : sp.cpr;       // never reached when there is one matrix
             if (last) {
                 // running sums of the blocks the CTA before has added (it does them first)
-                const granule a = wait_granule(P.prefix + (size_t)(blockIdx.x - 1) * 32 + lane, tag, c.abort_flag, P.error_flag, 13);
+                const granule a = wait_granule(P, P.prefix + (size_t)(blockIdx.x - 1) * 32 + lane, tag, c.abort_flag, 13);
+                ok = ok && a.w == tag;
                 s = __uint_as_float(a.x); sg = __uint_as_float(a.y);
             }
             // a lane whose wait ran out goes on without waits; the warp leaves by a vote after the row group
@@ -730,10 +741,10 @@ __device__ __forceinline__ void gdn_phase(const StepParams& P, const StepLayer& 
     if (tid < 4 * GH) {
         const int r = tid / GH, first = r == 0 ? kh * SD : r == 1 ? P.qk + kh * SD : r == 2 ? 2 * P.qk + h * SD : P.cd + h * SD;
         const granule* gp = P.rows + (size_t)(first / 32) * ST_GPU + (tid - r * GH);
-        const granule g = wait_granule(gp, tag, c.abort_flag, P.error_flag, 17);
+        const granule g = wait_granule(P, gp, tag, c.abort_flag, 17);
         bool two; float* at = raw + r * SD + granule_row(tid - r * GH, two);
         at[0] = __uint_as_float(g.x); at[ST_GPU] = __uint_as_float(g.y); if (!two) at[2 * ST_GPU] = __uint_as_float(g.z);
-    } else if (tid >= ST_CT - 2) scs[2 + tid - (ST_CT - 2)] = ld_tagged(P.gate + (tid - (ST_CT - 2)) * P.nv + h, tag, c.abort_flag, P.error_flag, 18);
+    } else if (tid >= ST_CT - 2) scs[2 + tid - (ST_CT - 2)] = ld_tagged(P, P.gate + (tid - (ST_CT - 2)) * P.nv + h, tag, c.abort_flag, 18);
     float nw[SD / 32];
     if (warp == 0) {
 #pragma unroll
@@ -741,6 +752,7 @@ __device__ __forceinline__ void gdn_phase(const StepParams& P, const StepLayer& 
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     cons_sync();
+    const bool lost = *c.abort_flag;                                 // the rows or gates may not have come: the state stays, nothing is published
     const float q = raw[tid & (SD - 1)], k = raw[SD + (tid & (SD - 1))], v = raw[2 * SD + (tid & (SD - 1))], bt = scs[2], eg = scs[3];
     if (warp >= 4 && warp < 6 && lane == 0) { const float* r = raw + (warp - 4) * SD; scs[warp - 4] = __fdiv_rn(1.0f, fmaxf(__fsqrt_rn(chain_dot(r, r, SD)), P.eps)); }
     if (warp < 6) asm volatile("bar.sync 3, 192;" ::: "memory");
@@ -801,7 +813,7 @@ __device__ __forceinline__ void gdn_phase(const StepParams& P, const StepLayer& 
         // the new state to global memory, a 16-byte piece a thread at a time (coalesced), once the head's output is out
         asm volatile("bar.sync 6, 384;" ::: "memory");
 #pragma unroll 2
-        for (int f = tid - SD; f < SD * PPR; f += ST_CT - SD) {
+        for (int f = lost ? SD * PPR : tid - SD; f < SD * PPR; f += ST_CT - SD) {
             const int j = f / PPR, cc = f % PPR;
             const float4 o = *piece(j, cc), k4 = *reinterpret_cast<const float4*>(ks + 4 * cc);
             const float delta = dl[j];
@@ -816,7 +828,7 @@ __device__ __forceinline__ void gdn_phase(const StepParams& P, const StepLayer& 
         const int u0 = (P.v_grouped ? h / P.nk + P.nv / P.nk * kh : h) * (SD / 32);
         const unsigned otag = tag_of(c.base, il, PH_C);
 #pragma unroll
-        for (int i = 0; i < SD / 32; i++) { const int j = lane + 32 * i; publish(P.o, u0 + i, lane, it_mul(it_mul(it_mul(os[j], sc), nw[i]), raw[3 * SD + j]), otag); }
+        for (int i = 0; i < SD / 32; i++) { const int j = lane + 32 * i; publish(P.o, u0 + i, lane, it_mul(it_mul(it_mul(os[j], sc), nw[i]), raw[3 * SD + j]), otag, lost); }
         asm volatile("bar.arrive 6, 384;" ::: "memory");             // the other warps may form the new rows
     }
 }
@@ -855,7 +867,6 @@ __device__ __forceinline__ void attn_phase(const StepParams& P, const StepLayer&
     const int G = P.attn_g, h = hg / G, g = hg % G, epc = hd / G;   // elements of the output this CTA owns
     const int vs = it_vc_slice(hd);                                  // elements per V slice: epc is a multiple of it
     const int rep = P.nh / nkv, kh = h / rep;
-    const bool writer = h % rep == 0 && g == 0;
     const int pos = *P.pos, n = pos + 1, nold = pos;
     const int ntiles = (nold + 31) / 32;                             // K tiles = V tiles of 32 positions
     const int my_tiles = ntiles > g ? (ntiles - g + G - 1) / G : 0;  // tiles g, g + G, ... are scored here
@@ -888,12 +899,13 @@ __device__ __forceinline__ void attn_phase(const StepParams& P, const StepLayer&
         const int gh = hd / 32 * ST_GPU, r = tid / gh;                // granules of hd rows; hd <= 256: four parts of at most 88
         if (r < 4) {
             const int first = r < 2 ? (2 * h + r) * hd : P.nh * 2 * hd + (r - 2) * kvd + kh * hd;
-            const granule g = wait_granule(P.rows + (size_t)(first / 32) * ST_GPU + (tid - r * gh), tag, c.abort_flag, P.error_flag, 17);
+            const granule g = wait_granule(P, P.rows + (size_t)(first / 32) * ST_GPU + (tid - r * gh), tag, c.abort_flag, 17);
             bool two; float* at = (r == 0 ? qs : r == 1 ? gs : r == 2 ? kl : vl) + granule_row(tid - r * gh, two);
             at[0] = __uint_as_float(g.x); at[ST_GPU] = __uint_as_float(g.y); if (!two) at[2 * ST_GPU] = __uint_as_float(g.z);
         }
     }
     cons_sync();                                                     // all twelve warps, the loader included
+    const bool lost = *c.abort_flag, writer = h % rep == 0 && g == 0 && !lost;
     ST_EV(P, c, c.evt_base + 5);
     const __half* kc = L.kc; const __half* vc = L.vc;
 
@@ -989,7 +1001,7 @@ __device__ __forceinline__ void attn_phase(const StepParams& P, const StepLayer&
                     f = __half22float2(hh[3]); s = it_add(s, it_mul(qb.z, f.x)); s = it_add(s, it_mul(qb.w, f.y));
                 }
                 s = it_mul(s, scale); sc[p] = s;
-                if (G > 1) st_tagged(shared_sc + p, s, sc_tag);
+                if (G > 1 && !lost) st_tagged(shared_sc + p, s, sc_tag);
             }
             __syncwarp();
             if (lane == 0) mbar_arrive(ke + 8 * sl);
@@ -1011,7 +1023,7 @@ __device__ __forceinline__ void attn_phase(const StepParams& P, const StepLayer&
                 if ((int)(v - target) >= 0) break;
                 if ((it & 63u) == 63u) {
                     if (*reinterpret_cast<volatile unsigned*>(P.sync + 2)) { *c.abort_flag = 1; break; }
-                    if (clock64() - t0 > WAIT_CLOCKS) { atomicExch(P.error_flag, 112); atomicExch(P.sync + 2, 1u); *c.abort_flag = 1; break; }
+                    if (clock64() - t0 > WAIT_CLOCKS) { give_up(P, c.abort_flag, 112); break; }
                 }
             }
         }
@@ -1021,7 +1033,7 @@ __device__ __forceinline__ void attn_phase(const StepParams& P, const StepLayer&
             for (int i = 0; i < ntiles; i++) {
                 if (i % G == g) continue;
                 const int p = i * 32 + (tid & 31);
-                if ((tid >> 5) == (i % (ST_NCONS - 1)) && p < nold) sc[p] = ld_tagged(shared_sc + p, sc_tag, c.abort_flag, P.error_flag, 19);
+                if ((tid >> 5) == (i % (ST_NCONS - 1)) && p < nold) sc[p] = ld_tagged(P, shared_sc + p, sc_tag, c.abort_flag, 19);
             }
         }
         at_sync();
@@ -1087,7 +1099,7 @@ __device__ __forceinline__ void attn_phase(const StepParams& P, const StepLayer&
             acc = it_add(acc, it_mul(sc[nold], vl[e0]));
             acc = it_mul(acc, it_sigmoid(gs[e0]));
         }
-        publish(P.o, (h * hd + g * epc) / 32 + warp, lane, acc, sc_tag);      // epc is a multiple of 32
+        publish(P.o, (h * hd + g * epc) / 32 + warp, lane, acc, sc_tag, *c.abort_flag);      // epc is a multiple of 32; a wait since the rows came may have run out
     }
     ST_EV(P, c, c.evt_base + 10);
 }
@@ -1218,13 +1230,17 @@ __global__ void __launch_bounds__(ST_THREADS, 1) k_decode_step(const __grid_cons
     if (!count_wait(P, c, P.sync, c.target, 10, false)) return;
     if (logits && c.warp == 0) {
         Pick q{ -INFINITY, 0xffffffffu };
+        bool ok = true;
 #pragma unroll 1
         for (unsigned b = c.lane; b < gridDim.x * ST_NSUM; b += 32) {
-            const granule u = wait_granule(P.partials + b, tag_of(c.base, P.n_layer, PH_B), c.abort_flag, P.error_flag, 20);
+            const unsigned tag = tag_of(c.base, P.n_layer, PH_B);
+            const granule u = wait_granule(P, P.partials + b, tag, c.abort_flag, 20);
+            ok = ok && u.w == tag;
             q = pick_better(q, Pick{ __uint_as_float(u.x), u.y });
         }
 #pragma unroll
         for (unsigned mm = 16; mm > 0; mm >>= 1) { Pick o{ __shfl_xor_sync(0xffffffffu, q.v, mm), __shfl_xor_sync(0xffffffffu, q.i, mm) }; q = pick_better(q, o); }
+        if (!__all_sync(0xffffffffu, ok)) return;
         if (c.lane == 0) {
             const unsigned pick = q.i == 0xffffffffu ? 0u : q.i;
             A[P.amx] = __uint_as_float(pick);
@@ -1318,6 +1334,10 @@ int it_step_prepare(it_engine* e) {
     }
     std::vector<StepSpan> sp((size_t)st->grid * SP_KINDS);
     step_spans(sp, SP_IN_GDN, st->grid, it_cfg_conv_dim(c) + c.ssm_inner, c.n_embd, 1);
+    {   // tests drop one CTA's share here, so that the rows it should publish never come and the waits for them run out
+        const char* v = getenv("IT_STEP_DROP_CTA"); const int b = v ? atoi(v) : -1;
+        if (b >= 0 && b < st->grid) sp[(size_t)b * SP_KINDS + SP_IN_GDN] = step_span(0, 0, c.n_embd / 128, 1, 0);
+    }
     step_spans(sp, SP_IN_ATT, st->grid, (2 * c.n_head + 2 * c.n_head_kv) * c.head_dim, c.n_embd, 1);
     step_spans(sp, SP_OUT_GDN, st->grid, c.n_embd, c.ssm_inner, 1);
     step_spans(sp, SP_OUT_ATT, st->grid, c.n_embd, c.n_head * c.head_dim, 1);

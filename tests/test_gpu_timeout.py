@@ -52,3 +52,38 @@ def test_peer_wait_runs_out_and_the_context_stays_usable(orc):
         full.close(); half.close(); q.close()
     finally:
         b1.close(); b0.close()
+
+
+@pytest.mark.parametrize("over,cta", [(dict(), 3), (dict(n_embd=2048, n_ff=1024, ssm_groups=8, ssm_vheads=24, ssm_inner=3072, n_head=8), 30)])     # 80 row groups; 256, cut between CTAs
+def test_rows_that_never_come_end_a_decode_step(monkeypatch, over, cta):
+    """One CTA of the decode step kernel is dealt none of its input-projection rows (on the host), so the waits for their values run out:
+    the call reports it, nothing is computed from values that did not come (later layers' state stays), and the engine goes on working."""
+    from irontimber_b200 import _lib
+    from irontimber_b200.engine import CudaEngine, ModelConfig
+    from tests.util import tiny_config
+    cfg = tiny_config(ModelConfig)
+    for k, v in over.items():
+        setattr(cfg, k, v)
+    prompt = [5, 77, 901, 13, 640, 2, 999, 0, 321, 45, 600]
+    good = CudaEngine(cfg, seed=3, with_mtp=False)
+    try:
+        want = bits(good.eval(prompt)).copy()
+    finally:
+        good.close()
+    monkeypatch.setenv("IT_STEP_DROP_CTA", str(cta))
+    eng = CudaEngine(cfg, seed=3, with_mtp=False)
+    try:
+        assert np.array_equal(bits(eng.eval(prompt)), want)                       # a pass of several rows does not use the kernel
+        later = [(il, k) for il in range(1, cfg.n_layer) for k in ((0, 1) if cfg.is_recurrent(il) else (2, 3))]
+        before = [bits(eng.state(il, k)).copy() for il, k in later]
+        for _ in range(2):
+            t0 = time.perf_counter()
+            with pytest.raises(_lib.IronTimberError) as err:
+                eng.eval([7])
+            assert err.value.code == -5 and "bounded wait" in str(err.value)
+            assert time.perf_counter() - t0 < 4.0                                 # one wait's limit (about a second), not one after another
+            assert all(np.array_equal(bits(eng.state(il, k))[: b.size], b) for (il, k), b in zip(later, before))     # (the caches have a position more)
+        eng.reset()
+        assert np.array_equal(bits(eng.eval(prompt)), want)
+    finally:
+        eng.close()
