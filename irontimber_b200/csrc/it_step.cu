@@ -101,7 +101,7 @@ struct StepParams {
     unsigned long long* gate;          // per value head beta, then decay: value and tag
     granule* prefix;                   // [grid][32] running sums of a cut row group (two matrices' worth) and the tag
     granule* partials;                 // one greedy-pick partial per sum warp: value, row, tag
-    unsigned long long* att_sc; int att_stride; unsigned* att_cnt;   // per head: the scores its CTAs exchange [nh][att_stride] (value and tag), their arrival counter [nh]
+    unsigned long long* att_sc; int att_stride;   // per head: the scores its CTAs exchange [nh][att_stride] (value and tag)
     const uint32_t* sg[4]; int sg_off[4], sg_words[4];   // sign bits of the four widths (n_embd, ssm_inner, attention output, n_ff): words, and where they start in shared memory
     const float *tok_embd, *output_norm; const uint8_t* output;
     uint32_t* toks; int* pos;
@@ -133,8 +133,7 @@ struct Cta {
     const uint32_t* sg;                // sign bits of the four widths (P.sg_off)
     unsigned base, target;             // tags of this launch start here; what the counter reaches when the transforms so far have begun
     int nsync;                         // waits in front of matrix phases passed so far (index into the trace)
-    unsigned att_seq;                  // attention blocks this CTA has run in this launch (a sum warp: dense rows)
-    unsigned att_base;                 // the head's arrival counter at the start of the launch (thread 0)
+    unsigned dense_seq;                // dense rows this sum warp has finished in this launch
     float inv_sqrt_sd, inv_sqrt_hd;    // 1 / sqrt(state size), 1 / sqrt(head dimension): formed once per launch
     int evt_on, evt_base;              // diagnostics: this thread records fine-grained events into slots evt_base ..
 };
@@ -581,7 +580,7 @@ __device__ __forceinline__ void sum_warps(const StepParams& P, Cta& c) {
         const int drow = (int)gridDim.x - 1 - (int)blockIdx.x;
         if (gdn_in && jw == 1 && drow < 2 * P.nv) {
             // the dense row of this CTA: beta (sigmoid) or alpha (decay) gate of a value head
-            if (!mbar_wait_warp(c.dn, (unsigned)(c.att_seq++) & 1u, c.abort_flag, P.error_flag, 12)) break;
+            if (!mbar_wait_warp(c.dn, (c.dense_seq++) & 1u, c.abort_flag, P.error_flag, 12)) break;
             if (lane == 0) {
                 const double* ws = reinterpret_cast<const double*>(c.scratch);
                 double tt = ws[0];
@@ -858,8 +857,8 @@ constexpr int ST_AT_MAXS = 8, ST_AT_LOADER = ST_NCONS - 1, ST_AT_T = (ST_NCONS -
 // the block's own barrier: every consumer warp but the loader, which runs ahead and only joins the next phase
 __device__ __forceinline__ void at_sync() { asm volatile("bar.sync 4, %0;" :: "n"(ST_AT_T) : "memory"); }
 // G = P.attn_g CTAs share a head (hg = G h + g).  Each forms q and the new position's k and v for itself, scores the K
-// tiles i with i % G == g, publishes those scores, meets the head's other CTAs at a counter of their own, reads their
-// scores, runs the softmax for itself (one thread adds the exponentials in position order) and accumulates the
+// tiles i with i % G == g, publishes those scores, reads the others' as they come (the tag is the exchange: a
+// counter would need a base that nobody's late start can miss), runs the softmax for itself (one thread adds the exponentials in position order) and accumulates the
 // head_dim / G output elements [g head_dim / G, ...) over all positions from row slices of the V tiles.  A single SM can
 // keep only so many bytes in flight, so a head's cache traffic is spread over G SMs.
 __device__ __forceinline__ void attn_phase(const StepParams& P, const StepLayer& L, Cta& c, int hg, int il) {
@@ -885,7 +884,6 @@ __device__ __forceinline__ void attn_phase(const StepParams& P, const StepLayer&
     const int S = max(1, min(ST_AT_MAXS, room / tile_bytes)), SV = max(1, min(ST_AT_MAXS, room / vslot_bytes));
     const int vwarps = (epc + 31) / 32;                              // output warps: one element per thread
     const unsigned kf = c.at, ke = c.at + 8 * ST_AT_MAXS, vf = c.at + 16 * ST_AT_MAXS, ve = c.at + 24 * ST_AT_MAXS;
-    c.att_seq++;
     if (tid == 0) {
 #pragma unroll 1
         for (int k = 0; k < 4 * ST_AT_MAXS; k++) asm volatile("mbarrier.inval.shared::cta.b64 [%0];" :: "r"(c.at + 8 * k) : "memory");
@@ -1011,33 +1009,15 @@ __device__ __forceinline__ void attn_phase(const StepParams& P, const StepLayer&
     }
     ST_EV(P, c, c.evt_base + 7);
     if (G > 1) {
-        // ---- the head's CTAs meet: arrival counter of the head (zeroed at the start of the launch), then everyone reads the others' scores
-        at_sync();
-        if (tid == 0) {
-            unsigned* cnt = P.att_cnt + h;
-            const unsigned target = c.att_base + (unsigned)G * c.att_seq;
-            count_up(cnt);
-            const long long t0 = clock64();
-            for (unsigned it = 0;; it++) {
-                unsigned v; asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(cnt) : "memory");
-                if ((int)(v - target) >= 0) break;
-                if ((it & 63u) == 63u) {
-                    if (*reinterpret_cast<volatile unsigned*>(P.sync + 2)) { *c.abort_flag = 1; break; }
-                    if (clock64() - t0 > WAIT_CLOCKS) { give_up(P, c.abort_flag, 112); break; }
-                }
-            }
-        }
-        at_sync();
-        if (!*c.abort_flag) {
+        // ---- the other CTAs' scores, as they come: their tags say that they are this layer's
 #pragma unroll 1
-            for (int i = 0; i < ntiles; i++) {
-                if (i % G == g) continue;
-                const int p = i * 32 + (tid & 31);
-                if ((tid >> 5) == (i % (ST_NCONS - 1)) && p < nold) sc[p] = ld_tagged(P, shared_sc + p, sc_tag, c.abort_flag, 19);
-            }
+        for (int i = 0; i < ntiles; i++) {
+            if (i % G == g) continue;
+            const int p = i * 32 + lane;
+            if (warp == i % (ST_NCONS - 1) && p < nold) sc[p] = ld_tagged(P, shared_sc + p, sc_tag, c.abort_flag, 19);
         }
-        at_sync();
-    } else at_sync();
+    }
+    at_sync();
     ST_EV(P, c, c.evt_base + 8);
     float mx = -INFINITY;
 #pragma unroll 1
@@ -1122,7 +1102,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) k_decode_step(const __grid_cons
     c.sp = reinterpret_cast<const StepSpan*>(tail + ST_BARS);
     c.sg = reinterpret_cast<const uint32_t*>(tail + ST_BARS + SP_KINDS * sizeof(StepSpan));
     c.tid = threadIdx.x; c.warp = c.tid >> 5; c.lane = c.tid & 31;
-    c.q = 0u; c.nsync = 0; c.evt_on = 0; c.att_seq = 0u; c.mph = 0u;
+    c.q = 0u; c.nsync = 0; c.evt_on = 0; c.dense_seq = 0u; c.mph = 0u;
     if (c.tid == 0) {
         *c.abort_flag = *reinterpret_cast<volatile unsigned*>(P.sync + 2) ? 1 : 0;      // a step that was given up earlier: nothing runs until the host has cleared the words
         for (int s = 0; s < P.slots; s++) { mbar_init(c.bars + 8 * s, 1); mbar_init(c.bars + 8 * (P.slots + s), 1); mbar_init(c.tf + 8 * s, ST_CW); }
@@ -1147,8 +1127,6 @@ __global__ void __launch_bounds__(ST_THREADS, 1) k_decode_step(const __grid_cons
     float* A = P.arena;
     const int cta = (int)blockIdx.x, grid = (int)gridDim.x, drow = grid - 1 - cta, ah = cta - P.attn_base;
     const int hb = cta % P.had_step == 0 && cta / P.had_step < P.widest / 1024 ? cta / P.had_step : -1;      // the block this CTA transforms, of every row that has as many
-    // the heads' arrival counters only grow; nobody counts before this CTA has taken part in the first layer
-    c.att_base = c.tid == 0 && ah >= 0 && ah < P.nh * P.attn_g ? *reinterpret_cast<volatile unsigned*>(P.att_cnt + ah / P.attn_g) : 0u;
     const uint32_t tok = (P.flags & 1) ? __float_as_uint(*reinterpret_cast<volatile float*>(A + P.amx)) : *reinterpret_cast<volatile uint32_t*>(P.toks);
     float* wb = reinterpret_cast<float*>(c.scratch + P.w_off);
     // the norms' weights are wanted where a block of a normed row is transformed and where a dense row is multiplied
@@ -1261,7 +1239,7 @@ struct it_step_state {
     unsigned long long* gate;
     int had_step;
     int grid, slots, scratch, gdn_off, attn_base, attn_g, att_stride;
-    unsigned long long* att_sc; unsigned* att_cnt;
+    unsigned long long* att_sc;
     bool cooperative;
 };
 
@@ -1320,7 +1298,7 @@ int it_step_prepare(it_engine* e) {
     for (int g = 4; g > 1; g /= 2) if (c.head_dim % (32 * g) == 0 && (c.head_dim / g) % it_vc_slice(c.head_dim) == 0 && g * c.n_head <= st->grid) { st->attn_g = g; break; }
     { const char* v = getenv("IT_STEP_ATTN_G"); if (v && (atoi(v) == 1 || atoi(v) == 2) && atoi(v) < st->attn_g) st->attn_g = atoi(v); }
     st->attn_base = (c.ssm_vheads + st->attn_g * c.n_head <= st->grid) ? c.ssm_vheads : 0;
-    st->layers_dev = nullptr; st->spans_dev = nullptr; st->partials = nullptr; st->gate = nullptr; st->trace = nullptr; st->had_step = st->grid / (step_widest(c) / 1024); st->att_sc = nullptr; st->att_cnt = nullptr;
+    st->layers_dev = nullptr; st->spans_dev = nullptr; st->partials = nullptr; st->gate = nullptr; st->trace = nullptr; st->had_step = st->grid / (step_widest(c) / 1024); st->att_sc = nullptr;
     st->att_stride = (c.ctx_len + 32 + 3) / 4 * 4;
     { const char* v = getenv("IT_STEP_COOP"); st->cooperative = !v || atoi(v) != 0; }
     std::vector<StepLayer> hl(c.n_layer);
@@ -1353,7 +1331,6 @@ int it_step_prepare(it_engine* e) {
     granules(&st->codes, (size_t)(step_widest(c) / 1024) * 128 * ST_COPIES * 2); granules(&st->prefix, (size_t)st->grid * 32); granules(&st->partials, (size_t)st->grid * ST_NSUM);
     if (r == IT_OK) r = it_engine_dev_alloc(e, (void**)&st->gate, 2 * (size_t)c.ssm_vheads * sizeof(unsigned long long), true);
     if (r == IT_OK) r = it_engine_dev_alloc(e, (void**)&st->att_sc, (size_t)c.n_head * st->att_stride * sizeof(unsigned long long), true);
-    if (r == IT_OK) r = it_engine_dev_alloc(e, (void**)&st->att_cnt, (size_t)c.n_head * sizeof(unsigned), true);
     { const char* v = getenv("IT_STEP_TRACE"); if (r == IT_OK && v && atoi(v) != 0) r = it_engine_dev_alloc(e, (void**)&st->trace, (2 * ST_TRACE_MAX * 2 + ST_EVT_MAX) * sizeof(unsigned long long), true); }
     if (r) { delete st; return r; }
     IT_CUDA(cudaMemcpyAsync(st->layers_dev, hl.data(), hl.size() * sizeof(StepLayer), cudaMemcpyHostToDevice, cx->stream));
@@ -1378,7 +1355,7 @@ int it_step_launch(it_engine* e, int flags) {
     P.tok_embd = e->tok_embd; P.output_norm = e->output_norm; P.output = e->output->tiles;
     P.toks = e->toks_dev; P.pos = e->pos_dev;
     P.sync = cx->grid_sync; P.partials = st->partials; P.error_flag = cx->error_flag_dev;
-    P.slots = st->slots; P.scratch = st->scratch; P.w_off = st->scratch - (int)step_w_bytes(c); P.flags = flags; P.trace = st->trace; P.gdn_off = st->gdn_off; P.attn_base = st->attn_base; P.attn_g = st->attn_g; P.att_sc = st->att_sc; P.att_stride = st->att_stride; P.att_cnt = st->att_cnt;
+    P.slots = st->slots; P.scratch = st->scratch; P.w_off = st->scratch - (int)step_w_bytes(c); P.flags = flags; P.trace = st->trace; P.gdn_off = st->gdn_off; P.attn_base = st->attn_base; P.attn_g = st->attn_g; P.att_sc = st->att_sc; P.att_stride = st->att_stride;
     it_note_op(cx);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)st->grid); cfg.blockDim = dim3(ST_THREADS); cfg.dynamicSmemBytes = step_smem_bytes(c, st->slots); cfg.stream = cx->stream;

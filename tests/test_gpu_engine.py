@@ -402,7 +402,8 @@ def test_a_short_context_keeps_short_row_buffers():
     dict(n_embd=3072, n_ff=5120, ssm_vheads=16, ssm_groups=4, ssm_inner=2048, n_head=8, head_dim=128, conv_k=3, gdn_v_grouped=0, n_vocab=5000),   # gate/up and head cut across CTAs, general conv
     dict(n_embd=2048, n_ff=5120, ssm_vheads=24, ssm_groups=8, ssm_inner=3072, n_head=16, n_head_kv=4, head_dim=64, n_vocab=4767, conv_k=2),      # 149 row groups of the head, the last one short
     dict(n_embd=5120, n_ff=1024, ssm_vheads=48, ssm_groups=16, ssm_inner=6144, full_attn_interval=2, n_vocab=64),                                # 160 row groups for the residual, CTAs without any of the head
-    dict(n_embd=8192, n_ff=2048, n_vocab=200)])                                                                                                  # widest norm row: fewer ring slots
+    dict(n_embd=8192, n_ff=2048, n_vocab=200),                                                                                                   # widest norm row: fewer ring slots
+    dict(full_attn_interval=1)])                                                                                                                 # attention in the first layer
 def test_step_kernel_geometries(monkeypatch, over):
     """Matrices that cut a row group between two CTAs, leave CTAs without work, or leave the ring fewer slots: logits, picks and
     state of the persistent kernel equal the per-op schedule's bit for bit."""

@@ -223,6 +223,20 @@ def test_the_model_sees_an_early_overwrite(plan):
     assert len(late) > SM // 2                                          # most CTAs give block 0 nothing
 
 
+def test_a_count_read_at_the_start_can_come_late(plan):
+    """Why the CTAs of an attention head exchange nothing but tagged scores: a count that a CTA reads at its own start may already hold a
+    sibling's arrival when layer 0 is an attention layer, or when nobody needs anything of the late CTA's."""
+    def late(g):
+        step = Step(plan, g, plan.codes_half)
+        return [(c, d) for ctas, c, ev in step.score_events for d in ctas if d != c and not step.before[ev] >> step.start[d] & 1]
+    assert late(Geometry()) == []
+    assert late(Geometry(interval=1, layers=1))
+    assert late(Geometry(**dict(GEOMETRIES["one block a row"], attn_g=4)))            # CTAs without row groups
+    with open(os.path.join(CSRC, "it_step.cu")) as f:
+        phase = re.search(r"void attn_phase\(.*?\n}\n", f.read(), re.S).group()
+    assert "st_tagged(shared_sc" in phase and "ld_tagged(P, shared_sc" in phase and "count_up" not in phase and "count_wait" not in phase
+
+
 def test_the_kernel_uses_the_plan():
     """Both sides of the quantised row take their half from the plan."""
     with open(os.path.join(CSRC, "it_step.cu")) as f:
