@@ -259,6 +259,16 @@ __device__ __forceinline__ bool count_wait(const StepParams& P, Cta& c, const un
 __device__ __forceinline__ int mat_count(const StepParams& P) { return 4 * P.n_layer + ((P.flags & 4) ? 1 : 0); }
 __device__ __forceinline__ int span_kind(int sub, int recurrent) { return sub == 0 ? (recurrent ? SP_IN_GDN : SP_IN_ATT) : sub == 1 ? (recurrent ? SP_OUT_GDN : SP_OUT_ATT) : sub == 2 ? SP_GATE_UP : SP_DOWN; }
 
+// Whoever starts bulk copies leaves only when they have landed, also where nobody waits for them any more: the last `issued` copies of
+// a ring of `slots` with full barriers at `full` (each wait bounded by the clock limit).
+__device__ __noinline__ void drain_copies(unsigned full, unsigned slots, unsigned issued) {
+#pragma unroll 1
+    for (unsigned k = issued > slots ? issued - slots : 0u; k < issued; k++) {
+        const long long t0 = clock64();
+        while (!mbar_test(full + 8 * (k % slots), (k / slots) & 1u) && clock64() - t0 < WAIT_CLOCKS) { }
+    }
+}
+
 // ---------------------------------------------------------------- producer
 __device__ __forceinline__ void producer(const StepParams& P, const Cta& c) {
     int s = 0, issued = 0; unsigned ph = 0u;
@@ -285,14 +295,7 @@ __device__ __forceinline__ void producer(const StepParams& P, const Cta& c) {
             if (++cq == cpu) { cq = 0; unit++; }
         }
     }
-    if (!ok || *c.abort_flag) {
-        // leave only after every copy this thread started has landed (each wait bounded by the clock limit)
-        const int first = issued > P.slots ? issued - P.slots : 0;
-        for (int k = first; k < issued; k++) {
-            const long long t0 = clock64();
-            while (!mbar_test(c.bars + 8 * (k % P.slots), (unsigned)(k / P.slots) & 1u) && clock64() - t0 < WAIT_CLOCKS) { }
-        }
-    }
+    drain_copies(c.bars, (unsigned)P.slots, (unsigned)issued);
 }
 
 // Vectors that a later phase reads once: on their way into L2 while the weight stream would make them wait (lines of 128 bytes, a thread each).
@@ -909,21 +912,20 @@ __device__ __forceinline__ void attn_phase(const StepParams& P, const StepLayer&
 
     if (warp == ST_AT_LOADER) {
         // ---- loader: this CTA's K tiles, then its slice of every V tile, as far ahead as the rings allow
+        unsigned kn = 0, vn = 0; bool ok = true;
 #pragma unroll 1
-        for (int j = 0; j < my_tiles; j++) {
+        for (int j = 0; j < my_tiles; j++, kn++) {
             const unsigned sl = (unsigned)j % (unsigned)S, u = (unsigned)j / (unsigned)S;
-            if (!mbar_wait(ke + 8 * sl, (u & 1u) ^ 1u, c.abort_flag, P.error_flag, 8)) break;
+            if (!(ok = mbar_wait(ke + 8 * sl, (u & 1u) ^ 1u, c.abort_flag, P.error_flag, 8))) break;
             if (lane == 0) {
                 mbar_expect_tx(kf + 8 * sl, (unsigned)tile_bytes);
                 bulk_load(smem_u32(ring + sl * tile_bytes), kc + it_kc_index((size_t)(g + G * j) * 32, kh, 0, nkv, hd), (unsigned)tile_bytes, kf + 8 * sl);
             }
         }
         // the V slices go through the same bytes: not before the last K tile of every slot has been scored
-        for (int j = my_tiles > S ? my_tiles - S : 0; j < my_tiles; j++) {
-            if (!mbar_wait(ke + 8 * (j % S), (unsigned)(j / S) & 1u, c.abort_flag, P.error_flag, 8)) break;
-        }
+        for (int j = my_tiles > S ? my_tiles - S : 0; j < my_tiles; j++) ok = ok && mbar_wait(ke + 8 * (j % S), (unsigned)(j / S) & 1u, c.abort_flag, P.error_flag, 8);
 #pragma unroll 1
-        for (int i = 0; i < ntiles; i++) {
+        for (int i = 0; i < ntiles && ok; i++, vn++) {
             const unsigned sl = (unsigned)i % (unsigned)SV, u = (unsigned)i / (unsigned)SV;
             if (!mbar_wait(ve + 8 * sl, (u & 1u) ^ 1u, c.abort_flag, P.error_flag, 9)) break;
             if (lane == 0) {
@@ -932,6 +934,8 @@ __device__ __forceinline__ void attn_phase(const StepParams& P, const StepLayer&
                 bulk_load(smem_u32(ring + sl * vslot_bytes), vc + it_vc_index((size_t)i * 32, kh, g * epc, nkv, hd), (unsigned)vslot_bytes, vf + 8 * sl);
             }
         }
+        if (lane == 0) { drain_copies(kf, (unsigned)S, kn); drain_copies(vf, (unsigned)SV, vn); }
+        __syncwarp();
         return;                                                      // the loader meets the others at the next phase
     }
     if (warp < 2) {
@@ -1161,17 +1165,17 @@ __global__ void __launch_bounds__(ST_THREADS, 1) k_decode_step(const __grid_cons
                 else {
                     in.x = (ph == PH_D ? P.o : P.act) + (size_t)hb * ST_GPB; in.tag = tag_of(c.base, il, ph == PH_D ? PH_C : PH_G); in.nblk = 1; in.blk = 0;
                 }
-                if (!owner && !count_wait(P, c, P.sync, c.target + (unsigned)row_blocks, 1 + ph, false)) return;      // a dense row's owner follows the blocks' owners
+                if (!owner && !count_wait(P, c, P.sync, c.target + (unsigned)row_blocks, 1 + ph, false)) goto leave;      // a dense row's owner follows the blocks' owners
                 ST_EV(P, c, c.evt_base + 0);
                 block_transform(P, c, in);
                 ST_EV(P, c, c.evt_base + 1);
             }
-            if (tail_ph && !logits) { if (cta != 0) return; break; }
+            if (tail_ph && !logits) { if (cta != 0) goto leave; break; }
             c.target += (unsigned)row_blocks;
         } else {
             const int sub = ph == PH_B ? 0 : ph == PH_E ? 1 : ph == PH_G ? 2 : 3;
             const int kind = tail_ph ? SP_HEAD : span_kind(sub, L.recurrent);
-            if (!count_wait(P, c, P.sync, c.target, 1 + ph)) return;
+            if (!count_wait(P, c, P.sync, c.target, 1 + ph)) goto leave;
             ST_EV(P, c, c.evt_base + 0);
             if (c.tid == 0) mbar_arrive(c.ps);                       // the sum warps may enter this phase
             // (a CTA without row groups does not read the codes: nobody waits for it, so nothing would keep them)
@@ -1196,7 +1200,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) k_decode_step(const __grid_cons
                 const bool more = il + 1 < P.n_layer; const StepLayer& N = c.lay[(il + 1) & 1];
                 want_norm(more ? N.attn_norm : P.output_norm, more ? dense_row(P, N, drow) : nullptr);
             }
-            if (tail_ph) { if (cta != 0) return; break; }
+            if (tail_ph) { if (cta != 0) goto leave; break; }
             // the scratch is the next phase's once this CTA's sum warps are through (they are before anything the next phase needs has arrived)
             mbar_wait(c.pd, c.mph & 1u, c.abort_flag, P.error_flag, 5);
             c.mph++;
@@ -1205,7 +1209,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) k_decode_step(const __grid_cons
     }
     // every sum warp counts when it is through: nobody is left who could still read the words written below
     c.target += ST_NSUM * (unsigned)grid;
-    if (!count_wait(P, c, P.sync, c.target, 10, false)) return;
+    if (!count_wait(P, c, P.sync, c.target, 10, false)) goto leave;
     if (logits && c.warp == 0) {
         Pick q{ -INFINITY, 0xffffffffu };
         bool ok = true;
@@ -1218,7 +1222,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) k_decode_step(const __grid_cons
         }
 #pragma unroll
         for (unsigned mm = 16; mm > 0; mm >>= 1) { Pick o{ __shfl_xor_sync(0xffffffffu, q.v, mm), __shfl_xor_sync(0xffffffffu, q.i, mm) }; q = pick_better(q, o); }
-        if (!__all_sync(0xffffffffu, ok)) return;
+        if (!__all_sync(0xffffffffu, ok)) goto leave;
         if (c.lane == 0) {
             const unsigned pick = q.i == 0xffffffffu ? 0u : q.i;
             A[P.amx] = __uint_as_float(pick);
@@ -1226,6 +1230,8 @@ __global__ void __launch_bounds__(ST_THREADS, 1) k_decode_step(const __grid_cons
         }
     }
     if (c.tid == 0) { P.sync[1] = c.target; P.sync[3] = c.base + (unsigned)(ST_SUBS * (P.n_layer + 1) + 1); }
+leave:
+    asm volatile("cp.async.wait_all;" ::: "memory");                 // a norm's weights, a state tile that nobody waited for
 }
 
 }  // namespace

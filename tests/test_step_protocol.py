@@ -243,3 +243,20 @@ def test_the_kernel_uses_the_plan():
         src = f.read()
     uses = re.findall(r"P\.codes \+ ([^;]*?)P\.codes_half", src)
     assert uses == ["step_codes_half(ph) * "] * 2, uses
+
+
+def test_copies_are_waited_for_on_every_way_out():
+    """A CTA that leaves with copies in flight lets them land in the shared memory of the next one: whoever starts bulk copies drains its
+    rings at its end, and the consumer warps have one way out, behind a wait for their asynchronous copies."""
+    with open(os.path.join(CSRC, "it_step.cu")) as f:
+        src = re.sub(r"//[^\n]*", "", f.read())
+    producer = re.search(r"void producer\(.*?\n}\n", src, re.S).group()
+    assert producer.count("bulk_load(") == 1 and re.search(r"drain_copies\(c\.bars, [^;]*;\s*}\n$", producer) and "return" not in producer
+    attn = re.search(r"void attn_phase\(.*?\n}\n", src, re.S).group()
+    loader = attn[attn.index("warp == ST_AT_LOADER"):]
+    loader = loader[:loader.index("return;")]
+    assert attn.count("bulk_load(") == loader.count("bulk_load(") == loader.count("drain_copies(") == 2
+    consumers = src[src.index("c.base = *reinterpret_cast<volatile unsigned*>(P.sync + 3)"):]
+    consumers = consumers[:consumers.index("leave:")]
+    assert not re.search(r"\breturn;", consumers)
+    assert re.search(r"leave:\s*asm volatile\(\"cp\.async\.wait_all;", src)
