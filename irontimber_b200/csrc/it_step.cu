@@ -126,6 +126,7 @@ struct Cta {
     int tid, warp, lane;
     unsigned q;                        // chunks of the CTA's stream passed so far (slot = q % slots, phase = (q / slots) & 1; slots is a power of two)
     unsigned tf, ps, pd, dn;           // mbarriers: terms of a slot's chunk in place [slots], phase started, phase summed, dense row's warp sums in place
+    unsigned issued;                   // where the producer says how many chunks of the stream it has issued
     unsigned mph;                      // matrix phases so far
     unsigned at;                       // mbarriers of the attention block: K full / free, V full / free, eight of each
     const StepLayer* lay;              // the two shared-memory copies of layer descriptions (layer il at lay[il & 1])
@@ -259,6 +260,34 @@ __device__ __forceinline__ bool count_wait(const StepParams& P, Cta& c, const un
 __device__ __forceinline__ int mat_count(const StepParams& P) { return 4 * P.n_layer + ((P.flags & 4) ? 1 : 0); }
 __device__ __forceinline__ int span_kind(int sub, int recurrent) { return sub == 0 ? (recurrent ? SP_IN_GDN : SP_IN_ATT) : sub == 1 ? (recurrent ? SP_OUT_GDN : SP_OUT_ATT) : sub == 2 ? SP_GATE_UP : SP_DOWN; }
 
+// A wait on an mbarrier sees the parity of a phase only, so whoever waits for chunk q of a slot must know that the chunk before it in that
+// slot is through: a sum warp that leaves a row group of more chunks than the ring has slots to the other one, or a consumer group
+// whose chunk's predecessor was another group's, otherwise takes the phase before for its own - it adds terms that are not there yet, or
+// hands a slot back twice.  The producer issues a chunk when its slot has been handed back, so it says how many chunks it has
+// issued, and nobody looks at a chunk's barriers before it is among them (the first `slots` of a phase follow chunks of the phase
+// before, which everyone knows to be through).
+__device__ __forceinline__ void st_issued(unsigned at, unsigned n) { asm volatile("st.release.cta.shared::cta.u32 [%0], %1;" :: "r"(at), "r"(n) : "memory"); }
+__device__ __forceinline__ unsigned ld_issued(unsigned at) { unsigned v; asm volatile("ld.acquire.cta.shared::cta.u32 %0, [%1];" : "=r"(v) : "r"(at) : "memory"); return v; }
+// The chunks issued once chunk q is one of them; fewer when the wait had to end without it.
+__device__ __noinline__ unsigned issued_past(unsigned at, unsigned q, volatile int* abort_flag, int* error_flag, int site) {
+    const long long t0 = clock64();
+#pragma unroll 1
+    for (;;) {
+        const unsigned v = ld_issued(at);
+        if ((int)(v - q) > 0 || *abort_flag) return v;
+        if (clock64() - t0 > WAIT_CLOCKS) { if (!*abort_flag) atomicExch(error_flag, site); *abort_flag = 1; return v; }
+        __nanosleep(32);
+    }
+}
+// Waits for the chunk's bytes; `issued`: chunks known to have been issued, or to follow a phase that is through.
+__device__ __forceinline__ bool chunk_wait(unsigned bar, unsigned parity, unsigned q, unsigned& issued, const StepParams& P, const Cta& c, int site) {
+    if ((int)(issued - q) <= 0) {
+        issued = issued_past(c.issued, q, c.abort_flag, P.error_flag, site);
+        if ((int)(issued - q) <= 0) return false;
+    }
+    return mbar_wait(bar, parity, c.abort_flag, P.error_flag, site);
+}
+
 // Whoever starts bulk copies leaves only when they have landed, also where nobody waits for them any more: the last `issued` copies of
 // a ring of `slots` with full barriers at `full` (each wait bounded by the clock limit).
 __device__ __noinline__ void drain_copies(unsigned full, unsigned slots, unsigned issued) {
@@ -287,6 +316,7 @@ __device__ __forceinline__ void producer(const StepParams& P, const Cta& c) {
             if (i == sp.hl) { unit = sp.uf; cq = 0; }
             if (i == sp.n - sp.tl) { unit = sp.ut; cq = sp.lead; }
             if (!mbar_wait(c.bars + 8 * (P.slots + s), ph ^ 1u, c.abort_flag, P.error_flag, 2)) { ok = false; break; }
+            st_issued(c.issued, (unsigned)issued + 1u);
             const bool second = cq >= sp.cpr;
             mbar_expect_tx(c.bars + 8 * s, ST_CHUNK);
             bulk_load(smem_u32(c.smem + s * ST_CHUNK), tiles + ((size_t)(second ? unit + sp.units : unit) * sp.cpr + (second ? cq - sp.cpr : cq)) * ST_CHUNK, ST_CHUNK, c.bars + 8 * s);
@@ -531,13 +561,14 @@ __device__ __forceinline__ void matvec_phase(const StepParams& P, Cta& c, const 
         return __fmul_rn(__fmul_rn(__half2float(dwh), dxs[b >> 1]), (float)((S >> (2 * t)) - sss[b]));
     };
     bool ok = !*c.abort_flag;                                        // (the row may not have come) a lane whose wait ran out goes on without waits and arrivals; the CTA leaves at its next wait
+    unsigned issued = c.q + (unsigned)P.slots;                       // the slots of these were another phase's
 #pragma unroll 1
     for (int i = warp / ST_CW; i < n; i += ST_NG) {
         const unsigned q = c.q + (unsigned)i;
         const int cs = (int)(q & smask);
         const unsigned r = (unsigned)(i < hl ? i : i < whole ? i - hl : i + lead);
         const int b0 = (cpr == 1 ? 0 : (int)(r - __umulhi(r, magic) * (unsigned)cpr)) * ST_TPC + wi, b1 = b0 + ST_CW;      // r modulo cpr: the chunk's index within its row of blocks
-        if (ok) ok = mbar_wait(c.bars + 8 * cs, (q >> sshift) & 1u, c.abort_flag, P.error_flag, 3);
+        if (ok) ok = chunk_wait(c.bars + 8 * cs, (q >> sshift) & 1u, q, issued, P, c, 3);
         const unsigned char *tile0 = c.smem + cs * ST_CHUNK + wi * IT_TILE_BYTES, *tile1 = tile0 + ST_CW * IT_TILE_BYTES;
         int a0[4], a1[4];
         dots(tile0, b0, a0); dots(tile1, b1, a1);
@@ -594,6 +625,7 @@ __device__ __forceinline__ void sum_warps(const StepParams& P, Cta& c) {
             }
             __syncwarp();
         }
+        unsigned issued = c.q + (unsigned)P.slots;
         int unit = sp.uf;
 #pragma unroll 1
         for (int i = 0, ord = 0, len; i < n; i += len, ord++) {
@@ -624,6 +656,10 @@ __device__ __forceinline__ void sum_warps(const StepParams& P, Cta& c) {
             }
             // a lane whose wait ran out goes on without waits; the warp leaves by a vote after the row group
             unsigned q = c.q + (unsigned)i;
+            // the chunks before this row group's first `slots` in their slots may be the other warp's (behind those come its own): one look a row
+            // group is 1 % of a step less than one a chunk
+            const unsigned want = q + (unsigned)min(len, P.slots);
+            if (ok && (int)(want - issued) > 0) { issued = issued_past(c.issued, want - 1u, c.abort_flag, P.error_flag, 6); ok = (int)(want - issued) <= 0; }
 #pragma unroll 1
             for (int k = 0; k < len; k += 2, q += 2) {               // two chunks a turn: this warp has one issue slot in four, and half a turn is overhead
                 const int c0 = (int)(q & smask), c1 = (int)((q + 1) & smask);
@@ -1102,12 +1138,13 @@ __global__ void __launch_bounds__(ST_THREADS, 1) k_decode_step(const __grid_cons
     c.bars = smem_u32(tail);                                         // full[s] at bars + 8 s, empty[s] at bars + 8 (slots + s), terms full[s] at tf + 8 s
     c.tf = c.bars + 16 * P.slots; c.ps = c.tf + 8 * P.slots; c.pd = c.ps + 8; c.dn = c.pd + 8; c.at = c.dn + 8;
     c.lay = reinterpret_cast<const StepLayer*>(tail + 704);         // two layer descriptions
-    c.abort_flag = reinterpret_cast<volatile int*>(tail + ST_BARS - 16); c.verdict = c.abort_flag + 1;
+    c.abort_flag = reinterpret_cast<volatile int*>(tail + ST_BARS - 16); c.verdict = c.abort_flag + 1; c.issued = smem_u32(tail + ST_BARS - 8);
     c.sp = reinterpret_cast<const StepSpan*>(tail + ST_BARS);
     c.sg = reinterpret_cast<const uint32_t*>(tail + ST_BARS + SP_KINDS * sizeof(StepSpan));
     c.tid = threadIdx.x; c.warp = c.tid >> 5; c.lane = c.tid & 31;
     c.q = 0u; c.nsync = 0; c.evt_on = 0; c.dense_seq = 0u; c.mph = 0u;
     if (c.tid == 0) {
+        st_issued(c.issued, 0u);
         *c.abort_flag = *reinterpret_cast<volatile unsigned*>(P.sync + 2) ? 1 : 0;      // a step that was given up earlier: nothing runs until the host has cleared the words
         for (int s = 0; s < P.slots; s++) { mbar_init(c.bars + 8 * s, 1); mbar_init(c.bars + 8 * (P.slots + s), 1); mbar_init(c.tf + 8 * s, ST_CW); }
         mbar_init(c.ps, 1); mbar_init(c.pd, ST_NSUM); mbar_init(c.dn, 8);

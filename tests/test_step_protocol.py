@@ -8,6 +8,7 @@ waits for.  Any CTA may be arbitrarily late; a write is safe only if every read 
 matrices and the halves of the quantised row come from the kernel's own plan (it_step_plan.h).
 """
 import ctypes as C
+import graphlib
 import os
 import re
 import subprocess
@@ -243,6 +244,98 @@ def test_the_kernel_uses_the_plan():
         src = f.read()
     uses = re.findall(r"P\.codes \+ ([^;]*?)P\.codes_half", src)
     assert uses == ["step_codes_half(ph) * "] * 2, uses
+
+
+class Ring:
+    """One CTA's ring over the matrices of its spans: chunks are issued in order, land in any order, are multiplied by one of three groups of
+    warps and summed by one of two warps.  A wait sees the parity of its barrier only, so when it begins the phase before must surely be
+    complete, and the phase after must not complete before it has ended."""
+
+    GROUPS, SUMS = 3, 2
+
+    def __init__(self, spans, slots, gated):
+        self.after, self.slots = {}, slots
+        edge = lambda e, *before: self.after.setdefault(e, set()).update(b for b in before if b is not None)
+        group, sums, phase, q0 = [None] * self.GROUPS, [None] * self.SUMS, None, 0
+        self.chunks = sum(s["n"] for s in spans)
+        for q in range(self.chunks):
+            edge(("issue", q), ("issue", q - 1) if q else None, ("free", q - slots) if q >= slots else None)
+            edge(("land", q), ("issue", q))
+        for p, s in enumerate(spans):
+            edge(("phase", p), phase, *sums)
+            for i in range(s["n"]):                          # consumer groups
+                q, g = q0 + i, i % self.GROUPS
+                edge(("full wait", q), group[g], ("phase", p), ("issue", q) if gated and i >= slots else None)
+                edge(("use", q), ("full wait", q), ("land", q))
+                group[g] = ("use", q)
+            i, sums = 0, [("phase", p)] * self.SUMS
+            for o, (u, part) in enumerate(units_of(s)):
+                n, w = {"first": s["hl"], "last": s["tl"], "whole": s["cpr"] * s["parts"]}[part], o % self.SUMS
+                if gated and i + min(n, slots) > slots:      # one look a row group: its first `slots` chunks have been issued
+                    edge(("group", p, o), sums[w], ("issue", q0 + i + min(n, slots) - 1))
+                    sums[w] = ("group", p, o)
+                for k in range(0, n, 2):
+                    turn = [q0 + i + k + d for d in range(min(2, n - k))]
+                    for q in turn:
+                        edge(("sum wait", q), sums[w])
+                        edge(("sum", q), ("sum wait", q), ("use", q))
+                        sums[w] = ("sum", q)
+                    for q in turn:
+                        edge(("free", q), sums[w])
+                i += n
+            assert i == s["n"]
+            q0 += s["n"]
+        self.before, order = {}, list(graphlib.TopologicalSorter(self.after).static_order())
+        bit = {e: 1 << k for k, e in enumerate(order)}
+        for e in order:
+            m = 0
+            for b in self.after.get(e, ()):
+                m |= self.before[b] | bit[b]
+            self.before[e] = m
+        self.bit = bit
+
+    def surely(self, a, b):
+        return self.before[b] & self.bit[a]
+
+    def aliased(self):
+        out = []
+        for q in range(self.chunks):
+            if q >= self.slots:
+                out += [(w, q) for w, done in (("full wait", "land"), ("sum wait", "use")) if not self.surely((done, q - self.slots), (w, q))]
+            if q + self.slots < self.chunks:
+                assert self.surely(("use", q), ("land", q + self.slots)) and self.surely(("sum", q), ("use", q + self.slots))
+        return out
+
+
+def ring_spans(plan, g, cta, layers=2):
+    kinds = sum(([("in_gdn" if g.recurrent(il) else "in_att"), "out_gdn" if g.recurrent(il) else "out_att", "gate_up", "down"] for il in range(layers)), []) + ["head"]
+    return [spans(plan, g, k)[cta] for k in kinds]
+
+
+@pytest.mark.parametrize("slots", [16, 8, 4])
+@pytest.mark.parametrize("name", GEOMETRIES)
+def test_no_chunk_wait_takes_another_phase_for_its_own(plan, name, slots):
+    g = Geometry(**GEOMETRIES[name])
+    for cta in (0, 1, 20, 86, g.grid - 1):
+        assert Ring(ring_spans(plan, g, cta), slots, True).aliased() == []
+
+
+def test_the_model_sees_a_wait_a_phase_early(plan):
+    """A row of the down projection is 17 chunks: the sum warp that has the row group behind it waits on a slot of the ring of 16 whose chunk
+    the other one may not have summed; and a group's chunk may have been preceded in its slot by one of another group's that has yet to land."""
+    g = Geometry()
+    found = Ring(ring_spans(plan, g, 86), 16, False).aliased()
+    down = sum(s["n"] for s in ring_spans(plan, g, 86)[:3])
+    assert ("sum wait", down + 17) in found and any(w == "full wait" for w, _ in found)
+    with open(os.path.join(CSRC, "it_step.cu")) as f:
+        src = f.read()
+    loops = re.search(r"void matvec_phase\(.*?\n}\n.*?void sum_warps\(.*?\n}\n", src, re.S).group()
+    assert len(re.findall(r"chunk_wait\(c\.bars \+ 8 \* cs,", loops)) == 1 and not re.findall(r"mbar_wait\w*\(c\.bars", loops)
+    gate, tf = re.search(r"want = q \+ \(unsigned\)min\(len, P\.slots\);\s*if \(ok && \(int\)\(want - issued\) > 0\) { issued = issued_past\(c\.issued, want - 1u,", loops), [m.start() for m in re.finditer(r"mbar_wait\(c\.tf", loops)]
+    assert len(tf) == 2 and gate.start() < tf[0]
+    producer = re.search(r"void producer\(.*?\n}\n", src, re.S).group()
+    assert loops.count("unsigned issued = c.q + (unsigned)P.slots;") == 2              # the first chunks of a phase follow a phase that is through
+    assert producer.index("mbar_wait(") < producer.index("st_issued(c.issued, (unsigned)issued + 1u)") < producer.index("issued++")
 
 
 def test_copies_are_waited_for_on_every_way_out():
