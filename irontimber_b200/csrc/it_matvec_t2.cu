@@ -29,6 +29,7 @@
 // + 4*ntok*rows (x2 when accumulating).  The kernel is HBM-bound.
 #include "it_internal.h"
 #include "it_pipe.cuh"
+#include "it_route.h"
 #include <algorithm>
 
 namespace {
@@ -325,7 +326,7 @@ int launch(it_ctx* c, const it_mat* w, int ntok, const it_q8* x, size_t xrow0, f
         if (per_sm == 3) return launch_cfg<MT, 1, 3, false>(c, w, ntok, x, xrow0, y, y_stride, accum, nullptr, slots, nbuf, grid);
         if (per_sm == 2) return launch_cfg<MT, 1, 2, false>(c, w, ntok, x, xrow0, y, y_stride, accum, nullptr, slots, nbuf, grid);
         // a single CTA per SM: long rows get three consumer groups so that the per-warp chain stays short
-        if (long_rows) return launch_cfg<MT, 3, 1, false>(c, w, ntok, x, xrow0, y, y_stride, accum, nullptr, slots, nbuf, grid);
+        if (long_rows) return launch_cfg<MT, 3, 1, false>(c, w, ntok, x, xrow0, y, y_stride, accum, nullptr, it_mv_ring(slots, 3), nbuf, grid);
         return launch_cfg<MT, 1, 1, false>(c, w, ntok, x, xrow0, y, y_stride, accum, nullptr, slots, nbuf, grid);
     }
     return it_fail(IT_EINVAL, "it_matvec_t2: %d rows of width %zu exceed the shared-memory budget", MT, w->cols);

@@ -2,6 +2,12 @@
 #pragma once
 #include <cstddef>
 
+// ---- ternary products of up to eight rows -----------------------------------------------------------------------------------
+// Ring slots of a CTA of k_matvec_t2 (it_matvec_t2.cu) whose chunks `groups` groups of warps take in turn: a multiple of them, so that a slot
+// is always the same group's.  A wait on an mbarrier sees a parity: in a ring of another size a group's chunk follows another group's in
+// its slot, and a copy that lands that much late would let the group take the phase before for its own.
+static inline int it_mv_ring(int slots, int groups) { return slots - slots % groups; }
+
 // ---- ternary products of more than eight rows -----------------------------------------------------------------------------
 // Row groups (of 32 matrix rows) a CTA of the mma.sync kernel owns: 128-row tiles with sixteen consumer warps when that still gives
 // the grid at least 0.6 CTAs per SM, else 64-row tiles (eight warps, two CTAs per SM), else 32-row tiles.

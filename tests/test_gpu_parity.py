@@ -171,6 +171,15 @@ def test_matvec_t2_kparity_grid_bit_exact(be, orc, rows, ntok, acc):
     assert np.array_equal(bits(got), bits(want))
 
 
+# long rows on one CTA per SM: three groups of warps over rings of nine (of eleven), six (of seven) and three (of four) slots
+@pytest.mark.parametrize("rows,cols,ntok", [(1001, 10240, 4), (5000, 12288, 3), (333, 14336, 4), (9600, 19456, 2)])
+def test_matvec_t2_three_groups_bit_exact(be, orc, rows, cols, ntok):
+    rng = np.random.default_rng(rows + cols)
+    raw = synth_pq2(rows + cols, rows, cols)
+    got, want = run_mv(be, orc, raw, rows, cols, rng.standard_normal((ntok, cols)).astype(np.float32))
+    assert np.array_equal(bits(got), bits(want))
+
+
 @pytest.mark.parametrize("rows,cols", [(17408, 5120), (5120, 6144), (5120, 17408), (1024, 5120)])
 def test_matvec_t2_model_shapes_bit_exact(be, orc, rows, cols):
     rng = np.random.default_rng(rows + cols)

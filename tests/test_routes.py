@@ -1,6 +1,7 @@
 """The rules that pick a kernel by sizes (csrc/it_route.h), held to their edges on the CPU.  148 SMs are a B200's."""
 import ctypes as C
 import os
+import re
 import subprocess
 
 import pytest
@@ -19,6 +20,7 @@ def routes(tmp_path_factory):
                    'extern "C" int tc_tile(long rg, long ntok, int sm) { return it_tc_tile(rg, ntok, sm); }\n'
                    'extern "C" int attn_tiled(int slot0, int nt, int blk, int sm) { return it_attn_takes_tiled(256, 24, 4, slot0, nt, blk, sm); }\n'
                    'extern "C" int attn_group(int hd, int nh, int nkv, int npos) { auto g = it_attn_grouping(hd, nh, nkv, npos); return 10 * g.heads + g.rows; }\n'
+                   'extern "C" int mv_ring(int slots, int groups) { return it_mv_ring(slots, groups); }\n'
                    'extern "C" int gdn_rows(int sd, int nt) { return it_gdn_rows_takes(sd, nt); }\n')
     subprocess.run(["g++", "-std=c++17", "-Wall", "-Werror", "-Wno-unused-function", "-shared", "-fPIC", "-I", CSRC, str(src), "-o", str(lib)], check=True)
     return C.CDLL(str(lib))
@@ -69,3 +71,27 @@ def test_grouping_of_attention_heads(routes, hd, nh, nkv, npos, heads, rows):
 def test_prompt_delta_rule(routes, sd, nt, takes):
     """One or two tokens are refused: one warp would store a state row that the other may not have read yet."""
     assert routes.gdn_rows(sd, nt) == takes
+
+
+def overtaken_copy(slots, groups):
+    """A chunk whose group can find its slot a phase behind: the chunk before it in the slot may still be landing when the group, through with
+    its own chunks up to then, begins to wait.  Copies land in any order; a chunk is issued when its slot's last one has been read."""
+    for q in range(slots, 4 * slots):
+        own = range(q - groups, -1, -groups)                       # chunks this group has read
+        read = set(own)
+        for c in own:                                              # a chunk that was read had been issued, and so had all before it: their slots' last ones were read
+            read |= set(range(0, c - slots + 1))
+        if q - slots not in read:
+            return q
+    return None
+
+
+@pytest.mark.parametrize("slots", range(4, 17))
+def test_ring_of_several_groups(routes, slots):
+    """Three groups of k_matvec_t2 on the ring that the launch gives them; sizes that are no multiple of three can be overtaken."""
+    ring = routes.mv_ring(slots, 3)
+    assert 3 <= ring <= slots and overtaken_copy(ring, 3) is None
+    assert slots % 3 == 0 or overtaken_copy(slots, 3) is not None
+    with open(os.path.join(CSRC, "it_matvec_t2.cu")) as f:
+        src = f.read()
+    assert re.findall(r"launch_cfg<MT, 3,[^;]*;", src) == re.findall(r"launch_cfg<MT, 3,[^;]*it_mv_ring\(slots, 3\)[^;]*;", src) != []
