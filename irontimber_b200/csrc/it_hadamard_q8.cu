@@ -28,30 +28,16 @@ k_hadamard(const float* arena_in, size_t in_off, size_t in_stride,
                              perm_hd, perm_nk, perm_rep, qs, qd, qsum, q_stride, pro);
 }
 
-// Hadamard + q8k, 64 threads a block (it_had16_*).  ROW: a CTA takes a whole row, a pair of warps per block (at most eight), so that a
-// norm is formed once; else a CTA of 64 threads takes one block and, where there is a norm, forms it for itself.
-// silu(a) * b of four elements, the operations of it_silu.  CUDA's division branches, which puts sixteen of them behind one another; with
-// a denominator 1 + exp(-x) inside the normal range and a numerator that cannot lose digits, the quotient is formed from a
-// correctly rounded reciprocal and an exact residual (Markstein, IBM J. Res. Dev. 34, 1990: the result is the rounded quotient unless
-// the denominator's digits are all ones), four side by side; anything else in the warp takes the division.
+// silu(a) * b of four elements, the operations of it_silu.  CUDA's division branches, which puts sixteen of them behind one another; where every
+// lane's operands suit it (it_quot_fits), the quotient is formed without branches, four side by side; else the warp takes the division.
 __device__ __forceinline__ float4 silu_mul4(const float4 a4, const float4 b4) {
     const float a[4] = { a4.x, a4.y, a4.z, a4.w }, b[4] = { b4.x, b4.y, b4.z, b4.w };
     float d[4], q[4]; bool plain = true;
 #pragma unroll
-    for (int i = 0; i < 4; i++) {
-        d[i] = it_add(1.0f, it_expf_inline(-a[i]));
-        const float m = fabsf(a[i]);
-        plain = plain && d[i] < 1e15f && m < 1e15f && (m > 1e-15f || m == 0.f) && (__float_as_uint(d[i]) & 0x7fffffu) != 0x7fffffu;
-    }
+    for (int i = 0; i < 4; i++) { d[i] = it_add(1.0f, it_expf_inline(-a[i])); plain = plain && it_quot_fits(a[i], d[i]); }
     if (__all_sync(0xffffffffu, plain)) {
 #pragma unroll
-        for (int i = 0; i < 4; i++) {
-            float r; asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d[i]));
-            r = it_fma(it_fma(-d[i], r, 1.0f), r, r);
-            r = it_fma(it_fma(-d[i], r, 1.0f), r, r);
-            const float t = it_mul(a[i], r);
-            q[i] = it_fma(it_fma(-d[i], t, a[i]), r, t);
-        }
+        for (int i = 0; i < 4; i++) { float r; asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d[i])); q[i] = it_quot(a[i], d[i], r); }
     } else {
 #pragma unroll 1
         for (int i = 0; i < 4; i++) { const float x = i == 0 ? a[0] : i == 1 ? a[1] : i == 2 ? a[2] : a[3], y = i == 0 ? d[0] : i == 1 ? d[1] : i == 2 ? d[2] : d[3], z = it_div(x, y); if (i == 0) q[0] = z; else if (i == 1) q[1] = z; else if (i == 2) q[2] = z; else q[3] = z; }
@@ -59,6 +45,8 @@ __device__ __forceinline__ float4 silu_mul4(const float4 a4, const float4 b4) {
     return make_float4(it_mul(q[0], b[0]), it_mul(q[1], b[1]), it_mul(q[2], b[2]), it_mul(q[3], b[3]));
 }
 
+// Hadamard + q8k, 64 threads a block (it_had16_*).  ROW: a CTA takes a whole row, a pair of warps per block (at most eight), so that a
+// norm is formed once; else a CTA of 64 threads takes one block and, where there is a norm, forms it for itself.
 struct Had16In {
     const float* x; size_t stride; const float* signs; int rotate, nblk;
     unsigned hd, nk, rep;

@@ -149,3 +149,17 @@ IT_HD_BIG void it_sincosf(float x, float* s, float* c) {
 IT_HD float it_silu(float x) { return it_div(x, it_add(1.0f, it_expf(-x))); }          // x / (1 + exp(-x))
 IT_HD float it_sigmoid(float x) { return it_div(1.0f, it_add(1.0f, it_expf(-x))); }    // 1 / (1 + exp(-x))
 IT_HD float it_softplus(float x) { return x > 20.0f ? x : it_logf(it_add(1.0f, it_expf(x))); }
+
+// a / d without a branch, so that several overlap: from r, 1 / d to a few units in the last place, through a correctly rounded reciprocal
+// and an exact residual (Markstein, IBM J. Res. Dev. 34, 1990: the rounded quotient unless the denominator's digits are all ones).  A zero
+// keeps its sign, which the residual would lose.  it_quot_fits: whether a and a d of at least 1 are where no step leaves the normal range.
+IT_HD bool it_quot_fits(float a, float d) {
+    const float m = fabsf(a);
+    return d < 1e15f && m < 1e15f && (m > 1e-15f || m == 0.f) && (it_float_to_bits(d) & 0x7fffffu) != 0x7fffffu;
+}
+IT_HD float it_quot(float a, float d, float r) {
+    r = it_fma(it_fma(-d, r, 1.0f), r, r);
+    r = it_fma(it_fma(-d, r, 1.0f), r, r);
+    const float t = it_mul(a, r), q = it_fma(it_fma(-d, t, a), r, t);
+    return a == 0.f ? a : q;
+}
