@@ -54,14 +54,9 @@ constexpr int ST_CW = 4;                               // warps per consumer gro
 constexpr int ST_NG = 3;                               // consumer groups; group j takes the chunks i of a phase with i % ST_NG == j
 constexpr int ST_NCONS = ST_CW * ST_NG;                // consumer warps
 constexpr int ST_CT = ST_NCONS * 32;                   // consumer threads
+static_assert(ST_CHUNK == ST_TPC * IT_TILE_BYTES && ST_PITCH == IT_HAD_PITCH, "it_step_plan.h");
 constexpr int ST_NSUM = 2;                             // warps that only add the per-block terms in block order
 constexpr int ST_THREADS = ST_CT + (ST_NSUM + 1) * 32; // + the sum warps + the producer warp
-constexpr int ST_CHUNK = ST_TPC * IT_TILE_BYTES;       // bytes of one ring slot
-constexpr int ST_TERMS = ST_TPC * 32;                  // terms of one chunk (floats)
-constexpr int ST_SMEM = 227 * 1024;                    // dynamic shared memory of the CTA
-constexpr int ST_BARS = 1024;                          // bytes reserved for mbarriers, flags, layer descriptions and spans
-constexpr int ST_SD = 128;                             // delta-rule state size this kernel is built for
-constexpr int ST_RED = 384;                            // bytes: the dense row's eight f64 warp sums, then the transform's [8] sums of squares and [4][2] group maxima
 
 struct StepLayer {
     const uint8_t *in_proj, *out_proj, *gate_up, *down;
@@ -102,7 +97,7 @@ struct StepParams {
     granule* prefix;                   // [grid][32] running sums of a cut row group (two matrices' worth) and the tag
     granule* partials;                 // one greedy-pick partial per sum warp: value, row, tag
     unsigned long long* att_sc; int att_stride;   // per head: the scores its CTAs exchange [nh][att_stride] (value and tag)
-    const uint32_t* sg[4]; int sg_off[4], sg_words[4];   // sign bits of the four widths (n_embd, ssm_inner, attention output, n_ff): words, and where they start in shared memory
+    const uint32_t* sg[4];             // sign bits of the four widths (n_embd, ssm_inner, attention output, n_ff), 32 words a block of 1024
     const float *tok_embd, *output_norm; const uint8_t* output;
     uint32_t* toks; int* pos;
     unsigned* sync;                    // [0] arrivals, [1] arrivals at the end of the last launch, [2] abort word
@@ -131,7 +126,6 @@ struct Cta {
     unsigned at;                       // mbarriers of the attention block: K full / free, V full / free, eight of each
     const StepLayer* lay;              // the two shared-memory copies of layer descriptions (layer il at lay[il & 1])
     const StepSpan* sp;                // this CTA's spans, by matrix kind
-    const uint32_t* sg;                // sign bits of the four widths (P.sg_off)
     unsigned base, target;             // tags of this launch start here; what the counter reaches when the transforms so far have begun
     int nsync;                         // waits in front of matrix phases passed so far (index into the trace)
     unsigned dense_seq;                // dense rows this sum warp has finished in this launch
@@ -213,10 +207,6 @@ __device__ __forceinline__ void publish(granule* dst, int u, int lane, float v, 
 // Granule i of a run of row groups holds rows r, r + 11 and (unless it is the last of its row group) r + 22.
 __device__ __forceinline__ int granule_row(int i, bool& two) { const int u = i / ST_GPU, l = i - u * ST_GPU; two = l == ST_GPU - 1; return u * 32 + l; }
 __device__ __forceinline__ unsigned tag_of(unsigned base, int il, int sub) { return base + 1u + (unsigned)(ST_SUBS * il + sub); }
-// Scratch of a matrix phase of nb blocks a row: ST_RED bytes of sums, the q8k row with its scales (a float per 256) and block sums
-// (an int per 128), then the transform's exchange area and, after it, the terms [slots][ST_TPC][32] of the ring's chunks.
-__host__ __device__ __forceinline__ int terms_at(int nb) { return ST_RED + ((nb * 134 + 127) & ~127); }
-
 // Nothing waits for everyone: a phase starts where its granules are, and polls them.  All CTAs polling a row through the whole of
 // the phases that lead to it would take bandwidth from the weights, so they wait on a counter until the owners of the row's
 // blocks have begun to transform them (a hint: it orders nothing and needs no fence), about 1500 cycles before the codes come.
@@ -400,6 +390,7 @@ __device__ __forceinline__ void block_transform(const StepParams& P, const Cta& 
     float* ex0 = reinterpret_cast<float*>(c.scratch + ST_RED);
     float* red = reinterpret_cast<float*>(c.scratch + 64);   // [8] warp sums of squares, [4][2] group maxima
     const float* wb = reinterpret_cast<const float*>(c.scratch + P.w_off);
+    const unsigned m16 = warp < 2 && in.codes ? reinterpret_cast<const unsigned short*>(in.signs)[j] : 0u;      // the thread's sixteen signs, here long before the row
     cons_sync();                                             // the scratch is nobody's any more (the block before may still have been writing state)
     if (in.plain) {
 #pragma unroll 1
@@ -472,7 +463,6 @@ __device__ __forceinline__ void block_transform(const StepParams& P, const Cta& 
                     v[4 * u + 2] = it_mul(it_mul(v[4 * u + 2], sc), w.z); v[4 * u + 3] = it_mul(it_mul(v[4 * u + 3], sc), w.w);
                 }
             }
-            const unsigned m16 = reinterpret_cast<const unsigned short*>(in.signs)[j];
 #pragma unroll
             for (int i = 0; i < 16; i++) v[i] = __uint_as_float(__float_as_uint(v[i]) ^ ((m16 << (31 - i)) & 0x80000000u));     // times +-1
             it_had16_rotate(v, ex, j, [] { pair_sync(); });
@@ -876,8 +866,8 @@ __device__ __forceinline__ void gdn_phase(const StepParams& P, const StepLayer& 
 // k_attn_prep and k_attention (it_support.cu; src/cpu.rs:252-272): every score a sequential dot over the head dimension,
 // the exponentials added in ascending position order by one thread, every output element accumulating w[p] * v[p][j] in
 // ascending position order.  The k and v rows of the new position are recomputed by each of the heads that share the KV
-// head and used from shared memory (after the same f16 rounding the cache applies); the first head of the group stores
-// them into the cache.
+// head and used from shared memory (after the same f16 rounding the cache applies); the CTAs of the first head of the
+// group store them into the cache.
 // Data movement: both caches are tiled (32 positions x head_dim halves = one contiguous 16 KB block per KV head), so a
 // loader warp brings whole tiles into a ring of 16 KB slots with one bulk copy each.  One warp per slot scores its K
 // tiles, a position per lane, from shared memory; the V tiles follow through the same ring and four warps (two output
@@ -895,7 +885,7 @@ __device__ __forceinline__ void attn_prefetch(const StepParams& P, const StepLay
 constexpr int ST_AT_MAXS = 8, ST_AT_LOADER = ST_NCONS - 1, ST_AT_T = (ST_NCONS - 1) * 32;
 // the block's own barrier: every consumer warp but the loader, which runs ahead and only joins the next phase
 __device__ __forceinline__ void at_sync() { asm volatile("bar.sync 4, %0;" :: "n"(ST_AT_T) : "memory"); }
-// G = P.attn_g CTAs share a head (hg = G h + g).  Each forms q and the new position's k and v for itself, scores the K
+// G = P.attn_g CTAs share a head (hg = G h + g).  Each forms q and the new position's k for itself, and its elements of v, scores the K
 // tiles i with i % G == g, publishes those scores, reads the others' as they come (the tag is the exchange: a
 // counter would need a base that nobody's late start can miss), runs the softmax for itself (one thread adds the exponentials in position order) and accumulates the
 // head_dim / G output elements [g head_dim / G, ...) over all positions from row slices of the V tiles.  A single SM can
@@ -913,10 +903,10 @@ __device__ __forceinline__ void attn_phase(const StepParams& P, const StepLayer&
     float* sc = reinterpret_cast<float*>(c.scratch);                 // [n] scores
     float* qs = sc + ((n + 3) & ~3);                                 // [hd] q head after norm + rope
     float* kl = qs + hd;                                             // [hd] k row of the new position as the cache holds it
-    float* vl = kl + hd;                                             // [hd] v row of the new position as the cache holds it
-    float* gs = vl + hd;                                             // [hd] gate row of the head
-    float* red = gs + hd;                                            // [32] + the sum
-    unsigned char* ring = reinterpret_cast<unsigned char*>(red + 48) + ((128u - (smem_u32(red + 48) & 127u)) & 127u);
+    float* vl = kl + hd;                                             // [epc] this CTA's elements of the v row of the new position, as the cache holds them
+    float* gs = vl + epc;                                            // [epc] and of the head's gate row
+    float* red = gs + epc;                                           // [32] + the sum
+    unsigned char* ring = reinterpret_cast<unsigned char*>(red + ST_AT_RED) + (-smem_u32(red + ST_AT_RED) & 15u);
     const int room = (int)((c.scratch + P.scratch) - ring);
     // K: tile j of this CTA goes to slot j % S and is scored by warp j % S, so every slot is filled and emptied by the same two
     // warps in order.  V: slice j goes to slot j % SV; the output warps walk the slices in order.
@@ -931,18 +921,19 @@ __device__ __forceinline__ void attn_phase(const StepParams& P, const StepLayer&
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     ST_EV(P, c, c.evt_base + 4);
-    {   // the head's q and gate rows (adjacent in the stacked output, and here with k, v between them) and the KV head's k and v rows
+    {   // the head's q row and the KV head's k row whole, of the gate and v rows this CTA's elements
         const unsigned tag = tag_of(c.base, il, PH_B);
-        const int gh = hd / 32 * ST_GPU, r = tid / gh;                // granules of hd rows; hd <= 256: four parts of at most 88
-        if (r < 4) {
-            const int first = r < 2 ? (2 * h + r) * hd : P.nh * 2 * hd + (r - 2) * kvd + kh * hd;
-            const granule g = wait_granule(P, P.rows + (size_t)(first / 32) * ST_GPU + (tid - r * gh), tag, c.abort_flag, 17);
-            bool two; float* at = (r == 0 ? qs : r == 1 ? gs : r == 2 ? kl : vl) + granule_row(tid - r * gh, two);
-            at[0] = __uint_as_float(g.x); at[ST_GPU] = __uint_as_float(g.y); if (!two) at[2 * ST_GPU] = __uint_as_float(g.z);
+        const int gh = hd / 32 * ST_GPU, ge = epc / 32 * ST_GPU;      // granules of hd and of epc rows; hd <= 256: at most 88 each
+        const int r = tid < 2 * gh ? (tid < gh ? 0 : 1) : tid < 2 * gh + ge ? 2 : 3, k = r < 2 ? tid - r * gh : tid - 2 * gh - (r - 2) * ge;
+        if (tid < 2 * (gh + ge)) {
+            const int first = r == 0 ? 2 * h * hd : r == 1 ? 2 * P.nh * hd + kh * hd : r == 2 ? (2 * h + 1) * hd + g * epc : 2 * P.nh * hd + kvd + kh * hd + g * epc;
+            const granule v = wait_granule(P, P.rows + (size_t)(first / 32) * ST_GPU + k, tag, c.abort_flag, 17);
+            bool two; float* at = (r == 0 ? qs : r == 1 ? kl : r == 2 ? gs : vl) + granule_row(k, two);
+            at[0] = __uint_as_float(v.x); at[ST_GPU] = __uint_as_float(v.y); if (!two) at[2 * ST_GPU] = __uint_as_float(v.z);
         }
     }
     cons_sync();                                                     // all twelve warps, the loader included
-    const bool lost = *c.abort_flag, writer = h % rep == 0 && g == 0 && !lost;
+    const bool lost = *c.abort_flag, writer = h % rep == 0 && !lost;      // the group's first head stores the new position: k by its first CTA, v by all, their elements
     ST_EV(P, c, c.evt_base + 5);
     const __half* kc = L.kc; const __half* vc = L.vc;
 
@@ -1003,13 +994,13 @@ __device__ __forceinline__ void attn_phase(const StepParams& P, const StepLayer&
         __syncwarp();
         if (warp == 1) for (int i = lane; i < hd; i += 32) {
             const __half hv = __float2half_rn(buf[i]);
-            if (writer) const_cast<__half*>(kc)[it_kc_index(pos, kh, i, nkv, hd)] = hv;
+            if (writer && g == 0) const_cast<__half*>(kc)[it_kc_index(pos, kh, i, nkv, hd)] = hv;
             buf[i] = __half2float(hv);
         }
     } else if (warp == 2) {
-        for (int i = lane; i < hd; i += 32) {
+        for (int i = lane; i < epc; i += 32) {
             const __half hv = __float2half_rn(vl[i]);
-            if (writer) const_cast<__half*>(vc)[it_vc_index(pos, kh, i, nkv, hd)] = hv;
+            if (writer) const_cast<__half*>(vc)[it_vc_index(pos, kh, g * epc + i, nkv, hd)] = hv;
             vl[i] = __half2float(hv);
         }
     }
@@ -1115,9 +1106,8 @@ __device__ __forceinline__ void attn_phase(const StepParams& P, const StepLayer&
             if (lane == 0) mbar_arrive(ve + 8 * sl);
         }
         if (live) {
-            const int e0 = g * epc + tid;
-            acc = it_add(acc, it_mul(sc[nold], vl[e0]));
-            acc = it_mul(acc, it_sigmoid(gs[e0]));
+            acc = it_add(acc, it_mul(sc[nold], vl[tid]));
+            acc = it_mul(acc, it_sigmoid(gs[tid]));
         }
         publish(P.o, (h * hd + g * epc) / 32 + warp, lane, acc, sc_tag, *c.abort_flag);      // epc is a multiple of 32; a wait since the rows came may have run out
     }
@@ -1140,7 +1130,6 @@ __global__ void __launch_bounds__(ST_THREADS, 1) k_decode_step(const __grid_cons
     c.lay = reinterpret_cast<const StepLayer*>(tail + 704);         // two layer descriptions
     c.abort_flag = reinterpret_cast<volatile int*>(tail + ST_BARS - 16); c.verdict = c.abort_flag + 1; c.issued = smem_u32(tail + ST_BARS - 8);
     c.sp = reinterpret_cast<const StepSpan*>(tail + ST_BARS);
-    c.sg = reinterpret_cast<const uint32_t*>(tail + ST_BARS + SP_KINDS * sizeof(StepSpan));
     c.tid = threadIdx.x; c.warp = c.tid >> 5; c.lane = c.tid & 31;
     c.q = 0u; c.nsync = 0; c.evt_on = 0; c.dense_seq = 0u; c.mph = 0u;
     if (c.tid == 0) {
@@ -1155,8 +1144,6 @@ __global__ void __launch_bounds__(ST_THREADS, 1) k_decode_step(const __grid_cons
         constexpr int words = (int)(sizeof(StepLayer) / 4), sw = (int)(SP_KINDS * sizeof(StepSpan) / 4);
         if (c.tid < words) reinterpret_cast<uint32_t*>(tail + 704)[c.tid] = reinterpret_cast<const uint32_t*>(P.layers)[c.tid];
         if (c.tid < sw) reinterpret_cast<uint32_t*>(tail + ST_BARS)[c.tid] = reinterpret_cast<const uint32_t*>(P.spans + (size_t)blockIdx.x * SP_KINDS)[c.tid];
-#pragma unroll 1
-        for (int k = 0; k < 4; k++) for (int i = c.tid; i < P.sg_words[k]; i += ST_THREADS) const_cast<uint32_t*>(c.sg)[P.sg_off[k] + i] = P.sg[k][i];
     }
     __syncthreads();
     if (*c.abort_flag) return;
@@ -1193,7 +1180,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) k_decode_step(const __grid_cons
             if (owner || in.dense) {
                 in.codes = owner && (!tail_ph || logits) ? P.codes + step_codes_half(ph) * P.codes_half + hb * 128 : nullptr; in.codes_copy = row_blocks * 128; in.code_tag = tag_of(c.base, il, ph);
                 in.nblk = row_blocks; in.blk = hb;
-                in.signs = c.sg + (hb >= 0 ? 32 * hb : 0) + P.sg_off[ph == PH_D ? (L.recurrent ? 1 : 2) : ph == PH_H ? 3 : 0];
+                in.signs = P.sg[ph == PH_D ? (L.recurrent ? 1 : 2) : ph == PH_H ? 3 : 0] + (hb >= 0 ? 32 * hb : 0);
                 if (ph == PH_A) {
                     in.x = P.xi; in.tag = tag_of(c.base, il - 1, PH_I);
                     if (il == 0) in.plain = P.tok_embd + (size_t)tok * P.e;      // the residual row of layer 0 is the embedding row (Model::embed, src/cpu.rs:118-122)
@@ -1286,36 +1273,6 @@ struct it_step_state {
     bool cooperative;
 };
 
-static int step_widest(const it_model_config& c) { return std::max(std::max(c.n_embd, c.n_ff), std::max(c.ssm_inner, c.n_head * c.head_dim)); }
-// the state tile of the delta-net block comes in while the input projection's chunks run: behind their terms
-static size_t step_gdn_off(const it_model_config& c, int slots) { return (size_t)terms_at(c.n_embd / 128) + (size_t)slots * ST_TERMS * 4; }
-static size_t step_w_bytes(const it_model_config& c) { return (size_t)(c.n_embd / 1024) * IT_HAD_PITCH * 4; }
-static size_t step_scratch_bytes(const it_model_config& c, int slots) {
-    size_t s = (size_t)terms_at(step_widest(c) / 128) + (size_t)slots * ST_TERMS * 4;
-    s = std::max(s, (size_t)ST_RED + (size_t)(c.n_embd / 1024) * IT_HAD_PITCH * 4 + (size_t)c.n_embd * 4 + step_w_bytes(c));      // a normed row, a dense row, the norm's weights
-    s = std::max(s, step_gdn_off(c, slots) + (size_t)ST_SD * ST_SD * 4);
-    // a norm's weights and a dense row come in while the widest matrix's chunks run, and stay while their row is transformed
-    const size_t below = std::max((size_t)terms_at(step_widest(c) / 128) + (size_t)slots * ST_TERMS * 4, (size_t)terms_at(c.n_embd / 128) + (size_t)(c.n_embd / 1024) * IT_HAD_PITCH * 4);
-    s = std::max(s, below + (size_t)c.n_embd * 4 + step_w_bytes(c));
-    s = std::max(s, ((size_t)c.ctx_len + 4 + 4 * c.head_dim + 48) * 4 + 128 + 3 * (size_t)c.head_dim * 64);
-    return (s + 127) / 128 * 128;
-}
-// where the sign bits of the four widths start (words): a width that occurs twice is kept once
-static int step_sign_words(const it_model_config& c, int (&off)[4], int (&words)[4]) {
-    const int n[4] = { c.n_embd, c.ssm_inner, c.n_head * c.head_dim, c.n_ff };
-    int o = 0;
-    for (int k = 0; k < 4; k++) {
-        int same = -1;
-        for (int j = 0; j < k; j++) if (n[j] == n[k]) same = j;
-        off[k] = same >= 0 ? off[same] : o; words[k] = same >= 0 ? 0 : n[k] / 32; o += words[k];
-    }
-    return o;
-}
-static size_t step_smem_bytes(const it_model_config& c, int slots) {
-    int off[4], words[4];
-    return (size_t)slots * ST_CHUNK + step_scratch_bytes(c, slots) + ST_BARS + SP_KINDS * sizeof(StepSpan) + 4 * (size_t)step_sign_words(c, off, words);
-}
-
 // Whether this engine's decode step can run as the persistent kernel, and with which geometry.
 int it_step_prepare(it_engine* e) {
     const it_model_config& c = e->cfg; it_ctx* cx = e->ctx;
@@ -1324,22 +1281,20 @@ int it_step_prepare(it_engine* e) {
     if (e->world != 1) return IT_OK;                                  // row shards exchange results inside the per-op kernels
     if (c.ssm_state != ST_SD || c.conv_k > 8 || c.head_dim > 256 || c.head_dim % 32 || c.n_embd > 8192 || c.n_embd % 1024 || c.n_ff % 1024 || c.ssm_inner % 1024 || (c.n_head * c.head_dim) % 1024) return IT_OK;
     if (2 * c.ssm_vheads > cx->sm_count || c.n_head > cx->sm_count || step_widest(c) / 1024 > cx->sm_count || c.n_embd % 32 || c.ssm_vheads % c.ssm_groups) return IT_OK;
-    int slots = 16;                                                   // a power of two: slot = chunk index & (slots - 1)
-    while (slots > 2 && step_smem_bytes(c, slots) > (size_t)ST_SMEM) slots /= 2;
-    if (slots < 4) return IT_OK;
+    // several CTAs per attention head when the grid has them: each takes a share of the K tiles and of the output elements
+    int attn_g = step_attn_split(c, cx->sm_count);
+    { const char* v = getenv("IT_STEP_ATTN_G"); if (v && (atoi(v) == 1 || atoi(v) == 2) && atoi(v) < attn_g) attn_g = atoi(v); }
+    const int slots = step_ring_slots(c, attn_g);
+    if (!slots) return IT_OK;
     IT_CUDA(cudaSetDevice(cx->device));
     static bool attr_set[16] = {};
     if (!attr_set[cx->device & 15]) { IT_CUDA(cudaFuncSetAttribute(k_decode_step, cudaFuncAttributeMaxDynamicSharedMemorySize, ST_SMEM)); attr_set[cx->device & 15] = true; }
     int per_sm = 0;
-    IT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_decode_step, ST_THREADS, step_smem_bytes(c, slots)));
+    IT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_decode_step, ST_THREADS, step_smem_bytes(c, slots, attn_g)));
     if (per_sm < 1) return IT_OK;
     it_step_state* st = new it_step_state();
-    st->grid = cx->sm_count; st->slots = slots; st->scratch = (int)step_scratch_bytes(c, slots); st->gdn_off = (int)step_gdn_off(c, slots);
-    // several CTAs per attention head when the grid has them: each takes a share of the K tiles and of the output elements;
-    // attention heads sit behind the value heads when they all fit side by side
-    st->attn_g = 1;
-    for (int g = 4; g > 1; g /= 2) if (c.head_dim % (32 * g) == 0 && (c.head_dim / g) % it_vc_slice(c.head_dim) == 0 && g * c.n_head <= st->grid) { st->attn_g = g; break; }
-    { const char* v = getenv("IT_STEP_ATTN_G"); if (v && (atoi(v) == 1 || atoi(v) == 2) && atoi(v) < st->attn_g) st->attn_g = atoi(v); }
+    st->grid = cx->sm_count; st->slots = slots; st->scratch = (int)step_scratch_bytes(c, slots, attn_g); st->gdn_off = (int)step_gdn_off(c, slots);
+    st->attn_g = attn_g;                                              // attention heads sit behind the value heads when they all fit side by side
     st->attn_base = (c.ssm_vheads + st->attn_g * c.n_head <= st->grid) ? c.ssm_vheads : 0;
     st->layers_dev = nullptr; st->spans_dev = nullptr; st->partials = nullptr; st->gate = nullptr; st->trace = nullptr; st->had_step = st->grid / (step_widest(c) / 1024); st->att_sc = nullptr;
     st->att_stride = (c.ctx_len + 32 + 3) / 4 * 4;
@@ -1394,14 +1349,13 @@ int it_step_launch(it_engine* e, int flags) {
     P.eps = c.eps; P.theta_scale = e->theta_scale; for (int i = 0; i < 4; i++) P.sec[i] = c.rope_sections[i]; P.v_grouped = c.gdn_v_grouped;
     P.arena = cx->arena; P.xe = st->xe; P.xi = st->xi; P.rows = st->rows; P.o = st->o; P.act = st->act; P.codes = st->codes; P.codes_half = step_widest(c) / 1024 * 128 * ST_COPIES; P.prefix = st->prefix; P.had_step = st->had_step; P.hrow = L.hrow; P.logits = L.logits; P.amx = L.amx; P.gate = st->gate;
     { const size_t w[4] = { (size_t)c.n_embd, (size_t)c.ssm_inner, (size_t)c.n_head * c.head_dim, (size_t)c.n_ff }; for (int k = 0; k < 4; k++) P.sg[k] = reinterpret_cast<const uint32_t*>(cx->signs[w[k]] + w[k]); }
-    step_sign_words(c, P.sg_off, P.sg_words);
     P.tok_embd = e->tok_embd; P.output_norm = e->output_norm; P.output = e->output->tiles;
     P.toks = e->toks_dev; P.pos = e->pos_dev;
     P.sync = cx->grid_sync; P.partials = st->partials; P.error_flag = cx->error_flag_dev;
     P.slots = st->slots; P.scratch = st->scratch; P.w_off = st->scratch - (int)step_w_bytes(c); P.flags = flags; P.trace = st->trace; P.gdn_off = st->gdn_off; P.attn_base = st->attn_base; P.attn_g = st->attn_g; P.att_sc = st->att_sc; P.att_stride = st->att_stride;
     it_note_op(cx);
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)st->grid); cfg.blockDim = dim3(ST_THREADS); cfg.dynamicSmemBytes = step_smem_bytes(c, st->slots); cfg.stream = cx->stream;
+    cfg.gridDim = dim3((unsigned)st->grid); cfg.blockDim = dim3(ST_THREADS); cfg.dynamicSmemBytes = step_smem_bytes(c, st->slots, st->attn_g); cfg.stream = cx->stream;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeCooperative; attr[0].val.cooperative = 1;
     cfg.attrs = attr; cfg.numAttrs = st->cooperative ? 1 : 0;

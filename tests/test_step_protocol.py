@@ -30,7 +30,8 @@ def plan(tmp_path_factory):
                    'extern "C" int codes_half(int ph) { return step_codes_half(ph); }\n'
                    'extern "C" void spans(int grid, int rows, int cols, int parts, int* out) {\n'
                    '  std::vector<StepSpan> v((size_t)grid * SP_KINDS); step_spans(v, 0, grid, rows, cols, parts);\n'
-                   '  for (int b = 0; b < grid; b++) { const StepSpan& s = v[(size_t)b * SP_KINDS]; const int f[11] = { s.n, s.hl, s.tl, s.lead, s.uh, s.uf, s.ut, s.nb, s.cpr, s.parts, s.units }; memcpy(out + 11 * b, f, sizeof f); } }\n')
+                   '  for (int b = 0; b < grid; b++) { const StepSpan& s = v[(size_t)b * SP_KINDS]; const int f[11] = { s.n, s.hl, s.tl, s.lead, s.uh, s.uf, s.ut, s.nb, s.cpr, s.parts, s.units }; memcpy(out + 11 * b, f, sizeof f); } }\n'
+                   'extern "C" int ring_slots(const it_model_config* c, int sm) { return step_ring_slots(*c, step_attn_split(*c, sm)); }\n')
     subprocess.run(["g++", "-std=c++17", "-shared", "-fPIC", "-I", CSRC, str(src), "-o", str(lib)], check=True)
     return C.CDLL(str(lib))
 
@@ -353,3 +354,22 @@ def test_copies_are_waited_for_on_every_way_out():
     consumers = consumers[:consumers.index("leave:")]
     assert not re.search(r"\breturn;", consumers)
     assert re.search(r"leave:\s*asm volatile\(\"cp\.async\.wait_all;", src)
+
+
+@pytest.mark.parametrize("ctx,slots", [(8192, 16), (9900, 16), (9988, 16), (9989, 8), (16384, 8), (27000, 8), (32768, 4)])
+def test_ring_depth_by_context(plan, ctx, slots):
+    """The 27B widths: the scores of an attention CTA share its shared memory with the ring."""
+    from irontimber_b200.engine import config_27b
+    assert plan.ring_slots(C.byref(config_27b(ctx_len=ctx)), SM) == slots
+
+
+def test_ring_depth_by_widths(plan):
+    """Wide rows at a short context: a norm's weights and a dense row come in beside the widest matrix's terms."""
+    from irontimber_b200.engine import config_27b
+    def depth(**over):
+        cfg = config_27b(ctx_len=1024)
+        for k, v in over.items():
+            setattr(cfg, k, v)
+        return plan.ring_slots(C.byref(cfg), SM)
+    assert depth(n_head=32, n_head_kv=8, head_dim=128, n_embd=4096, n_ff=12288, ssm_inner=4096, ssm_vheads=32, ctx_len=16384) == 16
+    assert depth(n_ff=22528) == 16 and depth(n_ff=32768) == 8 and depth(n_embd=8192, n_ff=40960) == 8
