@@ -92,6 +92,7 @@ struct StepParams {
     float eps, theta_scale; int sec[4]; int v_grouped;
     float* arena; size_t hrow, logits, amx;
     granule *xe, *xi, *rows, *o, *act; // residual row after the output / down projection; input projection's rows; block output; silu(gate) * up
+    unsigned long long* o1;            // block output of attention heads whose dimension is no multiple of 32: a value and its tag an element (else null)
     granule* codes; int codes_half;    // the quantised row: 128 granules a block of 1024, ST_COPIES copies; codes_half granules further: the other half (step_codes_half)
     unsigned long long* gate;          // per value head beta, then decay: value and tag
     granule* prefix;                   // [grid][32] running sums of a cut row group (two matrices' worth) and the tag
@@ -347,7 +348,7 @@ __device__ __forceinline__ void warm_layer(const StepParams& P, const Cta& c, co
 // of the transform (64 bytes a thread straight into registers: 24 KB cost 2000 cycles with all SMs at it, in lane order 560).
 // The norm's weights and the dense row do not depend on the step and are in shared memory before the row is.
 struct RowIn {
-    const granule* x; unsigned tag; const float* plain;      // the row (norm) or its block, as granules of a phase, or (plain) as floats
+    const granule* x; unsigned tag; const float* plain; const unsigned long long* one;      // the row (norm) or its block, as granules of a phase, as floats (plain), or as tagged values (one)
     const uint32_t* signs; float* normed;                    // normed: where the normed row goes, or null
     granule* codes; unsigned code_tag; int codes_copy;       // where the quantised block goes (copies codes_copy granules apart), or null
     int nblk, blk; bool norm, dense;                         // blocks brought in, the one to transform; dense: multiply the normed row with this CTA's dense row
@@ -384,8 +385,8 @@ __device__ __noinline__ void norm_request(float* wb, const float* w, const float
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
 }
-__device__ __forceinline__ void block_transform(const StepParams& P, const Cta& c, const RowIn in) {
-    const int tid = c.tid, warp = c.warp, lane = c.lane, half = warp & 1, j = tid & 63;
+template <bool ANY> __device__ __forceinline__ void block_transform(const StepParams& P, const Cta& c, const RowIn in) {
+    const int tid = c.tid, warp = c.warp, lane = c.lane, j = tid & 63;
     const int n = in.nblk * 1024;
     float* ex0 = reinterpret_cast<float*>(c.scratch + ST_RED);
     float* red = reinterpret_cast<float*>(c.scratch + 64);   // [8] warp sums of squares, [4][2] group maxima
@@ -395,6 +396,9 @@ __device__ __forceinline__ void block_transform(const StepParams& P, const Cta& 
     if (in.plain) {
 #pragma unroll 1
         for (int i = 4 * tid; i < n; i += 4 * ST_CT) *reinterpret_cast<float4*>(ex0 + it_had_at(i)) = *reinterpret_cast<const float4*>(in.plain + i);
+    } else if (ANY && in.one) {
+#pragma unroll 1
+        for (int i = tid; i < n; i += ST_CT) ex0[it_had_at(i)] = ld_tagged(P, in.one + i, in.tag, c.abort_flag, 14);
     } else row_place(P, c, ex0, in.x, in.nblk, in.tag);
     asm volatile("cp.async.wait_group 0;" ::: "memory");             // the norm's weights
     cons_sync();
@@ -732,8 +736,8 @@ __device__ __forceinline__ void gdn_prefetch(const StepParams& P, const StepLaye
     for (int f = c.tid; f < SD * PPR; f += ST_CT) { const int j = f / PPR, cc = f % PPR; cp_async16(tile + j * SD + ((cc ^ (j & 7)) << 2), m + f); }
     asm volatile("cp.async.commit_group;" ::: "memory");
 }
-// sum of a[i] * b[i] in index order (one lane); n a multiple of 16, both 16-byte aligned
-__device__ __noinline__ float chain_dot(const float* a, const float* b, int n) {
+// sum of a[i] * b[i] in index order (one lane); both 16-byte aligned, n a multiple of 16, with ANY of 8 (up to eight elements behind them are read)
+template <bool ANY> __device__ __noinline__ float chain_dot(const float* a, const float* b, int n) {
     float s = 0.f;
     float4 x[4], y[4];
 #pragma unroll
@@ -749,6 +753,9 @@ __device__ __noinline__ float chain_dot(const float* a, const float* b, int n) {
 #pragma unroll
         for (int u = 0; u < 16; u++) s = it_add(s, p[u]);
     }
+    if (ANY)
+#pragma unroll 1
+        for (int i = n & ~15; i < n; i++) s = it_add(s, it_mul(a[i], b[i]));
     return s;
 }
 __device__ __forceinline__ void gdn_phase(const StepParams& P, const StepLayer& L, const Cta& c, int h, int il) {
@@ -782,7 +789,7 @@ __device__ __forceinline__ void gdn_phase(const StepParams& P, const StepLayer& 
     cons_sync();
     const bool lost = *c.abort_flag;                                 // the rows or gates may not have come: the state stays, nothing is published
     const float q = raw[tid & (SD - 1)], k = raw[SD + (tid & (SD - 1))], v = raw[2 * SD + (tid & (SD - 1))], bt = scs[2], eg = scs[3];
-    if (warp >= 4 && warp < 6 && lane == 0) { const float* r = raw + (warp - 4) * SD; scs[warp - 4] = __fdiv_rn(1.0f, fmaxf(__fsqrt_rn(chain_dot(r, r, SD)), P.eps)); }
+    if (warp >= 4 && warp < 6 && lane == 0) { const float* r = raw + (warp - 4) * SD; scs[warp - 4] = __fdiv_rn(1.0f, fmaxf(__fsqrt_rn(chain_dot<false>(r, r, SD)), P.eps)); }
     if (warp < 6) asm volatile("bar.sync 3, 192;" ::: "memory");
     if (tid < SD) {
         qs[tid] = it_mul(q, scs[0]); ks[tid] = it_mul(k, scs[1]);
@@ -850,7 +857,7 @@ __device__ __forceinline__ void gdn_phase(const StepParams& P, const StepLayer& 
     }
     if (warp == 0) {
         float sc = 0.f;
-        if (lane == 0) sc = __fdiv_rn(1.0f, __fsqrt_rn(it_add(__fdiv_rn(chain_dot(os, os, SD), (float)SD), P.eps)));
+        if (lane == 0) sc = __fdiv_rn(1.0f, __fsqrt_rn(it_add(__fdiv_rn(chain_dot<false>(os, os, SD), (float)SD), P.eps)));
         sc = __shfl_sync(0xffffffffu, sc, 0);
         // the output projection's columns may be grouped [rep][key head] where value heads are [key head][rep]
         const int u0 = (P.v_grouped ? h / P.nk + P.nv / P.nk * kh : h) * (SD / 32);
@@ -890,7 +897,7 @@ __device__ __forceinline__ void at_sync() { asm volatile("bar.sync 4, %0;" :: "n
 // counter would need a base that nobody's late start can miss), runs the softmax for itself (one thread adds the exponentials in position order) and accumulates the
 // head_dim / G output elements [g head_dim / G, ...) over all positions from row slices of the V tiles.  A single SM can
 // keep only so many bytes in flight, so a head's cache traffic is spread over G SMs.
-__device__ __forceinline__ void attn_phase(const StepParams& P, const StepLayer& L, Cta& c, int hg, int il) {
+template <bool ANY> __device__ __forceinline__ void attn_phase(const StepParams& P, const StepLayer& L, Cta& c, int hg, int il) {
     const int tid = c.tid, warp = c.warp, lane = c.lane, hd = P.hd, nkv = P.nkv, kvd = nkv * hd;
     const int G = P.attn_g, h = hg / G, g = hg % G, epc = hd / G;   // elements of the output this CTA owns
     const int vs = it_vc_slice(hd);                                  // elements per V slice: epc is a multiple of it
@@ -925,11 +932,17 @@ __device__ __forceinline__ void attn_phase(const StepParams& P, const StepLayer&
         const unsigned tag = tag_of(c.base, il, PH_B);
         const int gh = hd / 32 * ST_GPU, ge = epc / 32 * ST_GPU;      // granules of hd and of epc rows; hd <= 256: at most 88 each
         const int r = tid < 2 * gh ? (tid < gh ? 0 : 1) : tid < 2 * gh + ge ? 2 : 3, k = r < 2 ? tid - r * gh : tid - 2 * gh - (r - 2) * ge;
-        if (tid < 2 * (gh + ge)) {
+        if ((!ANY || hd % 32 == 0) && tid < 2 * (gh + ge)) {
             const int first = r == 0 ? 2 * h * hd : r == 1 ? 2 * P.nh * hd + kh * hd : r == 2 ? (2 * h + 1) * hd + g * epc : 2 * P.nh * hd + kvd + kh * hd + g * epc;
             const granule v = wait_granule(P, P.rows + (size_t)(first / 32) * ST_GPU + k, tag, c.abort_flag, 17);
             bool two; float* at = (r == 0 ? qs : r == 1 ? kl : r == 2 ? gs : vl) + granule_row(k, two);
             at[0] = __uint_as_float(v.x); at[ST_GPU] = __uint_as_float(v.y); if (!two) at[2 * ST_GPU] = __uint_as_float(v.z);
+        }
+        // a head dimension that is no multiple of 32 (then G is 1): heads begin inside row groups, every row is looked up by itself
+        if (ANY && hd % 32) for (int i = tid; i < 4 * hd; i += ST_CT) {
+            const int r = i / hd, k = i - r * hd, row = (r == 0 ? 2 * h * hd : r == 1 ? 2 * P.nh * hd + kh * hd : r == 2 ? (2 * h + 1) * hd : 2 * P.nh * hd + kvd + kh * hd) + k, l = row & 31;
+            const granule v = wait_granule(P, P.rows + (size_t)(row / 32) * ST_GPU + l % ST_GPU, tag, c.abort_flag, 17);
+            (r == 0 ? qs : r == 1 ? kl : r == 2 ? gs : vl)[k] = __uint_as_float(l < ST_GPU ? v.x : l < 2 * ST_GPU ? v.y : v.z);
         }
     }
     cons_sync();                                                     // all twelve warps, the loader included
@@ -973,7 +986,7 @@ __device__ __forceinline__ void attn_phase(const StepParams& P, const StepLayer&
 #pragma unroll
         for (int k = 0; k < 8; k++) wr[k] = lane + 32 * k < hd ? w[lane + 32 * k] : 0.f;
         float s = 0.f;
-        if (lane == 0) s = chain_dot(buf, buf, hd);
+        if (lane == 0) s = chain_dot<ANY>(buf, buf, hd);
         s = __shfl_sync(0xffffffffu, s, 0);
         const float scl = it_div(1.0f, it_sqrt(it_add(it_div(s, (float)hd), P.eps)));
 #pragma unroll
@@ -1036,7 +1049,7 @@ __device__ __forceinline__ void attn_phase(const StepParams& P, const StepLayer&
             if (lane == 0) mbar_arrive(ke + 8 * sl);
         }
     } else if (warp == ST_AT_MAXS && lane == 0) {
-        sc[nold] = it_mul(chain_dot(qs, kl, hd), scale);             // the new position, from its row in shared memory (every CTA of the head for itself)
+        sc[nold] = it_mul(chain_dot<ANY>(qs, kl, hd), scale);             // the new position, from its row in shared memory (every CTA of the head for itself)
     }
     ST_EV(P, c, c.evt_base + 7);
     if (G > 1) {
@@ -1109,7 +1122,9 @@ __device__ __forceinline__ void attn_phase(const StepParams& P, const StepLayer&
             acc = it_add(acc, it_mul(sc[nold], vl[tid]));
             acc = it_mul(acc, it_sigmoid(gs[tid]));
         }
-        publish(P.o, (h * hd + g * epc) / 32 + warp, lane, acc, sc_tag, *c.abort_flag);      // epc is a multiple of 32; a wait since the rows came may have run out
+        const bool gone = *c.abort_flag;                             // a wait since the rows came may have run out
+        if (!ANY || hd % 32 == 0) publish(P.o, (h * hd + g * epc) / 32 + warp, lane, acc, sc_tag, gone);      // epc is a multiple of 32
+        else if (live && !gone) st_tagged(P.o1 + h * hd + tid, acc, sc_tag);
     }
     ST_EV(P, c, c.evt_base + 10);
 }
@@ -1120,7 +1135,9 @@ __device__ __forceinline__ const float* dense_row(const StepParams& P, const Ste
 }
 
 // ---------------------------------------------------------------- the step
-__global__ void __launch_bounds__(ST_THREADS, 1) k_decode_step(const __grid_constant__ StepParams P) {
+// ANY: head dimensions that are no multiple of 32 as well.  Their few branches cost the usual step 0.6 % (155.0 instead of 154.0 ms for 48 steps of
+// 64 layers behind a 9-token prompt), so that they have a copy of the kernel.
+template <bool ANY> __global__ void __launch_bounds__(ST_THREADS, 1) k_decode_step(const __grid_constant__ StepParams P) {
     extern __shared__ __align__(128) unsigned char smem[];
     Cta c;
     c.smem = smem; c.scratch = smem + P.slots * ST_CHUNK;
@@ -1173,9 +1190,9 @@ __global__ void __launch_bounds__(ST_THREADS, 1) k_decode_step(const __grid_cons
         if (ph == PH_C) {
             const int heads = L.recurrent ? P.nv : P.nh * P.attn_g;
             if (L.recurrent) { if (cta < P.nv) { cons_sync(); gdn_phase(P, L, c, cta, il); } }
-            else if (ah >= 0 && ah < heads) { cons_sync(); attn_phase(P, L, c, ah, il); }
+            else if (ah >= 0 && ah < heads) { cons_sync(); attn_phase<ANY>(P, L, c, ah, il); }
         } else if (ph == PH_A || ph == PH_D || ph == PH_F || ph == PH_H) {
-            RowIn in; in.normed = nullptr; in.plain = nullptr; in.norm = ph == PH_A || ph == PH_F; in.dense = ph == PH_A && !tail_ph && L.recurrent && drow < 2 * P.nv;
+            RowIn in; in.normed = nullptr; in.plain = nullptr; in.one = nullptr; in.norm = ph == PH_A || ph == PH_F; in.dense = ph == PH_A && !tail_ph && L.recurrent && drow < 2 * P.nv;
             const bool owner = hb >= 0 && hb < row_blocks && (!tail_ph || logits || cta == 0);
             if (owner || in.dense) {
                 in.codes = owner && (!tail_ph || logits) ? P.codes + step_codes_half(ph) * P.codes_half + hb * 128 : nullptr; in.codes_copy = row_blocks * 128; in.code_tag = tag_of(c.base, il, ph);
@@ -1188,10 +1205,11 @@ __global__ void __launch_bounds__(ST_THREADS, 1) k_decode_step(const __grid_cons
                 } else if (ph == PH_F) { in.x = P.xe; in.tag = tag_of(c.base, il, PH_E); }
                 else {
                     in.x = (ph == PH_D ? P.o : P.act) + (size_t)hb * ST_GPB; in.tag = tag_of(c.base, il, ph == PH_D ? PH_C : PH_G); in.nblk = 1; in.blk = 0;
+                    if (ANY && ph == PH_D && !L.recurrent && P.o1) in.one = P.o1 + (size_t)hb * 1024;
                 }
                 if (!owner && !count_wait(P, c, P.sync, c.target + (unsigned)row_blocks, 1 + ph, false)) goto leave;      // a dense row's owner follows the blocks' owners
                 ST_EV(P, c, c.evt_base + 0);
-                block_transform(P, c, in);
+                block_transform<ANY>(P, c, in);
                 ST_EV(P, c, c.evt_base + 1);
             }
             if (tail_ph && !logits) { if (cta != 0) goto leave; break; }
@@ -1266,11 +1284,11 @@ struct it_step_state {
     StepSpan* spans_dev;
     unsigned long long* trace;
     granule *xe, *xi, *rows, *o, *act, *codes, *prefix, *partials;
-    unsigned long long* gate;
+    unsigned long long *gate, *o1;
     int had_step;
     int grid, slots, scratch, gdn_off, attn_base, attn_g, att_stride;
     unsigned long long* att_sc;
-    bool cooperative;
+    bool cooperative, any;
 };
 
 // Whether this engine's decode step can run as the persistent kernel, and with which geometry.
@@ -1279,7 +1297,7 @@ int it_step_prepare(it_engine* e) {
     e->step = nullptr;
     { const char* v = getenv("IT_STEP_KERNEL"); if (v && atoi(v) == 0) return IT_OK; }
     if (e->world != 1) return IT_OK;                                  // row shards exchange results inside the per-op kernels
-    if (c.ssm_state != ST_SD || c.conv_k > 8 || c.head_dim > 256 || c.head_dim % 32 || c.n_embd > 8192 || c.n_embd % 1024 || c.n_ff % 1024 || c.ssm_inner % 1024 || (c.n_head * c.head_dim) % 1024) return IT_OK;
+    if (c.ssm_state != ST_SD || c.conv_k > 8 || c.head_dim > 256 || c.head_dim % 8 || c.n_embd > 8192 || c.n_embd % 1024 || c.n_ff % 1024 || c.ssm_inner % 1024 || (c.n_head * c.head_dim) % 1024) return IT_OK;
     if (2 * c.ssm_vheads > cx->sm_count || c.n_head > cx->sm_count || step_widest(c) / 1024 > cx->sm_count || c.n_embd % 32 || c.ssm_vheads % c.ssm_groups) return IT_OK;
     // several CTAs per attention head when the grid has them: each takes a share of the K tiles and of the output elements
     int attn_g = step_attn_split(c, cx->sm_count);
@@ -1288,15 +1306,20 @@ int it_step_prepare(it_engine* e) {
     if (!slots) return IT_OK;
     IT_CUDA(cudaSetDevice(cx->device));
     static bool attr_set[16] = {};
-    if (!attr_set[cx->device & 15]) { IT_CUDA(cudaFuncSetAttribute(k_decode_step, cudaFuncAttributeMaxDynamicSharedMemorySize, ST_SMEM)); attr_set[cx->device & 15] = true; }
+    if (!attr_set[cx->device & 15]) {
+        IT_CUDA(cudaFuncSetAttribute(k_decode_step<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, ST_SMEM));
+        IT_CUDA(cudaFuncSetAttribute(k_decode_step<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, ST_SMEM));
+        attr_set[cx->device & 15] = true;
+    }
+    const bool any = c.head_dim % 32 != 0;
     int per_sm = 0;
-    IT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_decode_step, ST_THREADS, step_smem_bytes(c, slots, attn_g)));
+    IT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, any ? k_decode_step<true> : k_decode_step<false>, ST_THREADS, step_smem_bytes(c, slots, attn_g)));
     if (per_sm < 1) return IT_OK;
     it_step_state* st = new it_step_state();
-    st->grid = cx->sm_count; st->slots = slots; st->scratch = (int)step_scratch_bytes(c, slots, attn_g); st->gdn_off = (int)step_gdn_off(c, slots);
+    st->any = any; st->grid = cx->sm_count; st->slots = slots; st->scratch = (int)step_scratch_bytes(c, slots, attn_g); st->gdn_off = (int)step_gdn_off(c, slots);
     st->attn_g = attn_g;                                              // attention heads sit behind the value heads when they all fit side by side
     st->attn_base = (c.ssm_vheads + st->attn_g * c.n_head <= st->grid) ? c.ssm_vheads : 0;
-    st->layers_dev = nullptr; st->spans_dev = nullptr; st->partials = nullptr; st->gate = nullptr; st->trace = nullptr; st->had_step = st->grid / (step_widest(c) / 1024); st->att_sc = nullptr;
+    st->layers_dev = nullptr; st->spans_dev = nullptr; st->partials = nullptr; st->gate = nullptr; st->o1 = nullptr; st->trace = nullptr; st->had_step = st->grid / (step_widest(c) / 1024); st->att_sc = nullptr;
     st->att_stride = (c.ctx_len + 32 + 3) / 4 * 4;
     { const char* v = getenv("IT_STEP_COOP"); st->cooperative = !v || atoi(v) != 0; }
     std::vector<StepLayer> hl(c.n_layer);
@@ -1328,6 +1351,7 @@ int it_step_prepare(it_engine* e) {
     row_of(&st->o, std::max(c.ssm_inner, c.n_head * c.head_dim)); row_of(&st->act, c.n_ff);
     granules(&st->codes, (size_t)(step_widest(c) / 1024) * 128 * ST_COPIES * 2); granules(&st->prefix, (size_t)st->grid * 32); granules(&st->partials, (size_t)st->grid * ST_NSUM);
     if (r == IT_OK) r = it_engine_dev_alloc(e, (void**)&st->gate, 2 * (size_t)c.ssm_vheads * sizeof(unsigned long long), true);
+    if (r == IT_OK && c.head_dim % 32) r = it_engine_dev_alloc(e, (void**)&st->o1, (size_t)c.n_head * c.head_dim * sizeof(unsigned long long), true);
     if (r == IT_OK) r = it_engine_dev_alloc(e, (void**)&st->att_sc, (size_t)c.n_head * st->att_stride * sizeof(unsigned long long), true);
     { const char* v = getenv("IT_STEP_TRACE"); if (r == IT_OK && v && atoi(v) != 0) r = it_engine_dev_alloc(e, (void**)&st->trace, (2 * ST_TRACE_MAX * 2 + ST_EVT_MAX) * sizeof(unsigned long long), true); }
     if (r) { delete st; return r; }
@@ -1347,7 +1371,7 @@ int it_step_launch(it_engine* e, int flags) {
     P.e = c.n_embd; P.ff = c.n_ff; P.widest = step_widest(c); P.hd = c.head_dim; P.nh = c.n_head; P.nkv = c.n_head_kv; P.cd = it_cfg_conv_dim(c); P.inner = c.ssm_inner; P.nv = c.ssm_vheads;
     P.nk = c.ssm_groups; P.qk = it_cfg_qk(c); P.conv_k = c.conv_k; P.n_rot = c.n_rot; P.n_vocab = c.n_vocab;
     P.eps = c.eps; P.theta_scale = e->theta_scale; for (int i = 0; i < 4; i++) P.sec[i] = c.rope_sections[i]; P.v_grouped = c.gdn_v_grouped;
-    P.arena = cx->arena; P.xe = st->xe; P.xi = st->xi; P.rows = st->rows; P.o = st->o; P.act = st->act; P.codes = st->codes; P.codes_half = step_widest(c) / 1024 * 128 * ST_COPIES; P.prefix = st->prefix; P.had_step = st->had_step; P.hrow = L.hrow; P.logits = L.logits; P.amx = L.amx; P.gate = st->gate;
+    P.arena = cx->arena; P.xe = st->xe; P.xi = st->xi; P.rows = st->rows; P.o = st->o; P.o1 = st->o1; P.act = st->act; P.codes = st->codes; P.codes_half = step_widest(c) / 1024 * 128 * ST_COPIES; P.prefix = st->prefix; P.had_step = st->had_step; P.hrow = L.hrow; P.logits = L.logits; P.amx = L.amx; P.gate = st->gate;
     { const size_t w[4] = { (size_t)c.n_embd, (size_t)c.ssm_inner, (size_t)c.n_head * c.head_dim, (size_t)c.n_ff }; for (int k = 0; k < 4; k++) P.sg[k] = reinterpret_cast<const uint32_t*>(cx->signs[w[k]] + w[k]); }
     P.tok_embd = e->tok_embd; P.output_norm = e->output_norm; P.output = e->output->tiles;
     P.toks = e->toks_dev; P.pos = e->pos_dev;
@@ -1359,7 +1383,7 @@ int it_step_launch(it_engine* e, int flags) {
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeCooperative; attr[0].val.cooperative = 1;
     cfg.attrs = attr; cfg.numAttrs = st->cooperative ? 1 : 0;
-    IT_CUDA(cudaLaunchKernelEx(&cfg, k_decode_step, P));
+    IT_CUDA(cudaLaunchKernelEx(&cfg, st->any ? k_decode_step<true> : k_decode_step<false>, P));
     return IT_OK;
 }
 

@@ -403,6 +403,8 @@ def test_a_short_context_keeps_short_row_buffers():
     dict(n_embd=2048, n_ff=5120, ssm_vheads=24, ssm_groups=8, ssm_inner=3072, n_head=16, n_head_kv=4, head_dim=64, n_vocab=4767, conv_k=2),      # 149 row groups of the head, the last one short
     dict(n_embd=5120, n_ff=1024, ssm_vheads=48, ssm_groups=16, ssm_inner=6144, full_attn_interval=2, n_vocab=64),                                # 160 row groups for the residual, CTAs without any of the head
     dict(n_embd=8192, n_ff=2048, n_vocab=200),                                                                                                   # widest norm row: fewer ring slots
+    dict(head_dim=80, n_head=64, n_head_kv=2, n_rot=40),                                                                                         # heads that begin inside row groups
+    dict(head_dim=24, n_head=128, n_head_kv=4, n_rot=16, full_attn_interval=2), dict(head_dim=8, n_head=128, n_head_kv=4, n_rot=8),              # ... down to the smallest dimension
     dict(full_attn_interval=1)])                                                                                                                 # attention in the first layer
 def test_step_kernel_geometries(monkeypatch, over):
     """Matrices that cut a row group between two CTAs, leave CTAs without work, or leave the ring fewer slots: logits, picks and
