@@ -352,6 +352,7 @@ struct RowIn {
     const uint32_t* signs; float* normed;                    // normed: where the normed row goes, or null
     granule* codes; unsigned code_tag; int codes_copy;       // where the quantised block goes (copies codes_copy granules apart), or null
     int nblk, blk; bool norm, dense;                         // blocks brought in, the one to transform; dense: multiply the normed row with this CTA's dense row
+    const float* dense2;                                     // ... and with this second one (in global memory), or null
 };
 __device__ __forceinline__ void pair_sync() { asm volatile("bar.sync 5, 64;" ::: "memory"); }
 // nblk blocks of 1024 rows (32 row groups, 352 granules: a thread each) from `x` into the padded layout at `ex`
@@ -446,6 +447,15 @@ template <bool ANY> __device__ __forceinline__ void block_transform(const StepPa
                 for (int k = 0; k < in.nblk * 4; k++) d += (double)it_mul(dp[256 * k], it_mul(it_mul(xp[336 * k], sc), wp[336 * k]));
 #pragma unroll
                 for (int m = 16; m >= 1; m >>= 1) d += __shfl_xor_sync(0xffffffffu, d, m);
+                if (ANY && in.dense2) {
+                    double d2 = 0.0;
+                    dp = in.dense2 + tid;
+#pragma unroll 1
+                    for (int k = 0; k < in.nblk * 4; k++) d2 += (double)it_mul(dp[256 * k], it_mul(it_mul(xp[336 * k], sc), wp[336 * k]));
+#pragma unroll
+                    for (int m = 16; m >= 1; m >>= 1) d2 += __shfl_xor_sync(0xffffffffu, d2, m);
+                    if (lane == 0) reinterpret_cast<double*>(c.scratch + ST_DENSE2)[warp] = d2;
+                }
                 if (lane == 0 && !lost) { reinterpret_cast<double*>(c.scratch)[warp] = d; mbar_arrive(c.dn); }
             }
             cons_sync();                                     // the row is about to be overwritten
@@ -577,7 +587,7 @@ __device__ __forceinline__ void matvec_phase(const StepParams& P, Cta& c, const 
 
 // The sum warps' side: warp j takes every second row group (in the order of the CTA's chunks), adds its terms in block order
 // and finishes the row: into the residual, through conv and SiLU, through silu(gate) * up, or plainly.
-__device__ __forceinline__ void sum_warps(const StepParams& P, Cta& c) {
+template <bool ANY> __device__ __forceinline__ void sum_warps(const StepParams& P, Cta& c) {
     const int jw = c.warp - ST_NCONS, lane = c.lane;
     float* A = P.arena;
     Pick best{ -INFINITY, 0xffffffffu };
@@ -611,11 +621,14 @@ __device__ __forceinline__ void sum_warps(const StepParams& P, Cta& c) {
             if (!mbar_wait_warp(c.dn, (c.dense_seq++) & 1u, c.abort_flag, P.error_flag, 12)) break;
             if (lane == 0) {
                 const double* ws = reinterpret_cast<const double*>(c.scratch);
-                double tt = ws[0];
-                for (int k = 1; k < 8; k++) tt += ws[k];
-                const float tf = (float)tt;
-                const int h = drow % P.nv;
-                st_tagged(P.gate + drow, drow < P.nv ? it_sigmoid(tf) : it_expf(it_mul(it_softplus(it_add(tf, L.dt[h])), L.a[h])), tag);
+#pragma unroll 1
+                for (int r = drow; r < (ANY ? 2 * P.nv : drow + 1); r += (int)gridDim.x, ws += ST_DENSE2 / 8) {
+                    double tt = ws[0];
+                    for (int k = 1; k < 8; k++) tt += ws[k];
+                    const float tf = (float)tt;
+                    const int h = r % P.nv;
+                    st_tagged(P.gate + r, r < P.nv ? it_sigmoid(tf) : it_expf(it_mul(it_softplus(it_add(tf, L.dt[h])), L.a[h])), tag);
+                }
             }
             __syncwarp();
         }
@@ -1135,7 +1148,7 @@ __device__ __forceinline__ const float* dense_row(const StepParams& P, const Ste
 }
 
 // ---------------------------------------------------------------- the step
-// ANY: head dimensions that are no multiple of 32 as well.  Their few branches cost the usual step 0.6 % (155.0 instead of 154.0 ms for 48 steps of
+// ANY: head dimensions that are no multiple of 32, and more dense rows than CTAs, as well.  Their few branches cost the usual step 0.6 % (155.0 instead of 154.0 ms for 48 steps of
 // 64 layers behind a 9-token prompt), so that they have a copy of the kernel.
 template <bool ANY> __global__ void __launch_bounds__(ST_THREADS, 1) k_decode_step(const __grid_constant__ StepParams P) {
     extern __shared__ __align__(128) unsigned char smem[];
@@ -1165,7 +1178,7 @@ template <bool ANY> __global__ void __launch_bounds__(ST_THREADS, 1) k_decode_st
     __syncthreads();
     if (*c.abort_flag) return;
     if (c.warp == ST_NCONS + ST_NSUM) { if (c.lane == 0) producer(P, c); return; }
-    if (c.warp >= ST_NCONS) { sum_warps(P, c); return; }
+    if (c.warp >= ST_NCONS) { sum_warps<ANY>(P, c); return; }
 
     c.base = *reinterpret_cast<volatile unsigned*>(P.sync + 3); c.target = *reinterpret_cast<volatile unsigned*>(P.sync + 1);
     c.inv_sqrt_sd = it_div(1.0f, it_sqrt((float)ST_SD)); c.inv_sqrt_hd = it_div(1.0f, it_sqrt((float)P.hd));
@@ -1196,7 +1209,7 @@ template <bool ANY> __global__ void __launch_bounds__(ST_THREADS, 1) k_decode_st
             const bool owner = hb >= 0 && hb < row_blocks && (!tail_ph || logits || cta == 0);
             if (owner || in.dense) {
                 in.codes = owner && (!tail_ph || logits) ? P.codes + step_codes_half(ph) * P.codes_half + hb * 128 : nullptr; in.codes_copy = row_blocks * 128; in.code_tag = tag_of(c.base, il, ph);
-                in.nblk = row_blocks; in.blk = hb;
+                in.nblk = row_blocks; in.blk = hb; in.dense2 = ANY && in.dense ? dense_row(P, L, drow + grid) : nullptr;
                 in.signs = P.sg[ph == PH_D ? (L.recurrent ? 1 : 2) : ph == PH_H ? 3 : 0] + (hb >= 0 ? 32 * hb : 0);
                 if (ph == PH_A) {
                     in.x = P.xi; in.tag = tag_of(c.base, il - 1, PH_I);
@@ -1298,7 +1311,7 @@ int it_step_prepare(it_engine* e) {
     { const char* v = getenv("IT_STEP_KERNEL"); if (v && atoi(v) == 0) return IT_OK; }
     if (e->world != 1) return IT_OK;                                  // row shards exchange results inside the per-op kernels
     if (c.ssm_state != ST_SD || c.conv_k > 8 || c.head_dim > 256 || c.head_dim % 8 || c.n_embd > 8192 || c.n_embd % 1024 || c.n_ff % 1024 || c.ssm_inner % 1024 || (c.n_head * c.head_dim) % 1024) return IT_OK;
-    if (2 * c.ssm_vheads > cx->sm_count || c.n_head > cx->sm_count || step_widest(c) / 1024 > cx->sm_count || c.n_embd % 32 || c.ssm_vheads % c.ssm_groups) return IT_OK;
+    if (c.ssm_vheads > cx->sm_count || c.n_head > cx->sm_count || step_widest(c) / 1024 > cx->sm_count || c.n_embd % 32 || c.ssm_vheads % c.ssm_groups) return IT_OK;
     // several CTAs per attention head when the grid has them: each takes a share of the K tiles and of the output elements
     int attn_g = step_attn_split(c, cx->sm_count);
     { const char* v = getenv("IT_STEP_ATTN_G"); if (v && (atoi(v) == 1 || atoi(v) == 2) && atoi(v) < attn_g) attn_g = atoi(v); }
@@ -1311,7 +1324,7 @@ int it_step_prepare(it_engine* e) {
         IT_CUDA(cudaFuncSetAttribute(k_decode_step<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, ST_SMEM));
         attr_set[cx->device & 15] = true;
     }
-    const bool any = c.head_dim % 32 != 0;
+    const bool any = c.head_dim % 32 != 0 || 2 * c.ssm_vheads > cx->sm_count;
     int per_sm = 0;
     IT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, any ? k_decode_step<true> : k_decode_step<false>, ST_THREADS, step_smem_bytes(c, slots, attn_g)));
     if (per_sm < 1) return IT_OK;

@@ -22,6 +22,7 @@ constexpr int ST_SMEM = 227 * 1024;                    // dynamic shared memory 
 constexpr int ST_BARS = 1024;                          // bytes reserved for mbarriers, flags and layer descriptions
 constexpr int ST_SD = 128;                             // delta-rule state size this kernel is built for
 constexpr int ST_RED = 384;                            // bytes: the dense row's eight f64 warp sums, then the transform's [8] sums of squares and [4][2] group maxima
+constexpr int ST_DENSE2 = 128;                         // bytes: where in it a second dense row's warp sums are
 constexpr int ST_AT_RED = 36;                          // floats of the attention block's reductions: one a warp, at 32 the sum
 constexpr int ST_PITCH = 1344;                         // floats of a block of 1024 in the transform's padded layout (IT_HAD_PITCH)
 

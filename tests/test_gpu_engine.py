@@ -405,6 +405,7 @@ def test_a_short_context_keeps_short_row_buffers():
     dict(n_embd=8192, n_ff=2048, n_vocab=200),                                                                                                   # widest norm row: fewer ring slots
     dict(head_dim=80, n_head=64, n_head_kv=2, n_rot=40),                                                                                         # heads that begin inside row groups
     dict(head_dim=24, n_head=128, n_head_kv=4, n_rot=16, full_attn_interval=2), dict(head_dim=8, n_head=128, n_head_kv=4, n_rot=8),              # ... down to the smallest dimension
+    dict(ssm_vheads=80, ssm_inner=10240, ssm_groups=8), dict(ssm_vheads=144, ssm_inner=18432, ssm_groups=16, full_attn_interval=2),                # two dense rows for some CTAs, for most
     dict(full_attn_interval=1)])                                                                                                                 # attention in the first layer
 def test_step_kernel_geometries(monkeypatch, over):
     """Matrices that cut a row group between two CTAs, leave CTAs without work, or leave the ring fewer slots: logits, picks and

@@ -170,7 +170,7 @@ class Step:
         eb, ob, fb = g.e // 1024, (g.inner if rec else g.att) // 1024, g.ff // 1024
         row = lambda buf: [(buf, u) for u in range(g.e // 32)]
         block = lambda buf: lambda b: [(buf, 32 * b + i) for i in range(32)]
-        gates = [g.grid - 1 - r for r in range(2 * g.nv)] if rec else []
+        gates = [g.grid - 1 - r % g.grid for r in range(2 * g.nv)] if rec else []
         self.transform(n + "A", "A", eb, lambda b: row("xi") if il else [], gates)
         self.matrix(n + "B", "B", "in_gdn" if rec else "in_att", eb, "rows", gates=gates)
         self.heads(n + "C", rec)
@@ -205,6 +205,8 @@ GEOMETRIES = {
     "one block a row": dict(e=1024, ff=2048, nh=4, nkv=2, nv=8, nk=2, vocab=1000),
     "cut gate / up pairs": dict(e=3072, ff=5120, nv=16, nk=4, nh=8, nkv=2, hd=128, attn_g=2, grouped=0, vocab=5000),
     "149 row groups of the head": dict(e=2048, ff=5120, nv=24, nk=8, nh=16, nkv=4, hd=64, attn_g=1, vocab=4767),
+    "two dense rows for some CTAs": dict(e=1024, ff=2048, nh=4, nkv=2, nv=80, nk=8, vocab=1000),
+    "as many value heads as CTAs allow": dict(e=1024, ff=2048, nh=4, nkv=2, nv=144, nk=16, vocab=1000, interval=2),
     "8192 wide": dict(e=8192, ff=2048, nh=4, nkv=2, nv=8, nk=2, vocab=200),
 }
 
