@@ -1,7 +1,7 @@
 """The hand-over protocol of the tensor-memory tile kernel (it_matmul_tc.cu), without a GPU.
 
 A wait on an mbarrier sees one bit, the parity of the phase: a role that has not yet seen phase q complete must be sure that phase
-q + 1 of the same barrier cannot complete first, or it waits for good.  The model below has the kernel's roles as step counters and
+q + 1 of the same barrier cannot complete first, or it waits for good, and that phase q - 1 is complete, or it goes on too early.  The model below has the kernel's roles as step counters and
 walks every order in which they can proceed; how many barriers the steps commit to in turn is read from the source.
 """
 import os
@@ -26,9 +26,18 @@ def commit_barriers(acc):
     return acc if rings == {"TC_ND"} else int(re.search(rings.pop() + r" = (\d+)", src).group(1))
 
 
-def overtaken(acc, boxes, commits):
+def most_pairs():
+    """Pairs of expanded tiles where they fit; else two."""
+    src = source("it_matmul_tc.cu")
+    assert re.search(r"if \(gp >= na\) ok = ok && mbar_wait\(dfull0 \+ 8 \* dp", src) and re.search(r"\bdp = TC_NC - na\b", src)      # step n waits for the commit of step n - na
+    assert re.search(r"if \(\+\+pair == na\) pair = 0;", src) and re.search(r"na = TC_NA_MAX;\s*if \(!fits\(2, 2\)\) na = 2;", src)
+    return int(re.search(r"TC_NA_MAX = (\d+)", src).group(1))
+
+
+def overtaken(acc, boxes, commits, pairs):
     """(role, step) of a wait whose barrier can be two phases on; None when there is no such order.  acc: steps of accumulators, boxes:
-    slots of the activation ring, commits: barriers the steps commit to in turn."""
+    slots of the activation ring, commits: barriers the steps commit to in turn, pairs: pairs of expanded tiles, which both sets of
+    expanders fill in turn."""
     seen, todo = set(), [(0, 0, 0, 0, 0, 0)]
     while todo:
         st = todo.pop()
@@ -36,14 +45,14 @@ def overtaken(acc, boxes, commits):
             continue
         seen.add(st)
         x, e0, e1, m, c, p = st                     # boxes issued, steps expanded by either set, MMAs issued, committed, steps folded
-        for role, q in (("producer", x - boxes), ("expanders 0", 2 * e0 - 2), ("expanders 1", 2 * e1 - 1), ("epilogue", p)):
-            if q >= 0 and c > q + commits:
+        for role, q in (("producer", x - boxes), ("expanders 0", 2 * e0 - pairs), ("expanders 1", 2 * e1 + 1 - pairs), ("epilogue", p)):
+            if q >= 0 and (c > q + commits or c <= q - commits):       # the phase after is complete, or the one before is not: either is taken for phase q
                 return role, q
         if x < STEPS and (x < boxes or c > x - boxes):
             todo.append((x + 1, e0, e1, m, c, p))
-        if 2 * e0 < STEPS and c > 2 * e0 - 2:
+        if 2 * e0 < STEPS and c > 2 * e0 - pairs:
             todo.append((x, e0 + 1, e1, m, c, p))
-        if 2 * e1 + 1 < STEPS and c > 2 * e1 - 1:
+        if 2 * e1 + 1 < STEPS and c > 2 * e1 + 1 - pairs:
             todo.append((x, e0, e1 + 1, m, c, p))
         if m < x and (e1 if m & 1 else e0) > m // 2 and p > m - acc:
             todo.append((x, e0, e1, m + 1, c, p))
@@ -57,13 +66,23 @@ def overtaken(acc, boxes, commits):
 
 @pytest.mark.parametrize("acc,boxes", [(4, 2), (4, 3), (2, 2), (2, 3)])      # 64- and 128-row tiles, with two and three steps of boxes
 def test_no_wait_can_be_overtaken(acc, boxes):
-    assert overtaken(acc, boxes, commit_barriers(acc)) is None
+    for pairs in range(2, most_pairs() + 1):
+        assert overtaken(acc, boxes, commit_barriers(acc), pairs) is None
 
 
 def test_the_model_sees_an_overtaken_wait():
     """A barrier per accumulator, two of them, and three slots of boxes: box n - 1 is in place while the producer waits for step n - 3, and
     both commit to one barrier."""
-    assert overtaken(2, 3, 2) == ("producer", 0)
+    assert overtaken(2, 3, 2, 2) == ("producer", 0)
+
+
+@pytest.mark.parametrize("acc,boxes", [(4, 2), (4, 3), (2, 2), (2, 3)])
+def test_more_pairs_than_commit_barriers_are_too_many(acc, boxes):
+    """As many pairs as barriers are the limit that the kernel asserts: step n, which commits to the barrier of step n - 4, waits for its
+    expanders.  With a fifth pair step n - 1 commits to the barrier of step n - 5, which a late set of expanders is still to see."""
+    assert overtaken(acc, boxes, 4, 4) is None
+    assert overtaken(acc, boxes, 4, 5)[0].startswith("expanders")
+    assert "static_assert(TC_NA_MAX <= TC_NC" in source("it_matmul_tc.cu")
 
 
 def warp_statements(src, pattern):
