@@ -207,7 +207,7 @@ int mm_launch(it_ctx* c, const it_mat* w, int ntok, const it_q8* x, float* y, si
 
 }  // namespace
 
-// Tile policy: it_mm_groups, it_mm_takes_tc and it_mm_takes_tc64 (it_route.h).
+// Tile policy: it_mm_groups and it_mm_takes_tc (it_route.h).
 int it_matmul_t2_launch(it_ctx* c, const it_mat* w, int ntok, const it_q8* x, float* y, size_t y_stride, int accum) {
     const int wr = it_mm_groups((long)w->row_groups, ntok, c->sm_count);
     if (mm_layout(wr, (int)(w->cols / 128), 2).total + 1024 > MM_SMEM_MAX)
@@ -217,7 +217,7 @@ int it_matmul_t2_launch(it_ctx* c, const it_mat* w, int ntok, const it_q8* x, fl
     const char* fv = getenv("IT_MATMUL");      // read on every call so that a test can exercise both kernels on one shape
     const int force = !fv ? 0 : !strcmp(fv, "legacy") ? 1 : !strcmp(fv, "tc") ? 2 : 0;
     const long rgs = (long)w->row_groups;
-    if (force != 1 && (force == 2 || it_mm_takes_tc(rgs, ntok, c->sm_count) || it_mm_takes_tc64(rgs, (long)w->cols, ntok, c->sm_count))) {
+    if (force != 1 && (force == 2 || it_mm_takes_tc(rgs, (long)w->cols, ntok, c->sm_count))) {
         const int r = it_matmul_tc_launch(c, w, ntok, x, y, y_stride, accum); if (r <= 0) return r;
     }
     if (wr == 4) return mm_launch<4, 4>(c, w, ntok, x, y, y_stride, accum);

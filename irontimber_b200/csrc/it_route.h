@@ -15,20 +15,14 @@ static inline int it_mm_groups(long row_groups, long ntok, int sm_count) {
     const long tok_tiles = (ntok + 63) / 64, want = (long)sm_count * 6 / 10;
     return (row_groups + 3) / 4 * tok_tiles >= want ? 4 : (row_groups + 1) / 2 * tok_tiles >= want ? 2 : 1;
 }
-// Whether the tensor-memory kernel (it_matmul_tc.cu, one CTA per SM) goes first by its 128-row tiles alone: matrices that give such tiles to most
-// SMs, and smaller ones of more row groups than SMs from the activation rows on at which the mma.sync kernel starts a second wave.
-static inline bool it_mm_takes_tc(long row_groups, long ntok, int sm_count) {
-    const int wr = it_mm_groups(row_groups, ntok, sm_count);
-    return wr == 4 || (row_groups > sm_count && ntok > (wr == 2 ? 32 : 40));
-}
-
-// The same by its 64-row tiles: everything but short rows and few of them, where both kernels are all start-up and the mma.sync kernel's is shorter.
+// Whether the tensor-memory kernel (it_matmul_tc.cu, one CTA per SM) goes first: for everything but short rows and few of them, where both kernels
+// are all start-up and the mma.sync kernel's is shorter.
 // us, mma.sync / tensor memory:
 //   5120 x 17408 at 9 rows 44.1 / 34.7, at 33 58.9 / 37.9, at 64 67.5 / 38.1, at 128 103.5 / 53.8;  1024 x 17408 at 9 rows 33.9 / 33.3, at 64 44.5 / 36.8
 //   5120 x 5120 at 9 rows 15.0 / 12.4, at 64 22.0 / 13.6;  4736 x 5120 at 9 12.2 / 11.8, at 64 15.2 / 13.0;  96 x 5120 at 9 11.5 / 11.2, at 64 14.5 / 12.5
 //   9000 x 5120 at 9 rows 20.8 / 13.1, at 64 21.7 / 14.2;  2560 x 3072 at 9 8.3 / 8.0;  5120 x 2048 at 9 7.4 / 6.9;  640 x 2048 at 9 to 32 6.0 / 6.0
 //   2560 x 2048 at 9 rows 6.1 / 6.2, at 33 7.3 / 6.7;  5000 x 1024 at 9 4.9 / 5.0, at 33 5.7 / 5.4;  512 x 1024 at 9 4.2 / 4.3, at 32 4.2 / 4.4, at 33 4.7 / 4.6
-static inline bool it_mm_takes_tc64(long row_groups, long cols, long ntok, int sm_count) {
+static inline bool it_mm_takes_tc(long row_groups, long cols, long ntok, int sm_count) {
     return ntok > 32 || cols > 2048 || (row_groups > sm_count && cols > 1024) || it_mm_groups(row_groups, ntok, sm_count) > 1;
 }
 // Which tiles it cuts a product into, matrix rows x activation rows: what the busiest SM's tiles take, a step of theirs some 1980, 1480 and 1080

@@ -15,8 +15,7 @@ def routes(tmp_path_factory):
     d = tmp_path_factory.mktemp("routes")
     src, lib = d / "routes.cpp", d / "routes.so"
     src.write_text('#include "it_route.h"\n'
-                   'extern "C" int takes_tc(long rg, long ntok, int sm) { return it_mm_takes_tc(rg, ntok, sm); }\n'
-                   'extern "C" int takes_tc64(long rg, long cols, long ntok, int sm) { return it_mm_takes_tc64(rg, cols, ntok, sm); }\n'
+                   'extern "C" int takes_tc(long rg, long cols, long ntok, int sm) { return it_mm_takes_tc(rg, cols, ntok, sm); }\n'
                    'extern "C" int tc_tile(long rg, long ntok, int sm) { return it_tc_tile(rg, ntok, sm); }\n'
                    'extern "C" int attn_tiled(int slot0, int nt, int blk, int sm) { return it_attn_takes_tiled(256, 24, 4, slot0, nt, blk, sm); }\n'
                    'extern "C" int attn_group(int hd, int nh, int nkv, int npos) { auto g = it_attn_grouping(hd, nh, nkv, npos); return 10 * g.heads + g.rows; }\n'
@@ -26,19 +25,10 @@ def routes(tmp_path_factory):
     return C.CDLL(str(lib))
 
 
-@pytest.mark.parametrize("rows,ntok,tc", [
-    (5120, 32, 0), (5120, 40, 0), (5120, 41, 1), (5120, 64, 1), (5120, 65, 1), (5120, 128, 1), (5120, 236, 1),      # one wave and twelve CTAs of 32-row tiles
-    (4736, 64, 0), (4737, 64, 1), (4736, 65, 0), (2560, 64, 0), (1024, 512, 0),                                     # no more row groups than SMs
-    (5568, 40, 0), (5569, 40, 1), (5569, 32, 0), (6144, 32, 0), (6144, 33, 1), (11136, 33, 1),                       # from 5569 on: 64-row tiles
-    (11137, 9, 1), (34816, 9, 1), (2689, 256, 1), (2688, 256, 0)])                                  # 128-row tiles for 0.6 of the SMs
-def test_tile_kernel_of_a_product(routes, rows, ntok, tc):
-    assert routes.takes_tc(C.c_long((rows + 31) // 32), C.c_long(ntok), SM) == tc
-
-
 @pytest.mark.parametrize("rows,cols,ntok,tc", [
     (512, 1024, 32, 0), (512, 1024, 33, 1), (5000, 1024, 9, 0), (9000, 1024, 9, 1), (4736, 2048, 32, 0), (4737, 2048, 9, 1), (32, 3072, 9, 1)])
-def test_64_row_tiles_of_a_product(routes, rows, cols, ntok, tc):
-    assert routes.takes_tc64(C.c_long((rows + 31) // 32), C.c_long(cols), C.c_long(ntok), SM) == tc
+def test_tile_kernel_of_a_product(routes, rows, cols, ntok, tc):
+    assert routes.takes_tc(C.c_long((rows + 31) // 32), C.c_long(cols), C.c_long(ntok), SM) == tc
 
 
 @pytest.mark.parametrize("rows,ntok,tile", [
