@@ -45,8 +45,8 @@ __device__ __forceinline__ float4 silu_mul4(const float4 a4, const float4 b4) {
     return make_float4(it_mul(q[0], b[0]), it_mul(q[1], b[1]), it_mul(q[2], b[2]), it_mul(q[3], b[3]));
 }
 
-// Hadamard + q8k, 64 threads a block (it_had16_*).  ROW: a CTA takes a whole row, a pair of warps per block (at most eight), so that a
-// norm is formed once; else a CTA of 64 threads takes one block and, where there is a norm, forms it for itself.
+// Hadamard + q8k, 64 threads a block (it_had16_*).  ROW: a norm first, formed once by a CTA that takes the whole row, a pair of warps per block (at
+// most eight); else a CTA of 64 threads takes one block.
 struct Had16In {
     const float* x; size_t stride; const float* signs; int rotate, nblk;
     unsigned hd, nk, rep;
@@ -55,10 +55,10 @@ struct Had16In {
 template <bool ROW>
 __global__ void __launch_bounds__(ROW ? 512 : 64) k_hadamard16(const Had16In in, const it_had_prologue pro) {
     IT_PDL_TRIGGER(); IT_PDL_WAIT();
-    extern __shared__ __align__(16) float sm[];                  // [pairs][IT_HAD_PITCH], [pairs][8] group maxima, [8] warp sums of squares
+    extern __shared__ __align__(16) float sm[];                  // [pairs][IT_HAD_PITCH], [pairs][8] group maxima; ROW: [8] warp sums of squares
     const int tid = threadIdx.x, j = tid & 63, pair = ROW ? tid >> 6 : 0, pairs = ROW ? (int)blockDim.x >> 6 : 1, lane = tid & 31;
     const int blk = ROW ? pair : (int)blockIdx.x; const size_t tok = ROW ? blockIdx.x : blockIdx.y;
-    float* ex = sm + pair * IT_HAD_PITCH; float* mx = sm + pairs * IT_HAD_PITCH + pair * 8; float* ws = sm + pairs * (IT_HAD_PITCH + 8);
+    float* ex = sm + pair * IT_HAD_PITCH; float* mx = sm + pairs * IT_HAD_PITCH + pair * 8;
     auto sync = [&] { if (ROW) asm volatile("bar.sync %0, 64;" :: "r"(1 + pair) : "memory"); else __syncthreads(); };
     const float* x = in.x + tok * in.stride;
     const int g0 = blk * 1024 + 4 * j;                           // thread j comes in with elements g0 + 256 u .. + 3 (16-byte pieces in lane order)
@@ -77,43 +77,37 @@ __global__ void __launch_bounds__(ROW ? 512 : 64) k_hadamard16(const Had16In in,
         if (!in.hd || in.hd % 4 == 0) r[u] = *reinterpret_cast<const float4*>(x + at);
         sg[u] = in.signs ? *reinterpret_cast<const float4*>(in.signs + g0 + 256 * u) : make_float4(1.f, 1.f, 1.f, 1.f);
     }
-    if (pro.mode == 1) {
+    if (!ROW && pro.mode == 1) {
         // silu(a) * b on the way in (src/cpu.rs:183)
         const float* b = pro.b + tok * pro.b_stride + g0;
 #pragma unroll
         for (int u = 0; u < 4; u++) r[u] = silu_mul4(r[u], *reinterpret_cast<const float4*>(b + 256 * u));
-    } else if (pro.mode == 2) {
+    }
+    if constexpr (ROW) {
         // rmsnorm of the whole row first (src/cpu.rs:14-18), in the order of k_rmsnorm_wide: thread i of 256 adds x[i]^2,
         // x[i + 256]^2, ...; warp butterflies; eight warp sums in ascending order
+        float* ws = sm + pairs * (IT_HAD_PITCH + 8);
         float4 w[4];
 #pragma unroll
         for (int u = 0; u < 4; u++) w[u] = *reinterpret_cast<const float4*>(pro.w + g0 + 256 * u);
-        // four neighbours of the 256 at a time: their butterflies over lanes 16, 8, 4 are this thread's over 4, 2, 1
-        auto finish = [&](float4 s, int i4) {
+#pragma unroll
+        for (int u = 0; u < 4; u++) *reinterpret_cast<float4*>(ex + it_had_at(4 * j) + 336 * u) = r[u];
+        __syncthreads();
+        if (tid < 64) {
+            // four neighbours of the 256 at a time: their butterflies over lanes 16, 8, 4 are this thread's over 4, 2, 1
+            float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+            const float* xp = sm + it_had_at(4 * tid);
+#pragma unroll 4
+            for (int k = 0; k < in.nblk * 4; k++) {
+                const float4 t = *reinterpret_cast<const float4*>(xp + 336 * k);
+                s.x = it_add(s.x, it_mul(t.x, t.x)); s.y = it_add(s.y, it_mul(t.y, t.y)); s.z = it_add(s.z, it_mul(t.z, t.z)); s.w = it_add(s.w, it_mul(t.w, t.w));
+            }
 #pragma unroll
             for (int m = 4; m >= 1; m >>= 1) {
                 s.x = it_add(s.x, __shfl_xor_sync(0xffffffffu, s.x, m)); s.y = it_add(s.y, __shfl_xor_sync(0xffffffffu, s.y, m));
                 s.z = it_add(s.z, __shfl_xor_sync(0xffffffffu, s.z, m)); s.w = it_add(s.w, __shfl_xor_sync(0xffffffffu, s.w, m));
             }
-            if ((lane & 7) == 0) ws[i4 >> 3] = it_add(it_add(s.x, s.z), it_add(s.y, s.w));
-        };
-        auto squares = [&](float4& s, const float4 t) { s.x = it_add(s.x, it_mul(t.x, t.x)); s.y = it_add(s.y, it_mul(t.y, t.y)); s.z = it_add(s.z, it_mul(t.z, t.z)); s.w = it_add(s.w, it_mul(t.w, t.w)); };
-        float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (ROW) {
-#pragma unroll
-            for (int u = 0; u < 4; u++) *reinterpret_cast<float4*>(ex + it_had_at(4 * j) + 336 * u) = r[u];
-            __syncthreads();
-            if (tid < 64) {
-                const float* xp = sm + it_had_at(4 * tid);
-#pragma unroll 4
-                for (int k = 0; k < in.nblk * 4; k++) squares(s, *reinterpret_cast<const float4*>(xp + 336 * k));
-                finish(s, tid);
-            }
-        } else {
-            const float* xp = x + 4 * tid;
-#pragma unroll 8
-            for (int k = 0; k < in.nblk * 4; k++) squares(s, *reinterpret_cast<const float4*>(xp + 256 * k));
-            finish(s, tid);
+            if ((lane & 7) == 0) ws[tid >> 3] = it_add(it_add(s.x, s.z), it_add(s.y, s.w));
         }
         __syncthreads();
         float tot = ws[0];
@@ -161,8 +155,8 @@ void launch_q8(it_ctx* c, size_t n, size_t ntok, size_t x_off, size_t x_stride, 
     }
     const Had16In in{ c->arena + x_off, x_stride, signs, rotate, (int)nblk, (unsigned)hd, (unsigned)nk, (unsigned)rep, out->qs, out->d, out->sum128, out->max_n };
     const size_t per = (IT_HAD_PITCH + 8) * sizeof(float);
-    if (pro.mode == 2 && nblk <= 8) it_pdl(k_hadamard16<true>, dim3((unsigned)ntok), dim3((unsigned)(64 * nblk)), nblk * per + 32, c->stream, in, pro);      // at most 43.3 KB
-    else it_pdl(k_hadamard16<false>, dim3((unsigned)nblk, (unsigned)ntok), dim3(64), per + 32, c->stream, in, pro);
+    if (pro.mode == 2) it_pdl(k_hadamard16<true>, dim3((unsigned)ntok), dim3((unsigned)(64 * nblk)), nblk * per + 32, c->stream, in, pro);      // normed rows are at most 8192 wide: 43.3 KB
+    else it_pdl(k_hadamard16<false>, dim3((unsigned)nblk, (unsigned)ntok), dim3(64), per, c->stream, in, pro);
 }
 
 int check_common(it_ctx* c, size_t n, size_t ntok, size_t in_off, size_t in_stride, int use_signs,
