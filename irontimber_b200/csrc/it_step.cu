@@ -890,8 +890,8 @@ __device__ __forceinline__ void gdn_phase(const StepParams& P, const StepLayer& 
 // group store them into the cache.
 // Data movement: both caches are tiled (32 positions x head_dim halves = one contiguous 16 KB block per KV head), so a
 // loader warp brings whole tiles into a ring of 16 KB slots with one bulk copy each.  One warp per slot scores its K
-// tiles, a position per lane, from shared memory; the V tiles follow through the same ring and four warps (two output
-// elements per thread) walk them in order.  Full / free mbarriers pace both; they are set up afresh by every attention
+// tiles, a position per lane, from shared memory; slices of the V tiles follow through the same ring and a warp per 32 output
+// elements (one a thread) walks them in order.  Full / free mbarriers pace both; they are set up afresh by every attention
 // block.  The tiles were sent on their way into L2 while the input projection ran (attn_prefetch).
 __device__ __forceinline__ void attn_prefetch(const StepParams& P, const StepLayer& L, const Cta& c, int hg) {
     if (c.warp != 0 || hg < 0 || hg >= P.nh * P.attn_g) return;
